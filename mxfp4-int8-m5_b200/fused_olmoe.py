@@ -11,11 +11,13 @@ import os
 import numpy as np
 import torch
 
+from . import _lib
 from . import host_model as HM
 from . import packed_io
 from . import sc_format as F
 from . import sc_kernels as S
 from . import sc_moe as M_
+from .fused_moe import MoeBlock
 from .w4a8 import PackedWeight
 
 ATTN = ["self_attn.q_proj", "self_attn.k_proj", "self_attn.v_proj", "self_attn.o_proj"]
@@ -120,6 +122,13 @@ class FusedOlmoe:
         logits = torch.nn.functional.linear(xn[:M], layer.mlp.gate.weight)
         return M_.router_topk(logits.float(), self.args.num_experts_per_tok)
 
+    def _packed(self, R):
+        """Whether the grouped GEMMs read the packed weights (scmx_moe_mm_w4) although the experts could be decoded ahead: MoeBlock's
+        rule.  An expert's INT8 copy costs three passes over its bytes, which few rows do not repay: two layers of 64 experts of
+        2048 x 1024 at 128 rows per expert take 592 us with the rest of a prompt against 765 us, the bits being the same."""
+        return (self.two_pass is not True and M_.FUSED_UNPACK and R // self.args.num_experts < MoeBlock.FUSED_BELOW and self.args.num_experts <= 512
+                and all(_lib.lib().scmx_w4_supported(F.DEFAULT.c_struct(), k) for k in (self.args.hidden_size, self.args.intermediate_size)))
+
     def _decode_experts(self, i):
         """Layer i's experts -> INT8 in ring[i % 2] on the side stream; waits for the GEMMs that last read that pair."""
         a = self.args
@@ -140,7 +149,7 @@ class FusedOlmoe:
         a = self.args
         k, E, F2, D = a.num_experts_per_tok, a.num_experts, 2 * a.intermediate_size, a.hidden_size
         R = L * k
-        two_pass = self.two_pass if self.two_pass != "auto" else R // E >= 256
+        two_pass = self.two_pass if self.two_pass != "auto" else R // E >= 256 and not self._packed(R)
         pos, tok_p, e_sorted, off, tstart, maxt = M_.route_sort(inds, E, M_.TM)
         xq_s, xs_s = M_.gather_rows(xq, xs, tok_p, R)
         (cg, bg, sg), (cd, bd, sd) = ex["gu"], ex["down"]
@@ -172,14 +181,15 @@ class FusedOlmoe:
         h = h.contiguous()
         nl = len(self.layers)
         main = torch.cuda.current_stream()
-        if self.prefetch:
+        ahead = self.prefetch and not self._packed(L * a.num_experts_per_tok)
+        if ahead:
             self._ready, self._done = [None] * nl, [None] * nl
             self.side.wait_stream(main)
             self._decode_experts(0)
         xq, xs = S.rmsnorm_quant(h, self.layers[0][0].input_layernorm.weight, self.eps, Mp)
         for i, (layer, ws, ex) in enumerate(self.layers):
             at, c = layer.self_attn, cache[i]
-            if self.prefetch and i + 1 < nl:
+            if ahead and i + 1 < nl:
                 self._decode_experts(i + 1)                    # under this layer's attention and GEMMs
             wq, wo = ws["qkv"], ws["o"]
             y = S.mm_epi(xq, wq.unpack(), xs, wq.wscale, 1)
@@ -191,10 +201,10 @@ class FusedOlmoe:
             h = S.mm_epi(xq, wo.unpack(), xs, wo.wscale, 2, res=h)
             xq, xs, xn = S.rmsnorm_quant_n(h, layer.post_attention_layernorm.weight, self.eps)
             inds, scores = self.route(layer, xn, L)
-            if self.prefetch:
+            if ahead:
                 main.wait_event(self._ready[i])
-            yd, pos, rec = self.experts(ex, xq, xs, inds, L, self.ring[i % 2] if self.prefetch else None)
-            if self.prefetch:
+            yd, pos, rec = self.experts(ex, xq, xs, inds, L, self.ring[i % 2] if ahead else None)
+            if ahead:
                 self._done[i] = torch.cuda.Event()
                 self._done[i].record(main)
             nn = self.layers[i + 1][0].input_layernorm.weight if i + 1 < nl else self.model.model.norm.weight
@@ -202,7 +212,7 @@ class FusedOlmoe:
             h, xq, xs = M_.moe_combine(yd, pos, scores, h, nn, self.eps, L)
             if self.record is not None and i in self.record_layers:
                 self.record[(i, "experts")] = (h_in, xn, inds, scores, yd, pos, *rec)
-        if self.prefetch:
+        if ahead:
             main.wait_stream(self.side)
         xn = S.rmsnorm_quant_n(h, self.model.model.norm.weight, self.eps, Mp)[2]
         return xn[:L][None]
