@@ -2,8 +2,8 @@
 // and scaled.  Keys are cached after their norm: K [2 G, cap, d] (map m of key/value head g at row 2 g + m), V [G, cap, dv].
 //
 // qk_norm_append_kernel   q / k RMS norm per head and map, K / V rows appended to the cache
-// diff_attn_kernel        prompt portions, any sizes and storage types, float32 arithmetic on the CUDA cores (bfloat16 with head
-//                         sizes up to 128: diff_attn_tc, tensor cores)
+// diff_attn_tile_kernel   prompt portions in float32 on the CUDA cores, head sizes that are multiples of 4, up to 256 values
+// diff_attn_kernel        the same for other sizes and for bfloat16 (bfloat16 with head sizes up to 128: diff_attn_tc, tensor cores)
 // diff_decode_kernel      one query row: positions split over CTAs, the last CTA of a key/value head combines
 #include "mix_common.cuh"
 
@@ -191,6 +191,155 @@ __global__ void __launch_bounds__(256) diff_attn_kernel(const DiffAttnArgs<T> a)
         }
         const float inv = rms_inv_f32(warp_sumf(ss), dv, a.eps) * (1.0f - a.diff);
         for (int e = lane; e < dv; e += 32) stf(a.o + ((q0 + t) * a.H + h) * dv + e, (o1[e] * i1 - o2[e] * i2) * inv);
+    }
+}
+
+// Float32 storage: both maps of 16 queries, tiles of 32 keys.  Bound by fused multiply-adds and the shared-memory reads that feed
+// them, so a thread computes 2 x 2 scores from 16-byte reads (rows pitched by d + 4: no bank conflicts for d a multiple of 8) and 4 rows x
+// 4 CV output columns in registers; softmax sums stay in registers, and the next tile arrives by asynchronous copies under the present
+// one.  8 heads of 64 / 128, 300 queries: 215 us as diff_attn_kernel (one score per thread and scalar reads, outputs in shared memory).
+constexpr int DT_P = 36;      // pitch of the weights, [DG_K][rows]: row (t / 2) 4 + 2 map + t % 2 for query t, so a warp owns both maps of two queries
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool ok) {      // zeros when !ok
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+
+template <int CV>
+__global__ void __launch_bounds__(256) diff_attn_tile_kernel(const DiffAttnArgs<float> a) {
+    extern __shared__ __align__(16) float sm[];
+    const int d = a.d, dv = a.dv, dp = d + 4, tile = 2 * DG_K * dp + DG_K * dv;
+    float* sq = sm;                           // [2 DG_Q][dp]
+    float* sp = sq + 2 * DG_Q * dp;           // [DG_K][DT_P] weights
+    float* sc = sp + DG_K * DT_P;             // [2 DG_Q] corrections, at the end sums
+    float* ring = sc + 2 * DG_Q;              // 2 tiles: keys [2][DG_K][dp], values [DG_K][dv]
+    pdl_launch_dependents();
+    pdl_wait();
+    const int h = blockIdx.y, g = h / (a.H / a.G), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t q0 = (int64_t)(gridDim.x - 1 - blockIdx.x) * DG_Q;      // the longest rows first
+    const int nq = (int)min((int64_t)DG_Q, a.n - q0);
+    const int64_t last = a.pos + q0 + nq;     // first key no row of the tile sees
+    const int d4 = d / 4, v4 = dv / 4;
+    auto fetch = [&](int64_t k0, float* to) {
+        for (int i = tid; i < 2 * DG_K * d4; i += 256) {
+            const int r = i / d4, e = 4 * (i - r * d4), m = r / DG_K, t = r - m * DG_K;
+            const bool ok = k0 + t < last;
+            cp_async16(to + r * dp + e, a.k + ((int64_t)(2 * g + m) * a.cap + (ok ? k0 + t : 0)) * d + e, ok);
+        }
+        to += 2 * DG_K * dp;
+        for (int i = tid; i < DG_K * v4; i += 256) {
+            const int t = i / v4, e = 4 * (i - t * v4);
+            const bool ok = k0 + t < last;
+            cp_async16(to + t * dv + e, a.v + ((int64_t)g * a.cap + (ok ? k0 + t : 0)) * dv + e, ok);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0, ring);
+    for (int i = tid; i < 2 * DG_Q * d4; i += 256) {
+        const int r = i / d4, e = 4 * (i - r * d4), m = r / DG_Q, t = r - m * DG_Q;
+        float4 x = make_float4(0, 0, 0, 0);
+        if (t < nq) x = *reinterpret_cast<const float4*>(a.q + ((int64_t)(2 * h + m) * a.n + q0 + t) * d + e);
+        *reinterpret_cast<float4*>(sq + r * dp + e) = make_float4(x.x * a.scale, x.y * a.scale, x.z * a.scale, x.w * a.scale);
+    }
+    // scores: map tm, queries 2 tr and 2 tr + 1, keys tk and tk + 16 of the tile
+    const int tm = tid >> 7, tr = (tid >> 4) & 7, tk = tid & 15, prow = 4 * tr + 2 * tm;
+    const float* qr = sq + (tm * DG_Q + 2 * tr) * dp;
+    float mx[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f}, acc[4][4 * CV];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 4 * CV; ++c) acc[r][c] = 0.0f;
+    int slot = 0;
+    for (int64_t k0 = 0; k0 < last; k0 += DG_K, slot ^= 1) {
+        const float* kt = ring + slot * tile;
+        if (k0 + DG_K < last) {
+            fetch(k0 + DG_K, ring + (slot ^ 1) * tile);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        const float* kr = kt + (tm * DG_K + tk) * dp;
+        float s[2][2] = {};
+#pragma unroll 4
+        for (int e = 0; e < d; e += 4) {
+            const float4 a0 = *reinterpret_cast<const float4*>(qr + e), a1 = *reinterpret_cast<const float4*>(qr + dp + e);
+            const float4 b0 = *reinterpret_cast<const float4*>(kr + e), b1 = *reinterpret_cast<const float4*>(kr + 16 * dp + e);
+            s[0][0] = fmaf(a0.x, b0.x, s[0][0]); s[0][1] = fmaf(a0.x, b1.x, s[0][1]); s[1][0] = fmaf(a1.x, b0.x, s[1][0]); s[1][1] = fmaf(a1.x, b1.x, s[1][1]);
+            s[0][0] = fmaf(a0.y, b0.y, s[0][0]); s[0][1] = fmaf(a0.y, b1.y, s[0][1]); s[1][0] = fmaf(a1.y, b0.y, s[1][0]); s[1][1] = fmaf(a1.y, b1.y, s[1][1]);
+            s[0][0] = fmaf(a0.z, b0.z, s[0][0]); s[0][1] = fmaf(a0.z, b1.z, s[0][1]); s[1][0] = fmaf(a1.z, b0.z, s[1][0]); s[1][1] = fmaf(a1.z, b1.z, s[1][1]);
+            s[0][0] = fmaf(a0.w, b0.w, s[0][0]); s[0][1] = fmaf(a0.w, b1.w, s[0][1]); s[1][0] = fmaf(a1.w, b0.w, s[1][0]); s[1][1] = fmaf(a1.w, b1.w, s[1][1]);
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int64_t lim = a.pos + q0 + 2 * tr + r - k0;       // the row sees keys 0 .. lim of the tile
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+                if (tk + 16 * c > lim) s[r][c] = -INFINITY;
+            float t = fmaxf(s[r][0], s[r][1]);
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) t = fmaxf(t, __shfl_xor_sync(0xffffffffu, t, o));
+            const float mn = fmaxf(mx[r], t);      // finite from the first tile on: every row sees key 0 (unless a score is not a number)
+            const float corr = mn == -INFINITY ? 1.0f : expf(mx[r] - mn);
+            mx[r] = mn;
+            l[r] *= corr;
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const float p = mn == -INFINITY ? 0.0f : expf(s[r][c] - mn);
+                l[r] += p;
+                sp[(tk + 16 * c) * DT_P + prow + r] = p;
+            }
+            if (tk == 0) sc[prow + r] = corr;
+        }
+        __syncthreads();
+        const float4 corr = *reinterpret_cast<const float4*>(sc + 4 * warp);
+        const float cr[4] = {corr.x, corr.y, corr.z, corr.w};
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int c = 0; c < 4 * CV; ++c) acc[r][c] *= cr[r];
+        const float* vt = kt + 2 * DG_K * dp + 4 * lane;
+#pragma unroll
+        for (int j = 0; j < CV; ++j)
+            if (4 * lane + 128 * j < dv)
+#pragma unroll 8
+                for (int kk = 0; kk < DG_K; ++kk) {
+                    const float4 w = *reinterpret_cast<const float4*>(sp + kk * DT_P + 4 * warp);
+                    const float4 x = *reinterpret_cast<const float4*>(vt + kk * dv + 128 * j);
+                    const float ww[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        acc[r][4 * j] = fmaf(ww[r], x.x, acc[r][4 * j]);
+                        acc[r][4 * j + 1] = fmaf(ww[r], x.y, acc[r][4 * j + 1]);
+                        acc[r][4 * j + 2] = fmaf(ww[r], x.z, acc[r][4 * j + 2]);
+                        acc[r][4 * j + 3] = fmaf(ww[r], x.w, acc[r][4 * j + 3]);
+                    }
+                }
+        __syncthreads();                      // the tile's slot and the weights are free
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) l[r] += __shfl_xor_sync(0xffffffffu, l[r], o);
+        if (tk == 0) sc[prow + r] = l[r];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int t = 2 * warp + i;
+        const float i1 = 1.0f / sc[4 * warp + i], i2 = a.lambda / sc[4 * warp + 2 + i];
+        float ss = 0.0f;
+#pragma unroll
+        for (int c = 0; c < 4 * CV; ++c) {
+            acc[i][c] = acc[i][c] * i1 - acc[2 + i][c] * i2;      // columns above dv were never added to
+            ss += acc[i][c] * acc[i][c];
+        }
+        const float inv = rms_inv_f32(warp_sumf(ss), dv, a.eps) * (1.0f - a.diff);
+        if (t < nq)
+#pragma unroll
+            for (int j = 0; j < CV; ++j)
+                if (4 * lane + 128 * j < dv)
+                    st4(a.o + ((q0 + t) * a.H + h) * dv + 4 * lane + 128 * j, acc[i][4 * j] * inv, acc[i][4 * j + 1] * inv, acc[i][4 * j + 2] * inv,
+                        acc[i][4 * j + 3] * inv);
     }
 }
 
@@ -425,6 +574,20 @@ static int run_diff_attn(const DiffAttnArgs<T>& a, cudaStream_t st) {
     return SCMX_OK;
 }
 
+template <int CV>
+static int run_diff_tile(const DiffAttnArgs<float>& a, size_t smem, cudaStream_t st) {
+    SCMX_CUDA_OK(cudaFuncSetAttribute(diff_attn_tile_kernel<CV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    SCMX_PDL_OK("diff_attn_tile_kernel", launch_pdl(diff_attn_tile_kernel<CV>, dim3((unsigned)((a.n + DG_Q - 1) / DG_Q), a.H), dim3(256), smem, st, a));
+    return SCMX_OK;
+}
+static int run_diff_attn_f32(const DiffAttnArgs<float>& a, cudaStream_t st) {
+    // 16-byte copies of keys and values, output columns of a warp in registers
+    const size_t smem = ((size_t)2 * DG_Q * (a.d + 4) + DG_K * DT_P + 2 * DG_Q + 2 * ((size_t)2 * DG_K * (a.d + 4) + (size_t)DG_K * a.dv)) * 4;
+    const uintptr_t bits = (uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.v | (uintptr_t)a.o;
+    if (a.d % 4 || a.dv % 4 || a.dv > 256 || (bits & 15) || smem > 220 * 1024) return run_diff_attn<float>(a, st);
+    return a.dv <= 128 ? run_diff_tile<1>(a, smem, st) : run_diff_tile<2>(a, smem, st);
+}
+
 template <typename T, int QP>
 static int run_diff_decode_q(const DiffDecodeArgs<T>& a, cudaStream_t st) {
     const int Q = 2 * (a.H / a.G), groups = 256 / a.ct;
@@ -520,7 +683,7 @@ extern "C" int scmx_diff_attn(const void* q, const void* k_cache, const void* v_
         return run_diff_attn<bf16_t>(a, (cudaStream_t)stream);
     }
     FILL(float);
-    return run_diff_attn<float>(a, (cudaStream_t)stream);
+    return run_diff_attn_f32(a, (cudaStream_t)stream);
 #undef FILL
 }
 

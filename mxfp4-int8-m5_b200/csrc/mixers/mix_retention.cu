@@ -1,7 +1,8 @@
 // Retention: linear attention with a fixed decay per head.  S_t = decay S_(t-1) + k_t v_t^T, o_t = S_t^T q_t; q and k are rotated
 // (rotate-half, table of cosines and sines per position) and k is scaled when they are read, in float32.
 //
-// retention_scan_kernel   any sizes, any storage type: token by token, float32 (bfloat16 prompts: retention_tc, tensor cores)
+// retention_cols_kernel   heads of up to 256, any storage type: token by token, float32, the state in registers
+// retention_scan_kernel   larger heads: the same with the state in shared memory (bfloat16 prompts: retention_tc, tensor cores)
 // retention_step_kernel   one token: state update, output, head norm and gate, a cluster of CTAs per head
 #include <cooperative_groups.h>
 #include "mix_common.cuh"
@@ -87,6 +88,101 @@ __global__ void __launch_bounds__(256) retention_scan_kernel(const RetArgs<T> a)
         if (ok) gS[(int64_t)i * a.dv] = S[i * 32 + lane];
 }
 
+// Grid (heads, column slices of 16): thread (row group g, column c) holds NR consecutive rows of its column in registers.  A chain of
+// fused multiply-adds per token and, before this form, of shared-memory reads of the state: 8 heads of 128 x 256, 300 tokens took 380 us
+// as retention_scan_kernel (three scalar reads per two multiply-adds, staging exposed in every 8 tokens) on 64 CTAs.  Rows in registers
+// read q and k as 16-byte broadcasts, twice as many CTAs share the columns, and the next 16 tokens are loaded under the present ones.
+constexpr int RC_T = 16;                    // tokens staged together
+constexpr int RC_PITCH = 16 * RC_T + 16;    // outputs of a row group; row groups of a warp fall on different banks
+template <int NR> constexpr size_t rc_smem() { return (size_t)(2 * RC_T * 16 * NR + RC_T * 16 + 16 * RC_PITCH) * 4; }
+
+template <typename T, int NR>
+__global__ void __launch_bounds__(256) retention_cols_kernel(const RetArgs<T> a) {
+    constexpr int DP = 16 * NR, J = DP / 2, TI = 256 / J, NI = RC_T / TI;      // J pairs of elements per token, TI tokens at a time
+    extern __shared__ __align__(16) float sm[];
+    float* sq = sm;                         // [RC_T][DP], zero above d
+    float* sk = sq + RC_T * DP;
+    float* sv = sk + RC_T * DP;             // [RC_T][16]
+    float* so = sv + RC_T * 16;             // [16 row groups][RC_PITCH]
+    pdl_launch_dependents();
+    const int h = blockIdx.x, e0 = blockIdx.y * 16, tid = threadIdx.x, c = tid & 15, g = tid >> 4;
+    // the pair of elements that this thread stages: (j, j + half) of the rotated part, two neighbours above it
+    const int j = tid % J, tj = tid / J, half = a.dims >> 1;
+    const bool rot = j < half;
+    const int ea = rot ? j : a.dims + 2 * (j - half), eb = rot ? j + half : ea + 1;
+    const T* q = a.q + (int64_t)h * a.d;
+    const T* k = a.k + (int64_t)h * a.d;
+    const T* v = a.v + (int64_t)h * a.dv + e0 + c;
+    const bool okc = e0 + c < a.dv;
+    float rq[NI][2], rk[NI][2], rc[NI][2], rv = 0.0f;
+    auto fetch = [&](int64_t t0) {
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            const int64_t t = t0 + tj + TI * i;
+            const bool ok = t < a.n;
+            rq[i][0] = ok && ea < a.d ? ldf(q + t * a.ldq + ea) : 0.0f;
+            rq[i][1] = ok && eb < a.d ? ldf(q + t * a.ldq + eb) : 0.0f;
+            rk[i][0] = ok && ea < a.d ? ldf(k + t * a.ldk + ea) : 0.0f;
+            rk[i][1] = ok && eb < a.d ? ldf(k + t * a.ldk + eb) : 0.0f;
+            rc[i][0] = ok && rot ? a.cs[t * a.dims + j] : 1.0f;
+            rc[i][1] = ok && rot ? a.cs[t * a.dims + half + j] : 0.0f;
+        }
+        rv = okc && t0 + g < a.n ? ldf(v + (t0 + g) * a.ldv) : 0.0f;      // 16 tokens x 16 columns
+    };
+    pdl_wait();
+    float s[NR];
+    float* S = a.state + ((int64_t)h * a.d + g * NR) * a.dv + e0 + c;
+#pragma unroll
+    for (int i = 0; i < NR; ++i) s[i] = okc && g * NR + i < a.d ? S[(int64_t)i * a.dv] : 0.0f;
+    const float decay = a.decay[h];
+    fetch(0);
+    for (int64_t t0 = 0; t0 < a.n; t0 += RC_T) {
+        const int nt = (int)min((int64_t)RC_T, a.n - t0);
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            const int t = tj + TI * i;
+            const float cs = rc[i][0], sn = rc[i][1];
+            if (ea < DP) {
+                sq[t * DP + ea] = rot ? rq[i][0] * cs - rq[i][1] * sn : rq[i][0];
+                sk[t * DP + ea] = (rot ? rk[i][0] * cs - rk[i][1] * sn : rk[i][0]) * a.kscale;
+            }
+            if (eb < DP) {
+                sq[t * DP + eb] = rot ? rq[i][1] * cs + rq[i][0] * sn : rq[i][1];
+                sk[t * DP + eb] = (rot ? rk[i][1] * cs + rk[i][0] * sn : rk[i][1]) * a.kscale;
+            }
+        }
+        sv[tid] = rv;
+        __syncthreads();
+        if (t0 + RC_T < a.n) fetch(t0 + RC_T);
+#pragma unroll 4
+        for (int t = 0; t < RC_T; ++t)
+            if (t < nt) {
+                const float x = sv[t * 16 + c];
+                float part = 0.0f;
+#pragma unroll
+                for (int i = 0; i < NR; i += 4) {
+                    const float4 k4 = *reinterpret_cast<const float4*>(sk + t * DP + g * NR + i);
+                    const float4 q4 = *reinterpret_cast<const float4*>(sq + t * DP + g * NR + i);
+                    s[i] = fmaf(decay, s[i], k4.x * x); part = fmaf(q4.x, s[i], part);
+                    s[i + 1] = fmaf(decay, s[i + 1], k4.y * x); part = fmaf(q4.y, s[i + 1], part);
+                    s[i + 2] = fmaf(decay, s[i + 2], k4.z * x); part = fmaf(q4.z, s[i + 2], part);
+                    s[i + 3] = fmaf(decay, s[i + 3], k4.w * x); part = fmaf(q4.w, s[i + 3], part);
+                }
+                so[g * RC_PITCH + t * 16 + c] = part;
+            }
+        __syncthreads();
+        if (g < nt && okc) {                // token g, column c
+            float o = 0.0f;
+#pragma unroll
+            for (int r = 0; r < 16; ++r) o += so[r * RC_PITCH + tid];
+            a.o[((t0 + g) * a.H + h) * a.dv + e0 + c] = o;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < NR; ++i)
+        if (okc && g * NR + i < a.d) S[(int64_t)i * a.dv] = s[i];
+}
+
 // ---- one token ------------------------------------------------------------------------------------------------------------
 struct RetStepArgs {
     const float *q, *k, *v, *g;      // one row each
@@ -170,8 +266,21 @@ __global__ void __launch_bounds__(256) retention_step_kernel(const RetStepArgs a
     }
 }
 
+template <typename T, int NR>
+static int run_ret_cols(const RetArgs<T>& a, cudaStream_t st) {
+    if (rc_smem<NR>() > 48 * 1024)
+        SCMX_CUDA_OK(cudaFuncSetAttribute(retention_cols_kernel<T, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rc_smem<NR>()));
+    SCMX_PDL_OK("retention_cols_kernel",
+                launch_pdl(retention_cols_kernel<T, NR>, dim3(a.H, (a.dv + 15) / 16), dim3(256), rc_smem<NR>(), st, a));
+    return SCMX_OK;
+}
+
 template <typename T>
 static int run_ret_scan(const RetArgs<T>& a, cudaStream_t st) {
+    // rows of a column per thread: registers hold 16 at most, so heads above 256 keep the state in shared memory
+    if (a.d <= 64) return run_ret_cols<T, 4>(a, st);
+    if (a.d <= 128) return run_ret_cols<T, 8>(a, st);
+    if (a.d <= 256) return run_ret_cols<T, 16>(a, st);
     const size_t smem = ((size_t)a.d * 32 + 2 * RS_T * a.d + RS_T * 32 + 8 * RS_T * 32) * 4;
     SCMX_REQUIRE(smem <= 200 * 1024, SCMX_ELIMIT, "retention: head size %d", a.d);
     if (smem > 48 * 1024)
