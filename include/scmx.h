@@ -377,6 +377,9 @@ int scmx_decode_step_dense(const scmx_decode_layer* layers, int n_layers, int D,
                            float scale, const float* inv_freq, const float* rope_table, int64_t rope_rows, int64_t capacity,
                            const int32_t* pos_dev, uint16_t* h, uint16_t* y, uint16_t* act, uint16_t* o, float* partials,
                            int nsplit, int32_t* counters, uint32_t* barrier, int32_t* status, void* stream);
+/* Greedy choice inside a captured decode step: *tok = out[*count] = index of the largest of V logits (bf16 or float; the lowest of equal ones, a
+ * not-a-number value counts as the largest), *count += 1, *pos += 1.  Nothing is stored in out at cap or beyond.  In libscmx_mixers too. */
+int scmx_select_token(const void* logits, int is_f32, int64_t V, int64_t* tok, int32_t* pos, int32_t* count, int64_t* out, int64_t cap, void* stream);
 /* Diagnostic: while device_buf is set, CTA 0 of scmx_decode_step_dense stores its SM cycle counter in device_buf[0 .. n)
  * at every barrier entry and exit and, in the attention phase, after the q/k/v preparation and after the split's positions,
  * layer after layer; with

@@ -96,6 +96,7 @@ SIGNATURES = {
     "scmx_decode_step_dense": [c_vp, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_vp, c_vp, c_i64, c_i64, c_vp,
                                c_vp, c_vp, c_vp, c_vp, c_vp, c_int, c_vp, c_vp, c_vp, c_vp],
     "scmx_set_decode_trace": [c_vp, c_int],
+    "scmx_select_token": [c_vp, c_int, c_i64, c_vp, c_vp, c_vp, c_vp, c_i64, c_vp],
     "scmx_gemv_pro": [c_vp, c_int, c_vp, c_float, c_vp, c_vp, c_vp, c_i64, c_i64, _FMT_P, c_int, c_vp, c_vp, c_int, c_int, c_int,
                       c_vp, c_int, c_vp],
     "scmx_gemv_multi_plan": [c_vp, c_int, _FMT_P],
@@ -112,6 +113,7 @@ MIXER_SIGNATURES = {
     "scmx_embed_pair": [c_vp, c_vp, c_vp, c_int, c_i64, c_i64, c_int, c_float, c_i64, c_i64, c_i64, c_vp, c_vp, c_vp],
     "scmx_add_norm": [c_vp, c_i64, c_vp, c_vp, c_float, c_float, c_i64, c_int, c_vp, c_vp, c_int, c_vp],
     "scmx_head_norm_gate": [c_vp, c_vp, c_i64, c_int, c_vp, c_int, c_i64, c_int, c_int, c_float, c_vp, c_vp],
+    "scmx_select_token": [c_vp, c_int, c_i64, c_vp, c_vp, c_vp, c_vp, c_i64, c_vp],
     "scmx_gated_gelu": [c_vp, c_i64, c_i64, c_int, c_vp, c_vp],
     "scmx_delta_scratch": [c_i64, c_int, c_int, c_int, c_i64],
     "scmx_delta": [c_vp, c_i64, c_vp, c_i64, c_vp, c_i64, c_vp, c_i64, c_vp, c_i64, c_int, c_int, c_i64, c_int, c_int, c_int, c_int, c_vp, c_vp,

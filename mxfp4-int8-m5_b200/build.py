@@ -13,7 +13,7 @@ CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(HERE, "..", "include")
 LIBS = {"scmx": os.path.join(HERE, "libscmx.so"), "mixers": os.path.join(HERE, "libscmx_mixers.so")}
 LIB = LIBS["scmx"]
-SHARED = ("scmx_abi.cu", "scmx_tma.cu")        # error reporting and tensor maps: part of both libraries
+SHARED = ("scmx_abi.cu", "scmx_tma.cu", "scmx_select.cu")        # error reporting, tensor maps, choice of a token: part of both libraries
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
               "--shared", "-cudart", "static"]
 

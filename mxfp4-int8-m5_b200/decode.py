@@ -78,37 +78,48 @@ class _Decoder:
             # the warm-up run below writes the cache row at `pos`: point it at the row the first real step overwrites
             tok_buf = tok.reshape(1, 1).to(torch.long).clone()
             pos = torch.full((1,), offsets[0], dtype=torch.int32, device=dev)
+            count = torch.zeros(1, dtype=torch.int32, device=dev)
+            chosen = torch.empty(cache[0].capacity, dtype=torch.long, device=dev)
             for c in cache:
                 c.offset = 0                                   # rows and rotary positions come from `pos` on the device
             s = torch.cuda.Stream(device=dev)
             s.wait_stream(torch.cuda.current_stream())
             with torch.cuda.stream(s):
                 kept = [(t, t.clone()) for c in cache for t in c.carried()]
-                self._step(tok_buf, cache, pos)                # warm-up outside the capture (lazy initialisations)
+                logits = self._step(tok_buf, cache, pos)       # warm-up outside the capture (lazy initialisations)
+                self._select(logits, tok_buf, pos, count, chosen)
                 for t, old in kept:                            # recurrent states must not see the warm-up token
                     t.copy_(old)
                 torch.cuda.synchronize()
                 g = torch.cuda.CUDAGraph()
                 with torch.cuda.graph(g, stream=s):
                     logits = self._step(tok_buf, cache, pos)
-                    tok_buf.copy_(logits[:, -1].argmax(-1, keepdim=True))
-                    pos.add_(1)
+                    self._select(logits, tok_buf, pos, count, chosen)
             torch.cuda.current_stream().wait_stream(s)
             for c, o in zip(cache, offsets):
                 c.offset = o
-            self._graph = (cache, g, tok_buf, pos, logits)
-        _, g, tok_buf, pos, _ = self._graph
+            self._graph = (cache, g, tok_buf, pos, count, chosen, logits)
+        _, g, tok_buf, pos, count, chosen, _ = self._graph
         start = cache[0].offset
         assert start + n <= cache[0].capacity, "KV cache capacity exceeded"
         tok_buf.copy_(tok.reshape(1, 1))
         pos.fill_(start)
-        out = torch.empty(n, dtype=torch.long, device=dev)
-        for i in range(n):
+        count.zero_()
+        for _ in range(n):
             g.replay()
-            out[i:i + 1].copy_(tok_buf.reshape(1))
+        out = chosen[:n].clone()
         for c in cache:
             c.offset = start + n
         return out
+
+
+    _call = staticmethod(_lib.call)      # the library that the decoder's kernels are in
+
+    def _select(self, logits, tok, pos, count, chosen):
+        """The next token (greedy) as the step's input and in the list of chosen ones, and the step's counters, in one kernel."""
+        row = logits[:, -1].reshape(-1)
+        self._call("scmx_select_token", _lib.ptr(row), int(row.dtype == torch.float32), row.numel(), _lib.ptr(tok), _lib.ptr(pos), _lib.ptr(count),
+                   _lib.ptr(chosen), chosen.numel(), _lib.stream())
 
 
 class DecodeQwen3(_Decoder):
@@ -231,6 +242,7 @@ class DecodeOlmoe(_Decoder):
 class DecodeHybrid(_Decoder):
     """Built from a FusedHybrid.  Activations of a step are float32 vectors in buffers that live with the decoder."""
     replayable = True
+    _call = staticmethod(_lib.mcall)
 
     def __init__(self, fused):
         self.f, self.model, self.args, self._graph = fused, fused.model, fused.args, None
