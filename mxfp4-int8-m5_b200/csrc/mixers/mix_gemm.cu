@@ -315,6 +315,13 @@ __global__ void __launch_bounds__(256) gemm_reduce_kernel(const float* part, int
     else st4(static_cast<bf16_t*>(out) + r * ldo + c, s.x, s.y, s.z, s.w);
 }
 
+int gemm_reduce(const float* part, int splits, int64_t stride, int64_t rows, int64_t ldp, int out_f32, void* out, int64_t ldo, cudaStream_t st) {
+    const int quads = (int)(ldp / 4);
+    SCMX_PDL_OK("gemm_reduce_kernel", launch_pdl(gemm_reduce_kernel, dim3((unsigned)((rows * quads + 255) / 256)), dim3(256), 0, st, part, splits, stride,
+                                                 rows, quads, ldp, out_f32, out, ldo));
+    return SCMX_OK;
+}
+
 }  // namespace scmx
 
 using namespace scmx;
@@ -350,11 +357,7 @@ extern "C" int scmx_gemm_bf16(const void* A, int64_t lda, const void* W, int64_t
         a.out = part; a.out_f32 = 1; a.ldo = ldp; a.splits = splits; a.split_stride = M * ldp;
         const int rc = tile == 256 ? launch_bg<256, 5, true>(A, lda, W, ldw, a, st)
                      : tile == 128 ? launch_bg<128, 5, false>(A, lda, W, ldw, a, st) : launch_bg<64, 7, false>(A, lda, W, ldw, a, st);
-        if (rc) return rc;
-        const int quads = (int)(ldp / 4);
-        SCMX_PDL_OK("gemm_reduce_kernel", launch_pdl(gemm_reduce_kernel, dim3((unsigned)((M * quads + 255) / 256)), dim3(256), 0, st, (const float*)part,
-                                                     splits, a.split_stride, M, quads, ldp, out_f32 ? 1 : 0, out, ldo));
-        return SCMX_OK;
+        return rc ? rc : gemm_reduce(part, splits, a.split_stride, M, ldp, out_f32 ? 1 : 0, out, ldo, st);
     }
     if (tile == 256) return launch_bg<256, 5, true>(A, lda, W, ldw, a, st);
     if (tile == 128) return launch_bg<128, 5, false>(A, lda, W, ldw, a, st);

@@ -1,0 +1,413 @@
+// float32 GEMM, out = A [M, K] . W [N, K]^T, on tcgen05.mma kind::f16: every operand value is the exact sum of three bfloat16 parts
+// (8 bits of mantissa each), and the six part products above 2^-24 of the whole are summed.
+// The tensor core's float32 accumulator cuts bits off instead of rounding, so its error grows with the number of instructions that add to
+// it.  Therefore the products of the leading parts have an accumulator of their own (the other five are 2^-8 of it), an accumulator takes
+// 256 values of K at most, and the epilogue warps add both to float32 registers, rounded to nearest.
+// Error against 64-bit sums (2-norm, normal operands), K = 1024 / 2048 / 6144: 2.4e-7 / 2.4e-7 / 2.5e-7; sums of CUDA-core multiply-adds
+// 5.7e-7 / 8.1e-7 / 1.4e-6; accumulators over the whole of K 1.0e-6 / 2.1e-6 / 6.7e-6; all six products in one accumulator 1.4e-6.
+//
+// Structure of gemm_bf16 (TMA producer warp, one MMA-issuing thread, 8 epilogue warps, two accumulators, persistent tiles; CTA pairs for
+// large shapes).  A stage holds the three parts of 64 values of both operands: six products use every part loaded twice.
+// Infinities, not-a-number values and values that round to infinity in 16 bits make a sum not a number here; such outputs are
+// computed once more by plain multiply-adds on the float32 operands.
+#include "mix_tc.cuh"
+
+namespace scmx {
+
+int gemm_reduce(const float* part, int splits, int64_t stride, int64_t rows, int64_t ldp, int out_f32, void* out, int64_t ldo, cudaStream_t st);
+
+struct GfArgs {
+    int M, N, K;
+    int part_bytes;              // bytes of one part of a row: K rounded up to 64, times 2
+    int act;                     // 0: none, 1: xIELU, 2: gelu(gate) up, columns alternate 16 gate and 16 up
+    float a_pos, a_neg;
+    const float *A, *W;          // the operands themselves
+    int64_t lda, ldw;
+    float* out;
+    int64_t ldo;
+    int splits;                  // > 1: range s of K goes to out + s * split_stride (no activation)
+    int64_t split_stride;
+    int32_t* status;
+    uint64_t wait_ns;
+};
+
+constexpr int GF_CHUNK = 4;                            // blocks of 64 values per accumulator
+constexpr int GF_PITCH = 80;                           // staged row of 16 outputs; conflict-free 16-byte stores
+constexpr int GF_STAGE_WARP = 32 * GF_PITCH;
+
+// x = p0 + p1 + p2; out [rows][3][kp], zero above K.
+template <int V>
+__global__ void __launch_bounds__(256) split3_kernel(const float* x, int64_t ldx, int64_t rows, int K, int kp, bf16_t* out) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    const int per = kp / V;
+    if (i >= rows * per) return;
+    const int64_t r = i / per;
+    const int c = V * (int)(i - r * per);
+    float v[V];
+    if (V == 4) {
+        const float4 q = c < K ? *reinterpret_cast<const float4*>(x + r * ldx + c) : make_float4(0, 0, 0, 0);
+        v[0] = q.x; v[1 % V] = q.y; v[2 % V] = q.z; v[3 % V] = q.w;
+    } else {
+#pragma unroll
+        for (int e = 0; e < V; ++e) v[e] = c + e < K ? x[r * ldx + c + e] : 0.0f;
+    }
+    bf16_t* o = out + r * 3 * kp + c;
+#pragma unroll
+    for (int p = 0; p < 3; ++p, o += kp) {
+        uint32_t w[V / 2];
+#pragma unroll
+        for (int e = 0; e < V; e += 2) {
+            w[e / 2] = pack_bf16x2(v[e], v[e + 1]);
+            v[e] -= bf16_lo(w[e / 2]);
+            v[e + 1] -= bf16_hi(w[e / 2]);
+        }
+        if (V == 4) *reinterpret_cast<uint2*>(o) = make_uint2(w[0], w[(V / 2) - 1]);
+        else *reinterpret_cast<uint32_t*>(o) = w[0];
+    }
+}
+
+// One output by multiply-adds over values [k0, k1).
+__device__ __noinline__ float gf_dot(const GfArgs& a, int row, int col, int k0, int k1) {
+    const float *x = a.A + (int64_t)row * a.lda, *w = a.W + (int64_t)col * a.ldw;
+    float s = 0.0f;
+    for (int k = k0; k < k1; ++k) s = fmaf(x[k], w[k], s);
+    return s;
+}
+
+template <int BN_, bool PAIR>
+struct GfSmem {
+    static constexpr int BN = BN_, STAGES = 2;
+    static constexpr int ACCS = BN == 256 ? 1 : 2;          // pairs of accumulators in tensor memory
+    static constexpr int A_BYTES = BM * BK;
+    static constexpr int B_BYTES = (PAIR ? BN / 2 : BN) * BK;
+    static constexpr int STAGE_BYTES = 3 * (A_BYTES + B_BYTES);
+    static constexpr int BAR_OFF = STAGES * STAGE_BYTES;
+    static constexpr int MISC_OFF = BAR_OFF + 8 * (2 * STAGES + 4);
+    static constexpr int EPI_OFF = (MISC_OFF + 16 + 127) & ~127;
+    static constexpr int TOTAL = EPI_OFF + EPI_WARPS * GF_STAGE_WARP + 1024;
+};
+
+template <int BN, bool PAIR>
+__device__ __forceinline__ void gemm_f32_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const GfArgs& a) {
+    using L = GfSmem<BN, PAIR>;
+    constexpr int STAGES = L::STAGES;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    const uint32_t sbase = smem_u32(smem);
+    const uint32_t bar_full = sbase + L::BAR_OFF, bar_empty = bar_full + 8 * STAGES;
+    const uint32_t bar_tfull = bar_empty + 8 * STAGES, bar_tempty = bar_tfull + 16;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::MISC_OFF);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::MISC_OFF + 4);
+    constexpr uint32_t TMEM_COLS = 2 * BN * L::ACCS;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = PAIR ? cluster_ctarank() : 0;
+    const bool leader = rank == 0;
+
+    if (threadIdx.x == 0) {
+        prefetch_map(&tmA);
+        prefetch_map(&tmB);
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(bar_full + 8 * s, 1);
+            mbar_init(bar_empty + 8 * s, 1);
+        }
+        for (int i = 0; i < L::ACCS; ++i) {
+            mbar_init(bar_tfull + 8 * i, 1);
+            mbar_init(bar_tempty + 8 * i, PAIR ? 2 * EPI_WARPS : EPI_WARPS);
+        }
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 1) {
+        if (PAIR) {
+            tmem_alloc2(smem_u32(tmem_slot), TMEM_COLS);
+            tmem_relinquish2();
+        } else {
+            tmem_alloc(smem_u32(tmem_slot), TMEM_COLS);
+            tmem_relinquish();
+        }
+    }
+    pdl_launch_dependents();
+    tc_fence_before();
+    __syncthreads();
+    if (PAIR) cluster_sync_all();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();
+
+    const uint32_t full_leader = PAIR ? mapa_u32(bar_full, 0) : bar_full;
+    const uint32_t tempty_leader = PAIR ? mapa_u32(bar_tempty, 0) : bar_tempty;
+    constexpr int TM_ROWS = PAIR ? 2 * BM : BM;
+    const int worker = PAIR ? blockIdx.x >> 1 : blockIdx.x, nworkers = PAIR ? gridDim.x >> 1 : gridDim.x;
+    const int tiles_m = (a.M + TM_ROWS - 1) / TM_ROWS, tiles_n = (a.N + BN - 1) / BN;
+    const int per_split = tiles_m * tiles_n, total = per_split * a.splits;
+    const int all_kb = a.part_bytes / BK, chunks = (all_kb + GF_CHUNK - 1) / GF_CHUNK;
+    // blocks of 64 values of range sp: whole chunks
+    auto first_kb = [&](int sp) { return min(all_kb, GF_CHUNK * (int)((int64_t)chunks * sp / a.splits)); };
+    int fail = 0;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int stage = 0;
+            uint32_t phase = 0;
+            for (int t = worker; t < total && fail == 0; t += nworkers) {
+                const int sp = t / per_split, tt = t - sp * per_split, nt = tt / tiles_m, mt = tt - nt * tiles_m;
+                const int kb0 = first_kb(sp), kb1 = first_kb(sp + 1);
+                const int row0 = mt * TM_ROWS + (int)rank * BM, brow = nt * BN + (PAIR ? (int)rank * (BN / 2) : 0);
+                for (int kb = kb0; kb < kb1; ++kb) {
+                    if (int w = mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, a.wait_ns)) { fail = w == 1 ? 1 : -1; break; }
+                    const uint32_t sa = sbase + stage * L::STAGE_BYTES, sb = sa + 3 * L::A_BYTES;
+                    if (!PAIR) mbar_expect_tx(bar_full + 8 * stage, L::STAGE_BYTES);
+                    else if (leader) mbar_expect_tx(bar_full + 8 * stage, 2 * L::STAGE_BYTES);
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) {
+                        const int x = p * a.part_bytes + kb * BK;
+                        if (PAIR) {
+                            tma_load_2d_pair(sa + p * L::A_BYTES, &tmA, x, row0, full_leader + 8 * stage);
+                            tma_load_2d_pair(sb + p * L::B_BYTES, &tmB, x, brow, full_leader + 8 * stage);
+                        } else {
+                            tma_load_2d(sa + p * L::A_BYTES, &tmA, x, row0, bar_full + 8 * stage);
+                            tma_load_2d(sb + p * L::B_BYTES, &tmB, x, brow, bar_full + 8 * stage);
+                        }
+                    }
+                    if (++stage == STAGES) { stage = 0; phase ^= 1; }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0 && leader) {
+            constexpr uint32_t idesc = umma_idesc_bf16(TM_ROWS, BN);
+            int stage = 0;
+            uint32_t phase = 0, acc = 0, acc_phase = 0;
+            for (int t = worker; t < total && fail == 0; t += nworkers) {
+                const int sp = t / per_split, kb0 = first_kb(sp), kb1 = first_kb(sp + 1);
+                uint32_t d_tmem = 0;
+                for (int kb = kb0; kb < kb1; ++kb) {
+                    const bool fresh = (kb - kb0) % GF_CHUNK == 0;
+                    if (fresh) {
+                        const int w0 = PAIR ? mbar_wait_cluster(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, a.wait_ns)
+                                            : mbar_wait(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, a.wait_ns);
+                        if (w0) { fail = w0 == 1 ? 2 : -1; break; }
+                        tc_fence_after();
+                        d_tmem = tmem_base + acc * 2 * BN;
+                    }
+                    if (int w = mbar_wait(bar_full + 8 * stage, phase, abort_flag, a.wait_ns)) { fail = w == 1 ? 3 : -1; break; }
+                    tc_fence_after();
+                    const uint32_t sa = sbase + stage * L::STAGE_BYTES, sb = sa + 3 * L::A_BYTES;
+#pragma unroll
+                    for (int i = 0; i < 6; ++i) {
+                        constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};
+                        const uint64_t da = umma_desc(sa + PA[i] * L::A_BYTES), db = umma_desc(sb + PB[i] * L::B_BYTES);
+#pragma unroll
+                        for (int k = 0; k < BK / UMMA_K; ++k) {
+                            const uint64_t o = (uint64_t)(k * (UMMA_K >> 4));
+                            const uint32_t on = fresh && k == 0 && (i == 0 || i == 5) ? 0u : 1u, d = d_tmem + (i == 5 ? 0 : BN);
+                            if (PAIR) umma_bf16_pair(d, da + o, db + o, idesc, on);
+                            else umma_bf16(d, da + o, db + o, idesc, on);
+                        }
+                    }
+                    if (PAIR) umma_commit_pair(bar_empty + 8 * stage);
+                    else umma_commit(bar_empty + 8 * stage);
+                    if (++stage == STAGES) { stage = 0; phase ^= 1; }
+                    if (kb + 1 == kb1 || (kb + 1 - kb0) % GF_CHUNK == 0) {
+                        if (PAIR) umma_commit_pair(bar_tfull + 8 * acc);
+                        else umma_commit(bar_tfull + 8 * acc);
+                        if (++acc == L::ACCS) { acc = 0; acc_phase ^= 1; }
+                    }
+                }
+            }
+        }
+    } else {
+        constexpr int COLS = BN / 2;              // of this warp
+        const int q = warp & 3, chalf = (warp - 2) >> 2;
+        uint8_t* stg = smem + L::EPI_OFF + (warp - 2) * GF_STAGE_WARP;
+        uint32_t acc = 0, acc_phase = 0;
+        for (int t = worker; t < total && fail == 0; t += nworkers) {
+            const int sp = t / per_split, tt = t - sp * per_split, nt = tt / tiles_m, mt = tt - nt * tiles_m;
+            const int kb0 = first_kb(sp), kb1 = first_kb(sp + 1);
+            const int n0 = nt * BN + chalf * COLS, row0 = mt * TM_ROWS + (int)rank * BM + 32 * q;
+            float sum[COLS];
+#pragma unroll
+            for (int j = 0; j < COLS; ++j) sum[j] = 0.0f;
+            for (int kb = kb0; kb < kb1; kb += GF_CHUNK) {
+                if (int w = mbar_wait(bar_tfull + 8 * acc, acc_phase, abort_flag, a.wait_ns)) fail = w == 1 ? 4 : -1;
+                epilogue_bar();         // the epilogue threads agree on giving up before anyone touches TMEM
+                if (*abort_flag) { if (!fail) fail = -1; break; }
+                tc_fence_after();
+                const uint32_t taddr = tmem_base + acc * 2 * BN + chalf * COLS + ((uint32_t)(32 * q) << 16);
+#pragma unroll
+                for (int c = 0; c < COLS / 32; ++c) {
+                    uint32_t r[32];
+                    tmem_ld32(taddr + BN + 32 * c, r);
+                    tmem_ld_fence(r);
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) sum[32 * c + j] += __uint_as_float(r[j]);
+                    tmem_ld32(taddr + 32 * c, r);
+                    tmem_ld_fence(r);
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) sum[32 * c + j] += __uint_as_float(r[j]);
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    if (!PAIR || leader) mbar_arrive(bar_tempty + 8 * acc);
+                    else mbar_arrive_cluster(tempty_leader + 8 * acc);
+                }
+                if (++acc == L::ACCS) { acc = 0; acc_phase ^= 1; }
+            }
+            if (fail) break;
+            bool bad = false;
+#pragma unroll
+            for (int j = 0; j < COLS; ++j) bad |= sum[j] != sum[j];
+            if (bad && row0 + lane < a.M) {
+#pragma unroll
+                for (int j = 0; j < COLS; ++j)
+                    if (sum[j] != sum[j] && n0 + j < a.N) sum[j] = gf_dot(a, row0 + lane, n0 + j, 64 * kb0, min(a.K, 64 * kb1));
+            }
+            __syncwarp();
+            float* out = a.out + (int64_t)sp * a.split_stride;
+            const int npad = ((a.act == 2 ? a.N / 2 : a.N) + 3) & ~3, piece = lane & 3, rsub = lane >> 2;
+            // units of 16 outputs: staged a row per lane, stored as 64-byte row pieces
+            auto unit = [&](const float (&v)[16], int col) {
+                float4* o = reinterpret_cast<float4*>(stg + lane * GF_PITCH);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) o[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int rl = 8 * i + rsub, row = row0 + rl;
+                    const float4 x = *reinterpret_cast<const float4*>(stg + rl * GF_PITCH + piece * 16);
+                    if (row < a.M && col + 4 * piece < npad) *reinterpret_cast<float4*>(out + (int64_t)row * a.ldo + col + 4 * piece) = x;
+                }
+                __syncwarp();
+            };
+#pragma unroll
+            for (int c = 0; c < COLS / 32; ++c) {
+                float v[16];
+                if (a.act == 2) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j] = gelu_tanh_f32(sum[32 * c + j]) * sum[32 * c + 16 + j];
+                    unit(v, n0 / 2 + 16 * c);
+                } else {
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            const float x = sum[32 * c + 16 * u + j];
+                            v[j] = a.act == 1 ? xielu_f32(x, a.a_pos, a.a_neg) : x;
+                        }
+                        unit(v, n0 + 32 * c + 16 * u);
+                    }
+                }
+            }
+        }
+    }
+
+    if (fail > 0) {
+        if (atomicCAS(a.status, 0, fail) == 0) {
+            a.status[1] = blockIdx.x;
+            a.status[2] = threadIdx.x;
+        }
+    }
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    if (*abort_flag) {
+        const uint64_t t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);   // 0.2 ms for outstanding TMA writes
+        __syncthreads();
+    }
+    if (PAIR) cluster_sync_all();
+    tc_fence_after();
+    if (warp == 1) {
+        if (PAIR) tmem_dealloc2(tmem_base, TMEM_COLS);
+        else tmem_dealloc(tmem_base, TMEM_COLS);
+    }
+}
+
+template <int BN>
+__global__ void __launch_bounds__(CTA_THREADS, 1) gemm_f32_kernel(const __grid_constant__ CUtensorMap tmA,
+                                                            const __grid_constant__ CUtensorMap tmB, const GfArgs a) {
+    gemm_f32_body<BN, false>(tmA, tmB, a);
+}
+template <int BN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CTA_THREADS, 1)
+    gemm_f32_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GfArgs a) {
+    gemm_f32_body<BN, true>(tmA, tmB, a);
+}
+
+template <int BN, bool PAIR>
+static int launch_gf(const void* A3, const void* W3, const GfArgs& a, cudaStream_t st) {
+    using L = GfSmem<BN, PAIR>;
+    static bool configured[64] = {};
+    const int dev = current_device();
+    SCMX_REQUIRE(dev >= 0, SCMX_ECUDA, "no current CUDA device (ordinal 0..63)");
+    void (*kernel)(CUtensorMap, CUtensorMap, GfArgs);
+    if constexpr (PAIR) kernel = gemm_f32_pair_kernel<BN>;
+    else kernel = gemm_f32_kernel<BN>;
+    if (!configured[dev]) {
+        SCMX_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
+        configured[dev] = true;
+    }
+    CUtensorMap tmA, tmB;
+    int rc = make_map_u8(&tmA, A3, a.M, 3 * (int64_t)a.part_bytes, BK, BM, 128, 3 * (int64_t)a.part_bytes);
+    if (rc) return rc;
+    rc = make_map_u8(&tmB, W3, a.N, 3 * (int64_t)a.part_bytes, BK, PAIR ? BN / 2 : BN, 128, 3 * (int64_t)a.part_bytes);
+    if (rc) return rc;
+    constexpr int rows = PAIR ? 2 * BM : BM;
+    const int64_t tiles = ((a.M + rows - 1) / rows) * (int64_t)((a.N + BN - 1) / BN) * a.splits;
+    int workers = PAIR ? sm_count() / 2 : sm_count();
+    if (tiles < workers) workers = (int)tiles;
+    SCMX_PDL_OK("gemm_f32", launch_pdl(kernel, dim3(PAIR ? 2 * workers : workers), dim3(CTA_THREADS), (size_t)L::TOTAL, st, tmA, tmB, a));
+    return SCMX_OK;
+}
+
+}  // namespace scmx
+
+using namespace scmx;
+
+extern "C" int scmx_split3(const float* x, int64_t ldx, int64_t rows, int64_t K, void* out, void* stream) {
+    SCMX_REQUIRE(x && out && rows >= 0 && K > 0 && K < (1ll << 28) && ldx >= K && ((uintptr_t)out & 15) == 0, SCMX_EINVAL, "split3: rows=%lld K=%lld",
+                 (long long)rows, (long long)K);
+    if (rows == 0) return SCMX_OK;
+    const int kp = (int)((K + 63) / 64 * 64);
+    const bool vec = K % 4 == 0 && ldx % 4 == 0 && ((uintptr_t)x & 15) == 0;
+    const int64_t items = rows * (kp / (vec ? 4 : 2));
+    SCMX_REQUIRE(items < (1ll << 38), SCMX_ELIMIT, "split3: %lld x %lld", (long long)rows, (long long)K);
+    SCMX_PDL_OK("split3_kernel", launch_pdl(vec ? split3_kernel<4> : split3_kernel<2>, dim3((unsigned)((items + 255) / 256)), dim3(256), 0,
+                                            (cudaStream_t)stream, x, ldx, rows, (int)K, kp, (bf16_t*)out));
+    return SCMX_OK;
+}
+
+extern "C" int scmx_gemm_f32(const float* A, int64_t lda, void* A3, const float* W, int64_t ldw, const void* W3, int64_t M, int64_t N, int64_t K,
+                             int act, float a_pos, float a_neg, float* out, int64_t ldo, int tile, int splits, float* part, int32_t* status,
+                             void* stream) {
+    SCMX_REQUIRE(A && A3 && W && W3 && out && status, SCMX_EINVAL, "gemm_f32: null buffer");
+    SCMX_REQUIRE(M >= 0 && N > 0 && K > 0 && M < (1ll << 30) && N < (1ll << 30) && K < (1ll << 28), SCMX_EINVAL, "gemm_f32: M=%lld N=%lld K=%lld",
+                 (long long)M, (long long)N, (long long)K);
+    SCMX_REQUIRE(lda >= K && ldw >= K, SCMX_EINVAL, "gemm_f32: the row pitches %lld, %lld must hold K=%lld", (long long)lda, (long long)ldw, (long long)K);
+    SCMX_REQUIRE(act >= 0 && act <= 2 && (act != 2 || N % 32 == 0), SCMX_EINVAL, "gemm_f32: act=%d on %lld columns", act, (long long)N);
+    const int64_t nout = act == 2 ? N / 2 : N;
+    SCMX_REQUIRE(ldo % 4 == 0 && ldo >= (nout + 3) / 4 * 4, SCMX_EINVAL, "gemm_f32: output pitch %lld for %lld columns", (long long)ldo, (long long)N);
+    SCMX_REQUIRE(((uintptr_t)A3 & 15) == 0 && ((uintptr_t)W3 & 15) == 0 && ((uintptr_t)out & 15) == 0, SCMX_EINVAL, "gemm_f32: pointer not 16-byte aligned");
+    SCMX_REQUIRE(tile == 64 || tile == 128 || tile == 256, SCMX_EINVAL, "gemm_f32: tile=%d", tile);
+    if (M == 0) return SCMX_OK;
+    GfArgs a;
+    a.M = (int)M; a.N = (int)N; a.K = (int)K; a.part_bytes = (int)((K + 63) / 64 * 128); a.act = act; a.a_pos = a_pos; a.a_neg = a_neg;
+    a.A = A; a.W = W; a.lda = lda; a.ldw = ldw; a.out = out; a.ldo = ldo; a.splits = 1; a.split_stride = 0; a.status = status; a.wait_ns = g_wait_limit_ns;
+    const cudaStream_t st = (cudaStream_t)stream;
+    const int64_t ldp = (N + 3) / 4 * 4;
+    if (splits > 1) {
+        SCMX_REQUIRE(part && ((uintptr_t)part & 15) == 0 && act == 0 && splits <= (a.part_bytes / BK + GF_CHUNK - 1) / GF_CHUNK, SCMX_EINVAL,
+                     "gemm_f32: %d ranges of K=%lld need a buffer and no activation", splits, (long long)K);
+        a.out = part; a.ldo = ldp; a.splits = splits; a.split_stride = M * ldp;
+    }
+    int rc = scmx_split3(A, lda, M, K, A3, stream);
+    if (rc) return rc;
+    rc = tile == 256 ? launch_gf<256, true>(A3, W3, a, st) : tile == 128 ? launch_gf<128, false>(A3, W3, a, st) : launch_gf<64, false>(A3, W3, a, st);
+    if (rc || a.splits == 1) return rc;
+    return gemm_reduce(part, splits, a.split_stride, M, ldp, 1, out, ldo, st);
+}

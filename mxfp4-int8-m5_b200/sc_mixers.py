@@ -2,6 +2,8 @@
 row kernels, selective scan, retention, differential attention, gated delta rules, latent attention.  Every function takes CUDA tensors and launches on torch's
 current stream; there is no CPU path.  Activations are bfloat16 or float32 (the weights' type); the residual stream, norms,
 scores and recurrent states are float32."""
+import functools
+
 import torch
 
 from . import _lib
@@ -55,9 +57,47 @@ class GatedGELU:
         return w.view(2, m // 16, 16, k).transpose(0, 1).reshape(2 * m, k)
 
 
+# Float32 portions of fewer rows, or with few columns, are multiplied by the library's float32 product: 16 x 1024 x 1024 takes 9.2 us there
+# and 11.6 us on tensor cores, 300 x 2048 x 64 6.0 and 6.8 us; 32 x 1024 x 1024 takes 13.6 and 11.2 us, 300 x 6144 x 1024 85 and 27 us.
+F32_TC_MIN, F32_TC_MIN_K = 24, 128
+
+
+def split3(x):
+    """float32 [M, K] -> bfloat16 [M, 3 Kp] of its three parts (x = p0 + p1 + p2), Kp = K rounded up to 64, zero padded."""
+    M, K = x.shape
+    out = torch.empty((M, 3 * ((K + 63) // 64 * 64)), dtype=torch.bfloat16, device=x.device)
+    _lib.mcall("scmx_split3", _lib.ptr(x), _ld(x), M, K, _lib.ptr(out), _lib.stream())
+    return out
+
+
+@functools.lru_cache(maxsize=4096)
+def _plan(M, N, K, splits, n_sm=148):
+    """(tile, ranges of K computed side by side) for a product with few output tiles: the fewest bytes staged per SM, counting
+    whole waves; at least 512 of K per range.  (0, 1): leave it to the kernel."""
+    tm = -(-M // 128)
+    if tm * -(-N // 64) >= n_sm or splits == 1:
+        return 0, splits or 1
+    cost = lambda tile, s: -(-tm * -(-N // tile) * s // n_sm) / s * (128 + tile)         # noqa: E731
+    return min(((t, s) for t in (64, 128) for s in ([splits] if splits else range(1, max(1, min(8, K // 512)) + 1))), key=lambda c: cost(*c))
+
+
+@functools.lru_cache(maxsize=4096)
+def _plan_f32(M, N, K, splits, n_sm=148):
+    """(tile, ranges of K) of a float32 product: steps of 64 values stage three parts of 128 + tile rows (CTA pairs: half of a 256 x 256
+    tile each), about 5 ns a row and step, 4 ns for pairs; 5 us around them.  Ranges are whole accumulators of 256 values and cost a summing launch, about 3 us
+    and their traffic.  300 x 4096 x 1024: 26 us as 128 x 128 tiles, 40 us as 128 x 64; 2048 x 2048 x 6144: 242 us as pairs, 257 us as 128 x 128."""
+    kb, chunks = -(-K // 64), -(-K // 256)
+
+    def cost(tile, s):
+        tiles, workers = (-(-M // 256) * -(-N // 256), n_sm // 2) if tile == 256 else (-(-M // 128) * -(-N // tile), n_sm)
+        step = 256 * 0.0105 if tile == 256 else (128 + tile) * 0.0055
+        return 5 + -(-tiles * s // workers) * min(kb, 4 * -(-chunks // s)) * step + (3 + s * M * N * 8 / 3e6 if s > 1 else 0)
+    return min(((t, s) for t in (64, 128, 256) for s in ([splits] if splits else range(1, min(8, chunks) + 1))), key=lambda c: cost(*c))
+
+
 class Linear:
-    """y = W x without bias.  W [N, K] bfloat16 (tcgen05 GEMM / GEMV kernels) or float32 (GEMV kernel for one row, the library's
-    float32 product without reduced-precision modes otherwise)."""
+    """y = W x without bias.  W [N, K] bfloat16 (tcgen05 GEMM / GEMV kernels) or float32 (GEMV kernel for one row, tcgen05 products of
+    three bfloat16 parts for portions, the library's float32 product without reduced-precision modes for a few rows)."""
 
     def __init__(self, w):
         self.N, self.K = w.shape
@@ -68,22 +108,14 @@ class Linear:
             self.w = torch.zeros((self.N, ld), dtype=w.dtype, device=w.device)
             self.w[:, :self.K] = w
         self.dt = _dt(w)
+        self.w3 = split3(self.w[:, :self.K]) if self.dt == 1 and w.is_cuda and self.K >= F32_TC_MIN_K else None
 
     def rows(self, r0, r1):
         """The product with some of the rows, on the same memory."""
         out = object.__new__(Linear)
         out.N, out.K, out.w, out.dt = r1 - r0, self.K, self.w[r0:r1], self.dt
+        out.w3 = None if self.w3 is None else self.w3[r0:r1]
         return out
-
-    def _plan(self, M, splits, n_sm=148):
-        """(tile, ranges of K computed side by side) for a product with few output tiles: the fewest bytes staged per SM, counting
-        whole waves; at least 512 of K per range.  (0, 1): leave it to the kernel."""
-        tm = -(-M // 128)
-        if tm * -(-self.N // 64) >= n_sm or splits == 1:
-            return 0, splits or 1
-        cost = lambda tile, s: -(-tm * -(-self.N // tile) * s // n_sm) / s * (128 + tile)         # noqa: E731
-        return min(((t, s) for t in (64, 128) for s in ([splits] if splits else range(1, max(1, min(8, self.K // 512)) + 1))),
-                   key=lambda c: cost(*c))
 
     def __call__(self, x, out_dtype=None, act=None, tile=0, splits=None):
         """x [M, K] -> [M, N] (N / 2 with a gated activation) in out_dtype (default: the weights' type)."""
@@ -91,6 +123,23 @@ class Linear:
         M = x.shape[0]
         assert x.shape[1] == self.K and x.dtype == self.w.dtype and x.is_cuda
         if self.dt == 1:
+            return self._call_f32(x, act, tile, splits)
+        if _ld(x) % 8 or x.data_ptr() % 16:
+            x = empty_rows(M, self.K, x.dtype, x.device).copy_(x)
+        nout = self.N // 2 if act is not None and act.code == 2 else self.N
+        y = empty_rows(M, nout, out_dtype, x.device)
+        if tile == 0:
+            tile, splits = _plan(M, self.N, self.K, 1 if act is not None else splits)
+        splits = splits or 1
+        part = torch.empty(splits * M * ((self.N + 3) // 4 * 4), dtype=torch.float32, device=x.device) if splits > 1 else None
+        _lib.mcall("scmx_gemm_bf16", _lib.ptr(x), _ld(x), _lib.ptr(self.w), self.w.shape[1], M, self.N, self.K, act.code if act else 0,
+                   act.a_pos if act else 0.0, act.a_neg if act else 0.0, _lib.ptr(y), int(out_dtype == torch.float32), _round8(nout), tile, splits,
+                   _lib.ptr(part), _lib.ptr(_lib.mixer_status_buffer()), _lib.stream())
+        return y
+
+    def _call_f32(self, x, act, tile, splits):
+        M = x.shape[0]
+        if self.w3 is None or M < F32_TC_MIN:
             with _full_float32():
                 y = x @ self.w[:, :self.K].T
             if act is not None and act.code == 2:
@@ -100,17 +149,16 @@ class Linear:
             if act is not None:
                 _lib.mcall("scmx_xielu", _lib.ptr(y), y.numel(), act.a_pos, act.a_neg, _lib.stream())
             return y
-        if _ld(x) % 8 or x.data_ptr() % 16:
-            x = empty_rows(M, self.K, x.dtype, x.device).copy_(x)
         nout = self.N // 2 if act is not None and act.code == 2 else self.N
-        y = empty_rows(M, nout, out_dtype, x.device)
+        y = empty_rows(M, nout, torch.float32, x.device)
         if tile == 0:
-            tile, splits = self._plan(M, 1 if act is not None else splits)
+            tile, splits = _plan_f32(M, self.N, self.K, 1 if act is not None else splits)
         splits = splits or 1
+        x3 = torch.empty((M, self.w3.shape[1]), dtype=torch.bfloat16, device=x.device)
         part = torch.empty(splits * M * ((self.N + 3) // 4 * 4), dtype=torch.float32, device=x.device) if splits > 1 else None
-        _lib.mcall("scmx_gemm_bf16", _lib.ptr(x), _ld(x), _lib.ptr(self.w), self.w.shape[1], M, self.N, self.K, act.code if act else 0,
-                   act.a_pos if act else 0.0, act.a_neg if act else 0.0, _lib.ptr(y), int(out_dtype == torch.float32), _round8(nout), tile, splits,
-                   _lib.ptr(part), _lib.ptr(_lib.mixer_status_buffer()), _lib.stream())
+        _lib.mcall("scmx_gemm_f32", _lib.ptr(x), _ld(x), _lib.ptr(x3), _lib.ptr(self.w), self.w.shape[1], _lib.ptr(self.w3), M, self.N, self.K,
+                   act.code if act else 0, act.a_pos if act else 0.0, act.a_neg if act else 0.0, _lib.ptr(y), _round8(nout), tile, splits, _lib.ptr(part),
+                   _lib.ptr(_lib.mixer_status_buffer()), _lib.stream())
         return y
 
     def vec(self, x, act=None, conv=None, out=None):
