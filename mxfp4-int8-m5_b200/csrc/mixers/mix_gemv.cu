@@ -1,6 +1,6 @@
 // Matrix-vector product of the decode step: out [N] = W [N, K] x, weights bfloat16 or float, x and out float32, float32
-// accumulation.  Each warp owns two rows (or a slice of their columns) and keeps up to 16 weight loads of 16 bytes per lane in
-// flight; the first batch is issued before the previous kernel of the chain has finished (weights never change).
+// accumulation.  Each warp sums two rows at a time (or a slice of their columns) and keeps two sets of 8 weight loads of 16 bytes per lane
+// in flight across its rows; the first are issued before the previous kernel of the chain has finished (weights never change).
 // Epilogues: none; xIELU; the causal convolution + SiLU of the first C rows, whose carried inputs are shifted in place; gelu(gate) up
 // of rows that alternate 16 gate and 16 up rows (a warp owns one of each).
 #include "mix_common.cuh"
@@ -47,28 +47,45 @@ template <> struct Vec8<float> {
 };
 
 template <typename T, int EPI>
-__global__ void __launch_bounds__(256) gemv_x_kernel(const GvArgs a) {
-    constexpr int U = sizeof(T) == 2 ? 8 : 4;          // vectors per lane and row in flight
+__global__ void __launch_bounds__(256, 2) gemv_x_kernel(const GvArgs a) {
+    constexpr int U = sizeof(T) == 2 ? 4 : 2;          // vectors per lane and row in a set
     extern __shared__ __align__(16) float4 xs[];       // [2][nv]: elements 0..3 and 4..7 of every vector of 8
-    __shared__ float part[8][GV_ROWS];
+    __shared__ float part[2][8][GV_ROWS];
+    float* ys = reinterpret_cast<float*>(xs + 2 * ((a.K + 7) >> 3));      // EPI 2: products of this CTA's rows
     pdl_launch_dependents();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nv = (a.K + 7) >> 3, ks = a.ks;
-    const int r0 = (blockIdx.x * (8 / ks) + warp / ks) * GV_ROWS, first = (warp % ks) * 32 + lane, step = 32 * ks;
+    const int nv = (a.K + 7) >> 3, ks = a.ks, team = warp / ks, slice = warp - team * ks, teams = 8 / ks;
+    const int first = slice * 32 + lane, step = 32 * ks;
+    const int sets = (nv + U * step - 1) / (U * step);                 // of a row pair
+    // row pairs of this CTA: equal shares, dealt to its teams in turn
+    const int all = (a.N + GV_ROWS - 1) / GV_ROWS;
+    const int base = (int)((int64_t)all * blockIdx.x / gridDim.x), pairs = (int)((int64_t)all * (blockIdx.x + 1) / gridDim.x);
+    const int p0 = base + team, pstep = teams;
     const T* W = static_cast<const T*>(a.W);
-    auto row_of = [&](int r) { return EPI == 3 ? 32 * (r0 >> 5) + ((r0 >> 1) & 15) + 16 * r : r0 + r; };
-    Vec8<T> w[GV_ROWS][U];
-    auto fetch = [&](int v0) {
+    auto row_of = [&](int r0, int r) { return EPI == 3 ? 32 * (r0 >> 5) + ((r0 >> 1) & 15) + 16 * r : r0 + r; };
+    using Set = Vec8<T>[GV_ROWS][U];
+    Set wa, wb;
+    // the next set to load: of pair lp (done at pairs), from vector lv on
+    int lp = p0, lv = first;
+    auto fetch = [&](Set& w) {
+        const bool on = lp < pairs;
+        const int r0 = lp * GV_ROWS;
 #pragma unroll
         for (int u = 0; u < U; ++u)
 #pragma unroll
             for (int r = 0; r < GV_ROWS; ++r) {
-                const int v = v0 + u * step;
-                if (v < nv && r0 + r < a.N) w[r][u].load(W + (int64_t)row_of(r) * a.ldw + 8 * (int64_t)v);
+                const int v = lv + u * step;
+                if (on && v < nv && r0 + r < a.N) w[r][u].load(W + (int64_t)row_of(r0, r) * a.ldw + 8 * (int64_t)v);
                 else w[r][u].zero();
             }
+        lv += U * step;
+        if (lv - first >= sets * U * step) {
+            lv = first;
+            lp += pstep;
+        }
     };
-    fetch(first);
+    fetch(wa);
+    fetch(wb);
     pdl_wait();
     if ((a.K & 3) == 0 && ((uintptr_t)a.x & 15) == 0) {
 #pragma unroll 8
@@ -82,63 +99,97 @@ __global__ void __launch_bounds__(256) gemv_x_kernel(const GvArgs a) {
     }
     __syncthreads();
     float s[GV_ROWS] = {};
-    for (int v0 = first; v0 < nv; v0 += U * step) {
+    int cp = p0, cv = first, turn = 0;
+    auto finish = [&]() {                               // row pair cp is summed
+        const int r0 = cp * GV_ROWS;
+#pragma unroll
+        for (int r = 0; r < GV_ROWS; ++r) s[r] = warp_sumf(s[r]);
+        if (ks > 1) {
+            if (lane == 0)
+#pragma unroll
+                for (int r = 0; r < GV_ROWS; ++r) part[turn][warp][r] = s[r];
+            // the team's warps meet once per pair; two sets of sums, so that the next pair's are not written over these
+            asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "r"(32 * ks) : "memory");
+            if (slice == 0)
+#pragma unroll
+                for (int r = 0; r < GV_ROWS; ++r) {
+                    s[r] = 0.0f;
+                    for (int i = 0; i < ks; ++i) s[r] += part[turn][warp + i][r];
+                }
+            turn ^= 1;
+        }
+        if (slice == 0) {
+            if (EPI == 3) {
+                if (lane == 0) a.out[r0 >> 1] = gelu_tanh_f32(s[0]) * s[1];
+            } else {
+                const int row = r0 + lane;
+                if (lane < GV_ROWS && row < a.N) {
+                    float y = lane == 0 ? s[0] : s[1];
+                    if (EPI == 1) y = xielu_f32(y, a.a_pos, a.a_neg);
+                    if (EPI == 2 && row < a.C) ys[row - GV_ROWS * base] = y;
+                    else a.out[row] = y;
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < GV_ROWS; ++r) s[r] = 0.0f;
+    };
+    auto consume = [&](Set& w) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const int v = v0 + u * step;
+            const int v = cv + u * step;
             if (v < nv) {
                 const float4 lo = xs[v], hi = xs[nv + v];
 #pragma unroll
                 for (int r = 0; r < GV_ROWS; ++r) s[r] = w[r][u].dot(lo, hi, s[r]);
             }
         }
-        if (v0 + U * step < nv) fetch(v0 + U * step);
+        if (lp < pairs) fetch(w);
+        cv += U * step;
+        if (cv - first >= sets * U * step) {
+            finish();
+            cv = first;
+            cp += pstep;
+        }
+    };
+    while (cp < pairs) {
+        consume(wa);
+        if (cp >= pairs) break;
+        consume(wb);
     }
-#pragma unroll
-    for (int r = 0; r < GV_ROWS; ++r) s[r] = warp_sumf(s[r]);
-    if (ks > 1) {
-        if (lane == 0)
-#pragma unroll
-            for (int r = 0; r < GV_ROWS; ++r) part[warp][r] = s[r];
+    if (EPI == 2) {
+        // the convolution of all rows at once: its loads would otherwise be a chain in every row pair (33 MB of weights: 14 us, then 9)
         __syncthreads();
-        if (warp % ks) return;
-#pragma unroll
-        for (int r = 0; r < GV_ROWS; ++r) {
-            s[r] = 0.0f;
-            for (int i = 0; i < ks; ++i) s[r] += part[warp + i][r];
+        const int row = GV_ROWS * base + tid;
+        for (int r = row; r < min(GV_ROWS * pairs, a.C); r += 256) {
+            const float y = ys[r - GV_ROWS * base];
+            const float* cw = a.cw + (int64_t)r * a.taps;
+            float* tl = a.tail + (int64_t)r * (a.taps - 1);
+            float c = fmaf(cw[a.taps - 1], y, a.cb == nullptr ? 0.0f : a.cb[r]);
+            for (int j = 0; j < a.taps - 1; ++j) {
+                c = fmaf(cw[j], tl[j], c);
+                tl[j] = j + 1 < a.taps - 1 ? tl[j + 1] : y;
+            }
+            a.out[r] = silu_f32(c);
         }
     }
-    if (EPI == 3) {
-        if (lane == 0 && r0 < a.N) a.out[r0 >> 1] = gelu_tanh_f32(s[0]) * s[1];
-        return;
-    }
-    const int row = r0 + lane;
-    if (lane >= GV_ROWS || row >= a.N) return;
-    float y = lane == 0 ? s[0] : s[1];
-    if (EPI == 1) y = xielu_f32(y, a.a_pos, a.a_neg);
-    if (EPI == 2 && row < a.C) {
-        const float* cw = a.cw + (int64_t)row * a.taps;
-        float* tl = a.tail + (int64_t)row * (a.taps - 1);
-        float c = fmaf(cw[a.taps - 1], y, a.cb == nullptr ? 0.0f : a.cb[row]);
-        for (int j = 0; j < a.taps - 1; ++j) {
-            c = fmaf(cw[j], tl[j], c);
-            tl[j] = j + 1 < a.taps - 1 ? tl[j + 1] : y;
-        }
-        y = silu_f32(c);
-    }
-    a.out[row] = y;
 }
 
 template <typename T>
 static int run_gemv(GvArgs a, int epi, cudaStream_t st) {
+    constexpr int U = sizeof(T) == 2 ? 4 : 2;
     const int nv = (a.K + 7) / 8;
-    const size_t smem = (size_t)nv * 32;
-    SCMX_REQUIRE(smem <= 200 * 1024, SCMX_ELIMIT, "gemv_x: K=%d", a.K);
-    int ks = 1;                                        // enough CTAs for every SM, at least a few vectors per lane
-    while (ks < 8 && (a.N + 16 / ks - 1) / (16 / ks) < 2 * sm_count() && nv > 64 * ks) ks *= 2;
+    SCMX_REQUIRE(nv * 32 <= 200 * 1024, SCMX_ELIMIT, "gemv_x: K=%d", a.K);
+    // Persistent CTAs: x is staged once per CTA, and as many as stay resident (registers: two per SM) leave no wave of new ones that starts
+    // with nothing in flight.  Rows are shared by as many warps as still fill a set of loads each.
+    const int resident = (nv * 32 + 4096) * 2 <= 220 * 1024 ? 2 : 1;
+    int ks = 1;
+    while (ks < 8 && nv >= 2 * ks * 32 * U) ks *= 2;
     a.ks = ks;
-    const int rows = 8 / ks * GV_ROWS;
-    const dim3 grid((unsigned)((a.N + rows - 1) / rows)), block(256);
+    const int rows = 8 / ks * GV_ROWS, groups = (a.N + rows - 1) / rows, most = resident * sm_count();
+    const dim3 grid((unsigned)(groups < most ? groups : most)), block(256);
+    const size_t smem = (size_t)nv * 32 + (epi == 2 ? (size_t)4 * GV_ROWS * ((a.N / GV_ROWS + 1) / grid.x + 2) : 0);
+    SCMX_REQUIRE(smem <= 220 * 1024, SCMX_ELIMIT, "gemv_x: N=%d K=%d", a.N, a.K);
     auto kernel = epi == 0 ? gemv_x_kernel<T, 0> : epi == 1 ? gemv_x_kernel<T, 1> : epi == 2 ? gemv_x_kernel<T, 2> : gemv_x_kernel<T, 3>;
     if (smem > 40 * 1024) SCMX_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     SCMX_PDL_OK("gemv_x_kernel", launch_pdl(kernel, grid, block, smem, st, a));

@@ -3,6 +3,7 @@
 // row norm, causal depthwise convolution + SiLU, per-head norm + gate.
 // The residual stream is float32; a bfloat16 copy for the next matrix product is written beside it.
 #include <cooperative_groups.h>
+#include <initializer_list>
 #include "mix_common.cuh"
 
 namespace cg = cooperative_groups;
@@ -10,17 +11,29 @@ namespace cg = cooperative_groups;
 namespace scmx {
 
 // ---- embedding ----------------------------------------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(256) embed_kernel(const int64_t* tok, const T* table, int64_t V, int W, float* x, T* h) {
+// V = 8: 16-byte loads of bfloat16, a thread's elements side by side (one row of 2048: 4 us as single elements, a chain of eight
+// loads and stores per thread); V = 1 for odd widths and unaligned buffers.
+template <typename T, int V>
+__global__ void __launch_bounds__(256) embed_kernel(const int64_t* tok, const T* table, int64_t N, int W, float* x, T* h) {
     pdl_launch_dependents();
     pdl_wait();
     const int64_t t = blockIdx.x;
     int64_t id = tok[t];
-    id = id < 0 ? 0 : (id >= V ? V - 1 : id);
-    for (int i = threadIdx.x; i < W; i += 256) {
-        const T raw = table[id * W + i];
-        x[t * W + i] = ldf(&raw);
-        if (h != nullptr) h[t * W + i] = raw;
+    id = id < 0 ? 0 : (id >= N ? N - 1 : id);
+    for (int i = V * threadIdx.x; i < W; i += 256 * V) {
+        if constexpr (V == 8) {
+            Raw8<T> raw;
+            float v[8];
+            raw.load(table + id * W + i);
+            raw.get(v);
+            st4(x + t * W + i, v[0], v[1], v[2], v[3]);
+            st4(x + t * W + i + 4, v[4], v[5], v[6], v[7]);
+            if (h != nullptr) raw.store(h + t * W + i);
+        } else {
+            const T raw = table[id * W + i];
+            x[t * W + i] = ldf(&raw);
+            if (h != nullptr) h[t * W + i] = raw;
+        }
     }
 }
 
@@ -34,7 +47,7 @@ struct EmbedPairArgs {
     int W;
     float scale;
 };
-template <typename T>
+template <typename T, int V>
 __global__ void __launch_bounds__(256) embed_pair_kernel(const T* table, const T* pairs, const EmbedPairArgs a) {
     pdl_launch_dependents();
     pdl_wait();
@@ -51,9 +64,19 @@ __global__ void __launch_bounds__(256) embed_pair_kernel(const T* table, const T
         }
         pr = pairs + row * a.W;
     }
-    for (int i = threadIdx.x; i < a.W; i += 256) {
-        const float e = ldf(table + id * a.W + i) * a.scale;
-        a.x[t * a.W + i] = pr != nullptr ? e + ldf(pr + i) : e;
+    for (int i = V * threadIdx.x; i < a.W; i += 256 * V) {
+        if constexpr (V == 8) {
+            float e[8], q[8] = {};
+            ld8(table + id * a.W + i, e);
+            if (pr != nullptr) ld8(pr + i, q);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) e[j] = pr != nullptr ? e[j] * a.scale + q[j] : e[j] * a.scale;
+            st4(a.x + t * a.W + i, e[0], e[1], e[2], e[3]);
+            st4(a.x + t * a.W + i + 4, e[4], e[5], e[6], e[7]);
+        } else {
+            const float e = ldf(table + id * a.W + i) * a.scale;
+            a.x[t * a.W + i] = pr != nullptr ? e + ldf(pr + i) : e;
+        }
     }
     if (t == 0 && a.prev != nullptr) {
         __syncthreads();
@@ -245,17 +268,47 @@ __global__ void __launch_bounds__(256) res_norm_kernel(const ResNormArgs a) {
 }
 
 // ---- row norm with gather -----------------------------------------------------------------------------------------------
-template <typename T>
+// V = 4: 16-byte accesses, the first 4096 elements of the row stay in registers (2048 rows of 2048: 17 us as single elements, read twice).
+template <typename T, int V>
 __global__ void __launch_bounds__(256) norm_rows_kernel(const float* x, const int64_t* rows, const float* w, float eps, int W, T* out) {
+    constexpr int KEEP = V == 4 ? 4 : 1;
     __shared__ float red[33];
     pdl_launch_dependents();
     pdl_wait();
     const int64_t m = blockIdx.x, r = rows != nullptr ? rows[m] : m;
     const float* p = x + r * W;
-    float ss = 0.0f;
-    for (int i = threadIdx.x; i < W; i += 256) ss += p[i] * p[i];
-    const float inv = rms_inv_f32(block_sumf(ss, red), W, eps);
-    for (int i = threadIdx.x; i < W; i += 256) stf(out + m * W + i, p[i] * inv * w[i]);
+    T* o = out + m * W;
+    if constexpr (V == 4) {
+        float4 keep[KEEP];
+        float ss = 0.0f;
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k) {
+            const int i = 4 * (threadIdx.x + 256 * k);
+            keep[k] = i < W ? ld4(p + i) : make_float4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k) ss += keep[k].x * keep[k].x + keep[k].y * keep[k].y + keep[k].z * keep[k].z + keep[k].w * keep[k].w;
+        for (int i = 4 * (threadIdx.x + 256 * KEEP); i < W; i += 1024) {
+            const float4 q = ld4(p + i);
+            ss += q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w;
+        }
+        const float inv = rms_inv_f32(block_sumf(ss, red), W, eps);
+        auto write = [&](int i, float4 q) {
+            const float4 u = ld4(w + i);
+            st4(o + i, q.x * inv * u.x, q.y * inv * u.y, q.z * inv * u.z, q.w * inv * u.w);
+        };
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k) {
+            const int i = 4 * (threadIdx.x + 256 * k);
+            if (i < W) write(i, keep[k]);
+        }
+        for (int i = 4 * (threadIdx.x + 256 * KEEP); i < W; i += 1024) write(i, ld4(p + i));
+    } else {
+        float ss = 0.0f;
+        for (int i = threadIdx.x; i < W; i += 256) ss += p[i] * p[i];
+        const float inv = rms_inv_f32(block_sumf(ss, red), W, eps);
+        for (int i = threadIdx.x; i < W; i += 256) stf(o + i, p[i] * inv * w[i]);
+    }
 }
 
 // ---- causal depthwise convolution + SiLU --------------------------------------------------------------------------------
@@ -476,16 +529,39 @@ static int run_conv(const T* x, int64_t ldx, int64_t n_tok, int C, int taps, con
 
 using namespace scmx;
 
+static bool aligned16(std::initializer_list<const void*> ps) {
+    uintptr_t bits = 0;
+    for (const void* p : ps) bits |= (uintptr_t)p;
+    return (bits & 15) == 0;
+}
+
+template <typename T>
+static int run_embed(const int64_t* tokens, const T* table, int64_t V, int64_t n, int W, float* x, T* h, cudaStream_t st) {
+    const bool vec = W % 8 == 0 && aligned16({table, x, h});
+    SCMX_PDL_OK("embed_kernel", launch_pdl(vec ? embed_kernel<T, 8> : embed_kernel<T, 1>, dim3((unsigned)n), dim3(256), 0, st, tokens, table, V, W, x, h));
+    return SCMX_OK;
+}
+template <typename T>
+static int run_embed_pair(const T* table, const T* pairs, const EmbedPairArgs& a, cudaStream_t st) {
+    const bool vec = a.W % 8 == 0 && aligned16({table, pairs, a.x});
+    SCMX_PDL_OK("embed_pair_kernel",
+                launch_pdl(vec ? embed_pair_kernel<T, 8> : embed_pair_kernel<T, 1>, dim3((unsigned)a.T), dim3(256), 0, st, table, pairs, a));
+    return SCMX_OK;
+}
+template <typename T>
+static int run_norm_rows(const float* x, const int64_t* rows, const float* w, float eps, int64_t M, int W, T* out, cudaStream_t st) {
+    const bool vec = W % 4 == 0 && aligned16({x, w, out});
+    SCMX_PDL_OK("norm_rows_kernel",
+                launch_pdl(vec ? norm_rows_kernel<T, 4> : norm_rows_kernel<T, 1>, dim3((unsigned)M), dim3(256), 0, st, x, rows, w, eps, W, out));
+    return SCMX_OK;
+}
+
 extern "C" int scmx_embed(const int64_t* tokens, const void* table, int dt, int64_t V, int64_t T, int W, float* x, void* h, void* stream) {
     SCMX_DT_OK("embed", dt);
     SCMX_REQUIRE(tokens && table && x && V > 0 && T >= 0 && W > 0, SCMX_EINVAL, "embed: bad argument");
     if (T == 0) return SCMX_OK;
-    const cudaStream_t st = (cudaStream_t)stream;
-    if (dt == 0)
-        SCMX_PDL_OK("embed_kernel", launch_pdl(embed_kernel<bf16_t>, dim3((unsigned)T), dim3(256), 0, st, tokens, (const bf16_t*)table, V, W, x, (bf16_t*)h));
-    else
-        SCMX_PDL_OK("embed_kernel", launch_pdl(embed_kernel<float>, dim3((unsigned)T), dim3(256), 0, st, tokens, (const float*)table, V, W, x, (float*)h));
-    return SCMX_OK;
+    return dt == 0 ? run_embed(tokens, (const bf16_t*)table, V, T, W, x, (bf16_t*)h, (cudaStream_t)stream)
+                   : run_embed(tokens, (const float*)table, V, T, W, x, (float*)h, (cudaStream_t)stream);
 }
 
 extern "C" int scmx_res_norm(const float* y, int64_t ldy, const float* x, const float* w, float eps, int64_t T, int W, float* xs,
@@ -504,12 +580,8 @@ extern "C" int scmx_norm_rows(const float* x, const int64_t* rows, const float* 
     SCMX_DT_OK("norm_rows", dt);
     SCMX_REQUIRE(x && w && out && M >= 0 && W > 0, SCMX_EINVAL, "norm_rows: bad argument");
     if (M == 0) return SCMX_OK;
-    const cudaStream_t st = (cudaStream_t)stream;
-    if (dt == 0)
-        SCMX_PDL_OK("norm_rows_kernel", launch_pdl(norm_rows_kernel<bf16_t>, dim3((unsigned)M), dim3(256), 0, st, x, rows, w, eps, W, (bf16_t*)out));
-    else
-        SCMX_PDL_OK("norm_rows_kernel", launch_pdl(norm_rows_kernel<float>, dim3((unsigned)M), dim3(256), 0, st, x, rows, w, eps, W, (float*)out));
-    return SCMX_OK;
+    return dt == 0 ? run_norm_rows(x, rows, w, eps, M, W, (bf16_t*)out, (cudaStream_t)stream)
+                   : run_norm_rows(x, rows, w, eps, M, W, (float*)out, (cudaStream_t)stream);
 }
 
 extern "C" int scmx_conv_silu(const void* x, int64_t ldx, int dt, int64_t T, int C, int taps, const float* w, const float* b, float* tail,
@@ -530,12 +602,8 @@ extern "C" int scmx_embed_pair(const int64_t* tokens, const void* table, const v
     if (T == 0) return SCMX_OK;
     EmbedPairArgs a;
     a.tok = tokens; a.prev = prev; a.x = x; a.V = V; a.T = T; a.buckets = buckets; a.mul_prev = mul_prev; a.mul_cur = mul_cur; a.W = W; a.scale = scale;
-    const cudaStream_t st = (cudaStream_t)stream;
-    if (dt == 0)
-        SCMX_PDL_OK("embed_pair_kernel", launch_pdl(embed_pair_kernel<bf16_t>, dim3((unsigned)T), dim3(256), 0, st, (const bf16_t*)table, (const bf16_t*)pairs, a));
-    else
-        SCMX_PDL_OK("embed_pair_kernel", launch_pdl(embed_pair_kernel<float>, dim3((unsigned)T), dim3(256), 0, st, (const float*)table, (const float*)pairs, a));
-    return SCMX_OK;
+    return dt == 0 ? run_embed_pair((const bf16_t*)table, (const bf16_t*)pairs, a, (cudaStream_t)stream)
+                   : run_embed_pair((const float*)table, (const float*)pairs, a, (cudaStream_t)stream);
 }
 
 extern "C" int scmx_add_norm(const float* y, int64_t ldy, const float* x, const float* w, float mult, float eps, int64_t T, int W, float* x_out,
