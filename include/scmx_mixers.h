@@ -132,6 +132,9 @@ int scmx_diff_decode(const float* q, const void* k_cache, const void* v_cache, i
                      int H, int G, int d, int dv, float scale, float lambda, float diff, float eps, int nsplit, float* part,
                      int32_t* counters, float* o, void* stream);
 
+/* Greedy choice of a token inside a captured decode step, as in scmx.h. */
+int scmx_select_token(const void* logits, int is_f32, int64_t V, int64_t* tok, int32_t* pos, int32_t* count, int64_t* out, int64_t cap, void* stream);
+
 /* out [M, N] = A [M, K] . W [N, K]^T, bfloat16 operands, float32 accumulation; act 1: xIELU with a_pos = softplus(p) and
  * a_neg = 1/2 + softplus(q); act 2: gelu(gate) up of columns that alternate 16 gate and 16 up (N / 2 outputs).  The pitches are multiples of 8; the output pitch covers N rounded up to 16 bytes (the padding is
  * written).  tile: 0 = choose, 64 / 128 = one CTA per 128 x tile, 256 = CTA pairs.  splits > 1: K is cut
