@@ -30,7 +30,9 @@ def _round8(n):
 
 def empty_rows(m, n, dtype, device):
     """[m, n] whose rows start 16-byte aligned."""
-    return torch.empty((m, _round8(n)), dtype=dtype, device=device)[:, :n]
+    r = _round8(n)
+    y = torch.empty((m, r), dtype=dtype, device=device)
+    return y if r == n else y[:, :n]
 
 
 class XIELU:
