@@ -135,6 +135,10 @@ int scmx_attn_decode(const uint16_t* q, const uint16_t* k_cache, const uint16_t*
  * once; non-zero afterwards means a bounded wait inside the kernel ran out (results invalid). */
 int scmx_mm_i8(const int8_t* xq, const int8_t* wq, int64_t M, int64_t N, int64_t K, int epi, const float* xscale,
                const float* wscale, const uint16_t* res, void* out, int32_t* status, void* stream);
+/* The same with K cut into `splits` ranges (2 to 16, at most one per 128 values) computed side by side, for products with few output tiles; part:
+ * int32 [splits][M][N].  Totals are exact, so the bits are the same.  wscale 16-byte aligned. */
+int scmx_mm_i8_split(const int8_t* xq, const int8_t* wq, int64_t M, int64_t N, int64_t K, int epi, const float* xscale,
+                     const float* wscale, const uint16_t* res, void* out, int splits, int32_t* part, int32_t* status, void* stream);
 
 /* Process-wide tuning hint for the N tile of the GEMM kernels: 0 = automatic, 128 or 256.  Counterpart of the
  * module-level tile constants TM, TN, NSG, GROUP_M (e2e/sc_kernels.py:25) and the `tile=` arguments. */

@@ -33,6 +33,9 @@ struct Smem {
     static constexpr int TOTAL = EPI_OFF + EPI_STAGE_BYTES + 1024;       // + slack for 1024-byte alignment
 };
 
+// First K block of range sp.
+__device__ __forceinline__ int range_kb(const GemmArgs& a, int all_kb, int sp) { return a.splits > 1 ? (int)((int64_t)all_kb * sp / a.splits) : sp * all_kb; }
+
 template <int BN, int STAGES>
 __global__ void __launch_bounds__(CTA_THREADS, 1) gemm_i8_kernel(const __grid_constant__ CUtensorMap tmA,
                                                           const __grid_constant__ CUtensorMap tmB, const GemmArgs a) {
@@ -76,8 +79,8 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) gemm_i8_kernel(const __grid_co
     pdl_wait();
 
     int tiles_m, slot0;
-    const int total = num_tiles<BN>(a, tiles_m, slot0);
-    const int num_kb = (a.K + BK - 1) / BK;
+    const int tiles = num_tiles<BN>(a, tiles_m, slot0), total = tiles * max(1, a.splits);
+    const int all_kb = (a.K + BK - 1) / BK;
     int fail = 0;
 
     if (warp == 0) {
@@ -86,8 +89,9 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) gemm_i8_kernel(const __grid_co
             int stage = 0;
             uint32_t phase = 0;
             for (int t = blockIdx.x; t < total && fail == 0; t += gridDim.x) {
-                const Tile tl = get_tile<BN>(a, t, tiles_m, slot0);
-                for (int kb = 0; kb < num_kb; ++kb) {
+                const int sp = t / tiles, kb1 = range_kb(a, all_kb, sp + 1);
+                const Tile tl = get_tile<BN>(a, t - sp * tiles, tiles_m, slot0);
+                for (int kb = range_kb(a, all_kb, sp); kb < kb1; ++kb) {
                     if (int w = mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, a.wait_ns)) { fail = w == 1 ? 1 : -1; break; }
                     const uint32_t sa = sbase + stage * L::STAGE_BYTES, sb = sa + L::A_BYTES;
                     mbar_expect_tx(bar_full + 8 * stage, L::STAGE_BYTES);
@@ -107,6 +111,7 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) gemm_i8_kernel(const __grid_co
                 if (int w = mbar_wait(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, a.wait_ns)) { fail = w == 1 ? 2 : -1; break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * BN;
+                const int sp = t / tiles, num_kb = range_kb(a, all_kb, sp + 1) - range_kb(a, all_kb, sp);
                 for (int kb = 0; kb < num_kb; ++kb) {
                     if (int w = mbar_wait(bar_full + 8 * stage, phase, abort_flag, a.wait_ns)) { fail = w == 1 ? 3 : -1; break; }
                     tc_fence_after();
@@ -133,7 +138,8 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) gemm_i8_kernel(const __grid_co
         const int et = threadIdx.x - 64;          // 0..255 among the epilogue threads
         uint32_t acc = 0, acc_phase = 0;
         for (int t = blockIdx.x; t < total && fail == 0; t += gridDim.x) {
-            const Tile tl = get_tile<BN>(a, t, tiles_m, slot0);
+            const int sp = t / tiles, up = sp * a.M;          // range sp of K is stored `up` rows further down
+            const Tile tl = get_tile<BN>(a, t - sp * tiles, tiles_m, slot0);
             float* ws = ws_stage + acc * BN;
             if (a.epi != 0) {
                 for (int i = et; i < BN; i += EPI_THREADS) ws[i] = (tl.n0 + i < a.N) ? a.wscale[tl.wrow + i] : 0.0f;
@@ -148,8 +154,8 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) gemm_i8_kernel(const __grid_co
             epilogue_bar();
             if (*abort_flag) { if (!fail) fail = -1; break; }
             tc_fence_after();
-            epilogue_warp<BN>(a, tmem_base + acc * BN + chalf * (BN / 2) + ((uint32_t)(32 * q) << 16), ws + chalf * (BN / 2), wrow0,
-                              tl.row_end, tl.n0 + chalf * (BN / 2), smem + L::EPI_OFF + (warp - 2) * EPI_STAGE_WARP, lane, xs, rp);
+            epilogue_warp<BN>(a, tmem_base + acc * BN + chalf * (BN / 2) + ((uint32_t)(32 * q) << 16), ws + chalf * (BN / 2), up + wrow0,
+                              up + tl.row_end, tl.n0 + chalf * (BN / 2), smem + L::EPI_OFF + (warp - 2) * EPI_STAGE_WARP, lane, xs, rp);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
@@ -253,8 +259,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CTA_THREADS, 1)
     const uint32_t full_leader = mapa_u32(bar_full, 0), tempty_leader = mapa_u32(bar_tempty, 0);
     const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
     const int tiles_m = (a.M + 2 * BM - 1) / (2 * BM), tiles_n = (a.N + BN - 1) / BN;
-    const int total = tiles_m * tiles_n;
-    const int num_kb = (a.K + BK - 1) / BK;
+    const int tiles = tiles_m * tiles_n, total = tiles * max(1, a.splits);
+    const int all_kb = (a.K + BK - 1) / BK;
     int fail = 0;
 
     if (warp == 0) {
@@ -262,9 +268,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CTA_THREADS, 1)
             int stage = 0;
             uint32_t phase = 0;
             for (int t = pair; t < total && fail == 0; t += npairs) {
-                const int nt = t / tiles_m, mt = t - nt * tiles_m;
+                const int sp = t / tiles, tt = t - sp * tiles, nt = tt / tiles_m, mt = tt - nt * tiles_m, kb1 = range_kb(a, all_kb, sp + 1);
                 const int row0 = mt * 2 * BM + (int)rank * BM, brow = nt * BN + (int)rank * (BN / 2);
-                for (int kb = 0; kb < num_kb; ++kb) {
+                for (int kb = range_kb(a, all_kb, sp); kb < kb1; ++kb) {
                     if (int w = mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, a.wait_ns)) { fail = w == 1 ? 1 : -1; break; }
                     const uint32_t sa = sbase + stage * L::STAGE_BYTES, sb = sa + L::A_BYTES;
                     if (leader) mbar_expect_tx(bar_full + 8 * stage, 2 * L::STAGE_BYTES);
@@ -283,6 +289,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CTA_THREADS, 1)
                 if (int w = mbar_wait_cluster(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, a.wait_ns)) { fail = w == 1 ? 2 : -1; break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * BN;
+                const int sp = t / tiles, num_kb = range_kb(a, all_kb, sp + 1) - range_kb(a, all_kb, sp);
                 for (int kb = 0; kb < num_kb; ++kb) {
                     if (int w = mbar_wait(bar_full + 8 * stage, phase, abort_flag, a.wait_ns)) { fail = w == 1 ? 3 : -1; break; }
                     tc_fence_after();
@@ -307,7 +314,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CTA_THREADS, 1)
         const int et = threadIdx.x - 64;
         uint32_t acc = 0, acc_phase = 0;
         for (int t = pair; t < total && fail == 0; t += npairs) {
-            const int nt = t / tiles_m, mt = t - nt * tiles_m;
+            const int sp = t / tiles, tt = t - sp * tiles, nt = tt / tiles_m, mt = tt - nt * tiles_m, up = sp * a.M;
             const int n0 = nt * BN, row0 = mt * 2 * BM + (int)rank * BM;
             float* ws = ws_stage + acc * BN;
             if (a.epi != 0) {
@@ -322,7 +329,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CTA_THREADS, 1)
             if (*abort_flag) { if (!fail) fail = -1; break; }
             tc_fence_after();
             epilogue_warp<BN, true, BCAST>(a, tmem_base + acc * BN + chalf * (BN / 2) + ((uint32_t)(32 * q) << 16), ws + chalf * (BN / 2),
-                                           wrow0, a.M, n0 + chalf * (BN / 2), smem + L::EPI_OFF + (warp - 2) * EPI_STAGE_WARP, lane, xs, rp);
+                                           up + wrow0, up + a.M, n0 + chalf * (BN / 2), smem + L::EPI_OFF + (warp - 2) * EPI_STAGE_WARP, lane, xs, rp);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) {
@@ -426,7 +433,7 @@ static int run_gemm(const int8_t* xq, int64_t a_rows, const int8_t* wq, int64_t 
     if (a.E == 0 && g_use_pair && !g_bn_override && a.M > BM && a.N >= PAIR_BN && a.ret_rank == nullptr) {
         rc = make_map(&tmB, wq, b_rows, a.K, PAIR_BN / 2);
         if (rc) return rc;
-        const int64_t tiles = ((a.M + 2 * BM - 1) / (2 * BM)) * (int64_t)((a.N + PAIR_BN - 1) / PAIR_BN);
+        const int64_t tiles = ((a.M + 2 * BM - 1) / (2 * BM)) * (int64_t)((a.N + PAIR_BN - 1) / PAIR_BN) * (a.splits > 1 ? a.splits : 1);
         int pairs = num_sms() / 2;
         if (tiles < pairs) pairs = (int)tiles;
         static bool configured[64] = {};
@@ -447,11 +454,64 @@ static int run_gemm(const int8_t* xq, int64_t a_rows, const int8_t* wq, int64_t 
     if (rc) return rc;
     int grid = num_sms();
     if (a.E == 0) {
-        const int64_t tiles = ((a.M + BM - 1) / BM) * (int64_t)((a.N + bn - 1) / bn);
+        const int64_t tiles = ((a.M + BM - 1) / BM) * (int64_t)((a.N + bn - 1) / bn) * (a.splits > 1 ? a.splits : 1);
         if (tiles < grid) grid = (int)tiles;
     }
     if (bn == 256) return launch_gemm<256, 3>(tmA, tmB, a, grid, st);
     return launch_gemm<128, 5>(tmA, tmB, a, grid, st);
+}
+
+// Totals of the K ranges (exact: INT32) -> the GEMM's epilogue, eight accumulator columns per thread.
+template <int EPI>
+__global__ void __launch_bounds__(256) split_epilogue_kernel(const int32_t* part, int splits, int M, int N, const float* xscale, const float* wscale,
+                                                             const uint16_t* res, const uint16_t* silu_lut, void* out) {
+    pdl_launch_dependents();
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    const int per = N / 8;
+    const int64_t m = i / per;
+    const int n = 8 * (int)(i - m * per);
+    if (m >= M) return;
+    pdl_wait();
+    float4 w0 = make_float4(0, 0, 0, 0), w1 = w0;
+    if (EPI != 0) {
+        w0 = __ldg(reinterpret_cast<const float4*>(wscale + n));
+        w1 = __ldg(reinterpret_cast<const float4*>(wscale + n + 4));
+    }
+    const int64_t e = m * N + n, stride = (int64_t)M * N;
+    int4 s0 = make_int4(0, 0, 0, 0), s1 = s0;
+#pragma unroll 8
+    for (int k = 0; k < splits; ++k) {
+        const int4 a = __ldcg(reinterpret_cast<const int4*>(part + k * stride + e)), b = __ldcg(reinterpret_cast<const int4*>(part + k * stride + e) + 1);
+        s0.x += a.x; s0.y += a.y; s0.z += a.z; s0.w += a.w;
+        s1.x += b.x; s1.y += b.y; s1.z += b.z; s1.w += b.w;
+    }
+    if (EPI == 0) {
+        reinterpret_cast<int4*>(static_cast<int32_t*>(out) + e)[0] = s0;
+        reinterpret_cast<int4*>(static_cast<int32_t*>(out) + e)[1] = s1;
+        return;
+    }
+    const float xs = xscale[m];
+    uint32_t y[4] = {pack_bf16x2(scale2(s0.x, xs, w0.x), scale2(s0.y, xs, w0.y)), pack_bf16x2(scale2(s0.z, xs, w0.z), scale2(s0.w, xs, w0.w)),
+                     pack_bf16x2(scale2(s1.x, xs, w1.x), scale2(s1.y, xs, w1.y)), pack_bf16x2(scale2(s1.z, xs, w1.z), scale2(s1.w, xs, w1.w))};
+    uint16_t* o = static_cast<uint16_t*>(out);
+    if (EPI == 3) {                       // [g0 g1 u0 u1] [g2 g3 u2 u3]
+        uint32_t pk[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const uint32_t g = y[2 * j], u = y[2 * j + 1];
+            const float a = __uint_as_float((uint32_t)__ldg(silu_lut + (g & 0xFFFFu)) << 16), b = __uint_as_float((uint32_t)__ldg(silu_lut + (g >> 16)) << 16);
+            pk[j] = pack_bf16x2(__fmul_rn(a, bf16_lo(u)), __fmul_rn(b, bf16_hi(u)));
+        }
+        *reinterpret_cast<uint2*>(o + e / 2) = make_uint2(pk[0], pk[1]);
+        return;
+    }
+    if (EPI == 2) {
+        const uint4 r = *reinterpret_cast<const uint4*>(res + e);
+        const uint32_t rr[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) y[j] = pack_bf16x2(__fadd_rn(bf16_lo(rr[j]), bf16_lo(y[j])), __fadd_rn(bf16_hi(rr[j]), bf16_hi(y[j])));
+    }
+    *reinterpret_cast<uint4*>(o + e) = make_uint4(y[0], y[1], y[2], y[3]);
 }
 
 // A per-device side stream and the events that order it against the caller's stream (created on first use; event waits and
@@ -519,6 +579,30 @@ extern "C" int scmx_mm_i8(const int8_t* xq, const int8_t* wq, int64_t M, int64_t
     a.M = (int)M; a.N = (int)N; a.K = (int)K; a.epi = epi; a.xscale = xscale; a.wscale = wscale; a.res = res; a.out = out;
     a.status = status;
     return run_gemm(xq, M, wq, N, a, (cudaStream_t)stream);
+}
+
+extern "C" int scmx_mm_i8_split(const int8_t* xq, const int8_t* wq, int64_t M, int64_t N, int64_t K, int epi, const float* xscale,
+                                const float* wscale, const uint16_t* res, void* out, int splits, int32_t* part, int32_t* status, void* stream) {
+    int rc = check_common("mm_i8_split", N, K, epi, xscale, wscale, out, status);
+    if (rc) return rc;
+    SCMX_REQUIRE(M >= 0 && M < (1ll << 30), SCMX_EINVAL, "mm_i8_split: M=%lld out of range", (long long)M);
+    SCMX_REQUIRE(epi != 2 || res, SCMX_EINVAL, "mm_i8_split: epi 2 needs res");
+    SCMX_REQUIRE(splits >= 2 && splits <= 16 && splits <= (K + BK - 1) / BK && part && splits * M < (1ll << 30), SCMX_EINVAL,
+                 "mm_i8_split: %d ranges of K=%lld need a buffer", splits, (long long)K);
+    SCMX_REQUIRE(((reinterpret_cast<uintptr_t>(xq) | reinterpret_cast<uintptr_t>(wq) | reinterpret_cast<uintptr_t>(res) | reinterpret_cast<uintptr_t>(part) |
+                   reinterpret_cast<uintptr_t>(wscale)) & 15) == 0, SCMX_EINVAL, "mm_i8_split: xq, wq, wscale, res and part must be 16-byte aligned");
+    if (M == 0) return SCMX_OK;
+    const cudaStream_t st = (cudaStream_t)stream;
+    const uint16_t* lut = nullptr;
+    if (epi == 3 && (rc = silu_lut_ptr(st, &lut))) return rc;
+    GemmArgs a = {};
+    a.M = (int)M; a.N = (int)N; a.K = (int)K; a.epi = 0; a.out = part; a.status = status; a.splits = splits;
+    rc = run_gemm(xq, M, wq, N, a, st);
+    if (rc) return rc;
+    auto kernel = epi == 0 ? split_epilogue_kernel<0> : epi == 1 ? split_epilogue_kernel<1> : epi == 2 ? split_epilogue_kernel<2> : split_epilogue_kernel<3>;
+    SCMX_PDL_OK("split_epilogue_kernel", launch_pdl(kernel, dim3((unsigned)((M * (N / 8) + 255) / 256)), dim3(256), 0, st, (const int32_t*)part, splits, (int)M,
+                                                    (int)N, xscale, wscale, res, lut, out));
+    return SCMX_OK;
 }
 
 extern "C" int scmx_mm_i8_bcast(const int8_t* xq, const int8_t* wq, int64_t M, int64_t N, int64_t K, int epi, const float* xscale,

@@ -35,6 +35,7 @@ struct GemmArgs {
     int bcast;                   // > 0 (tensor parallelism): every output row is stored into peer_out[0 .. bcast) at the same row / column
     const int32_t* ret_row;
     uint16_t* peer_out[8];
+    int splits;                  // > 1 (dense, epi 0): K is cut into this many ranges; range s goes to rows s * M .. of `out`
 };
 
 // Barrier among the epilogue threads only (named barrier 1).

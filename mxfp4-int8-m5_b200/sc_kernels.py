@@ -7,6 +7,8 @@ allocated CUDA tensors, and accepts (and ignores) the reference's Metal tuning a
 
 All arithmetic happens in libscmx (CUDA, sm_100a); the GEMMs are tcgen05 kind::i8 kernels.
 """
+import functools
+
 import numpy as np
 import torch
 
@@ -102,6 +104,29 @@ def _rmsnorm_quant(x, w, eps, Mp, want_n):
     return xq, xs, xn
 
 
+@functools.lru_cache(maxsize=4096)
+def _ranges(M, N, K, n_sm=148):
+    """Ranges of K for a dense product whose tiles leave most SMs idle (CTA pairs of 256 x 256 tiles, single CTAs up to 128 rows).  Summing the
+    ranges costs a launch of 3 us and their traffic, which only a long K repays: 384 x 2048 x 6144 takes 21.7 us in one piece and
+    15.4 us in four, 128 x 1024 x 3072 14.3 and 10.4 us in eight, but 384 x 2048 x 2048 11.7 and 12.1 us."""
+    if K < 3072:
+        return 1
+    if M > 128 and N >= 256:
+        return max(1, min(4, n_sm // 2 // (-(-M // 256) * -(-N // 256))))
+    return max(1, min(8, n_sm // (-(-M // 128) * -(-N // (256 if N >= 256 else 128)))))
+
+
+def _mm_i8(xq, wq, M, N, K, epi, xscale, wscale, res, out, splits=None):
+    splits = splits or (_ranges(M, N, K) if wscale is None or wscale.data_ptr() % 16 == 0 else 1)
+    head = (_lib.ptr(xq), _lib.ptr(wq), M, N, K, epi, _lib.ptr(xscale), _lib.ptr(wscale), _lib.ptr(res), _lib.ptr(out))
+    if splits > 1:
+        part = torch.empty((splits, M, N), dtype=torch.int32, device=xq.device)
+        _lib.call("scmx_mm_i8_split", *head, splits, _lib.ptr(part), _lib.ptr(_lib.status_buffer()), _lib.stream())
+    else:
+        _lib.call("scmx_mm_i8", *head, _lib.ptr(_lib.status_buffer()), _lib.stream())
+    return out
+
+
 def mm_i8_i32(xq, wq, deps=(), tile=None):
     """INT8 [M, K] x INT8 [N, K]^T -> INT32 [M, N] (exact)."""
     _lib.require_cuda(xq, wq)
@@ -109,9 +134,7 @@ def mm_i8_i32(xq, wq, deps=(), tile=None):
     assert xq.dtype == torch.int8 and wq.dtype == torch.int8 and wq.shape[1] == K
     assert M % TM == 0 and N % 32 == 0, (M, N, TM)
     acc = torch.empty((M, N), dtype=torch.int32, device=xq.device)
-    _lib.call("scmx_mm_i8", _lib.ptr(xq), _lib.ptr(wq), M, N, K, 0, None, None, None, _lib.ptr(acc),
-              _lib.ptr(_lib.status_buffer()), _lib.stream())
-    return acc
+    return _mm_i8(xq, wq, M, N, K, 0, None, None, None, acc)
 
 
 def mm_epi(xq, wq, xscale, wscale, epi, dtype=torch.bfloat16, res=None, deps=(), tile=None):
@@ -123,9 +146,7 @@ def mm_epi(xq, wq, xscale, wscale, epi, dtype=torch.bfloat16, res=None, deps=(),
     assert M % TM == 0 and N % 32 == 0 and (epi != 2 or tuple(res.shape) == (M, N)), (M, N, TM)
     assert xscale.shape == (M,) and wscale.shape == (N,)
     out = torch.empty((M, N // 2 if epi == 3 else N), dtype=torch.bfloat16, device=xq.device)
-    _lib.call("scmx_mm_i8", _lib.ptr(xq), _lib.ptr(wq), M, N, K, epi, _lib.ptr(xscale), _lib.ptr(wscale),
-              _lib.ptr(res) if epi == 2 else None, _lib.ptr(out), _lib.ptr(_lib.status_buffer()), _lib.stream())
-    return out
+    return _mm_i8(xq, wq, M, N, K, epi, xscale, wscale, res if epi == 2 else None, out)
 
 
 def mm_w4_epi(xq, codes, bcodes, xscale, wscale, N, epi, dtype=torch.bfloat16, res=None):
