@@ -18,6 +18,7 @@ from . import sc_format as F
 from . import sc_kernels as S
 from . import sc_moe as M_
 from .fused_moe import MoeBlock
+from .fused_qwen3 import attend_quant
 from .w4a8 import PackedWeight
 
 ATTN = ["self_attn.q_proj", "self_attn.k_proj", "self_attn.v_proj", "self_attn.o_proj"]
@@ -196,8 +197,7 @@ class FusedOlmoe:
             q, kk, v = S.qkv_fullnorm_y(y, at.q_norm.weight, at.k_norm.weight, self.eps, L, H, d,
                                         rope=(self.inv_freq, c.offset, self.rope_cs), cache=c)
             c.offset += L
-            o = self.sdpa(q, kk, v, at.scale, True)
-            xq, xs = S.act_quant(o, Mp)
+            xq, xs = attend_quant(self.sdpa, q, kk, v, at.scale, Mp)
             h = S.mm_epi(xq, wo.unpack(), xs, wo.wscale, 2, res=h)
             xq, xs, xn = S.rmsnorm_quant_n(h, layer.post_attention_layernorm.weight, self.eps)
             inds, scores = self.route(layer, xn, L)

@@ -143,8 +143,8 @@ class TokenCache:
         return [self.prev]
 
 
-def sdpa(q, k, v, scale, causal):
-    """q [hq, L, d], k / v [hk, T, d] (T >= L: the last L keys are the queries' own positions) -> [L, hq * d]."""
+def sdpa_heads(q, k, v, scale, causal):
+    """q [hq, L, d], k / v [hk, T, d] (T >= L: the last L keys are the queries' own positions) -> [hq, L, d], strides as torch chooses."""
     hq, L, d = q.shape
     hk, T = k.shape[0], k.shape[1]
     mask = None
@@ -153,7 +153,13 @@ def sdpa(q, k, v, scale, causal):
         mask = torch.ones(L, T, dtype=torch.bool, device=q.device).tril(T - L)
     o = TF.scaled_dot_product_attention(q[None], k[None], v[None], attn_mask=mask, is_causal=is_causal, scale=scale,
                                         enable_gqa=hq != hk)
-    return o[0].transpose(0, 1).reshape(L, hq * d)
+    return o[0]
+
+
+def sdpa(q, k, v, scale, causal):
+    """The same -> [L, hq * d]."""
+    hq, L, d = q.shape
+    return sdpa_heads(q, k, v, scale, causal).transpose(0, 1).reshape(L, hq * d)
 
 
 def sdpa_f64(q, k, v, scale, causal):
