@@ -160,7 +160,21 @@ __global__ void __launch_bounds__(256) gemv_kernel(const GemvArgs a) {
             }
         }
     }
+    // row scales with the codes: loaded where they are used, they would cost a round trip to memory after the sum
+    float ws[4] = {};
+    if (rows_ok && a.epi != 0) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) ws[r] = __ldg(a.wscale + (size_t)ex * a.N + n0 + r);
+    }
     if (!a.eidx) asm volatile("griddepcontrol.wait;" ::: "memory");
+    float res[4] = {}, xs_in = 0.0f;
+    if (rows_ok && a.epi != 0) {
+        if (!PRO) xs_in = a.xscale[(size_t)slot * a.xstride];
+        if (a.epi == 2) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) res[r] = bf16_to_f32(a.res[n0 + r]);
+        }
+    }
 
     float xs_pro = 0.0f;
     if (PRO) xs_pro = gemv_prologue<PRO>(a, slot, xq_s, xn_s, red, dred);
@@ -209,14 +223,13 @@ __global__ void __launch_bounds__(256) gemv_kernel(const GemvArgs a) {
         }
     }
     if (lane != 0 || !rows_ok) return;
-    const float* ws = a.wscale + (size_t)ex * a.N + n0;
     if (a.epi == 0) {
         int32_t* o = reinterpret_cast<int32_t*>(a.out) + (size_t)slot * a.N + n0;
 #pragma unroll
         for (int r = 0; r < 4; ++r) o[r] = tot[r];
         return;
     }
-    const float xs = PRO ? xs_pro : a.xscale[(size_t)slot * a.xstride];
+    const float xs = PRO ? xs_pro : xs_in;
     float y[4];
 #pragma unroll
     for (int r = 0; r < 4; ++r) y[r] = scale_acc(tot[r], xs, ws[r]);
@@ -228,7 +241,7 @@ __global__ void __launch_bounds__(256) gemv_kernel(const GemvArgs a) {
     } else if (a.epi == 2) {
         uint16_t* o = out + (size_t)slot * a.N + n0;
 #pragma unroll
-        for (int r = 0; r < 4; ++r) o[r] = f32_to_bf16(__fadd_rn(bf16_to_f32(a.res[n0 + r]), y[r]));
+        for (int r = 0; r < 4; ++r) o[r] = f32_to_bf16(__fadd_rn(res[r], y[r]));
     } else {
         uint16_t* o = out + (size_t)slot * (a.N / 2) + n0 / 2;
         o[0] = f32_to_bf16(swiglu_bf16(y[0], y[2]));
