@@ -177,6 +177,8 @@ int scmx_route_sort(const int32_t* inds, int64_t M, int topk, int E, int tm, int
  * scores bf16 [M,topk]; scores_f32 (may be NULL) f32 [M,topk]. */
 int scmx_router_topk(const float* logits, int64_t M, int E, int topk, int32_t* inds, uint16_t* scores,
                      float* scores_f32, void* stream);
+/* The router of one token in one kernel: logits bf16(W xn) (W bf16 [E, D], xn bf16 [D], 16-byte aligned, D % 8 == 0), then as scmx_router_topk. */
+int scmx_route_token(const uint16_t* xn, const uint16_t* W, int D, int E, int topk, int32_t* inds, uint16_t* scores, void* stream);
 
 /* Row gather: dst_q[p] = xq[tok[p]] for p < rows_q, dst_s[p] = xs[tok[p]] for p < rows_s
  * (the `xq[tok_p], xs[tok_p[:R]]` of e2e/fused_olmoe.py:230). */

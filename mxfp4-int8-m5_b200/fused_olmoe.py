@@ -123,6 +123,13 @@ class FusedOlmoe:
         logits = torch.nn.functional.linear(xn[:M], layer.mlp.gate.weight)
         return M_.router_topk(logits.float(), self.args.num_experts_per_tok)
 
+    def route_token(self, layer, xn):
+        """route for one row, in one kernel where the sizes allow."""
+        w = layer.mlp.gate.weight
+        if w.dtype == xn.dtype == torch.bfloat16 and w.is_contiguous() and w.shape[1] % 8 == 0 and w.shape[0] <= 1024 and w.data_ptr() % 16 == 0:
+            return M_.route_token(xn, w, self.args.num_experts_per_tok)
+        return self.route(layer, xn, 1)
+
     def _packed(self, R):
         """Whether the grouped GEMMs read the packed weights (scmx_moe_mm_w4) although the experts could be decoded ahead: MoeBlock's
         rule.  An expert's INT8 copy costs three passes over its bytes, which few rows do not repay: two layers of 64 experts of

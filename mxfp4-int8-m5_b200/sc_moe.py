@@ -62,6 +62,16 @@ def router_topk(logits, k):
     return inds, scores
 
 
+def route_token(xn, w, k):
+    """Router of one token: xn bf16 [1, D], w bf16 [E, D] -> (inds int32 [1, k], scores bf16 [1, k]) of softmax(bf16(w xn))."""
+    _lib.require_cuda(xn, w)
+    E, D = w.shape
+    inds = torch.empty((1, k), dtype=torch.int32, device=xn.device)
+    scores = torch.empty((1, k), dtype=torch.bfloat16, device=xn.device)
+    _lib.call("scmx_route_token", _lib.ptr(xn), _lib.ptr(w), D, E, k, _lib.ptr(inds), _lib.ptr(scores), _lib.stream())
+    return inds, scores
+
+
 def gather_rows(xq, xs, tok, R):
     """(xq[tok], xs[tok[:R]]): INT8 rows and scales of the sorted assignments (tok has R + tm entries)."""
     _lib.require_cuda(xq, xs, tok)
