@@ -17,9 +17,17 @@ struct GvArgs {
     const float *cw, *cb;   // convolution weights [C, taps] and bias [C]
     float* tail;            // [C, taps - 1]
     int C, taps;
+    // The input row may be one that the sublayers before leave in parts (pro): 1: r = x + mult y, input r / rms(r) nw;
+    // 2: r = x + nw y / rms(y), then with n > 0 the weighted sum of n - 1 stored rows and r, input r, or r / rms(r) fw.
+    int pro, n, keep;       // keep: r goes to row n - 1 of the store before it is averaged
+    float mult, eps;
+    const float *y, *nw, *dwa, *fw;
+    float *store, *x_out;   // x_out: r (not normalized), written by the first CTA, or null
+    int64_t store_stride;
 };
 
 constexpr int GV_ROWS = 2;
+constexpr int GV_PRO_MAXK = 2048;      // two 16-byte pieces per thread
 
 template <typename T> struct Vec8;
 template <> struct Vec8<bf16_t> {
@@ -46,11 +54,75 @@ template <> struct Vec8<float> {
     }
 };
 
+// The residual and norm kernels between two products cost 2 - 5 us each in a chain of single rows, nearly all of it latency.  Every CTA computes
+// the whole row itself while its first weights arrive: a few reads from L2 and one or two sums over the CTA.
+__device__ __forceinline__ void gv_prologue(const GvArgs& a, float4* xs, int nv, float* red) {
+    const int tid = threadIdx.x, quads = a.K >> 2;
+    const bool first = blockIdx.x == 0;
+    float4 r[2], w[2], s[2];
+    float ss = 0.0f;
+    const float self = a.pro == 2 && a.n > 0 ? a.dwa[a.n - 1] : 1.0f;
+    auto sq = [](const float4& v) { return v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w; };
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int i = tid + 256 * k;
+        r[k] = w[k] = s[k] = make_float4(0, 0, 0, 0);
+        if (i >= quads) continue;
+        w[k] = ld4(a.nw + 4 * i);
+        const float4 x = ld4(a.x + 4 * i), y = a.y != nullptr ? ld4(a.y + 4 * i) : make_float4(0, 0, 0, 0);
+        if (a.pro == 1) {
+            r[k] = a.y != nullptr ? make_float4(fmaf(a.mult, y.x, x.x), fmaf(a.mult, y.y, x.y), fmaf(a.mult, y.z, x.z), fmaf(a.mult, y.w, x.w)) : x;
+            ss += sq(r[k]);
+        } else {
+            r[k] = y;
+            ss += sq(y);
+            s[k] = x;      // joined with the norm below
+        }
+    }
+    const float inv = rms_inv_f32(block_sumf(ss, red), a.K, a.eps);
+    if (a.pro == 2) {
+        ss = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int i = tid + 256 * k;
+            if (i >= quads) continue;
+            r[k] = make_float4(s[k].x + r[k].x * inv * w[k].x, s[k].y + r[k].y * inv * w[k].y, s[k].z + r[k].z * inv * w[k].z, s[k].w + r[k].w * inv * w[k].w);
+            if (a.n > 0) {
+                float4 m = make_float4(0, 0, 0, 0);
+#pragma unroll 4
+                for (int j = 0; j < a.n - 1; ++j) {
+                    const float c = a.dwa[j];
+                    const float4 q = ld4(a.store + j * a.store_stride + 4 * i);
+                    m.x += c * q.x; m.y += c * q.y; m.z += c * q.z; m.w += c * q.w;
+                }
+                if (a.keep && first) *reinterpret_cast<float4*>(a.store + (a.n - 1) * a.store_stride + 4 * i) = r[k];
+                r[k] = make_float4(m.x + self * r[k].x, m.y + self * r[k].y, m.z + self * r[k].z, m.w + self * r[k].w);
+            }
+            if (a.fw != nullptr) {
+                w[k] = ld4(a.fw + 4 * i);
+                ss += sq(r[k]);
+            }
+        }
+    }
+    const float scale = a.pro == 1 ? inv : a.fw != nullptr ? rms_inv_f32(block_sumf(ss, red), a.K, a.eps) : 1.0f;
+    const bool norm = a.pro == 1 || a.fw != nullptr;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int i = tid + 256 * k;
+        if (i < 2 * nv) {
+            float4 h = r[k];
+            if (norm) h = make_float4(h.x * scale * w[k].x, h.y * scale * w[k].y, h.z * scale * w[k].z, h.w * scale * w[k].w);
+            xs[(i & 1) * nv + (i >> 1)] = h;      // zero above K
+            if (first && a.x_out != nullptr && i < quads) *reinterpret_cast<float4*>(a.x_out + 4 * i) = r[k];
+        }
+    }
+}
+
 template <typename T, int EPI>
 __global__ void __launch_bounds__(256, 2) gemv_x_kernel(const GvArgs a) {
     constexpr int U = sizeof(T) == 2 ? 4 : 2;          // vectors per lane and row in a set
     extern __shared__ __align__(16) float4 xs[];       // [2][nv]: elements 0..3 and 4..7 of every vector of 8
-    __shared__ float part[2][8][GV_ROWS];
+    __shared__ float part[2][8][GV_ROWS], red[33];
     float* ys = reinterpret_cast<float*>(xs + 2 * ((a.K + 7) >> 3));      // EPI 2: products of this CTA's rows
     pdl_launch_dependents();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -87,7 +159,9 @@ __global__ void __launch_bounds__(256, 2) gemv_x_kernel(const GvArgs a) {
     fetch(wa);
     fetch(wb);
     pdl_wait();
-    if ((a.K & 3) == 0 && ((uintptr_t)a.x & 15) == 0) {
+    if (a.pro != 0) {
+        gv_prologue(a, xs, nv, red);
+    } else if ((a.K & 3) == 0 && ((uintptr_t)a.x & 15) == 0) {
 #pragma unroll 8
         for (int i = tid; i < 2 * nv; i += 256)
             xs[(i & 1) * nv + (i >> 1)] = 4 * i < a.K ? *reinterpret_cast<const float4*>(a.x + 4 * i) : make_float4(0, 0, 0, 0);
@@ -200,15 +274,35 @@ static int run_gemv(GvArgs a, int epi, cudaStream_t st) {
 
 using namespace scmx;
 
-extern "C" int scmx_gemv_x(const void* W, int64_t ldw, int dt, const float* x, int64_t N, int64_t K, int epi, float a_pos, float a_neg,
-                           const float* conv_w, const float* conv_b, float* tail, int C, int taps, float* out, void* stream) {
+static int gemv_x(const void* W, int64_t ldw, int dt, const float* x, int64_t N, int64_t K, int epi, float a_pos, float a_neg, const float* conv_w,
+                  const float* conv_b, float* tail, int C, int taps, float* out, GvArgs a, void* stream) {
     SCMX_DT_OK("gemv_x", dt);
     SCMX_REQUIRE(W && x && out && N > 0 && K > 0 && N < (1ll << 30) && K < (1ll << 30), SCMX_EINVAL, "gemv_x: N=%lld K=%lld", (long long)N, (long long)K);
     SCMX_REQUIRE(ldw % 8 == 0 && ldw >= K && ((uintptr_t)W & 15) == 0, SCMX_EINVAL, "gemv_x: row pitch %lld", (long long)ldw);
     SCMX_REQUIRE(epi >= 0 && epi <= 3 && (epi != 3 || N % 32 == 0), SCMX_EINVAL, "gemv_x: epi=%d on %lld rows", epi, (long long)N);
     SCMX_REQUIRE(epi != 2 || (conv_w && C > 0 && C <= N && taps >= 1 && (taps == 1 || tail)), SCMX_EINVAL, "gemv_x: convolution epilogue");
-    GvArgs a;
     a.W = W; a.x = x; a.out = out; a.ldw = ldw; a.N = (int)N; a.K = (int)K; a.ks = 1; a.a_pos = a_pos; a.a_neg = a_neg;
     a.cw = conv_w; a.cb = conv_b; a.tail = tail; a.C = C; a.taps = taps;
     return dt == 0 ? run_gemv<bf16_t>(a, epi, (cudaStream_t)stream) : run_gemv<float>(a, epi, (cudaStream_t)stream);
+}
+
+extern "C" int scmx_gemv_x(const void* W, int64_t ldw, int dt, const float* x, int64_t N, int64_t K, int epi, float a_pos, float a_neg,
+                           const float* conv_w, const float* conv_b, float* tail, int C, int taps, float* out, void* stream) {
+    return gemv_x(W, ldw, dt, x, N, K, epi, a_pos, a_neg, conv_w, conv_b, tail, C, taps, out, GvArgs{}, stream);
+}
+
+extern "C" int scmx_gemv_x_row(const void* W, int64_t ldw, int dt, const float* x, const float* y, const float* nw, int pro, float mult, float eps,
+                               float* store, int64_t store_stride, const float* dwa, int n, int keep, const float* fw, float* x_out, int64_t N,
+                               int64_t K, int epi, float a_pos, float a_neg, const float* conv_w, const float* conv_b, float* tail, int C, int taps,
+                               float* out, void* stream) {
+    SCMX_REQUIRE((pro == 1 || (pro == 2 && y)) && nw && K <= GV_PRO_MAXK && K % 4 == 0, SCMX_EINVAL, "gemv_x_row: pro=%d K=%lld", pro, (long long)K);
+    SCMX_REQUIRE(n >= 0 && (n == 0 || (pro == 2 && store && dwa && store_stride >= K && store_stride % 4 == 0)), SCMX_EINVAL,
+                 "gemv_x_row: average over %d results without a store", n);
+    SCMX_REQUIRE(x_out == nullptr || (x_out != x && x_out != y && x_out != out), SCMX_EINVAL, "gemv_x_row: the new row needs a place of its own");
+    SCMX_REQUIRE((((uintptr_t)x | (uintptr_t)y | (uintptr_t)nw | (uintptr_t)store | (uintptr_t)fw | (uintptr_t)x_out) & 15) == 0, SCMX_EINVAL,
+                 "gemv_x_row: rows must be 16-byte aligned");
+    GvArgs a = {};
+    a.pro = pro; a.n = n; a.keep = keep; a.mult = mult; a.eps = eps; a.y = y; a.nw = nw; a.dwa = dwa; a.fw = pro == 2 ? fw : nullptr;
+    a.store = store; a.x_out = x_out; a.store_stride = store_stride;
+    return gemv_x(W, ldw, dt, x, N, K, epi, a_pos, a_neg, conv_w, conv_b, tail, C, taps, out, a, stream);
 }

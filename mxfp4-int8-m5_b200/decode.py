@@ -248,7 +248,8 @@ class DecodeHybrid(_Decoder):
         self.f, self.model, self.args, self._graph = fused, fused.model, fused.args, None
         dev, a = fused.model.device, self.args
         f32 = lambda *s: torch.empty(s, dtype=torch.float32, device=dev)    # noqa: E731
-        self.x, self.h, self.y = f32(1, a.hidden_size), f32(1, a.hidden_size), f32(1, a.hidden_size)
+        # the residual row: a product that joins it reads one buffer and writes the other
+        self.x, self.y = (f32(1, a.hidden_size), f32(1, a.hidden_size)), f32(1, a.hidden_size)
         if not a.design.prenorm:     # the embedding's and every layer's result, for the depth average
             self.xs = f32(len(a.layers) + 1, 1, a.hidden_size)
         own = {}
@@ -266,34 +267,37 @@ class DecodeHybrid(_Decoder):
         f = self.f
         f.ensure_positions(cache[0].capacity)
         assert pos_dev is not None or cache[0].offset < cache[0].capacity, "KV cache capacity exceeded"
-        h = (self._prenorm if self.args.design.prenorm else self._postnorm)(tok.view(-1), cache, pos_dev)
-        return f.head.vec(h[0])[None, None]
+        row = (self._prenorm if self.args.design.prenorm else self._postnorm)(tok.view(-1), cache, pos_dev)
+        return f.head.vec(row)[None, None]
 
     def _prenorm(self, tok, cache, pos_dev):
-        f, x, h, y, mult = self.f, self.x, self.h, self.y, self.args.residual_mult
+        f, (x, spare), y, mult = self.f, self.x, self.y, self.args.residual_mult
         f.embed(tok, cache, x)
         nl = len(f.layers)
-        X.add_norm(None, x, f.layers[0].norm1 if nl else f.final_norm, mult, f.eps, h)
+        row = X.RowParts(x, None, f.layers[0].norm1 if nl else f.final_norm, mult, f.eps, None)
         for i, (ly, b, c) in enumerate(zip(f.layers, self.bufs, cache)):
             after = f.layers[i + 1].norm1 if i + 1 < nl else f.final_norm
-            self._mix(ly, b, h[0], c, pos_dev)
-            X.add_norm(y, x, after if ly.w_up is None else ly.norm2, mult, f.eps, h)
+            self._mix(ly, b, row, c, pos_dev)
+            row, x, spare = X.RowParts(x, y, after if ly.w_up is None else ly.norm2, mult, f.eps, spare), spare, x
             if ly.w_up is not None:
-                ly.feed_forward_vec(h[0], b["u"], y.view(-1))
-                X.add_norm(y, x, after, mult, f.eps, h)
-        return h
+                ly.feed_forward_vec(row, b["u"], y.view(-1))
+                row, x, spare = X.RowParts(x, y, after, mult, f.eps, spare), spare, x
+        return row
 
     def _postnorm(self, tok, cache, pos_dev):
-        f, y = self.f, self.y
+        f, y, nl = self.f, self.y, len(self.f.layers)
         f.embed(tok, cache, self.xs[0])
-        x = self.xs[0]
+        x, row, turn = self.xs[0], self.xs[0].view(-1), 0
+        if nl == 0:
+            return X.norm_rows(x, f.final_norm, f.eps, torch.float32).view(-1)
         for i, (ly, b, c) in enumerate(zip(f.layers, self.bufs, cache)):
-            self._mix(ly, b, x[0], c, pos_dev)
+            self._mix(ly, b, row, c, pos_dev)
+            last = i + 1 == nl
+            norm = ly.norm1
             if ly.w_up is not None:
-                X.res_norm(y, x, ly.norm1, f.eps, self.x)
-                x = self.x
-                ly.feed_forward_vec(x[0], b["u"], y.view(-1))
-            X.res_norm(y, x, ly.norm2 if ly.w_up is not None else ly.norm1, f.eps, self.x,
-                       average=(self.xs, ly.dwa, i + 1 < len(f.layers)))
-            x = self.x
-        return X.norm_rows(x, f.final_norm, f.eps, torch.float32)
+                row, x, turn = X.RowParts(x, y, norm, 1.0, f.eps, self.x[turn], ()), self.x[turn], 1 - turn
+                ly.feed_forward_vec(row, b["u"], y.view(-1))
+                norm = ly.norm2
+            row = X.RowParts(x, y, norm, 1.0, f.eps, self.x[turn], (self.xs, ly.dwa, not last), f.final_norm if last else None)
+            x, turn = self.x[turn], 1 - turn
+        return row

@@ -166,15 +166,50 @@ class Linear:
     def vec(self, x, act=None, conv=None, out=None):
         """One float32 row [K] -> float32 [N] (N / 2 with a gated activation); conv = (weights [C, taps], bias [C] or None, tail) for
         the convolution epilogue."""
-        assert x.dtype == torch.float32 and x.numel() == self.K and x.is_contiguous()
+        row = x if isinstance(x, RowParts) else None
+        if row is not None and not row.fits(self.K):
+            x, row = row.joined(), None
+        assert row is not None or (x.dtype == torch.float32 and x.numel() == self.K and x.is_contiguous())
         epi = 2 if conv is not None else 0 if act is None else (0, 1, 3)[act.code]
         if out is None:
-            out = torch.empty(self.N // 2 if epi == 3 else self.N, dtype=torch.float32, device=x.device)
+            out = torch.empty(self.N // 2 if epi == 3 else self.N, dtype=torch.float32, device=self.w.device)
         cw, cb, tail = conv if conv is not None else (None, None, None)
-        _lib.mcall("scmx_gemv_x", _lib.ptr(self.w), self.w.shape[1], self.dt, _lib.ptr(x), self.N, self.K, epi, act.a_pos if act else 0.0,
-                   act.a_neg if act else 0.0, _lib.ptr(cw), _lib.ptr(cb), _lib.ptr(tail), 0 if cw is None else cw.shape[0],
-                   0 if cw is None else cw.shape[1], _lib.ptr(out), _lib.stream())
+        rest = (self.N, self.K, epi, act.a_pos if act else 0.0, act.a_neg if act else 0.0, _lib.ptr(cw), _lib.ptr(cb), _lib.ptr(tail),
+                0 if cw is None else cw.shape[0], 0 if cw is None else cw.shape[1], _lib.ptr(out), _lib.stream())
+        if row is not None:
+            _lib.mcall("scmx_gemv_x_row", _lib.ptr(self.w), self.w.shape[1], self.dt, *row.args(), *rest)
+        else:
+            _lib.mcall("scmx_gemv_x", _lib.ptr(self.w), self.w.shape[1], self.dt, _lib.ptr(x), *rest)
         return out
+
+
+class RowParts:
+    """One row as the sublayers before leave it, to be joined by the product that reads it (Linear.vec): x + mult y, normalized with w
+    (average None), or x + w y / rms(y) (average = () or as in res_norm), normalized with `final` if given.  The joined row without its last norm
+    goes to x_out, another buffer than x and y.  Consumed by one product."""
+    __slots__ = ("x", "y", "w", "mult", "eps", "x_out", "average", "final")
+
+    def __init__(self, x, y, w, mult, eps, x_out, average=None, final=None):
+        self.x, self.y, self.w, self.mult, self.eps, self.x_out, self.average, self.final = x, y, w, mult, eps, x_out, average, final
+
+    def fits(self, K):
+        rows = (self.x, self.y, self.w, self.x_out, self.final, self.average[0] if self.average else None)
+        return K <= 2048 and K % 4 == 0 and all(t is None or t.data_ptr() % 16 == 0 for t in rows)
+
+    def args(self):
+        xs, dwa, keep = self.average if self.average else (None, None, False)
+        return (_lib.ptr(self.x), _lib.ptr(self.y), _lib.ptr(self.w), 1 if self.average is None else 2, self.mult, self.eps, _lib.ptr(xs),
+                0 if xs is None else xs.stride(0), _lib.ptr(dwa), 0 if dwa is None else dwa.numel(), int(keep), _lib.ptr(self.final), _lib.ptr(self.x_out))
+
+    def joined(self):
+        """The row itself, by the row kernels."""
+        h = torch.empty_like(self.x)
+        if self.average is None:
+            _lib.mcall("scmx_add_norm", _lib.ptr(self.y), 0 if self.y is None else _ld(self.y), _lib.ptr(self.x), _lib.ptr(self.w), self.mult, self.eps, 1,
+                       self.x.shape[1], _lib.ptr(self.x_out), _lib.ptr(h), _dt(h), _lib.stream())
+            return h.view(-1)
+        res_norm(self.y, self.x, self.w, self.eps, self.x_out, average=self.average or None)
+        return (self.x_out if self.final is None else norm_rows(self.x_out, self.final, self.eps, torch.float32)).view(-1)
 
 
 class _full_float32:
