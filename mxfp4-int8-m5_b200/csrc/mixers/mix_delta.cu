@@ -11,102 +11,151 @@ namespace cg = cooperative_groups;
 
 namespace scmx {
 
-constexpr int DS_T = 8;       // tokens staged together
+constexpr int DS_T = 16;      // tokens staged together
+constexpr int DS_COLS = 8;    // columns of the state per CTA
+template <int NR, bool CH> constexpr size_t ds_smem() { return (size_t)2 * DS_T * (64 * NR * (CH ? 3 : 2) + DS_COLS + 3) * 4; }
 
-// Grid (heads, column slices of 32), 128 threads: four lanes share a column of the state, each holds a quarter of its rows (float4
-// groups 4 r + sub).  With o = (g S)^T q + (q . k) u both sums over the old state are taken in one pass.
-template <typename T, int R4, bool CH>
-__global__ void __launch_bounds__(128) delta_scan_kernel(const DeltaArgs a) {
-    constexpr int D = 16 * R4;
-    __shared__ __align__(16) float sq[DS_T][D], sk[DS_T][D], sg[CH ? DS_T : 1][D];
-    __shared__ float sv[DS_T][32], sb[DS_T], sqk[DS_T], sgs[DS_T];
+// Grid (heads, column slices of 8).  Threads 0 .. 127 run the recurrence: 16 lanes share a column of the state, lane l holds rows 4 l + 64 r ..
+// 4 l + 64 r + 3 in registers.  With o = (g S)^T q + (q . k) u both sums over the old state are taken in one pass.  Threads 128 .. 255 stage the
+// next 16 tokens (unit vectors, decays) while the present ones run, their loads one tile ahead.
+// A chain per token (two sums over the column, one correction) bounds it, so the chain is cut short: 300 float32 tokens of 8 heads of 128 took
+// 320 us with a column on four lanes, 8 tokens staged in the open and 32 CTAs of 128 threads.
+template <typename T, int NR, bool CH>
+__global__ void __launch_bounds__(256) delta_scan_kernel(const DeltaArgs a) {
+    constexpr int D = 64 * NR, E = D / 32, TW = DS_T / 4;      // elements per staging lane, tokens per staging warp
+    extern __shared__ __align__(16) float sm[];
+    float* sq = sm;                              // [2][DS_T][D], zero above d
+    float* sk = sq + 2 * DS_T * D;
+    float* sg = sk + 2 * DS_T * D;               // CH: decays per channel
+    float* sv = sg + (CH ? 2 * DS_T * D : 0);    // [2][DS_T][DS_COLS]
+    float* sb = sv + 2 * DS_T * DS_COLS;         // [2][DS_T]: beta, q . k, decay of the head
+    float *sqk = sb + 2 * DS_T, *sgs = sqk + 2 * DS_T;
     pdl_launch_dependents();
     pdl_wait();
-    const int h = blockIdx.x, e0 = blockIdx.y * 32, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int kh = h / (a.H / a.G), sub = lane & 3, col = 8 * warp + (lane >> 2);
-    const bool ok = e0 + col < a.dv;
-    const T *q = static_cast<const T*>(a.q) + (int64_t)kh * a.d, *k = static_cast<const T*>(a.k) + (int64_t)kh * a.d;
-    const T *v = static_cast<const T*>(a.v) + (int64_t)h * a.dv + e0, *b = static_cast<const T*>(a.b) + h;
-    const float nA = a.nA[h], qs = rsqrtf((float)a.d);
-    float* gS = a.state + (int64_t)h * a.d * a.dv + e0 + col;
-    float4 S[R4];
+    const int h = blockIdx.x, e0 = blockIdx.y * DS_COLS, tid = threadIdx.x;
+    const int n = (int)a.n, tiles = (n + DS_T - 1) / DS_T;
+    if (tid >= 128) {
+        const int lane = tid & 31, w = (tid - 128) >> 5, kh = h / (a.H / a.G), col = tid & (DS_COLS - 1), row = (tid - 128) / DS_COLS;
+        const T *q = static_cast<const T*>(a.q) + (int64_t)kh * a.d, *k = static_cast<const T*>(a.k) + (int64_t)kh * a.d;
+        const T *v = static_cast<const T*>(a.v) + (int64_t)h * a.dv + e0 + col, *b = static_cast<const T*>(a.b) + h;
+        const float nA = a.nA[h], qs = rsqrtf((float)a.d);
+        float dtb[CH ? E : 1];
+        if (CH) {
 #pragma unroll
-    for (int r = 0; r < R4; ++r) {
-        const int i = 16 * r + 4 * sub;
+            for (int j = 0; j < E; ++j) dtb[CH ? j : 0] = lane + 32 * j < a.d ? a.dtb[(int64_t)h * a.d + lane + 32 * j] : 0.0f;
+        } else {
+            dtb[0] = a.dtb[h];
+        }
+        float x[TW][E], y[TW][E], g[TW][CH ? E : 1], bt[TW], vv;
+        auto fetch = [&](int t0) {
+#pragma unroll
+            for (int i = 0; i < TW; ++i) {
+                const int t = t0 + w + 4 * i;
+                const bool ok = t < n;
+#pragma unroll
+                for (int j = 0; j < E; ++j) {
+                    const int e = lane + 32 * j;
+                    const bool in = ok && e < a.d;
+                    x[i][j] = in ? ldf(q + (int64_t)t * a.ldq + e) : 0.0f;
+                    y[i][j] = in ? ldf(k + (int64_t)t * a.ldk + e) : 0.0f;
+                    if (CH) g[i][CH ? j : 0] = in ? static_cast<const float*>(a.a)[(int64_t)t * a.lda + (int64_t)h * a.d + e] : 0.0f;
+                }
+                if (!CH) g[i][0] = ok ? ldf(static_cast<const T*>(a.a) + (int64_t)t * a.lda + h) : 0.0f;
+                bt[i] = ok ? ldf(b + (int64_t)t * a.ldb) : 0.0f;
+            }
+            vv = t0 + row < n && e0 + col < a.dv ? ldf(v + (int64_t)(t0 + row) * a.ldv) : 0.0f;
+        };
+        auto put = [&](int buf) {
+#pragma unroll
+            for (int i = 0; i < TW; ++i) {
+                const int r = buf * DS_T + w + 4 * i;
+                float qq = 0.0f, kk = 0.0f, qk = 0.0f;
+#pragma unroll
+                for (int j = 0; j < E; ++j) {
+                    qq += x[i][j] * x[i][j];
+                    kk += y[i][j] * y[i][j];
+                    qk += x[i][j] * y[i][j];
+                }
+                const float iq = qs / sqrtf(warp_sumf(qq) + 1e-6f), ik = 1.0f / sqrtf(warp_sumf(kk) + 1e-6f);
+                qk = warp_sumf(qk);
+#pragma unroll
+                for (int j = 0; j < E; ++j) {
+                    const int e = lane + 32 * j;
+                    sq[r * D + e] = x[i][j] * iq;
+                    sk[r * D + e] = y[i][j] * ik;
+                    if (CH) sg[r * D + e] = e < a.d ? expf(nA * softplus_f32(g[i][CH ? j : 0] + dtb[CH ? j : 0])) : 0.0f;
+                }
+                if (lane == 0) {
+                    sqk[r] = qk * iq * ik;
+                    sb[r] = 1.0f / (1.0f + expf(-bt[i]));
+                    if (!CH) sgs[r] = expf(nA * softplus_f32(g[i][0] + dtb[0]));
+                }
+            }
+            sv[buf * DS_T * DS_COLS + tid - 128] = vv;
+        };
+        fetch(0);
+        put(0);
+        if (tiles > 1) fetch(DS_T);
+        __syncthreads();
+        for (int t = 0; t < tiles; ++t) {
+            if (t + 1 < tiles) put((t + 1) & 1);
+            if (t + 2 < tiles) fetch((t + 2) * DS_T);
+            __syncthreads();
+        }
+        return;
+    }
+    const int l = tid & 15, col = tid >> 4;
+    const bool ok = e0 + col < a.dv;
+    float* gS = a.state + (int64_t)h * a.d * a.dv + e0 + col;
+    float4 S[NR];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+        const int i = 64 * r + 4 * l;
         S[r].x = ok && i < a.d ? gS[(int64_t)i * a.dv] : 0.0f;
         S[r].y = ok && i + 1 < a.d ? gS[(int64_t)(i + 1) * a.dv] : 0.0f;
         S[r].z = ok && i + 2 < a.d ? gS[(int64_t)(i + 2) * a.dv] : 0.0f;
         S[r].w = ok && i + 3 < a.d ? gS[(int64_t)(i + 3) * a.dv] : 0.0f;
     }
-    for (int64_t t0 = 0; t0 < a.n; t0 += DS_T) {
-        const int nt = (int)min((int64_t)DS_T, a.n - t0);
-        __syncthreads();                       // the previous tokens are consumed
-        for (int t = warp; t < nt; t += 4) {
-            const T *qr = q + (t0 + t) * a.ldq, *kr = k + (t0 + t) * a.ldk;
-            constexpr int E = (D + 31) / 32;
-            float x[E], y[E], qq = 0.0f, kk = 0.0f, qk = 0.0f;
+    __syncthreads();
+    for (int tile = 0; tile < tiles; ++tile) {
+        const int r0 = (tile & 1) * DS_T, nt = min(DS_T, n - tile * DS_T);
+#pragma unroll 2
+        for (int t = 0; t < nt; ++t) {
+            const float4 *k4 = reinterpret_cast<const float4*>(sk + (r0 + t) * D), *q4 = reinterpret_cast<const float4*>(sq + (r0 + t) * D);
+            const float4* g4 = reinterpret_cast<const float4*>(sg + (CH ? (r0 + t) * D : 0));
+            const float gs = CH ? 0.0f : sgs[r0 + t];
+            float4 kk[NR];
+            float pk[NR], pq[NR];
 #pragma unroll
-            for (int j = 0; j < E; ++j) {
-                const int e = lane + 32 * j;
-                x[j] = e < a.d ? ldf(qr + e) : 0.0f;
-                y[j] = e < a.d ? ldf(kr + e) : 0.0f;
-                qq += x[j] * x[j];
-                kk += y[j] * y[j];
-                qk += x[j] * y[j];
+            for (int r = 0; r < NR; ++r) {
+                kk[r] = k4[16 * r + l];
+                const float4 qq = q4[16 * r + l], gg = CH ? g4[16 * r + l] : make_float4(gs, gs, gs, gs);
+                S[r].x *= gg.x; S[r].y *= gg.y; S[r].z *= gg.z; S[r].w *= gg.w;
+                pk[r] = S[r].x * kk[r].x; pk[r] = fmaf(S[r].y, kk[r].y, pk[r]); pk[r] = fmaf(S[r].z, kk[r].z, pk[r]); pk[r] = fmaf(S[r].w, kk[r].w, pk[r]);
+                pq[r] = S[r].x * qq.x; pq[r] = fmaf(S[r].y, qq.y, pq[r]); pq[r] = fmaf(S[r].z, qq.z, pq[r]); pq[r] = fmaf(S[r].w, qq.w, pq[r]);
             }
-            const float iq = qs / sqrtf(warp_sumf(qq) + 1e-6f), ik = 1.0f / sqrtf(warp_sumf(kk) + 1e-6f);
-            qk = warp_sumf(qk);
+            float sumk = pk[0], sumq = pq[0];
 #pragma unroll
-            for (int j = 0; j < E; ++j) {
-                const int e = lane + 32 * j;
-                if (e < D) {
-                    sq[t][e] = x[j] * iq;
-                    sk[t][e] = y[j] * ik;
-                    if (CH)
-                        sg[CH ? t : 0][e] = e < a.d ? expf(nA * softplus_f32(static_cast<const float*>(a.a)[(t0 + t) * a.lda + (int64_t)h * a.d + e] +
-                                                                             a.dtb[(int64_t)h * a.d + e])) : 0.0f;
-                }
+            for (int r = 1; r < NR; ++r) {
+                sumk += pk[r];
+                sumq += pq[r];
             }
-            if (lane == 0) {
-                sqk[t] = qk * iq * ik;
-                sb[t] = 1.0f / (1.0f + expf(-ldf(b + (t0 + t) * a.ldb)));
-                if (!CH) sgs[t] = expf(nA * softplus_f32(ldf(static_cast<const T*>(a.a) + (t0 + t) * a.lda + h) + a.dtb[h]));
+#pragma unroll
+            for (int o = 1; o < 16; o *= 2) sumk += __shfl_xor_sync(0xffffffffu, sumk, o);
+            const float u = sb[r0 + t] * (sv[(r0 + t) * DS_COLS + col] - sumk);
+#pragma unroll
+            for (int r = 0; r < NR; ++r) {
+                S[r].x = fmaf(kk[r].x, u, S[r].x); S[r].y = fmaf(kk[r].y, u, S[r].y); S[r].z = fmaf(kk[r].z, u, S[r].z); S[r].w = fmaf(kk[r].w, u, S[r].w);
             }
-        }
-        for (int i = tid; i < nt * 32; i += 128) {
-            const int t = i >> 5, e = i & 31;
-            sv[t][e] = e0 + e < a.dv ? ldf(v + (t0 + t) * a.ldv + e) : 0.0f;
+#pragma unroll
+            for (int o = 1; o < 16; o *= 2) sumq += __shfl_xor_sync(0xffffffffu, sumq, o);
+            if (l == 0 && ok) a.o[((int64_t)(tile * DS_T + t) * a.H + h) * a.dv + e0 + col] = fmaf(sqk[r0 + t], u, sumq);
         }
         __syncthreads();
-        for (int t = 0; t < nt; ++t) {
-            const float4 *k4 = reinterpret_cast<const float4*>(sk[t]), *q4 = reinterpret_cast<const float4*>(sq[t]);
-            const float4* g4 = reinterpret_cast<const float4*>(sg[CH ? t : 0]);
-            const float g = CH ? 0.0f : sgs[t];
-            float pk = 0.0f, pq = 0.0f;
-#pragma unroll
-            for (int r = 0; r < R4; ++r) {
-                const float4 kk = k4[4 * r + sub], qq = q4[4 * r + sub];
-                const float4 gg = CH ? g4[4 * r + sub] : make_float4(g, g, g, g);
-                S[r].x *= gg.x; S[r].y *= gg.y; S[r].z *= gg.z; S[r].w *= gg.w;
-                pk = fmaf(S[r].x, kk.x, pk); pk = fmaf(S[r].y, kk.y, pk); pk = fmaf(S[r].z, kk.z, pk); pk = fmaf(S[r].w, kk.w, pk);
-                pq = fmaf(S[r].x, qq.x, pq); pq = fmaf(S[r].y, qq.y, pq); pq = fmaf(S[r].z, qq.z, pq); pq = fmaf(S[r].w, qq.w, pq);
-            }
-            pk += __shfl_xor_sync(0xffffffffu, pk, 1);
-            pq += __shfl_xor_sync(0xffffffffu, pq, 1);
-            pk += __shfl_xor_sync(0xffffffffu, pk, 2);
-            pq += __shfl_xor_sync(0xffffffffu, pq, 2);
-            const float u = sb[t] * (sv[t][col] - pk);
-#pragma unroll
-            for (int r = 0; r < R4; ++r) {
-                const float4 kk = k4[4 * r + sub];
-                S[r].x = fmaf(kk.x, u, S[r].x); S[r].y = fmaf(kk.y, u, S[r].y); S[r].z = fmaf(kk.z, u, S[r].z); S[r].w = fmaf(kk.w, u, S[r].w);
-            }
-            if (sub == 0 && ok) a.o[((t0 + t) * a.H + h) * a.dv + e0 + col] = fmaf(sqk[t], u, pq);
-        }
     }
 #pragma unroll
-    for (int r = 0; r < R4; ++r) {
-        const int i = 16 * r + 4 * sub;
+    for (int r = 0; r < NR; ++r) {
+        const int i = 64 * r + 4 * l;
         if (ok && i < a.d) gS[(int64_t)i * a.dv] = S[r].x;
         if (ok && i + 1 < a.d) gS[(int64_t)(i + 1) * a.dv] = S[r].y;
         if (ok && i + 2 < a.d) gS[(int64_t)(i + 2) * a.dv] = S[r].z;
@@ -114,17 +163,21 @@ __global__ void __launch_bounds__(128) delta_scan_kernel(const DeltaArgs a) {
     }
 }
 
+template <typename T, int NR, bool CH>
+static int run_delta_rows(const DeltaArgs& a, cudaStream_t st) {
+    constexpr size_t smem = ds_smem<NR, CH>();
+    if (smem > 48 * 1024) SCMX_CUDA_OK(cudaFuncSetAttribute(delta_scan_kernel<T, NR, CH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    SCMX_PDL_OK("delta_scan_kernel",
+                launch_pdl(delta_scan_kernel<T, NR, CH>, dim3(a.H, (a.dv + DS_COLS - 1) / DS_COLS), dim3(256), smem, st, a));
+    return SCMX_OK;
+}
+
 template <typename T, bool CH>
 static int run_delta_scan(const DeltaArgs& a, cudaStream_t st) {
-    const dim3 grid(a.H, (a.dv + 31) / 32), block(128);
-    cudaError_t e;
-    if (a.d <= 16) e = launch_pdl(delta_scan_kernel<T, 1, CH>, grid, block, 0, st, a);
-    else if (a.d <= 32) e = launch_pdl(delta_scan_kernel<T, 2, CH>, grid, block, 0, st, a);
-    else if (a.d <= 64) e = launch_pdl(delta_scan_kernel<T, 4, CH>, grid, block, 0, st, a);
-    else if (a.d <= 128) e = launch_pdl(delta_scan_kernel<T, 8, CH>, grid, block, 0, st, a);
-    else e = launch_pdl(delta_scan_kernel<T, 16, CH>, grid, block, 0, st, a);
-    SCMX_PDL_OK("delta_scan_kernel", e);
-    return SCMX_OK;
+    SCMX_REQUIRE(a.n < (1ll << 30), SCMX_ELIMIT, "delta: %lld tokens", (long long)a.n);
+    if (a.d <= 64) return run_delta_rows<T, 1, CH>(a, st);
+    if (a.d <= 128) return run_delta_rows<T, 2, CH>(a, st);
+    return run_delta_rows<T, 4, CH>(a, st);
 }
 
 // ---- one token ------------------------------------------------------------------------------------------------------------

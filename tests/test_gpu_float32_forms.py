@@ -3,6 +3,7 @@ register limits and one above, portions around 16 tokens, 16 queries and 32 keys
 import pytest
 import torch
 
+from test_gpu_fabezen_kernels import DeltaCase
 from test_gpu_hybrid_kernels import BF, F32, Case, X, err, ret_case, run_ret  # noqa: F401
 
 pytestmark = pytest.mark.gpu
@@ -78,3 +79,13 @@ def test_float32_product_extreme_values(X):      # noqa: F811
         for r in (9, 20, 21, 30):
             ok = want[r].isfinite()
             assert rel(y[r][ok] / y[r][ok].abs().max(), want[r][ok] / y[r][ok].abs().max().double()) < 1e-6
+
+
+@pytest.mark.parametrize("H,G,d,dv", [(2, 1, 64, 8), (1, 1, 65, 9), (2, 2, 128, 128), (1, 1, 129, 7), (2, 1, 256, 24), (1, 1, 1, 1)])
+@pytest.mark.parametrize("channel", [False, True])
+@pytest.mark.parametrize("dt", [BF, F32])
+def test_delta_row_groups(X, H, G, d, dv, channel, dt):      # noqa: F811
+    for cuts in ([50], [16, 17, 1, 15, 1], [33, 17]):
+        c = DeltaCase(X, 50, H, G, d, dv, channel, dt)
+        o, S = c.oracle()
+        assert err(c.run(cuts, 1), o) < 2e-5 and err(c.state, S) < 2e-5, cuts
