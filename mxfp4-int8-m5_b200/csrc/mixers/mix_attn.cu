@@ -363,7 +363,13 @@ constexpr int DD_MIN_CHUNK = 64;  // positions per split at least
 // Query vectors of a key/value head: 2 r + m for head r of the group, map m; QP = their number padded to 4, 8, 16 or 32.  For the
 // weighted values a thread owns columns c and c + CT (CT a power of two, dv <= 2 CT) of every query vector over every
 // (256 / CT)-th position of a tile, so that a value read from shared memory serves all query vectors.
-template <typename T, int QP>
+//
+// FAST (few query vectors, keys and values in whole 16-byte pieces that fit a thread's registers): a tile's keys of both maps and its values are
+// requested together, the next tile's while the present one is weighted.  A chain of memory round trips bounds the kernel: 3000
+// positions of 8 key / value heads took 18 us with the keys of the two maps and the tiles one after the other.
+template <typename T> __host__ __device__ constexpr int dd_key_pieces() { return sizeof(T) == 2 ? 4 : 2; }      // of 32 elements over four lanes: d <= 32 of them
+
+template <typename T, int QP, bool FAST>
 __global__ void __launch_bounds__(256) diff_decode_kernel(const DiffDecodeArgs<T> a) {
     extern __shared__ __align__(16) float sm[];
     const int d = a.d, dv = a.dv, R = a.H / a.G, Q = 2 * R;
@@ -398,20 +404,56 @@ __global__ void __launch_bounds__(256) diff_decode_kernel(const DiffDecodeArgs<T
     for (int r = 0; r < QP; ++r) acc[r][0] = acc[r][1] = 0.0f;
     const bool vec = (d & 7) == 0, vecv = (dv & 7) == 0 && dv <= 256;
     const int p = tid >> 2, j4 = tid & 3;    // scores: four lanes per position
-    for (int64_t tb = t0; tb < t1; tb += DD_P) {
+    constexpr int VL = sizeof(T) == 2 ? 8 : 4, KC = FAST ? dd_key_pieces<T>() : 1;
+    Raw8<T> vreg[VL], kreg[2][KC];
+    const int nvec = DD_P * dv / 8;
+    // a tile's values: up to VL loads of 8 elements per thread, in flight while the scores are computed; FAST: its keys too
+    auto fetch = [&](int64_t tb) {
         const int np = (int)min((int64_t)DD_P, t1 - tb);
         const T* vr = a.v + ((int64_t)kvh * a.cap + tb) * dv;
-        // the tile's values: up to 8 loads of 8 elements per thread, in flight while the scores are computed
-        constexpr int VL = sizeof(T) == 2 ? 8 : 4;
-        Raw8<T> vreg[VL];
-        const int nvec = DD_P * dv / 8;
-        if (vecv) {
+        if (FAST) {
+            const T* kr = a.k + ((int64_t)(2 * kvh) * a.cap + (tb + p < t1 ? tb + p : t0)) * d + 8 * j4;
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int c = 0; c < KC; ++c)
+                    if (8 * j4 + 32 * c < d) kreg[m][c].load(kr + (int64_t)m * a.cap * d + 32 * c);
+        }
+        if (FAST || vecv) {
 #pragma unroll
             for (int i = 0; i < VL; ++i)
                 if (tid + 256 * i < nvec && 8 * (tid + 256 * i) < np * dv) vreg[i].load(vr + 8 * (tid + 256 * i));
         }
+    };
+    if (FAST) fetch(t0);
+    for (int64_t tb = t0; tb < t1; tb += DD_P) {
+        const int np = (int)min((int64_t)DD_P, t1 - tb);
+        const T* vr = a.v + ((int64_t)kvh * a.cap + tb) * dv;
+        if (!FAST) fetch(tb);
         __syncthreads();                     // queries staged; the previous tile's weights and values are consumed
         const int64_t t = tb + p;
+        if (FAST) {
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int r = 0; r < QP / 2; ++r)
+                    if (r < R) {
+                        float s = 0.0f;
+#pragma unroll
+                        for (int c = 0; c < KC; ++c)
+                            if (8 * j4 + 32 * c < d) {
+                                float kv[8];
+                                kreg[m][c].get(kv);
+                                const float4* qq = reinterpret_cast<const float4*>(sq + (2 * r + m) * dq + 8 * j4 + 32 * c);
+                                const float4 x = qq[0], y = qq[1];
+                                s = fmaf(x.x, kv[0], s); s = fmaf(x.y, kv[1], s); s = fmaf(x.z, kv[2], s); s = fmaf(x.w, kv[3], s);
+                                s = fmaf(y.x, kv[4], s); s = fmaf(y.y, kv[5], s); s = fmaf(y.z, kv[6], s); s = fmaf(y.w, kv[7], s);
+                            }
+                        s += __shfl_xor_sync(0xffffffffu, s, 1);
+                        s += __shfl_xor_sync(0xffffffffu, s, 2);
+                        if (j4 == 0) sp[p * QP + 2 * r + m] = t < t1 ? s : -INFINITY;
+                    }
+        } else
         for (int m = 0; m < 2; ++m) {
             const T* kr = a.k + ((int64_t)(2 * kvh + m) * a.cap + (t < t1 ? t : t0)) * d;
             for (int r0 = 0; r0 < R; r0 += 4) {
@@ -440,7 +482,7 @@ __global__ void __launch_bounds__(256) diff_decode_kernel(const DiffDecodeArgs<T
                 }
             }
         }
-        if (vecv) {
+        if (FAST || vecv) {
 #pragma unroll
             for (int i = 0; i < VL; ++i) {
                 const int o = 8 * (tid + 256 * i);
@@ -460,6 +502,7 @@ __global__ void __launch_bounds__(256) diff_decode_kernel(const DiffDecodeArgs<T
         } else {
             for (int i = tid; i < DD_P * dv; i += 256) sv[i] = i < np * dv ? ldf(vr + i) : 0.0f;
         }
+        if (FAST && tb + DD_P < t1) fetch(tb + DD_P);
         __syncthreads();
         for (int r = warp; r < Q; r += 8) {
             const float s0 = sp[lane * QP + r], s1 = sp[(32 + lane) * QP + r], m0 = ml[r][0];
@@ -523,10 +566,24 @@ __global__ void __launch_bounds__(256) diff_decode_kernel(const DiffDecodeArgs<T
     __syncthreads();
     if (ticket != active - 1) return;
     __threadfence();
-    // the last CTA of this key/value head: weights of the splits, then both maps, the difference, its norm
+    // the last CTA of this key/value head: weights of the splits, then both maps, the difference, its norm.  Partial outputs do not depend on
+    // the weights: those of the first splits are requested with the maxima and sums.
     const float* pg = a.part + (int64_t)g * a.nsplit * Q * ps;
     float* cf = sv;                          // [Q][32]: 2^(m_s - m) / sum
     float* sx = sv + Q * 32;                 // [R][dv]
+    constexpr int SB = 16;
+    float u[SB], v[SB];
+    auto load = [&](int i, int s0) {
+        const int r = i / dv, e = i - r * dv;
+        const float* pr = pg + 2 * r * ps + e;
+#pragma unroll
+        for (int s = 0; s < SB; ++s) {
+            const bool ok = s0 + s < active;
+            u[s] = ok ? __ldcg(pr + (int64_t)(s0 + s) * Q * ps) : 0.0f;
+            v[s] = ok ? __ldcg(pr + (int64_t)(s0 + s) * Q * ps + ps) : 0.0f;
+        }
+    };
+    if (tid < R * dv) load(tid, 0);
     for (int r = warp; r < Q; r += 8) {
         const float m = lane < active ? __ldcg(pg + ((int64_t)lane * Q + r) * ps + dv) : -INFINITY;
         const float l = lane < active ? __ldcg(pg + ((int64_t)lane * Q + r) * ps + dv + 1) : 0.0f;
@@ -536,19 +593,12 @@ __global__ void __launch_bounds__(256) diff_decode_kernel(const DiffDecodeArgs<T
     }
     __syncthreads();
     for (int i = tid; i < R * dv; i += 256) {
-        const int r = i / dv, e = i - r * dv;
-        const float* pr = pg + 2 * r * ps + e;
+        const int r = i / dv;
         float a1 = 0.0f, a2 = 0.0f;
-        for (int s0 = 0; s0 < active; s0 += 8) {
-            float u[8], v[8];
+        for (int s0 = 0; s0 < active; s0 += SB) {
+            if (i != tid || s0 != 0) load(i, s0);
 #pragma unroll
-            for (int s = 0; s < 8; ++s) {
-                const bool ok = s0 + s < active;
-                u[s] = ok ? __ldcg(pr + (int64_t)(s0 + s) * Q * ps) : 0.0f;
-                v[s] = ok ? __ldcg(pr + (int64_t)(s0 + s) * Q * ps + ps) : 0.0f;
-            }
-#pragma unroll
-            for (int s = 0; s < 8; ++s) {
+            for (int s = 0; s < SB; ++s) {      // weights of splits that do not exist are zero
                 a1 = fmaf(cf[(2 * r) * 32 + s0 + s], u[s], a1);
                 a2 = fmaf(cf[(2 * r + 1) * 32 + s0 + s], v[s], a2);
             }
@@ -588,7 +638,7 @@ static int run_diff_attn_f32(const DiffAttnArgs<float>& a, cudaStream_t st) {
     return a.dv <= 128 ? run_diff_tile<1>(a, smem, st) : run_diff_tile<2>(a, smem, st);
 }
 
-template <typename T, int QP>
+template <typename T, int QP, bool FAST>
 static int run_diff_decode_q(const DiffDecodeArgs<T>& a, cudaStream_t st) {
     const int Q = 2 * (a.H / a.G), groups = 256 / a.ct;
     size_t stage = (size_t)DD_P * a.dv;                                   // values, group sums, combination share this area
@@ -596,8 +646,8 @@ static int run_diff_decode_q(const DiffDecodeArgs<T>& a, cudaStream_t st) {
     stage = stage > (size_t)Q * 32 + (size_t)Q / 2 * a.dv ? stage : (size_t)Q * 32 + (size_t)Q / 2 * a.dv;
     const size_t smem = ((size_t)DD_P * QP + (size_t)Q * ((a.d + 7) & ~7) + stage) * 4;
     SCMX_REQUIRE(smem <= 220 * 1024, SCMX_ELIMIT, "diff_decode: %d query heads per key/value head of sizes %d / %d", Q / 2, a.d, a.dv);
-    SCMX_CUDA_OK(cudaFuncSetAttribute(diff_decode_kernel<T, QP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    SCMX_PDL_OK("diff_decode_kernel", launch_pdl(diff_decode_kernel<T, QP>, dim3(a.G, a.nsplit), dim3(256), smem, st, a));
+    SCMX_CUDA_OK(cudaFuncSetAttribute(diff_decode_kernel<T, QP, FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    SCMX_PDL_OK("diff_decode_kernel", launch_pdl(diff_decode_kernel<T, QP, FAST>, dim3(a.G, a.nsplit), dim3(256), smem, st, a));
     return SCMX_OK;
 }
 template <typename T>
@@ -612,10 +662,11 @@ static int run_diff_decode(DiffDecodeArgs<T> a, cudaStream_t st) {
     SCMX_REQUIRE(a.dv <= 512, SCMX_ELIMIT, "diff_decode: %d values per head (512 at most)", a.dv);
     a.ct = 1;
     while (2 * a.ct < a.dv) a.ct *= 2;
-    if (Q <= 4) return run_diff_decode_q<T, 4>(a, st);
-    if (Q <= 8) return run_diff_decode_q<T, 8>(a, st);
-    if (Q <= 16) return run_diff_decode_q<T, 16>(a, st);
-    return run_diff_decode_q<T, 32>(a, st);
+    const bool fast = a.d % 8 == 0 && a.d <= 32 * dd_key_pieces<T>() && a.dv % 8 == 0 && DD_P * a.dv / 8 <= 256 * (sizeof(T) == 2 ? 8 : 4);
+    if (Q <= 4) return fast ? run_diff_decode_q<T, 4, true>(a, st) : run_diff_decode_q<T, 4, false>(a, st);
+    if (Q <= 8) return fast ? run_diff_decode_q<T, 8, true>(a, st) : run_diff_decode_q<T, 8, false>(a, st);
+    if (Q <= 16) return run_diff_decode_q<T, 16, false>(a, st);
+    return run_diff_decode_q<T, 32, false>(a, st);
 }
 
 template <typename TI, typename TC, typename TQ>
