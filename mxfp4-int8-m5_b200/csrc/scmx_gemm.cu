@@ -421,7 +421,15 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const Gem
 }
 
 static int run_gemm(const int8_t* xq, int64_t a_rows, const int8_t* wq, int64_t b_rows, GemmArgs& a, cudaStream_t st) {
-    int bn = g_bn_override ? g_bn_override : (a.N >= 256 ? 256 : 128);
+    // Dense products whose 128 x 128 tiles fit one wave of single CTAs run as those: more SMs share the operand traffic and a CTA's
+    // K loop moves 32 KB per step instead of 48 (384 x 2048 x 2048: 9.2 us, CTA pairs 11.9 us, 128 x 256 tiles 12.3 us; 128 x 12288 x 2048 11.3
+    // and 14.3 us).  Above that pairs while their 256 x 256 tiles fit one wave (512 x 6144 x 2048: 12.3 us, 128 x 128 tiles 14.9 us), 128 x 256
+    // tiles where only these do (384 x 12288 x 2048: 15.0 us, pairs 18.2 us), pairs for the rest.
+    auto count = [&](int64_t tm, int64_t tn) { return (a.M + tm - 1) / tm * ((a.N + tn - 1) / tn); };
+    const bool dense = a.E == 0 && a.bcast == 0 && a.ret_rank == nullptr;
+    const bool small = dense && count(BM, 128) <= num_sms();
+    const bool wide = dense && !small && count(2 * BM, PAIR_BN) > num_sms() / 2 && count(BM, 256) <= num_sms();
+    int bn = g_bn_override ? g_bn_override : (a.N >= 256 && !(small && g_use_pair) ? 256 : 128);
     a.wait_ns = g_wait_limit_ns;
     if (a.epi == 3) {
         int rc3 = silu_lut_ptr(st, &a.silu_lut);
@@ -430,7 +438,7 @@ static int run_gemm(const int8_t* xq, int64_t a_rows, const int8_t* wq, int64_t 
     CUtensorMap tmA, tmB;
     int rc = make_map(&tmA, xq, a_rows, a.K, BM);
     if (rc) return rc;
-    if (a.E == 0 && g_use_pair && !g_bn_override && a.M > BM && a.N >= PAIR_BN && a.ret_rank == nullptr) {
+    if (a.E == 0 && g_use_pair && !g_bn_override && !small && !wide && a.M > BM && a.N >= PAIR_BN && a.ret_rank == nullptr) {
         rc = make_map(&tmB, wq, b_rows, a.K, PAIR_BN / 2);
         if (rc) return rc;
         const int64_t tiles = ((a.M + 2 * BM - 1) / (2 * BM)) * (int64_t)((a.N + PAIR_BN - 1) / PAIR_BN) * (a.splits > 1 ? a.splits : 1);

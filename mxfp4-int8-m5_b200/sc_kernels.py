@@ -106,14 +106,10 @@ def _rmsnorm_quant(x, w, eps, Mp, want_n):
 
 @functools.lru_cache(maxsize=4096)
 def _ranges(M, N, K, n_sm=148):
-    """Ranges of K for a dense product whose tiles leave most SMs idle (CTA pairs of 256 x 256 tiles, single CTAs up to 128 rows).  Summing the
-    ranges costs a launch of 3 us and their traffic, which only a long K repays: 384 x 2048 x 6144 takes 21.7 us in one piece and
-    15.4 us in four, 128 x 1024 x 3072 14.3 and 10.4 us in eight, but 384 x 2048 x 2048 11.7 and 12.1 us."""
-    if K < 3072:
-        return 1
-    if M > 128 and N >= 256:
-        return max(1, min(4, n_sm // 2 // (-(-M // 256) * -(-N // 256))))
-    return max(1, min(8, n_sm // (-(-M // 128) * -(-N // (256 if N >= 256 else 128)))))
+    """Ranges of K for a dense product whose 128 x 128 tiles leave most SMs idle.  Summing the ranges costs a launch of 3 us and their traffic,
+    which only a long K repays: 256 x 2048 x 6144 takes 18.2 us in one piece and 12.7 us in four, 128 x 1024 x 3072 10.9 and 8.6 us, but
+    256 x 2048 x 2048 9.0 and 9.4 us in two."""
+    return max(1, min(4, n_sm // (-(-M // 128) * -(-N // 128)))) if K >= 3072 else 1
 
 
 def _mm_i8(xq, wq, M, N, K, epi, xscale, wscale, res, out, splits=None):
