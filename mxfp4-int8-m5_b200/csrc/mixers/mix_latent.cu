@@ -8,6 +8,7 @@
 // latent_rows_*_kernel   attention of such queries over the cache, positions split over CTAs (decode, short portions, float32):
 //                        _mma for a bfloat16 cache, the plain one for float32
 // latent_value_kernel    combination of the splits and W_uv,h
+#include <cooperative_groups.h>
 #include "../scmx_ptx.cuh"
 #include "mix_common.cuh"
 
@@ -224,7 +225,7 @@ __global__ void __launch_bounds__(256) latent_absorb_kernel(const AbsorbArgs<TQ,
 
 // ---- attention of absorbed queries --------------------------------------------------------------------------------------
 constexpr int LR_P = 32;         // positions per tile
-constexpr int LR_SPLITS = 64;    // ranges of positions at most
+constexpr int LR_SPLITS = 128;   // ranges of positions at most
 
 // Pitch of a partial result: R values, maximum and sum, 16-byte aligned; maximum and sum start at column up4.
 __host__ __device__ __forceinline__ int up4(int n) { return (n + 3) & ~3; }
@@ -597,12 +598,21 @@ struct LatentValueArgs {
     int H, R, dv, nsplit;
 };
 constexpr int LV_ROWS = 32;      // values per CTA, four per warp
+constexpr int LV_BATCH = 8;      // ranges whose partial sums a thread requests together
+
+// Grid (heads, slices of 32 values, rows); the CTAs of a head form a cluster (up to 8).  Each combines its share of the latent's columns over the
+// ranges and hands it to the others through distributed shared memory: 8 heads, 64 ranges of 512 columns took 9.3 us in the chain of a decode
+// step when every CTA combined all of them, in two batches of reads that waited for the ranges' weights.  Partial sums do not depend on the
+// weights, so the first are requested with them.
 template <typename TW, typename TO>
 __global__ void __launch_bounds__(256) latent_value_kernel(const LatentValueArgs<TW, TO> a) {
-    extern __shared__ __align__(16) float ctx[];         // [2][ldw]: halves of the sum, then the latent in the first
+    extern __shared__ __align__(16) float ctx[];         // [ldw]
     __shared__ float cf[LR_SPLITS];
+    __shared__ __align__(16) float4 sums[256];
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
     pdl_launch_dependents();
     const int h = blockIdx.x, e0 = blockIdx.y * LV_ROWS, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nc = (int)cl.num_blocks(), rank = (int)cl.block_rank();
     // the first vectors of this warp's rows are requested before the previous kernel ends: weights never change
     constexpr int ROWS = LV_ROWS / 8, PRE = sizeof(TW) == 2 ? 2 : 1;
     const TW* w = a.wuv + ((int64_t)h * a.dv + e0 + warp) * a.ldw + 8 * lane;
@@ -612,46 +622,75 @@ __global__ void __launch_bounds__(256) latent_value_kernel(const LatentValueArgs
 #pragma unroll
         for (int k = 0; k < PRE; ++k)
             if (e0 + warp + 8 * j < a.dv && 8 * lane + 256 * k < a.ldw) pre[j][k].load(w + 8 * j * a.ldw + 256 * k);
+    if (nc > 1) cl.sync();               // every CTA of the cluster runs: its shared memory may be written
     pdl_wait();
     const int64_t row = blockIdx.z, pos = (a.pos_dev != nullptr ? (int64_t)a.pos_dev[0] : a.pos) + row;
     const int active = latent_span(pos, a.cap, a.window, a.nsplit).active;
     const int pp = part_pitch(a.R);
     const float* part = a.part + (row * a.H + h) * a.nsplit * pp;
-    if (warp == 0) {
-        float2 ml[2];
+    // this CTA's columns in groups of four: thread (col, grp) adds up every (256 / CT)-th range
+    const int quads = (int)(a.ldw / 4), per = (quads + nc - 1) / nc, q0 = rank * per, q1 = min(quads, q0 + per);
+    int CT = 1;
+    while (CT < 256 && CT < per) CT *= 2;
+    const int col = tid & (CT - 1), grp = tid / CT, groups = 256 / CT;
+    float4 v[LV_BATCH];
+    auto request = [&](int q, int i0) {
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int sp = lane + 32 * i;
-            ml[i] = sp < active ? *reinterpret_cast<const float2*>(part + sp * pp + up4(a.R)) : make_float2(-INFINITY, 0.0f);
+        for (int k = 0; k < LV_BATCH; ++k) {
+            const int i = i0 + k * groups;
+            v[k] = i < active && q < q1 && 4 * q < a.R ? *reinterpret_cast<const float4*>(part + (int64_t)i * pp + 4 * q) : make_float4(0, 0, 0, 0);
         }
-        const float mm = warp_max(fmaxf(ml[0].x, ml[1].x)), c0 = ex2_approx(ml[0].x - mm), c1 = ex2_approx(ml[1].x - mm);
-        const float inv = 1.0f / warp_sumf(c0 * ml[0].y + c1 * ml[1].y);
-        cf[lane] = c0 * inv;
-        cf[lane + 32] = c1 * inv;
+    };
+    request(q0 + col, grp);
+    if (warp == 0) {
+        float2 ml[LR_SPLITS / 32];
+        float mm = -INFINITY, sum = 0.0f;
+#pragma unroll
+        for (int i = 0; i < LR_SPLITS / 32; ++i) {
+            const int sp = lane + 32 * i;
+            ml[i] = sp < active ? *reinterpret_cast<const float2*>(part + (int64_t)sp * pp + up4(a.R)) : make_float2(-INFINITY, 0.0f);
+        }
+#pragma unroll
+        for (int i = 0; i < LR_SPLITS / 32; ++i) mm = fmaxf(mm, ml[i].x);
+        mm = warp_max(mm);
+#pragma unroll
+        for (int i = 0; i < LR_SPLITS / 32; ++i) {
+            ml[i].x = ex2_approx(ml[i].x - mm);
+            sum = fmaf(ml[i].x, ml[i].y, sum);
+        }
+        const float inv = 1.0f / warp_sumf(sum);
+#pragma unroll
+        for (int i = 0; i < LR_SPLITS / 32; ++i) cf[lane + 32 * i] = ml[i].x * inv;
     }
     __syncthreads();
-    // two halves of the CTA take every second range, four columns per thread; the halves meet in shared memory
-    {
-        const int half = tid >> 7;
-        for (int e0_ = 4 * (tid & 127); e0_ < a.ldw; e0_ += 512) {
-            float4 s = make_float4(0, 0, 0, 0);
-            if (e0_ < a.R)
-#pragma unroll 16
-                for (int i = half; i < active; i += 2) {
-                    const float c = cf[i];
-                    const float4 v = *reinterpret_cast<const float4*>(part + i * pp + e0_);
-                    s.x = fmaf(c, v.x, s.x); s.y = fmaf(c, v.y, s.y); s.z = fmaf(c, v.z, s.z); s.w = fmaf(c, v.w, s.w);
-                }
+    for (int q = q0 + col; q - col < q1; q += CT) {      // uniform over the CTA
+        float4 s = make_float4(0, 0, 0, 0);
+        for (int i0 = grp; i0 - grp < active; i0 += LV_BATCH * groups) {
+            if (i0 != grp || q != q0 + col) request(q, i0);
+#pragma unroll
+            for (int k = 0; k < LV_BATCH; ++k) {
+                const int i = i0 + k * groups;
+                const float c = i < active ? cf[i] : 0.0f;
+                s.x = fmaf(c, v[k].x, s.x); s.y = fmaf(c, v[k].y, s.y); s.z = fmaf(c, v[k].z, s.z); s.w = fmaf(c, v[k].w, s.w);
+            }
+        }
+        sums[tid] = s;
+        __syncthreads();
+        if (grp == 0 && q < q1) {
+            for (int k = 1; k < groups; ++k) {
+                const float4 u = sums[k * CT + col];
+                s.x += u.x; s.y += u.y; s.z += u.z; s.w += u.w;
+            }
             // columns from R on are not results
-            if (e0_ + 1 >= a.R) s.y = 0.0f;
-            if (e0_ + 2 >= a.R) s.z = 0.0f;
-            if (e0_ + 3 >= a.R) s.w = 0.0f;
-            *reinterpret_cast<float4*>(ctx + half * a.ldw + e0_) = s;
+            if (4 * q >= a.R) s.x = 0.0f;
+            if (4 * q + 1 >= a.R) s.y = 0.0f;
+            if (4 * q + 2 >= a.R) s.z = 0.0f;
+            if (4 * q + 3 >= a.R) s.w = 0.0f;
+            for (int k = 0; k < nc; ++k) *reinterpret_cast<float4*>(nc > 1 ? cl.map_shared_rank(ctx, k) + 4 * q : ctx + 4 * q) = s;
         }
         __syncthreads();
-        for (int e = tid; e < a.ldw; e += 256) ctx[e] += ctx[a.ldw + e];
     }
-    __syncthreads();
+    if (nc > 1) cl.sync();
 #pragma unroll
     for (int j = 0; j < ROWS; ++j) {
         const int e = e0 + warp + 8 * j;
@@ -827,7 +866,20 @@ extern "C" int scmx_latent_value(const float* part, const void* wuv, int64_t ldw
         LatentValueArgs<TW, TO> a;                                                                                         \
         a.part = part; a.wuv = (const TW*)wuv; a.out = (TO*)out; a.pos_dev = pos_dev; a.ldw = ldw; a.ldo = ldo; a.pos = pos; \
         a.cap = cap; a.window = window; a.H = H; a.R = R; a.dv = dv; a.nsplit = nsplit;                                    \
-        SCMX_PDL_OK("latent_value_kernel", launch_pdl(latent_value_kernel<TW, TO>, grid, block, (size_t)ldw * 8, (cudaStream_t)stream, a)); \
+        cudaLaunchConfig_t cfg = {};                                                                                       \
+        cfg.gridDim = grid;                                                                                                \
+        cfg.blockDim = block;                                                                                              \
+        cfg.dynamicSmemBytes = (size_t)ldw * 4;                                                                            \
+        cfg.stream = (cudaStream_t)stream;                                                                                 \
+        cudaLaunchAttribute at[2];                                                                                         \
+        at[0].id = cudaLaunchAttributeClusterDimension;                                                                    \
+        at[0].val.clusterDim.x = at[0].val.clusterDim.z = 1;                                                               \
+        at[0].val.clusterDim.y = grid.y <= 8 ? grid.y : 1;                                                                 \
+        at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;                                                     \
+        at[1].val.programmaticStreamSerializationAllowed = 1;                                                              \
+        cfg.attrs = at;                                                                                                    \
+        cfg.numAttrs = g_use_pdl ? 2 : 1;                                                                                  \
+        SCMX_PDL_OK("latent_value_kernel", cudaLaunchKernelEx(&cfg, latent_value_kernel<TW, TO>, a));                      \
         return SCMX_OK;                                                                                                    \
     } while (0)
     if (w_dt == 0 && out_dt == 0) GO(bf16_t, bf16_t);
