@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(256) latent_absorb_kernel(const AbsorbArgs<TQ,
 
 // ---- attention of absorbed queries --------------------------------------------------------------------------------------
 constexpr int LR_P = 32;         // positions per tile
-constexpr int LR_SPLITS = 128;   // ranges of positions at most
+constexpr int LR_SPLITS = 64;    // ranges of positions at most
 
 // Pitch of a partial result: R values, maximum and sum, 16-byte aligned; maximum and sum start at column up4.
 __host__ __device__ __forceinline__ int up4(int n) { return (n + 3) & ~3; }
