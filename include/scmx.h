@@ -383,6 +383,8 @@ int scmx_decode_step_dense(const scmx_decode_layer* layers, int n_layers, int D,
                            float scale, const float* inv_freq, const float* rope_table, int64_t rope_rows, int64_t capacity,
                            const int32_t* pos_dev, uint16_t* h, uint16_t* y, uint16_t* act, uint16_t* o, float* partials,
                            int nsplit, int32_t* counters, uint32_t* barrier, int32_t* status, void* stream);
+/* Output head of one row: out bf16 [N] = W bf16 [N, ldw] x, x bf16 [K], float32 sums.  K a multiple of 8 up to 6400, rows 16-byte aligned. */
+int scmx_head_bf16(const uint16_t* W, int64_t ldw, const uint16_t* x, int64_t N, int64_t K, uint16_t* out, void* stream);
 /* Greedy choice inside a captured decode step: *tok = out[*count] = index of the largest of V logits (bf16 or float; the lowest of equal ones, a
  * not-a-number value counts as the largest), *count += 1, *pos += 1.  Nothing is stored in out at cap or beyond.  In libscmx_mixers too. */
 int scmx_select_token(const void* logits, int is_f32, int64_t V, int64_t* tok, int32_t* pos, int32_t* count, int64_t* out, int64_t cap, void* stream);

@@ -98,6 +98,7 @@ SIGNATURES = {
                                c_vp, c_vp, c_vp, c_vp, c_vp, c_int, c_vp, c_vp, c_vp, c_vp],
     "scmx_set_decode_trace": [c_vp, c_int],
     "scmx_select_token": [c_vp, c_int, c_i64, c_vp, c_vp, c_vp, c_vp, c_i64, c_vp],
+    "scmx_head_bf16": [c_vp, c_i64, c_vp, c_i64, c_i64, c_vp, c_vp],
     "scmx_route_token": [c_vp, c_vp, c_int, c_int, c_int, c_vp, c_vp, c_vp],
     "scmx_gemv_pro": [c_vp, c_int, c_vp, c_float, c_vp, c_vp, c_vp, c_i64, c_i64, _FMT_P, c_int, c_vp, c_vp, c_int, c_int, c_int,
                       c_vp, c_int, c_vp],

@@ -13,7 +13,8 @@ CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(HERE, "..", "include")
 LIBS = {"scmx": os.path.join(HERE, "libscmx.so"), "mixers": os.path.join(HERE, "libscmx_mixers.so")}
 LIB = LIBS["scmx"]
-SHARED = ("scmx_abi.cu", "scmx_tma.cu", "scmx_select.cu")        # error reporting, tensor maps, choice of a token: part of both libraries
+# error reporting, tensor maps, choice of a token: part of both libraries, like the matrix-vector product of mixers/
+SHARED = ("scmx_abi.cu", "scmx_tma.cu", "scmx_select.cu")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
               "--shared", "-cudart", "static"]
 
@@ -21,11 +22,12 @@ NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", 
 def sources(which="scmx"):
     d = CSRC if which == "scmx" else os.path.join(CSRC, "mixers")
     own = [os.path.join(d, f) for f in os.listdir(d) if f.endswith(".cu")]
-    return sorted(own if which == "scmx" else own + [os.path.join(CSRC, f) for f in SHARED])
+    both = [os.path.join(CSRC, "mixers", "mix_gemv.cu")] if which == "scmx" else [os.path.join(CSRC, f) for f in SHARED]
+    return sorted(own + both)
 
 
 def _deps(which):
-    dirs = [CSRC, INCLUDE] + ([os.path.join(CSRC, "mixers")] if which == "mixers" else [])
+    dirs = [CSRC, INCLUDE, os.path.join(CSRC, "mixers")]
     files = [os.path.join(d, f) for d in dirs for f in os.listdir(d) if f.endswith((".cuh", ".h"))]
     return files + sources(which)
 

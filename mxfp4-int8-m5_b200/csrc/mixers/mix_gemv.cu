@@ -2,7 +2,8 @@
 // accumulation.  Each warp sums two rows at a time (or a slice of their columns) and keeps two sets of 8 weight loads of 16 bytes per lane
 // in flight across its rows; the first are issued before the previous kernel of the chain has finished (weights never change).
 // Epilogues: none; xIELU; the causal convolution + SiLU of the first C rows, whose carried inputs are shifted in place; gelu(gate) up
-// of rows that alternate 16 gate and 16 up rows (a warp owns one of each).
+// of rows that alternate 16 gate and 16 up rows (a warp owns one of each); a bfloat16 row in and out (the output head of the W4A8 decoders;
+// this file is part of both libraries).
 #include "mix_common.cuh"
 
 namespace scmx {
@@ -17,6 +18,8 @@ struct GvArgs {
     const float *cw, *cb;   // convolution weights [C, taps] and bias [C]
     float* tail;            // [C, taps - 1]
     int C, taps;
+    const bf16_t* xh;       // EPI 4: the input row and the outputs in bfloat16
+    bf16_t* outh;
     // The input row may be one that the sublayers before leave in parts (pro): 1: r = x + mult y, input r / rms(r) nw;
     // 2: r = x + nw y / rms(y), then with n > 0 the weighted sum of n - 1 stored rows and r, input r, or r / rms(r) fw.
     int pro, n, keep;       // keep: r goes to row n - 1 of the store before it is averaged
@@ -176,7 +179,14 @@ __global__ void __launch_bounds__(256, 2) gemv_x_kernel(const GvArgs a) {
     fetch(wa);
     fetch(wb);
     pdl_wait();
-    if (a.pro != 0) {
+    if (EPI == 4) {
+        for (int v = tid; v < nv; v += 256) {
+            float x[8];
+            ld8(a.xh + 8 * v, x);
+            xs[v] = make_float4(x[0], x[1], x[2], x[3]);
+            xs[nv + v] = make_float4(x[4], x[5], x[6], x[7]);
+        }
+    } else if (a.pro != 0) {
         gv_prologue(a, xs, nv, red);
     } else if ((a.K & 3) == 0 && ((uintptr_t)a.x & 15) == 0) {
 #pragma unroll 8
@@ -217,7 +227,8 @@ __global__ void __launch_bounds__(256, 2) gemv_x_kernel(const GvArgs a) {
                 if (lane < GV_ROWS && row < a.N) {
                     float y = lane == 0 ? s[0] : s[1];
                     if (EPI == 1) y = xielu_f32(y, a.a_pos, a.a_neg);
-                    if (EPI == 2 && row < a.C) ys[row - GV_ROWS * base] = y;
+                    if (EPI == 4) a.outh[row] = f32_to_bf16(y);
+                    else if (EPI == 2 && row < a.C) ys[row - GV_ROWS * base] = y;
                     else a.out[row] = y;
                 }
             }
@@ -281,7 +292,7 @@ static int run_gemv(GvArgs a, int epi, cudaStream_t st) {
     const dim3 grid((unsigned)(groups < most ? groups : most)), block(256);
     const size_t smem = (size_t)nv * 32 + (epi == 2 ? (size_t)4 * GV_ROWS * ((a.N / GV_ROWS + 1) / grid.x + 2) : 0);
     SCMX_REQUIRE(smem <= 220 * 1024, SCMX_ELIMIT, "gemv_x: N=%d K=%d", a.N, a.K);
-    auto kernel = epi == 0 ? gemv_x_kernel<T, 0> : epi == 1 ? gemv_x_kernel<T, 1> : epi == 2 ? gemv_x_kernel<T, 2> : gemv_x_kernel<T, 3>;
+    auto kernel = epi == 0 ? gemv_x_kernel<T, 0> : epi == 1 ? gemv_x_kernel<T, 1> : epi == 2 ? gemv_x_kernel<T, 2> : epi == 3 ? gemv_x_kernel<T, 3> : gemv_x_kernel<bf16_t, 4>;
     if (smem > 40 * 1024) SCMX_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     SCMX_PDL_OK("gemv_x_kernel", launch_pdl(kernel, grid, block, smem, st, a));
     return SCMX_OK;
@@ -322,4 +333,13 @@ extern "C" int scmx_gemv_x_row(const void* W, int64_t ldw, int dt, const float* 
     a.pro = pro; a.n = n; a.keep = keep; a.mult = mult; a.eps = eps; a.y = y; a.nw = nw; a.dwa = dwa; a.fw = pro == 2 ? fw : nullptr;
     a.store = store; a.x_out = x_out; a.store_stride = store_stride;
     return gemv_x(W, ldw, dt, x, N, K, epi, a_pos, a_neg, conv_w, conv_b, tail, C, taps, out, a, stream);
+}
+
+extern "C" int scmx_head_bf16(const uint16_t* W, int64_t ldw, const uint16_t* x, int64_t N, int64_t K, uint16_t* out, void* stream) {
+    SCMX_REQUIRE(W && x && out && N > 0 && K > 0 && N < (1ll << 30) && K % 8 == 0 && ldw % 8 == 0 && ldw >= K, SCMX_EINVAL, "head_bf16: N=%lld K=%lld pitch %lld",
+                 (long long)N, (long long)K, (long long)ldw);
+    SCMX_REQUIRE((((uintptr_t)W | (uintptr_t)x) & 15) == 0 && K <= 6400, SCMX_ELIMIT, "head_bf16: 16-byte aligned rows of at most 6400 (K=%lld)", (long long)K);
+    GvArgs a = {};
+    a.W = W; a.ldw = ldw; a.N = (int)N; a.K = (int)K; a.ks = 1; a.xh = x; a.outh = out;
+    return run_gemv<bf16_t>(a, 4, (cudaStream_t)stream);
 }

@@ -178,7 +178,7 @@ __device__ __forceinline__ void softmax_topk(float (&p)[PER], int E, int topk, i
             if (ov > bv || (ov == bv && oe < be)) { bv = ov; be = oe; }
         }
         if (lane == 0) {
-            inds[r] = be;
+            inds[r] = be < E ? be : 0;      // logits that are not numbers choose no expert: stay inside the tables
             scores[r] = f32_to_bf16(bv);
             if (scores_f32) scores_f32[r] = bv;
         }

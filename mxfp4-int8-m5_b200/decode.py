@@ -31,8 +31,20 @@ from . import sc_moe as M_
 
 
 def _head_fn(model, head):
+    """[1, 1, D] -> logits [1, 1, V].  A host_model head in bfloat16 is one streaming matrix-vector product that takes part in the chain of
+    launches and lets its weights leave L2 first (32000 x 2048: 23 us as torch's product); any other head is called."""
     src = model if head == "model" else head
-    return src.head
+    weight = getattr(src, "head_weight", lambda: None)
+
+    def product(h):
+        w, row = weight(), h.reshape(-1)
+        if (w is None or w.dtype != torch.bfloat16 or row.dtype != torch.bfloat16 or not w.is_contiguous() or w.shape[1] % 8 or w.shape[1] > 6400
+                or row.numel() != w.shape[1] or not row.is_cuda or w.device != row.device or w.data_ptr() % 16 or row.data_ptr() % 16):
+            return src.head(h)
+        out = torch.empty((1, 1, w.shape[0]), dtype=torch.bfloat16, device=row.device)
+        _lib.call("scmx_head_bf16", _lib.ptr(w), w.shape[1], _lib.ptr(row), w.shape[0], w.shape[1], _lib.ptr(out), _lib.stream())
+        return out
+    return product
 
 
 class _Decoder:
@@ -118,6 +130,12 @@ class _Decoder:
     def _select(self, logits, tok, pos, count, chosen):
         """The next token (greedy) as the step's input and in the list of chosen ones, and the step's counters, in one kernel."""
         row = logits[:, -1].reshape(-1)
+        if row.dtype not in (torch.bfloat16, torch.float32):      # a head of its own
+            tok.copy_(row.argmax(-1, keepdim=True).view_as(tok))
+            chosen.index_copy_(0, count.long(), tok.view(1))
+            count.add_(1)
+            pos.add_(1)
+            return
         self._call("scmx_select_token", _lib.ptr(row), int(row.dtype == torch.float32), row.numel(), _lib.ptr(tok), _lib.ptr(pos), _lib.ptr(count),
                    _lib.ptr(chosen), chosen.numel(), _lib.stream())
 

@@ -286,6 +286,16 @@ class CausalLM(torch.nn.Module):
     def head(self, h):
         return TF.linear(h, self.model.embed_tokens.weight) if self.lm_head is None else self.lm_head(h)
 
+    def head_weight(self):
+        """The output head's matrix, where `head` is nothing but a product with it, else None."""
+        if type(self).head is not CausalLM.head or "head" in self.__dict__:
+            return None
+        lin = self.lm_head
+        if lin is None:
+            return self.model.embed_tokens.weight
+        plain = type(lin) is torch.nn.Linear and lin.bias is None and not (lin._forward_hooks or lin._forward_pre_hooks)
+        return lin.weight if plain else None
+
     def forward(self, ids, cache=None):
         """ids int [1, L] -> logits [1, L, V]; prefill into a fresh or offset cache."""
         cache = cache if cache is not None else make_prompt_cache(self, ids.shape[1])
