@@ -149,6 +149,7 @@ MIXER_SIGNATURES = {
                          c_vp, c_vp, c_vp, c_vp],
     "scmx_gemm_bf16": [c_vp, c_i64, c_vp, c_i64, c_i64, c_i64, c_i64, c_int, c_float, c_float, c_vp, c_int, c_i64, c_int, c_int, c_vp,
                        c_vp, c_vp],
+    "scmx_gemv_bf16": [c_vp, c_i64, c_vp, c_i64, c_i64, c_vp, c_int, c_vp],
     "scmx_gemv_x_row": [c_vp, c_i64, c_int, c_vp, c_vp, c_vp, c_int, c_float, c_float, c_vp, c_i64, c_vp, c_int, c_int, c_vp, c_vp, c_i64, c_i64,
                         c_int, c_float, c_float, c_vp, c_vp, c_vp, c_int, c_int, c_vp, c_vp],
     "scmx_gemv_x": [c_vp, c_i64, c_int, c_vp, c_i64, c_i64, c_int, c_float, c_float, c_vp, c_vp, c_vp, c_int, c_int, c_vp, c_vp],

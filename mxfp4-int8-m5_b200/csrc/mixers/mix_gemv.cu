@@ -18,7 +18,7 @@ struct GvArgs {
     const float *cw, *cb;   // convolution weights [C, taps] and bias [C]
     float* tail;            // [C, taps - 1]
     int C, taps;
-    const bf16_t* xh;       // EPI 4: the input row and the outputs in bfloat16
+    const bf16_t* xh;       // EPI 4: the input row in bfloat16, and the outputs if outh is given
     bf16_t* outh;
     // The input row may be one that the sublayers before leave in parts (pro): 1: r = x + mult y, input r / rms(r) nw;
     // 2: r = x + nw y / rms(y), then with n > 0 the weighted sum of n - 1 stored rows and r, input r, or r / rms(r) fw.
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(256, 2) gemv_x_kernel(const GvArgs a) {
                 if (lane < GV_ROWS && row < a.N) {
                     float y = lane == 0 ? s[0] : s[1];
                     if (EPI == 1) y = xielu_f32(y, a.a_pos, a.a_neg);
-                    if (EPI == 4) a.outh[row] = f32_to_bf16(y);
+                    if (EPI == 4 && a.outh != nullptr) a.outh[row] = f32_to_bf16(y);
                     else if (EPI == 2 && row < a.C) ys[row - GV_ROWS * base] = y;
                     else a.out[row] = y;
                 }
@@ -335,11 +335,21 @@ extern "C" int scmx_gemv_x_row(const void* W, int64_t ldw, int dt, const float* 
     return gemv_x(W, ldw, dt, x, N, K, epi, a_pos, a_neg, conv_w, conv_b, tail, C, taps, out, a, stream);
 }
 
-extern "C" int scmx_head_bf16(const uint16_t* W, int64_t ldw, const uint16_t* x, int64_t N, int64_t K, uint16_t* out, void* stream) {
-    SCMX_REQUIRE(W && x && out && N > 0 && K > 0 && N < (1ll << 30) && K % 8 == 0 && ldw % 8 == 0 && ldw >= K, SCMX_EINVAL, "head_bf16: N=%lld K=%lld pitch %lld",
+static int row_product(const uint16_t* W, int64_t ldw, const uint16_t* x, int64_t N, int64_t K, void* out, int out_f32, void* stream) {
+    SCMX_REQUIRE(W && x && out && N > 0 && K > 0 && N < (1ll << 30) && K % 8 == 0 && ldw % 8 == 0 && ldw >= K, SCMX_EINVAL, "row product: N=%lld K=%lld pitch %lld",
                  (long long)N, (long long)K, (long long)ldw);
-    SCMX_REQUIRE((((uintptr_t)W | (uintptr_t)x) & 15) == 0 && K <= 6400, SCMX_ELIMIT, "head_bf16: 16-byte aligned rows of at most 6400 (K=%lld)", (long long)K);
+    SCMX_REQUIRE((((uintptr_t)W | (uintptr_t)x) & 15) == 0 && K <= 6400, SCMX_ELIMIT, "row product: 16-byte aligned rows of at most 6400 (K=%lld)", (long long)K);
     GvArgs a = {};
-    a.W = W; a.ldw = ldw; a.N = (int)N; a.K = (int)K; a.ks = 1; a.xh = x; a.outh = out;
+    a.W = W; a.ldw = ldw; a.N = (int)N; a.K = (int)K; a.ks = 1; a.xh = x;
+    if (out_f32) a.out = static_cast<float*>(out);
+    else a.outh = static_cast<bf16_t*>(out);
     return run_gemv<bf16_t>(a, 4, (cudaStream_t)stream);
+}
+
+extern "C" int scmx_head_bf16(const uint16_t* W, int64_t ldw, const uint16_t* x, int64_t N, int64_t K, uint16_t* out, void* stream) {
+    return row_product(W, ldw, x, N, K, out, 0, stream);
+}
+
+extern "C" int scmx_gemv_bf16(const void* W, int64_t ldw, const void* x, int64_t N, int64_t K, void* out, int out_f32, void* stream) {
+    return row_product((const uint16_t*)W, ldw, (const uint16_t*)x, N, K, out, out_f32, stream);
 }

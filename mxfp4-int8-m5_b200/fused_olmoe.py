@@ -14,6 +14,7 @@ import torch
 from . import _lib
 from . import host_model as HM
 from . import packed_io
+from . import sc_decode as G
 from . import sc_format as F
 from . import sc_kernels as S
 from . import sc_moe as M_
@@ -228,7 +229,7 @@ class FusedOlmoe:
         return HM.make_prompt_cache(self.model, capacity)
 
     def logits(self, h):
-        return self.model.head(h)
+        return G.head_product(self.model)(h) if h.dim() == 3 and h.shape[:2] == (1, 1) else self.model.head(h)
 
     def __call__(self, ids, cache=None):
         cache = cache if cache is not None else self.make_cache(max(ids.shape[1], 1))

@@ -19,6 +19,7 @@ import torch
 from . import fused_dense as FD
 from . import host_model as HM
 from . import packed_io
+from . import sc_decode as G
 from . import sc_format as F
 from . import sc_kernels as S
 from .w4a8 import PackedWeight
@@ -249,7 +250,7 @@ class FusedQwen3:
         return HM.make_prompt_cache(self.model, capacity)
 
     def logits(self, h):
-        return self.model.head(h)
+        return G.head_product(self.model)(h) if h.dim() == 3 and h.shape[:2] == (1, 1) else self.model.head(h)
 
     def __call__(self, ids, cache=None):
         """Logits for every position."""

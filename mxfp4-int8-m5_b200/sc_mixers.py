@@ -126,6 +126,15 @@ class Linear:
         out_dtype = out_dtype or self.w.dtype
         M = x.shape[0]
         assert x.shape[1] == self.K and x.dtype == self.w.dtype and x.is_cuda
+        if M == 1 and act is None and tile == 0 and self.K <= 6400 and self.N % 8 == 0 and x.is_contiguous() and x.data_ptr() % 16 == 0:
+            # one row (the logits of a prompt's last position) is a stream of the weights: 32000 x 2048 took 44 us as a tile of 128 rows, 25 us so
+            if self.dt == 1:
+                return self.vec(x.view(-1))[None]
+            if self.K % 8 == 0:
+                y = torch.empty((1, self.N), dtype=out_dtype, device=x.device)
+                _lib.mcall("scmx_gemv_bf16", _lib.ptr(self.w), self.w.shape[1], _lib.ptr(x), self.N, self.K, _lib.ptr(y), int(out_dtype == torch.float32),
+                           _lib.stream())
+                return y
         if self.dt == 1:
             return self._call_f32(x, act, tile, splits)
         if _ld(x) % 8 or x.data_ptr() % 16:

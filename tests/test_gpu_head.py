@@ -17,7 +17,7 @@ def test_head(scmx, V, K):
 
 
 def test_own_heads_are_called(scmx):
-    HM, D = scmx.host_model, scmx.decode
+    HM, head = scmx.host_model, scmx.sc_decode.head_product
     args = HM.ModelArgs(256, 512, 1, 2, 2, 128, 1e-6, 1e4, 500, True)
     with torch.device("cuda"):
         model = HM.CausalLM(args)
@@ -25,8 +25,8 @@ def test_own_heads_are_called(scmx):
     with torch.no_grad():
         model.model.embed_tokens.weight.normal_()
         want = model.head(h)
-        assert (D._head_fn(model, "model")(h).float() - want.float()).abs().max() <= 2.0 ** -6 * want.float().abs().max()
-        assert torch.equal(D._head_fn(model, "model")(h.float()[..., :0].new_zeros(1, 1, 256).to(torch.bfloat16)), torch.zeros_like(want))
+        assert (head(model)(h).float() - want.float()).abs().max() <= 2.0 ** -6 * want.float().abs().max()
+        assert torch.equal(head(model)(h.float()[..., :0].new_zeros(1, 1, 256).to(torch.bfloat16)), torch.zeros_like(want))
 
         class Own(HM.CausalLM):
             def head(self, h):
@@ -34,6 +34,20 @@ def test_own_heads_are_called(scmx):
 
         own = Own.__new__(Own)
         own.__dict__.update(model.__dict__)
-        assert torch.equal(D._head_fn(own, "model")(h), h[..., :3] * 2)
+        assert torch.equal(head(own)(h), h[..., :3] * 2)
         model.head = lambda h: h[..., :5]
-        assert torch.equal(D._head_fn(model, "model")(h), h[..., :5])
+        assert torch.equal(head(model)(h), h[..., :5])
+
+
+@pytest.mark.parametrize("N,K,dt", [(8, 8, torch.bfloat16), (32000, 1024, torch.bfloat16), (96, 6400, torch.bfloat16), (4096, 2048, torch.float32), (40, 100, torch.float32)])
+def test_one_row(scmx, N, K, dt):
+    """Products of one row run as streams of the weights, in both output types and from the last row of a portion."""
+    X, g = scmx.sc_mixers, torch.Generator("cuda").manual_seed(N + K)
+    w, x = (torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).to(dt), torch.randn(5, K, generator=g, device="cuda").to(dt)
+    want = x[-1:].double() @ w.double().T
+    lin = X.Linear(w)
+    y = lin(x[-1:], torch.float32)
+    assert y.dtype == torch.float32 and ((y.double() - want).norm() / want.norm()) < 2e-6
+    if dt == torch.bfloat16:
+        y = lin(x[-1:])
+        assert y.dtype == dt and ((y.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-5).all()
