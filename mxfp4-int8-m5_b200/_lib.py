@@ -117,8 +117,8 @@ MIXER_SIGNATURES = {
     "scmx_add_norm": [c_vp, c_i64, c_vp, c_vp, c_float, c_float, c_i64, c_int, c_vp, c_vp, c_int, c_vp],
     "scmx_head_norm_gate": [c_vp, c_vp, c_i64, c_int, c_vp, c_int, c_i64, c_int, c_int, c_float, c_vp, c_vp],
     "scmx_select_token": [c_vp, c_int, c_i64, c_vp, c_vp, c_vp, c_vp, c_i64, c_vp],
-    "scmx_split3": [c_vp, c_i64, c_i64, c_i64, c_vp, c_vp],
-    "scmx_gemm_f32": [c_vp, c_i64, c_vp, c_vp, c_i64, c_vp, c_i64, c_i64, c_i64, c_int, c_float, c_float, c_vp, c_i64, c_int, c_int, c_vp, c_vp, c_vp],
+    "scmx_gemm_f32": [c_vp, c_i64, c_vp, c_i64, c_i64, c_i64, c_i64, c_int, c_float, c_float, c_vp, c_i64, c_int, c_int, c_i64, c_vp, c_vp, c_vp,
+                      c_vp],
     "scmx_gated_gelu": [c_vp, c_i64, c_i64, c_int, c_vp, c_vp],
     "scmx_delta_scratch": [c_i64, c_int, c_int, c_int, c_i64],
     "scmx_delta": [c_vp, c_i64, c_vp, c_i64, c_vp, c_i64, c_vp, c_i64, c_vp, c_i64, c_int, c_int, c_i64, c_int, c_int, c_int, c_int, c_vp, c_vp,

@@ -7,7 +7,8 @@
 // 5.7e-7 / 8.1e-7 / 1.4e-6; accumulators over the whole of K 1.0e-6 / 2.1e-6 / 6.7e-6; all six products in one accumulator 1.4e-6.
 //
 // Structure of gemm_bf16 (TMA producer warp, one MMA-issuing thread, 8 epilogue warps, two accumulators, persistent tiles; CTA pairs for
-// large shapes).  A stage holds the three parts of 64 values of both operands: six products use every part loaded twice.
+// large shapes).  A stage holds the three parts of 64 values of both operands: six products use every part loaded twice.  The parts are
+// written by a kernel before.
 // Infinities, not-a-number values and values that round to infinity in 16 bits make a sum not a number here; such outputs are
 // computed once more by plain multiply-adds on the float32 operands.
 #include "mix_tc.cuh"
@@ -35,27 +36,30 @@ constexpr int GF_CHUNK = 4;                            // blocks of 64 values pe
 constexpr int GF_PITCH = 80;                           // staged row of 16 outputs; conflict-free 16-byte stores
 constexpr int GF_STAGE_WARP = 32 * GF_PITCH;
 
-// x = p0 + p1 + p2; out [rows][3][kp], zero above K.
+// Rows of an operand to be split: x = p0 + p1 + p2, out [rows][3][kp], zero above K.
+struct SplitRows {
+    const float* x;
+    int64_t ldx, rows;
+    bf16_t* out;
+    int vec;                     // 16-byte loads
+};
+
+// Activations and a band of the weights in one launch; `team` warps (1, 2, 4 or 8) share a row, so that four loads a lane are a row of up to 4096.
+// The weights' parts live for one call: kept ones would not follow a weight that is changed in place, and would hold 6 bytes beside every 4.
 template <int V>
-__global__ void __launch_bounds__(256) split3_kernel(const float* x, int64_t ldx, int64_t rows, int K, int kp, bf16_t* out) {
-    pdl_launch_dependents();
-    pdl_wait();
-    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
-    const int per = kp / V;
-    if (i >= rows * per) return;
-    const int64_t r = i / per;
-    const int c = V * (int)(i - r * per);
-    float v[V];
+__device__ __forceinline__ void load_row(const float* x, int K, int c, float (&v)[V]) {
     if (V == 4) {
-        const float4 q = c < K ? *reinterpret_cast<const float4*>(x + r * ldx + c) : make_float4(0, 0, 0, 0);
+        const float4 q = c < K ? __ldg(reinterpret_cast<const float4*>(x + c)) : make_float4(0, 0, 0, 0);
         v[0] = q.x; v[1 % V] = q.y; v[2 % V] = q.z; v[3 % V] = q.w;
     } else {
 #pragma unroll
-        for (int e = 0; e < V; ++e) v[e] = c + e < K ? x[r * ldx + c + e] : 0.0f;
+        for (int e = 0; e < V; ++e) v[e] = c + e < K ? __ldg(x + c + e) : 0.0f;
     }
-    bf16_t* o = out + r * 3 * kp + c;
+}
+template <int V>
+__device__ __forceinline__ void store_parts(float (&v)[V], bf16_t* o, int kp) {
 #pragma unroll
-    for (int p = 0; p < 3; ++p, o += kp) {
+    for (int p = 0; p < 3; ++p) {
         uint32_t w[V / 2];
 #pragma unroll
         for (int e = 0; e < V; e += 2) {
@@ -63,9 +67,42 @@ __global__ void __launch_bounds__(256) split3_kernel(const float* x, int64_t ldx
             v[e] -= bf16_lo(w[e / 2]);
             v[e + 1] -= bf16_hi(w[e / 2]);
         }
-        if (V == 4) *reinterpret_cast<uint2*>(o) = make_uint2(w[0], w[(V / 2) - 1]);
-        else *reinterpret_cast<uint32_t*>(o) = w[0];
+        if (V == 4) *reinterpret_cast<uint2*>(o + p * kp) = make_uint2(w[0], w[(V / 2) - 1]);
+        else *reinterpret_cast<uint32_t*>(o + p * kp) = w[0];
     }
+}
+template <int V>
+__device__ __forceinline__ void split_row(const float* x, int K, int kp, bf16_t* o, int at, int step) {
+    for (int c0 = V * at; c0 < kp; c0 += 4 * V * step) {
+        float v[4][V];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) load_row<V>(x, K, c0 + i * V * step, v[i]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (c0 + i * V * step < kp) store_parts<V>(v[i], o + c0 + i * V * step, kp);
+    }
+}
+__global__ void __launch_bounds__(256) split3_kernel(const SplitRows a, const SplitRows b, int K, int kp, int team) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int warp = threadIdx.x >> 5, at = (warp & (team - 1)) * 32 + (threadIdx.x & 31);
+    const int64_t g = ((int64_t)blockIdx.x * 8 + warp) / team, r = g < a.rows ? g : g - a.rows;
+    const SplitRows& s = g < a.rows ? a : b;
+    if (r >= s.rows) return;
+    const float* x = s.x + r * s.ldx;
+    bf16_t* o = s.out + r * 3 * kp;
+    if (s.vec) split_row<4>(x, K, kp, o, at, 32 * team);
+    else split_row<2>(x, K, kp, o, at, 32 * team);
+}
+
+static int run_split3(SplitRows a, SplitRows b, int K, int kp, cudaStream_t st) {
+    auto vec = [&](const SplitRows& s) { return K % 4 == 0 && s.ldx % 4 == 0 && ((uintptr_t)s.x & 15) == 0; };
+    a.vec = vec(a);
+    b.vec = vec(b);
+    int team = 1;
+    while (team < 8 && kp > 512 * team) team *= 2;
+    SCMX_PDL_OK("split3_kernel", launch_pdl(split3_kernel, dim3((unsigned)(((a.rows + b.rows) * team + 7) / 8)), dim3(256), 0, st, a, b, K, kp, team));
+    return SCMX_OK;
 }
 
 // One output by multiply-adds over values [k0, k1).
@@ -369,45 +406,39 @@ static int launch_gf(const void* A3, const void* W3, const GfArgs& a, cudaStream
 
 using namespace scmx;
 
-extern "C" int scmx_split3(const float* x, int64_t ldx, int64_t rows, int64_t K, void* out, void* stream) {
-    SCMX_REQUIRE(x && out && rows >= 0 && K > 0 && K < (1ll << 28) && ldx >= K && ((uintptr_t)out & 15) == 0, SCMX_EINVAL, "split3: rows=%lld K=%lld",
-                 (long long)rows, (long long)K);
-    if (rows == 0) return SCMX_OK;
-    const int kp = (int)((K + 63) / 64 * 64);
-    const bool vec = K % 4 == 0 && ldx % 4 == 0 && ((uintptr_t)x & 15) == 0;
-    const int64_t items = rows * (kp / (vec ? 4 : 2));
-    SCMX_REQUIRE(items < (1ll << 38), SCMX_ELIMIT, "split3: %lld x %lld", (long long)rows, (long long)K);
-    SCMX_PDL_OK("split3_kernel", launch_pdl(vec ? split3_kernel<4> : split3_kernel<2>, dim3((unsigned)((items + 255) / 256)), dim3(256), 0,
-                                            (cudaStream_t)stream, x, ldx, rows, (int)K, kp, (bf16_t*)out));
-    return SCMX_OK;
-}
-
-extern "C" int scmx_gemm_f32(const float* A, int64_t lda, void* A3, const float* W, int64_t ldw, const void* W3, int64_t M, int64_t N, int64_t K,
-                             int act, float a_pos, float a_neg, float* out, int64_t ldo, int tile, int splits, float* part, int32_t* status,
+extern "C" int scmx_gemm_f32(const float* A, int64_t lda, const float* W, int64_t ldw, int64_t M, int64_t N, int64_t K, int act, float a_pos,
+                             float a_neg, float* out, int64_t ldo, int tile, int splits, int64_t band, float* part, void* scratch, int32_t* status,
                              void* stream) {
-    SCMX_REQUIRE(A && A3 && W && W3 && out && status, SCMX_EINVAL, "gemm_f32: null buffer");
+    SCMX_REQUIRE(A && W && out && scratch && status, SCMX_EINVAL, "gemm_f32: null buffer");
     SCMX_REQUIRE(M >= 0 && N > 0 && K > 0 && M < (1ll << 30) && N < (1ll << 30) && K < (1ll << 28), SCMX_EINVAL, "gemm_f32: M=%lld N=%lld K=%lld",
                  (long long)M, (long long)N, (long long)K);
     SCMX_REQUIRE(lda >= K && ldw >= K, SCMX_EINVAL, "gemm_f32: the row pitches %lld, %lld must hold K=%lld", (long long)lda, (long long)ldw, (long long)K);
     SCMX_REQUIRE(act >= 0 && act <= 2 && (act != 2 || N % 32 == 0), SCMX_EINVAL, "gemm_f32: act=%d on %lld columns", act, (long long)N);
     const int64_t nout = act == 2 ? N / 2 : N;
     SCMX_REQUIRE(ldo % 4 == 0 && ldo >= (nout + 3) / 4 * 4, SCMX_EINVAL, "gemm_f32: output pitch %lld for %lld columns", (long long)ldo, (long long)N);
-    SCMX_REQUIRE(((uintptr_t)A3 & 15) == 0 && ((uintptr_t)W3 & 15) == 0 && ((uintptr_t)out & 15) == 0, SCMX_EINVAL, "gemm_f32: pointer not 16-byte aligned");
+    SCMX_REQUIRE(((uintptr_t)scratch & 15) == 0 && ((uintptr_t)out & 15) == 0, SCMX_EINVAL, "gemm_f32: pointer not 16-byte aligned");
     SCMX_REQUIRE(tile == 64 || tile == 128 || tile == 256, SCMX_EINVAL, "gemm_f32: tile=%d", tile);
+    SCMX_REQUIRE(band >= N || (band > 0 && band % 256 == 0), SCMX_EINVAL, "gemm_f32: bands of %lld rows", (long long)band);
     if (M == 0) return SCMX_OK;
     GfArgs a;
-    a.M = (int)M; a.N = (int)N; a.K = (int)K; a.part_bytes = (int)((K + 63) / 64 * 128); a.act = act; a.a_pos = a_pos; a.a_neg = a_neg;
-    a.A = A; a.W = W; a.lda = lda; a.ldw = ldw; a.out = out; a.ldo = ldo; a.splits = 1; a.split_stride = 0; a.status = status; a.wait_ns = g_wait_limit_ns;
-    const cudaStream_t st = (cudaStream_t)stream;
-    const int64_t ldp = (N + 3) / 4 * 4;
-    if (splits > 1) {
+    a.M = (int)M; a.K = (int)K; a.part_bytes = (int)((K + 63) / 64 * 128); a.act = act; a.a_pos = a_pos; a.a_neg = a_neg;
+    a.A = A; a.lda = lda; a.ldw = ldw; a.splits = splits > 1 ? splits : 1; a.status = status; a.wait_ns = g_wait_limit_ns;
+    if (splits > 1)
         SCMX_REQUIRE(part && ((uintptr_t)part & 15) == 0 && act == 0 && splits <= (a.part_bytes / BK + GF_CHUNK - 1) / GF_CHUNK, SCMX_EINVAL,
                      "gemm_f32: %d ranges of K=%lld need a buffer and no activation", splits, (long long)K);
-        a.out = part; a.ldo = ldp; a.splits = splits; a.split_stride = M * ldp;
+    const cudaStream_t st = (cudaStream_t)stream;
+    const int kp = a.part_bytes / 2;
+    bf16_t *a3 = (bf16_t*)scratch, *w3 = a3 + M * 3 * kp;
+    for (int64_t n0 = 0; n0 < N; n0 += band) {
+        const int64_t n = N - n0 < band ? N - n0 : band, ldp = (n + 3) / 4 * 4;
+        float* o = out + (act == 2 ? n0 / 2 : n0);
+        a.N = (int)n; a.W = W + n0 * ldw;
+        a.out = splits > 1 ? part : o; a.ldo = splits > 1 ? ldp : ldo; a.split_stride = splits > 1 ? M * ldp : 0;
+        int rc = run_split3(SplitRows{A, lda, n0 == 0 ? M : 0, a3, 0}, SplitRows{a.W, ldw, n, w3, 0}, (int)K, kp, st);
+        if (rc) return rc;
+        rc = tile == 256 ? launch_gf<256, true>(a3, w3, a, st) : tile == 128 ? launch_gf<128, false>(a3, w3, a, st) : launch_gf<64, false>(a3, w3, a, st);
+        if (rc) return rc;
+        if (splits > 1 && (rc = gemm_reduce(part, splits, a.split_stride, M, ldp, 1, o, ldo, st))) return rc;
     }
-    int rc = scmx_split3(A, lda, M, K, A3, stream);
-    if (rc) return rc;
-    rc = tile == 256 ? launch_gf<256, true>(A3, W3, a, st) : tile == 128 ? launch_gf<128, false>(A3, W3, a, st) : launch_gf<64, false>(A3, W3, a, st);
-    if (rc || a.splits == 1) return rc;
-    return gemm_reduce(part, splits, a.split_stride, M, ldp, 1, out, ldo, st);
+    return SCMX_OK;
 }

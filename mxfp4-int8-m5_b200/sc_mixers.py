@@ -59,17 +59,19 @@ class GatedGELU:
         return w.view(2, m // 16, 16, k).transpose(0, 1).reshape(2 * m, k)
 
 
-# Float32 portions of fewer rows, or with few columns, are multiplied by the library's float32 product: 16 x 1024 x 1024 takes 9.2 us there
-# and 11.6 us on tensor cores, 300 x 2048 x 64 6.0 and 6.8 us; 32 x 1024 x 1024 takes 13.6 and 11.2 us, 300 x 6144 x 1024 85 and 27 us.
+# Least rows and least K of a float32 product on tensor cores (an explicit tile asks for one); below, the library's float32 product.
 F32_TC_MIN, F32_TC_MIN_K = 24, 128
 
 
-def split3(x):
-    """float32 [M, K] -> bfloat16 [M, 3 Kp] of its three parts (x = p0 + p1 + p2), Kp = K rounded up to 64, zero padded."""
-    M, K = x.shape
-    out = torch.empty((M, 3 * ((K + 63) // 64 * 64)), dtype=torch.bfloat16, device=x.device)
-    _lib.mcall("scmx_split3", _lib.ptr(x), _ld(x), M, K, _lib.ptr(out), _lib.stream())
-    return out
+def _f32_tc(M, N, K):
+    """Whether a float32 product of M >= F32_TC_MIN rows runs on tensor cores, both times in us (library, tensor cores with the split of both operands).
+    A long K always: 24 x 1024 x 1024 13.7 and 13.0, 300 x 1024 x 1024 28 and 17, 24 x 96 x 2048 17 and 12, 300 x 6144 x 1024 84 and 35; but few rows of a large
+    matrix are bound by splitting it: 24 x 12288 x 2048 67 and 84, 40 rows 86 and 85.  A short K where the library has a wave of work:
+    300 x 1024 x 384 12.4 and 12.7, 1024 x 1024 x 384 20 and 14; 100 x 3072 x 256 9.2 and 11.0, 300 x 3072 x 256 15 and 12; 300 x 512 x 512 11.8 and 12.9,
+    1024 x 512 x 512 16.5 and 15.4."""
+    if K >= 768:
+        return M >= 40 or N <= 8192
+    return M * N >= (400000 if K >= 512 else 800000)
 
 
 @functools.lru_cache(maxsize=4096)
@@ -99,9 +101,17 @@ def _plan_f32(M, N, K, splits, n_sm=148):
     return min(((t, s) for t in (64, 128, 256) for s in ([splits] if splits else range(1, min(8, chunks) + 1))), key=lambda c: cost(*c))
 
 
+def _band(N, K):
+    """Rows of the weights that are split at a time: 256 MB of parts at most (6 bytes a value).  Bands that would stay in L2 leave SMs idle: 300 x 12288 x 2048
+    in bands of 48 MB takes 241 us."""
+    rows = max(256, int(256e6 / (6 * -(-K // 64) * 64)) // 256 * 256)
+    return N if N <= rows else rows
+
+
 class Linear:
     """y = W x without bias.  W [N, K] bfloat16 (tcgen05 GEMM / GEMV kernels) or float32 (GEMV kernel for one row, tcgen05 products of
-    three bfloat16 parts for portions, the library's float32 product without reduced-precision modes for a few rows)."""
+    three bfloat16 parts for portions, the library's float32 product without reduced-precision modes for a few rows).  A contiguous
+    weight with K a multiple of 8 is not copied: the layer follows changes of it."""
 
     def __init__(self, w):
         self.N, self.K = w.shape
@@ -112,13 +122,11 @@ class Linear:
             self.w = torch.zeros((self.N, ld), dtype=w.dtype, device=w.device)
             self.w[:, :self.K] = w
         self.dt = _dt(w)
-        self.w3 = split3(self.w[:, :self.K]) if self.dt == 1 and w.is_cuda and self.K >= F32_TC_MIN_K else None
 
     def rows(self, r0, r1):
         """The product with some of the rows, on the same memory."""
         out = object.__new__(Linear)
         out.N, out.K, out.w, out.dt = r1 - r0, self.K, self.w[r0:r1], self.dt
-        out.w3 = None if self.w3 is None else self.w3[r0:r1]
         return out
 
     def __call__(self, x, out_dtype=None, act=None, tile=0, splits=None):
@@ -152,7 +160,7 @@ class Linear:
 
     def _call_f32(self, x, act, tile, splits):
         M = x.shape[0]
-        if self.w3 is None or M < F32_TC_MIN:
+        if M < F32_TC_MIN or self.K < F32_TC_MIN_K or not (tile or _f32_tc(M, self.N, self.K)):
             with _full_float32():
                 y = x @ self.w[:, :self.K].T
             if act is not None and act.code == 2:
@@ -164,13 +172,14 @@ class Linear:
             return y
         nout = self.N // 2 if act is not None and act.code == 2 else self.N
         y = empty_rows(M, nout, torch.float32, x.device)
+        band = _band(self.N, self.K)
         if tile == 0:
-            tile, splits = _plan_f32(M, self.N, self.K, 1 if act is not None else splits)
+            tile, splits = _plan_f32(M, band, self.K, 1 if act is not None else splits)
         splits = splits or 1
-        x3 = torch.empty((M, self.w3.shape[1]), dtype=torch.bfloat16, device=x.device)
-        part = torch.empty(splits * M * ((self.N + 3) // 4 * 4), dtype=torch.float32, device=x.device) if splits > 1 else None
-        _lib.mcall("scmx_gemm_f32", _lib.ptr(x), _ld(x), _lib.ptr(x3), _lib.ptr(self.w), self.w.shape[1], _lib.ptr(self.w3), M, self.N, self.K,
-                   act.code if act else 0, act.a_pos if act else 0.0, act.a_neg if act else 0.0, _lib.ptr(y), _round8(nout), tile, splits, _lib.ptr(part),
+        scratch = torch.empty((M + band, 3 * -(-self.K // 64) * 64), dtype=torch.bfloat16, device=x.device)
+        part = torch.empty(splits * M * ((band + 3) // 4 * 4), dtype=torch.float32, device=x.device) if splits > 1 else None
+        _lib.mcall("scmx_gemm_f32", _lib.ptr(x), _ld(x), _lib.ptr(self.w), self.w.shape[1], M, self.N, self.K, act.code if act else 0,
+                   act.a_pos if act else 0.0, act.a_neg if act else 0.0, _lib.ptr(y), _round8(nout), tile, splits, band, _lib.ptr(part), _lib.ptr(scratch),
                    _lib.ptr(_lib.mixer_status_buffer()), _lib.stream())
         return y
 

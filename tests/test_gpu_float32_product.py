@@ -1,0 +1,46 @@
+"""GPU: float32 products of portions where they differ from a plain product: weights that change after the layer was built, weights taken in bands."""
+import pytest
+import torch
+
+from test_gpu_hybrid_kernels import F32, X  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(got, want):
+    return float((got.double() - want).norm() / want.norm())
+
+
+@pytest.mark.parametrize("M", [1, 2, 24, 130])
+def test_weights_changed_in_place(X, M):      # noqa: F811
+    """A layer on the caller's memory follows it, in a captured graph too, and keeps nothing beside it."""
+    x, w = torch.randn(M, 1024, device="cuda"), torch.randn(320, 1024, device="cuda") * 0.03
+    held = torch.cuda.memory_allocated()
+    lin = X.Linear(w)
+    assert torch.cuda.memory_allocated() == held
+    lin(x)
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=s):
+            z = lin(x)
+    torch.cuda.current_stream().wait_stream(s)
+    w.mul_(-0.5).add_(0.01)
+    graph.replay()
+    want = X.Linear(w.clone())(x)
+    assert rel(want, x.double() @ w.double().T) < 1e-6
+    assert torch.equal(lin(x), want) and torch.equal(z, want) and torch.equal(lin.rows(32, 96)(x), X.Linear(w[32:96].clone())(x))
+
+
+@pytest.mark.parametrize("tile,splits", [(0, None), (64, 3), (128, 1), (256, 1)])
+def test_bands_of_weights(X, monkeypatch, tile, splits):      # noqa: F811
+    M, N, K = 70, 600, 1100      # bands of 256, 256 and 88 rows
+    monkeypatch.setattr(X, "_band", lambda n, k: min(n, 256))
+    x, w = torch.randn(M, K, device="cuda"), torch.randn(N, K, device="cuda") * K ** -0.5
+    assert rel(X.Linear(w)(x, tile=tile, splits=splits), x.double() @ w.double().T) < 6e-7
+    if splits in (None, 1):
+        w = w[:576]
+        z = x.double() @ w.double().T
+        want = torch.nn.functional.gelu(z[:, :288], approximate="tanh") * z[:, 288:]
+        assert rel(X.Linear(X.GatedGELU.weight(w[:288], w[288:]))(x, act=X.GatedGELU(), tile=tile, splits=splits), want) < 2e-6
