@@ -1,13 +1,14 @@
 // float32 GEMM, out = A [M, K] . W [N, K]^T, on tcgen05.mma kind::f16: every operand value is the exact sum of three bfloat16 parts
 // (8 bits of mantissa each), and the six part products above 2^-24 of the whole are summed.
-// The tensor core's float32 accumulator cuts bits off instead of rounding, so its error grows with the number of instructions that add to
-// it.  Therefore the products of the leading parts have an accumulator of their own (the other five are 2^-8 of it), an accumulator takes
-// 256 values of K at most, and the epilogue warps add both to float32 registers, rounded to nearest.
-// Error against 64-bit sums (2-norm, normal operands), K = 1024 / 2048 / 6144: 2.4e-7 / 2.4e-7 / 2.5e-7; sums of CUDA-core multiply-adds
-// 5.7e-7 / 8.1e-7 / 1.4e-6; accumulators over the whole of K 1.0e-6 / 2.1e-6 / 6.7e-6; all six products in one accumulator 1.4e-6.
+// The tensor core's float32 accumulator cuts bits off instead of rounding: an error with a sign, which grows with the number of instructions that
+// add to it and which a scan over hundreds of tokens adds up.  Therefore the products of the leading parts have an accumulator of their own (the other
+// five are 2^-8 of it), an accumulator takes 64 values of K, and the epilogue warps add both to float32 registers, rounded to nearest.
+// Error against 64-bit sums (2-norm, normal operands), K = 1024 / 2048 / 6144: 1.2e-7 / 1.6e-7 / 2.6e-7, mean -5e-8; with accumulators of 256 values
+// 2.4e-7 / 2.4e-7 / 2.6e-7, mean -1.9e-7; sums of CUDA-core multiply-adds 5.7e-7 / 8.1e-7 / 1.4e-6, mean 0; accumulators over the whole of K 1.0e-6 / 2.1e-6 /
+// 6.7e-6.  State of the first scan after a prompt of 700 float32 tokens: 8.1e-7, with accumulators of 256 values 1.28e-6, with multiply-adds 1.0e-6.
 //
-// Structure of gemm_bf16 (TMA producer warp, one MMA-issuing thread, 8 epilogue warps, two accumulators, persistent tiles; CTA pairs for
-// large shapes).  A stage holds the three parts of 64 values of both operands: six products use every part loaded twice.  The parts are
+// Structure of gemm_bf16 (TMA producer warp, one MMA-issuing thread, 8 epilogue warps, two accumulators, persistent tiles; CTA pairs with
+// tile 256).  A stage holds the three parts of 64 values of both operands: six products use every part loaded twice.  The parts are
 // written by a kernel before.
 // Infinities, not-a-number values and values that round to infinity in 16 bits make a sum not a number here; such outputs are
 // computed once more by plain multiply-adds on the float32 operands.
@@ -32,7 +33,7 @@ struct GfArgs {
     uint64_t wait_ns;
 };
 
-constexpr int GF_CHUNK = 4;                            // blocks of 64 values per accumulator
+constexpr int GF_CHUNK = 1;                            // blocks of 64 values per accumulator (300 x 6144 x 1024: 35 us with 4, 36 us with 1)
 constexpr int GF_PITCH = 80;                           // staged row of 16 outputs; conflict-free 16-byte stores
 constexpr int GF_STAGE_WARP = 32 * GF_PITCH;
 

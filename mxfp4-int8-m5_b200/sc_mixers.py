@@ -89,16 +89,15 @@ def _plan(M, N, K, splits, n_sm=148):
 
 @functools.lru_cache(maxsize=4096)
 def _plan_f32(M, N, K, splits, n_sm=148):
-    """(tile, ranges of K) of a float32 product: steps of 64 values stage three parts of 128 + tile rows (CTA pairs: half of a 256 x 256
-    tile each), about 5 ns a row and step, 4 ns for pairs; 5 us around them.  Ranges are whole accumulators of 256 values and cost a summing launch, about 3 us
-    and their traffic.  300 x 4096 x 1024: 26 us as 128 x 128 tiles, 40 us as 128 x 64; 2048 x 2048 x 6144: 242 us as pairs, 257 us as 128 x 128."""
-    kb, chunks = -(-K // 64), -(-K // 256)
+    """(tile, ranges of K) of a float32 product: steps of 64 values stage three parts of 128 + tile rows, about 5.5 ns a row and step; 5 us around them.
+    Ranges cost a summing launch, about 3 us and their traffic.  300 x 6144 x 1024: 36 us as 128 x 128 tiles, 48 us as 128 x 64.  CTA pairs (tile 256), whose accumulators
+    leave no room for a second set, are only run when asked for: 2048 x 2048 x 6144 287 us as 128 x 128 tiles, 386 us as pairs."""
+    tm, kb = -(-M // 128), -(-K // 64)
 
     def cost(tile, s):
-        tiles, workers = (-(-M // 256) * -(-N // 256), n_sm // 2) if tile == 256 else (-(-M // 128) * -(-N // tile), n_sm)
-        step = 256 * 0.0105 if tile == 256 else (128 + tile) * 0.0055
-        return 5 + -(-tiles * s // workers) * min(kb, 4 * -(-chunks // s)) * step + (3 + s * M * N * 8 / 3e6 if s > 1 else 0)
-    return min(((t, s) for t in (64, 128, 256) for s in ([splits] if splits else range(1, min(8, chunks) + 1))), key=lambda c: cost(*c))
+        tiles = tm * -(-N // tile)
+        return 5 + -(-tiles * s // n_sm) * -(-kb // s) * (128 + tile) * 0.0055 + (3 + s * M * N * 8 / 3e6 if s > 1 else 0)
+    return min(((t, s) for t in (64, 128) for s in ([splits] if splits else range(1, min(8, -(-kb // 4)) + 1))), key=lambda c: cost(*c))
 
 
 def _band(N, K):
