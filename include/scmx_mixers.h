@@ -144,7 +144,7 @@ int scmx_gemm_bf16(const void* A, int64_t lda, const void* W, int64_t ldw, int64
                    void* out, int out_f32, int64_t ldo, int tile, int splits, float* part, int32_t* status, void* stream);
 
 /* out [M, N] = A [M, K] . W [N, K]^T in float32: both operands as three bfloat16 parts, sums over 64 values on tensor cores and float32 above
- * them.  scratch: (M + min(N, band)) * 6 * (K rounded up to 64) bytes for the parts, 16-byte aligned; W is taken in bands of `band` rows, a multiple of 256
+ * them.  scratch: (M + min(N, band)) * (6 * (K rounded up to 64) + 4) bytes, 16-byte aligned; W is taken in bands of `band` rows, a multiple of 256
  * or at least N.  act, tile (64, 128 or 256) and splits as above; part: float [splits][M][min(N, band) rounded up to 4]. */
 int scmx_gemm_f32(const float* A, int64_t lda, const float* W, int64_t ldw, int64_t M, int64_t N, int64_t K, int act, float a_pos, float a_neg,
                   float* out, int64_t ldo, int tile, int splits, int64_t band, float* part, void* scratch, int32_t* status, void* stream);

@@ -1,5 +1,7 @@
-// float32 GEMM, out = A [M, K] . W [N, K]^T, on tcgen05.mma kind::f16: every operand value is the exact sum of three bfloat16 parts
-// (8 bits of mantissa each), and the six part products above 2^-24 of the whole are summed.
+// float32 GEMM, out = A [M, K] . W [N, K]^T, on tcgen05.mma kind::f16: every operand value is the sum of three bfloat16 parts (8 bits of mantissa
+// each), and the six part products above 2^-24 of the whole are summed.  Rows of both operands are taken times a power of two that brings their largest
+// value into [1, 2), so the parts are exact down to 2^-110 of it (bfloat16 has no more exponents; unscaled, values below 2^-110 would lose bits) and
+// nothing overflows on the way; the epilogue scales back.
 // The tensor core's float32 accumulator cuts bits off instead of rounding: an error with a sign, which grows with the number of instructions that
 // add to it and which a scan over hundreds of tokens adds up.  Therefore the products of the leading parts have an accumulator of their own (the other
 // five are 2^-8 of it), an accumulator takes 64 values of K, and the epilogue warps add both to float32 registers, rounded to nearest.
@@ -10,8 +12,7 @@
 // Structure of gemm_bf16 (TMA producer warp, one MMA-issuing thread, 8 epilogue warps, two accumulators, persistent tiles; CTA pairs with
 // tile 256).  A stage holds the three parts of 64 values of both operands: six products use every part loaded twice.  The parts are
 // written by a kernel before.
-// Infinities, not-a-number values and values that round to infinity in 16 bits make a sum not a number here; such outputs are
-// computed once more by plain multiply-adds on the float32 operands.
+// Infinities and not-a-number values make a sum not a number here; such outputs are computed once more by plain multiply-adds on the float32 operands.
 #include "mix_tc.cuh"
 
 namespace scmx {
@@ -25,6 +26,7 @@ struct GfArgs {
     float a_pos, a_neg;
     const float *A, *W;          // the operands themselves
     int64_t lda, ldw;
+    const int32_t *ea, *ew;      // exponents of their rows
     float* out;
     int64_t ldo;
     int splits;                  // > 1: range s of K goes to out + s * split_stride (no activation)
@@ -37,11 +39,12 @@ constexpr int GF_CHUNK = 1;                            // blocks of 64 values pe
 constexpr int GF_PITCH = 80;                           // staged row of 16 outputs; conflict-free 16-byte stores
 constexpr int GF_STAGE_WARP = 32 * GF_PITCH;
 
-// Rows of an operand to be split: x = p0 + p1 + p2, out [rows][3][kp], zero above K.
+// Rows of an operand to be split: 2^-e x = p0 + p1 + p2, out [rows][3][kp], zero above K.
 struct SplitRows {
     const float* x;
     int64_t ldx, rows;
     bf16_t* out;
+    int32_t* e;
     int vec;                     // 16-byte loads
 };
 
@@ -72,28 +75,63 @@ __device__ __forceinline__ void store_parts(float (&v)[V], bf16_t* o, int kp) {
         else *reinterpret_cast<uint32_t*>(o + p * kp) = w[0];
     }
 }
+// Largest magnitude (bits) of this thread's share of a row.
 template <int V>
-__device__ __forceinline__ void split_row(const float* x, int K, int kp, bf16_t* o, int at, int step) {
+__device__ __forceinline__ uint32_t row_top(const float* x, int K, int at, int step) {
+    uint32_t m = 0;
+    for (int c0 = V * at; c0 < K; c0 += 4 * V * step) {
+        float v[4][V];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) load_row<V>(x, K, c0 + i * V * step, v[i]);
+#pragma unroll
+        for (int i = 0; i < 4 * V; ++i) m = max(m, __float_as_uint(v[i / V][i % V]) & 0x7FFFFFFFu);
+    }
+    return m;
+}
+// Its exponent, of subnormal numbers too; 0 for zero, infinities and not-a-number values.
+__device__ __forceinline__ int top_exponent(uint32_t m) {
+    if (m == 0 || m >= 0x7F800000u) return 0;
+    return m >= 0x00800000u ? (int)(m >> 23) - 127 : 31 - __clz((int)m) - 149;
+}
+template <int V>
+__device__ __forceinline__ void split_row(const float* x, int K, int kp, bf16_t* o, int at, int step, int exp) {
+    const int half = exp >> 1;      // -149 .. 127: 2^-exp in two factors
+    const float f1 = __int_as_float((127 - half) << 23), f2 = __int_as_float((127 - (exp - half)) << 23);
     for (int c0 = V * at; c0 < kp; c0 += 4 * V * step) {
         float v[4][V];
 #pragma unroll
         for (int i = 0; i < 4; ++i) load_row<V>(x, K, c0 + i * V * step, v[i]);
+#pragma unroll
+        for (int i = 0; i < 4 * V; ++i) v[i / V][i % V] *= f1;
+#pragma unroll
+        for (int i = 0; i < 4 * V; ++i) v[i / V][i % V] *= f2;
 #pragma unroll
         for (int i = 0; i < 4; ++i)
             if (c0 + i * V * step < kp) store_parts<V>(v[i], o + c0 + i * V * step, kp);
     }
 }
 __global__ void __launch_bounds__(256) split3_kernel(const SplitRows a, const SplitRows b, int K, int kp, int team) {
+    __shared__ uint32_t top[8];
     pdl_launch_dependents();
     pdl_wait();
     const int warp = threadIdx.x >> 5, at = (warp & (team - 1)) * 32 + (threadIdx.x & 31);
     const int64_t g = ((int64_t)blockIdx.x * 8 + warp) / team, r = g < a.rows ? g : g - a.rows;
     const SplitRows& s = g < a.rows ? a : b;
-    if (r >= s.rows) return;
+    const bool on = r < s.rows;
     const float* x = s.x + r * s.ldx;
+    uint32_t m = !on ? 0 : s.vec ? row_top<4>(x, K, at, 32 * team) : row_top<2>(x, K, at, 32 * team);
+    m = __reduce_max_sync(0xffffffffu, m);
+    if (team > 1) {
+        if ((threadIdx.x & 31) == 0) top[warp] = m;
+        __syncthreads();
+        for (int i = 0; i < team; ++i) m = max(m, top[(warp & ~(team - 1)) + i]);
+    }
+    if (!on) return;
+    const int exp = top_exponent(m);
+    if (at == 0) s.e[r] = exp;
     bf16_t* o = s.out + r * 3 * kp;
-    if (s.vec) split_row<4>(x, K, kp, o, at, 32 * team);
-    else split_row<2>(x, K, kp, o, at, 32 * team);
+    if (s.vec) split_row<4>(x, K, kp, o, at, 32 * team, exp);      // the row once more, from L1 or L2
+    else split_row<2>(x, K, kp, o, at, 32 * team, exp);
 }
 
 static int run_split3(SplitRows a, SplitRows b, int K, int kp, cudaStream_t st) {
@@ -104,6 +142,28 @@ static int run_split3(SplitRows a, SplitRows b, int K, int kp, cudaStream_t st) 
     while (team < 8 && kp > 512 * team) team *= 2;
     SCMX_PDL_OK("split3_kernel", launch_pdl(split3_kernel, dim3((unsigned)(((a.rows + b.rows) * team + 7) / 8)), dim3(256), 0, st, a, b, K, kp, team));
     return SCMX_OK;
+}
+
+// Sums of 32 columns times the powers of two of this lane's row (ea) and of the columns (ew: of column `lane`).  Powers up to 2^60 by multiplications, which
+// are exact; the others with one rounding at the ends of the number range.
+__device__ __noinline__ void gf_scale_far(float* s, int ea, int ew) {
+#pragma unroll 1
+    for (int j = 0; j < 32; ++j) s[j] = ldexpf(s[j], ea + __shfl_sync(0xffffffffu, ew, j));
+}
+__device__ __forceinline__ float gf_power(int e) { return __int_as_float((e + 127) << 23); }
+__device__ __forceinline__ void gf_scale(float* s, int ea, int ew) {
+    if (__all_sync(0xffffffffu, abs(ea) <= 60 && abs(ew) <= 60)) {
+        const float fa = gf_power(ea), fw = gf_power(ew);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) s[j] = s[j] * fa * __shfl_sync(0xffffffffu, fw, j);
+    } else {
+        float t[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) t[j] = s[j];
+        gf_scale_far(t, ea, ew);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) s[j] = t[j];
+    }
 }
 
 // One output by multiply-adds over values [k0, k1).
@@ -267,6 +327,10 @@ __device__ __forceinline__ void gemm_f32_body(const CUtensorMap& tmA, const CUte
             const int sp = t / per_split, tt = t - sp * per_split, nt = tt / tiles_m, mt = tt - nt * tiles_m;
             const int kb0 = first_kb(sp), kb1 = first_kb(sp + 1);
             const int n0 = nt * BN + chalf * COLS, row0 = mt * TM_ROWS + (int)rank * BM + 32 * q;
+            const int ea = row0 + lane < a.M ? a.ea[row0 + lane] : 0;
+            int ew[COLS / 32];
+#pragma unroll
+            for (int c = 0; c < COLS / 32; ++c) ew[c] = n0 + 32 * c + lane < a.N ? a.ew[n0 + 32 * c + lane] : 0;
             float sum[COLS];
 #pragma unroll
             for (int j = 0; j < COLS; ++j) sum[j] = 0.0f;
@@ -297,6 +361,8 @@ __device__ __forceinline__ void gemm_f32_body(const CUtensorMap& tmA, const CUte
                 if (++acc == L::ACCS) { acc = 0; acc_phase ^= 1; }
             }
             if (fail) break;
+#pragma unroll
+            for (int c = 0; c < COLS / 32; ++c) gf_scale(sum + 32 * c, ea, ew[c]);
             bool bad = false;
 #pragma unroll
             for (int j = 0; j < COLS; ++j) bad |= sum[j] != sum[j];
@@ -430,12 +496,14 @@ extern "C" int scmx_gemm_f32(const float* A, int64_t lda, const float* W, int64_
     const cudaStream_t st = (cudaStream_t)stream;
     const int kp = a.part_bytes / 2;
     bf16_t *a3 = (bf16_t*)scratch, *w3 = a3 + M * 3 * kp;
+    int32_t* e = (int32_t*)(w3 + (N < band ? N : band) * 3 * kp);
+    a.ea = e; a.ew = e + M;
     for (int64_t n0 = 0; n0 < N; n0 += band) {
         const int64_t n = N - n0 < band ? N - n0 : band, ldp = (n + 3) / 4 * 4;
         float* o = out + (act == 2 ? n0 / 2 : n0);
         a.N = (int)n; a.W = W + n0 * ldw;
         a.out = splits > 1 ? part : o; a.ldo = splits > 1 ? ldp : ldo; a.split_stride = splits > 1 ? M * ldp : 0;
-        int rc = run_split3(SplitRows{A, lda, n0 == 0 ? M : 0, a3, 0}, SplitRows{a.W, ldw, n, w3, 0}, (int)K, kp, st);
+        int rc = run_split3(SplitRows{A, lda, n0 == 0 ? M : 0, a3, e, 0}, SplitRows{a.W, ldw, n, w3, e + M, 0}, (int)K, kp, st);
         if (rc) return rc;
         rc = tile == 256 ? launch_gf<256, true>(a3, w3, a, st) : tile == 128 ? launch_gf<128, false>(a3, w3, a, st) : launch_gf<64, false>(a3, w3, a, st);
         if (rc) return rc;

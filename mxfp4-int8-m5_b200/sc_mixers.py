@@ -65,13 +65,12 @@ F32_TC_MIN, F32_TC_MIN_K = 24, 128
 
 def _f32_tc(M, N, K):
     """Whether a float32 product of M >= F32_TC_MIN rows runs on tensor cores, both times in us (library, tensor cores with the split of both operands).
-    A long K always: 24 x 1024 x 1024 13.7 and 13.0, 300 x 1024 x 1024 28 and 17, 24 x 96 x 2048 17 and 12, 300 x 6144 x 1024 84 and 35; but few rows of a large
-    matrix are bound by splitting it: 24 x 12288 x 2048 67 and 84, 40 rows 86 and 85.  A short K where the library has a wave of work:
-    300 x 1024 x 384 12.4 and 12.7, 1024 x 1024 x 384 20 and 14; 100 x 3072 x 256 9.2 and 11.0, 300 x 3072 x 256 15 and 12; 300 x 512 x 512 11.8 and 12.9,
-    1024 x 512 x 512 16.5 and 15.4."""
+    A long K: 100 x 1024 x 768 16.6 and 14.5, 300 x 6144 x 1024 84 and 39, 40 x 512 x 1024 14.2 and 13.3, 24 x 1024 x 1536 17.4 and 16.3, but 24 x 1024 x 1024 13.7
+    and 14.6; few rows of a large matrix are bound by splitting it: 64 x 8192 x 1024 34 and 37, 100 x 8192 x 1024 45 and 38.  A short K where the library has a wave
+    of work: 300 x 1024 x 384 12.4 and 13.5, 1024 x 1024 x 384 20 and 15.5; 300 x 3072 x 128 9.8 and 10.3, 2048 x 1024 x 128 15.4 and 13.3."""
     if K >= 768:
-        return M >= 40 or N <= 8192
-    return M * N >= (400000 if K >= 512 else 800000)
+        return M >= 100 or (N <= 6144 and (M >= 40 or K >= 1536))
+    return M >= 100 and M * N >= (800000 if K >= 192 else 1500000)
 
 
 @functools.lru_cache(maxsize=4096)
@@ -90,8 +89,8 @@ def _plan(M, N, K, splits, n_sm=148):
 @functools.lru_cache(maxsize=4096)
 def _plan_f32(M, N, K, splits, n_sm=148):
     """(tile, ranges of K) of a float32 product: steps of 64 values stage three parts of 128 + tile rows, about 5.5 ns a row and step; 5 us around them.
-    Ranges cost a summing launch, about 3 us and their traffic.  300 x 6144 x 1024: 36 us as 128 x 128 tiles, 48 us as 128 x 64.  CTA pairs (tile 256), whose accumulators
-    leave no room for a second set, are only run when asked for: 2048 x 2048 x 6144 287 us as 128 x 128 tiles, 386 us as pairs."""
+    Ranges cost a summing launch, about 3 us and their traffic.  300 x 6144 x 1024: 39 us as 128 x 128 tiles, 52 us as 128 x 64.  CTA pairs (tile 256), whose accumulators
+    leave no room for a second set, are only run when asked for: 2048 x 2048 x 6144 299 us as 128 x 128 tiles, 420 us as pairs."""
     tm, kb = -(-M // 128), -(-K // 64)
 
     def cost(tile, s):
@@ -175,7 +174,7 @@ class Linear:
         if tile == 0:
             tile, splits = _plan_f32(M, band, self.K, 1 if act is not None else splits)
         splits = splits or 1
-        scratch = torch.empty((M + band, 3 * -(-self.K // 64) * 64), dtype=torch.bfloat16, device=x.device)
+        scratch = torch.empty((M + band) * (192 * -(-self.K // 64) + 2), dtype=torch.bfloat16, device=x.device)
         part = torch.empty(splits * M * ((band + 3) // 4 * 4), dtype=torch.float32, device=x.device) if splits > 1 else None
         _lib.mcall("scmx_gemm_f32", _lib.ptr(x), _ld(x), _lib.ptr(self.w), self.w.shape[1], M, self.N, self.K, act.code if act else 0,
                    act.a_pos if act else 0.0, act.a_neg if act else 0.0, _lib.ptr(y), _round8(nout), tile, splits, band, _lib.ptr(part), _lib.ptr(scratch),

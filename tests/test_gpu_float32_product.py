@@ -1,5 +1,5 @@
 """GPU: float32 products of portions where they differ from a plain product: weights that change after the layer was built, weights taken in bands,
-errors that have a sign."""
+errors that have a sign, rows at the ends of the number range."""
 import pytest
 import torch
 
@@ -61,3 +61,23 @@ def test_error_has_little_sign(X, K, positive, tile):      # noqa: F811
     with X._full_float32():
         assert rel(y, want) <= rel(x @ w.T, want)
     assert abs(float(((y.double() - want) * want).sum() / (want * want).sum())) < 1.5e-7
+
+
+@pytest.mark.parametrize("tile,splits", [(64, 1), (128, 3), (256, 1)])
+@pytest.mark.parametrize("K", [301, 1028])
+def test_scale_of_rows(X, K, tile, splits):      # noqa: F811
+    """Rows of any size, to the ends of the number range, keep the precision of ordinary ones; the smallest results are off by a unit of the subnormal grid."""
+    g = torch.Generator("cuda").manual_seed(K)
+    x, w = torch.randn(160, K, generator=g, device="cuda"), torch.randn(200, K, generator=g, device="cuda")
+    x *= torch.logspace(-37.5, 37.5, 160, device="cuda")[:, None]
+    w *= torch.logspace(-37.5, 37.5, 200, device="cuda")[torch.randperm(200, generator=g, device="cuda")][:, None]
+    x[7], w[9] = x[7].sign() * 2.0 ** -141, 0.0      # subnormal numbers, zeros
+    x[8, 1:] = 0.0
+    want, y = x.double() @ w.double().T, X.Linear(w)(x, tile=tile, splits=splits)
+    top = torch.finfo(F32).max
+    scale = x.double().norm(dim=1)[:, None] * w.double().norm(dim=1)[None] / K ** 0.5      # of a typical sum of the row and column
+    far = ((y.double() - want).abs() - splits * 2.0 ** -149) / scale.clamp(min=1e-300)
+    ok = (want.abs() < 0.5 * top) & (scale < 0.01 * top)      # ranges of K are summed, so parts of a sum near the end may pass it
+    assert float(far[ok].max()) < 5e-6 and ok.float().mean() > 0.4
+    over = y[want.abs() > 2 * top]
+    assert (over.isinf() if splits == 1 else ~over.isfinite()).all() and (y[:, 9] == 0).all()
