@@ -12,7 +12,8 @@
 // Structure of gemm_bf16 (TMA producer warp, one MMA-issuing thread, 8 epilogue warps, two accumulators, persistent tiles; CTA pairs with
 // tile 256).  A stage holds the three parts of 64 values of both operands: six products use every part loaded twice.  The parts are
 // written by a kernel before.
-// Infinities and not-a-number values make a sum not a number here; such outputs are computed once more by plain multiply-adds on the float32 operands.
+// Infinities and not-a-number values make a sum not a number here.  That is the answer where a row of either operand has a not-a-number value; the
+// others are computed once more by plain multiply-adds on the float32 operands, 32 outputs of a row together.
 #include "mix_tc.cuh"
 
 namespace scmx {
@@ -27,6 +28,7 @@ struct GfArgs {
     const float *A, *W;          // the operands themselves
     int64_t lda, ldw;
     const int32_t *ea, *ew;      // exponents of their rows
+    int vec;                     // their rows start on 16 bytes
     float* out;
     int64_t ldo;
     int splits;                  // > 1: range s of K goes to out + s * split_stride (no activation)
@@ -35,7 +37,7 @@ struct GfArgs {
     uint64_t wait_ns;
 };
 
-constexpr int GF_CHUNK = 1;                            // blocks of 64 values per accumulator (300 x 6144 x 1024: 35 us with 4, 36 us with 1)
+constexpr int GF_CHUNK = 1;                            // blocks of 64 values per accumulator (300 x 6144 x 1024: 1 us more than with 4)
 constexpr int GF_PITCH = 80;                           // staged row of 16 outputs; conflict-free 16-byte stores
 constexpr int GF_STAGE_WARP = 32 * GF_PITCH;
 
@@ -88,7 +90,8 @@ __device__ __forceinline__ uint32_t row_top(const float* x, int K, int at, int s
     }
     return m;
 }
-// Its exponent, of subnormal numbers too; 0 for zero, infinities and not-a-number values.
+// Its exponent, of subnormal numbers too; 0 for zero, infinities and not-a-number values.  GF_NAN stands for the last in a row's entry.
+constexpr int GF_NAN = 1 << 16;
 __device__ __forceinline__ int top_exponent(uint32_t m) {
     if (m == 0 || m >= 0x7F800000u) return 0;
     return m >= 0x00800000u ? (int)(m >> 23) - 127 : 31 - __clz((int)m) - 149;
@@ -128,7 +131,7 @@ __global__ void __launch_bounds__(256) split3_kernel(const SplitRows a, const Sp
     }
     if (!on) return;
     const int exp = top_exponent(m);
-    if (at == 0) s.e[r] = exp;
+    if (at == 0) s.e[r] = m > 0x7F800000u ? GF_NAN : exp;
     bf16_t* o = s.out + r * 3 * kp;
     if (s.vec) split_row<4>(x, K, kp, o, at, 32 * team, exp);      // the row once more, from L1 or L2
     else split_row<2>(x, K, kp, o, at, 32 * team, exp);
@@ -166,12 +169,42 @@ __device__ __forceinline__ void gf_scale(float* s, int ea, int ew) {
     }
 }
 
-// One output by multiply-adds over values [k0, k1).
-__device__ __noinline__ float gf_dot(const GfArgs& a, int row, int col, int k0, int k1) {
-    const float *x = a.A + (int64_t)row * a.lda, *w = a.W + (int64_t)col * a.ldw;
-    float s = 0.0f;
-    for (int k = k0; k < k1; ++k) s = fmaf(x[k], w[k], s);
-    return s;
+// Four values of a row from k on, zero from k1 on.
+__device__ __forceinline__ float4 gf_four(const float* x, int k, int k1, int vec) {
+    if (vec && k + 4 <= k1) return *reinterpret_cast<const float4*>(x + k);
+    return make_float4(k < k1 ? x[k] : 0.0f, k + 1 < k1 ? x[k + 1] : 0.0f, k + 2 < k1 ? x[k + 2] : 0.0f, k + 3 < k1 ? x[k + 3] : 0.0f);
+}
+// Outputs col0 .. col0 + 31 of this lane's row by multiply-adds over values [k0, k1), run by whole warps that hold a sum which is not a number.  16 values of the 32
+// weight rows at a time in the warp's staging area (ws); a chain of scalar loads for every output took a hundred times as long.
+__device__ __noinline__ void gf_dots(const GfArgs& a, int row, int col0, int k0, int k1, float4* ws, float* out) {
+    const int lane = threadIdx.x & 31, piece = 4 * (lane & 3);
+    const float* x = a.A + (int64_t)min(row, a.M - 1) * a.lda;
+    float s[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) s[j] = 0.0f;
+#pragma unroll 1
+    for (int k = k0; k < k1; k += 16) {
+        float4 q[4], w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            w[i] = gf_four(a.W + (int64_t)min(col0 + 8 * i + (lane >> 2), a.N - 1) * a.ldw, k + piece, k1, a.vec);
+            q[i] = gf_four(x, k + 4 * i, k1, a.vec);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) ws[32 * i + lane] = w[i];
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+                const float4 u = ws[4 * j + i];
+                s[j] = fmaf(q[i].x, u.x, s[j]); s[j] = fmaf(q[i].y, u.y, s[j]); s[j] = fmaf(q[i].z, u.z, s[j]); s[j] = fmaf(q[i].w, u.w, s[j]);
+            }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < 32; ++j) out[j] = s[j];
 }
 
 template <int BN_, bool PAIR>
@@ -327,10 +360,10 @@ __device__ __forceinline__ void gemm_f32_body(const CUtensorMap& tmA, const CUte
             const int sp = t / per_split, tt = t - sp * per_split, nt = tt / tiles_m, mt = tt - nt * tiles_m;
             const int kb0 = first_kb(sp), kb1 = first_kb(sp + 1);
             const int n0 = nt * BN + chalf * COLS, row0 = mt * TM_ROWS + (int)rank * BM + 32 * q;
-            const int ea = row0 + lane < a.M ? a.ea[row0 + lane] : 0;
+            const int ea = row0 + lane < a.M ? a.ea[row0 + lane] : GF_NAN;      // rows and columns that do not exist need no repair
             int ew[COLS / 32];
 #pragma unroll
-            for (int c = 0; c < COLS / 32; ++c) ew[c] = n0 + 32 * c + lane < a.N ? a.ew[n0 + 32 * c + lane] : 0;
+            for (int c = 0; c < COLS / 32; ++c) ew[c] = n0 + 32 * c + lane < a.N ? a.ew[n0 + 32 * c + lane] : GF_NAN;
             float sum[COLS];
 #pragma unroll
             for (int j = 0; j < COLS; ++j) sum[j] = 0.0f;
@@ -362,14 +395,19 @@ __device__ __forceinline__ void gemm_f32_body(const CUtensorMap& tmA, const CUte
             }
             if (fail) break;
 #pragma unroll
-            for (int c = 0; c < COLS / 32; ++c) gf_scale(sum + 32 * c, ea, ew[c]);
-            bool bad = false;
+            for (int c = 0; c < COLS / 32; ++c) {
+                const uint32_t cols = __ballot_sync(0xffffffffu, ew[c] != GF_NAN);
+                bool bad = false;      // not a number although neither row has such a value
 #pragma unroll
-            for (int j = 0; j < COLS; ++j) bad |= sum[j] != sum[j];
-            if (bad && row0 + lane < a.M) {
+                for (int j = 0; j < 32; ++j) bad |= (cols >> j & 1) && sum[32 * c + j] != sum[32 * c + j];
+                gf_scale(sum + 32 * c, ea == GF_NAN ? 0 : ea, ew[c] == GF_NAN ? 0 : ew[c]);
+                if (__any_sync(0xffffffffu, bad && ea != GF_NAN)) {
+                    float t[32];
+                    gf_dots(a, row0 + lane, n0 + 32 * c, 64 * kb0, min(a.K, 64 * kb1), reinterpret_cast<float4*>(stg), t);
 #pragma unroll
-                for (int j = 0; j < COLS; ++j)
-                    if (sum[j] != sum[j] && n0 + j < a.N) sum[j] = gf_dot(a, row0 + lane, n0 + j, 64 * kb0, min(a.K, 64 * kb1));
+                    for (int j = 0; j < 32; ++j)
+                        if (sum[32 * c + j] != sum[32 * c + j]) sum[32 * c + j] = t[j];
+                }
             }
             __syncwarp();
             float* out = a.out + (int64_t)sp * a.split_stride;
@@ -498,6 +536,7 @@ extern "C" int scmx_gemm_f32(const float* A, int64_t lda, const float* W, int64_
     bf16_t *a3 = (bf16_t*)scratch, *w3 = a3 + M * 3 * kp;
     int32_t* e = (int32_t*)(w3 + (N < band ? N : band) * 3 * kp);
     a.ea = e; a.ew = e + M;
+    a.vec = lda % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
     for (int64_t n0 = 0; n0 < N; n0 += band) {
         const int64_t n = N - n0 < band ? N - n0 : band, ldp = (n + 3) / 4 * 4;
         float* o = out + (act == 2 ? n0 / 2 : n0);

@@ -65,7 +65,7 @@ F32_TC_MIN, F32_TC_MIN_K = 24, 128
 
 def _f32_tc(M, N, K):
     """Whether a float32 product of M >= F32_TC_MIN rows runs on tensor cores, both times in us (library, tensor cores with the split of both operands).
-    A long K: 100 x 1024 x 768 16.6 and 14.5, 300 x 6144 x 1024 84 and 39, 40 x 512 x 1024 14.2 and 13.3, 24 x 1024 x 1536 17.4 and 16.3, but 24 x 1024 x 1024 13.7
+    A long K: 100 x 1024 x 768 16.6 and 14.5, 300 x 6144 x 1024 84 and 40, 40 x 512 x 1024 14.2 and 13.3, 24 x 1024 x 1536 17.4 and 16.3, but 24 x 1024 x 1024 13.7
     and 14.6; few rows of a large matrix are bound by splitting it: 64 x 8192 x 1024 34 and 37, 100 x 8192 x 1024 45 and 38.  A short K where the library has a wave
     of work: 300 x 1024 x 384 12.4 and 13.5, 1024 x 1024 x 384 20 and 15.5; 300 x 3072 x 128 9.8 and 10.3, 2048 x 1024 x 128 15.4 and 13.3."""
     if K >= 768:
@@ -89,8 +89,8 @@ def _plan(M, N, K, splits, n_sm=148):
 @functools.lru_cache(maxsize=4096)
 def _plan_f32(M, N, K, splits, n_sm=148):
     """(tile, ranges of K) of a float32 product: steps of 64 values stage three parts of 128 + tile rows, about 5.5 ns a row and step; 5 us around them.
-    Ranges cost a summing launch, about 3 us and their traffic.  300 x 6144 x 1024: 39 us as 128 x 128 tiles, 52 us as 128 x 64.  CTA pairs (tile 256), whose accumulators
-    leave no room for a second set, are only run when asked for: 2048 x 2048 x 6144 299 us as 128 x 128 tiles, 420 us as pairs."""
+    Ranges cost a summing launch, about 3 us and their traffic.  300 x 6144 x 1024: 40 us as 128 x 128 tiles, 53 us as 128 x 64.  CTA pairs (tile 256), whose accumulators
+    leave no room for a second set, are only run when asked for: 2048 x 2048 x 6144 300 us as 128 x 128 tiles, 436 us as pairs."""
     tm, kb = -(-M // 128), -(-K // 64)
 
     def cost(tile, s):
