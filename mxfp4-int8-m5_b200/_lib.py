@@ -7,6 +7,7 @@ import ctypes
 import os
 
 import torch
+from torch.autograd import forward_ad
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libscmx.so")
@@ -221,6 +222,16 @@ def mcall(name, *args):
 def ptr(t):
     """Device pointer of a tensor (None -> NULL)."""
     return None if t is None else t.data_ptr()
+
+
+def unseen(*tensors):
+    """Whether torch would only multiply these tensors: no gradient is recorded, and no transform, mode, cast or tensor class sees the call.  A kernel that takes
+    the place of a torch operation is launched then; otherwise the operation runs."""
+    if torch.is_grad_enabled() and any(t.requires_grad for t in tensors):
+        return False
+    return not (torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack() or torch._C._are_functorch_transforms_active()
+                or forward_ad._current_level >= 0 or torch.is_autocast_enabled("cuda") or torch._C._get_tracing_state() is not None
+                or any(type(t) not in (torch.Tensor, torch.nn.Parameter) for t in tensors))
 
 
 def stream():

@@ -132,17 +132,13 @@ class Linear:
         out_dtype = out_dtype or self.w.dtype
         M = x.shape[0]
         assert x.shape[1] == self.K and x.dtype == self.w.dtype and x.is_cuda
-        if M == 1 and act is None and tile == 0 and self.K <= 6400 and self.N % 8 == 0 and x.is_contiguous() and x.data_ptr() % 16 == 0:
-            # one row (the logits of a prompt's last position) is a stream of the weights: 32000 x 2048 took 44 us as a tile of 128 rows, 25 us so
-            if self.dt == 1:
-                return self.vec(x.view(-1))[None]
-            if self.K % 8 == 0:
-                y = torch.empty((1, self.N), dtype=out_dtype, device=x.device)
-                _lib.mcall("scmx_gemv_bf16", _lib.ptr(self.w), self.w.shape[1], _lib.ptr(x), self.N, self.K, _lib.ptr(y), int(out_dtype == torch.float32),
-                           _lib.stream())
-                return y
         if self.dt == 1:
             return self._call_f32(x, act, tile, splits)
+        if M == 1 and act is None and tile == 0 and self.K % 8 == 0 and self._streams(x):
+            # one row (the logits of a prompt's last position) is a stream of the weights: 32000 x 2048 took 44 us as a tile of 128 rows, 25 us so
+            y = torch.empty((1, self.N), dtype=out_dtype, device=x.device)
+            _lib.mcall("scmx_gemv_bf16", _lib.ptr(self.w), self.w.shape[1], _lib.ptr(x), self.N, self.K, _lib.ptr(y), int(out_dtype == torch.float32), _lib.stream())
+            return y
         if _ld(x) % 8 or x.data_ptr() % 16:
             x = empty_rows(M, self.K, x.dtype, x.device).copy_(x)
         nout = self.N // 2 if act is not None and act.code == 2 else self.N
@@ -156,9 +152,16 @@ class Linear:
                    _lib.ptr(part), _lib.ptr(_lib.mixer_status_buffer()), _lib.stream())
         return y
 
+    def _streams(self, x):
+        return self.K <= 6400 and self.N % 8 == 0 and x.is_contiguous() and x.data_ptr() % 16 == 0
+
     def _call_f32(self, x, act, tile, splits):
-        M = x.shape[0]
-        if M < F32_TC_MIN or self.K < F32_TC_MIN_K or not (tile or _f32_tc(M, self.N, self.K)):
+        """torch's product, whatever the strides, with gradients and under transforms, unless one of the kernels gives the same sooner."""
+        M, unseen = x.shape[0], _lib.unseen(x, self.w)
+        if M == 1 and act is None and tile == 0 and unseen and self._streams(x):
+            return self.vec(x.view(-1))[None]
+        rows = unseen and x.stride(1) == 1 and x.stride(0) >= self.K
+        if not rows or M < F32_TC_MIN or self.K < F32_TC_MIN_K or not (tile or _f32_tc(M, self.N, self.K)):
             with _full_float32():
                 y = x @ self.w[:, :self.K].T
             if act is not None and act.code == 2:

@@ -1,5 +1,6 @@
 """GPU: float32 products of portions where they differ from a plain product: weights that change after the layer was built, weights taken in bands,
-errors that have a sign, rows at the ends of the number range, values that are not finite."""
+errors that have a sign, rows at the ends of the number range, values that are not finite, calls
+that torch's own product has to take."""
 import pytest
 import torch
 
@@ -105,3 +106,25 @@ def test_values_not_finite(X, K, tile, splits):      # noqa: F811
         b.record()
         b.synchronize()
         assert a.elapsed_time(b) < bound
+
+
+@pytest.mark.parametrize("M", [1, 2, 130])
+def test_forms_that_only_torch_takes(X, M):      # noqa: F811
+    """Columns first, rows that share memory, gradients, vmap, forward mode and autocast: the library's product, as before there was another."""
+    K, N = 1024, 96
+    w = torch.randn(N, K, device="cuda") * K ** -0.5
+    lin, tol = X.Linear(w), 2e-6
+    x = torch.randn(M, K, device="cuda")
+    want = x.double() @ w.double().T
+    assert rel(lin(x.T.contiguous().T), want) < tol
+    assert rel(lin(x[:1].expand(M, K)), want[:1].expand(M, N)) < tol
+    assert rel(torch.vmap(lambda r: lin(r[None])[0])(x), want) < tol
+    primal, tangent = torch.func.jvp(lambda t: lin(t), (x,), (x * 2,))
+    assert rel(primal, want) < tol and rel(tangent, 2 * want) < tol
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        assert lin(x).dtype == (x @ w.T).dtype
+    x.requires_grad_()
+    lin(x).sum().backward()
+    assert rel(x.grad, w.double().sum(0).expand(M, K)) < tol
+    with torch.no_grad():
+        assert rel(lin(x), want) < tol

@@ -6,6 +6,8 @@ import re
 
 import numpy as np
 import pytest
+import torch
+import torch.utils.flop_counter
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
@@ -138,3 +140,28 @@ def test_status_word_codes_have_texts(scmx):
         assert word in L.describe_status(code), code
     assert "grid barrier 3" in L.describe_status(103)
     assert L.describe_status(77) == "code 77"
+
+
+def test_calls_that_torch_has_to_see(scmx):
+    """A kernel takes the place of a torch operation only where nothing records, transforms or recasts it."""
+    unseen, x, w = scmx._lib.unseen, torch.randn(3), torch.nn.Parameter(torch.randn(3))
+    seen = []
+    assert unseen(x, x) and not unseen(x, w)
+    with torch.no_grad():
+        assert unseen(x, w)
+        torch.vmap(lambda t: seen.append(unseen(t)) or t)(x)
+        torch.func.jvp(lambda t: seen.append(unseen(t)) or t, (x,), (x,))
+        with torch.autograd.forward_ad.dual_level():
+            seen.append(unseen(x))
+        torch.set_autocast_enabled("cuda", True)      # as torch.autocast does where there is a GPU
+        seen.append(unseen(x))
+        torch.set_autocast_enabled("cuda", False)
+        with torch.utils.flop_counter.FlopCounterMode(display=False):
+            seen.append(unseen(x))
+        torch.jit.trace(lambda t: seen.append(unseen(t)) or t, x, check_trace=False)
+
+        class Own(torch.Tensor):
+            pass
+
+        seen.append(unseen(x.as_subclass(Own)))
+    assert seen == [False] * 7
