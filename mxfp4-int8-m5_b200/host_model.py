@@ -10,8 +10,11 @@ from dataclasses import dataclass
 
 import torch
 import torch.nn.functional as TF
+import torch.nn.modules.module as MODULE
 
 from . import sc_kernels as S
+
+_LINEAR_FORWARD = torch.nn.Linear.forward      # as torch defines it
 
 
 @dataclass
@@ -287,14 +290,16 @@ class CausalLM(torch.nn.Module):
         return TF.linear(h, self.model.embed_tokens.weight) if self.lm_head is None else self.lm_head(h)
 
     def head_weight(self):
-        """The output head's matrix, where `head` is nothing but a product with it, else None."""
-        if type(self).head is not CausalLM.head or "head" in self.__dict__:
+        """The output head's matrix, where `head` is nothing but a product with it, else None: replaced methods and hooks want the call."""
+        if type(self).head is not _HEAD or "head" in self.__dict__:
             return None
         lin = self.lm_head
         if lin is None:
             return self.model.embed_tokens.weight
-        plain = type(lin) is torch.nn.Linear and lin.bias is None and not (lin._forward_hooks or lin._forward_pre_hooks)
-        return lin.weight if plain else None
+        plain = type(lin) is torch.nn.Linear and lin.bias is None and torch.nn.Linear.forward is _LINEAR_FORWARD and "forward" not in lin.__dict__
+        hooks = (lin._forward_hooks or lin._forward_pre_hooks or lin._backward_hooks or lin._backward_pre_hooks or MODULE._global_forward_hooks
+                 or MODULE._global_forward_pre_hooks or MODULE._global_backward_hooks or MODULE._global_backward_pre_hooks)
+        return lin.weight if plain and not hooks else None
 
     def forward(self, ids, cache=None):
         """ids int [1, L] -> logits [1, L, V]; prefill into a fresh or offset cache."""
@@ -329,6 +334,9 @@ class CausalLM(torch.nn.Module):
             else:
                 p.copy_(sd[k].to(p.dtype))
         return self
+
+
+_HEAD = CausalLM.head      # as this file defines it
 
 
 # ---- hybrid decoders: every layer names its own mixer -------------------------------------------------------------------------

@@ -39,6 +39,20 @@ def test_own_heads_are_called(scmx):
         assert torch.equal(head(model)(h), h[..., :5])
 
 
+def test_gradient_of_one_position(scmx):
+    """Logits of one position carry a gradient where those of two do."""
+    HM = scmx.host_model
+    with torch.device("cuda"):
+        model = HM.CausalLM(HM.ModelArgs(256, 512, 1, 2, 2, 128, 1e-6, 1e4, 500, False))
+    model.lm_head.weight.requires_grad_()
+    head = scmx.sc_decode.head_product(model)
+    h = torch.randn(1, 1, 256, device="cuda").to(torch.bfloat16).requires_grad_()
+    head(h).float().sum().backward()
+    assert torch.equal(model.lm_head.weight.grad[7], h.detach()[0, 0]) and h.grad is not None
+    with torch.no_grad():
+        assert (head(h).float() - model.head(h).float()).abs().max() <= 2.0 ** -6 * model.head(h).float().abs().max()
+
+
 @pytest.mark.parametrize("N,K,dt", [(8, 8, torch.bfloat16), (32000, 1024, torch.bfloat16), (96, 6400, torch.bfloat16), (4096, 2048, torch.float32), (40, 100, torch.float32)])
 def test_one_row(scmx, N, K, dt):
     """Products of one row run as streams of the weights, in both output types and from the last row of a portion."""

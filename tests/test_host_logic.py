@@ -165,3 +165,41 @@ def test_calls_that_torch_has_to_see(scmx):
 
         seen.append(unseen(x.as_subclass(Own)))
     assert seen == [False] * 7
+
+
+@pytest.mark.parametrize("tied", [False, True])
+def test_heads_that_want_the_call(scmx, monkeypatch, tied):
+    """The head's matrix is handed out only while `head` is a product with it and nobody watches or replaces the call."""
+    HM = scmx.host_model
+    model = HM.CausalLM(HM.ModelArgs(256, 512, 1, 2, 2, 128, 1e-6, 1e4, 500, tied))
+    matrix = model.model.embed_tokens.weight if tied else model.lm_head.weight
+    assert model.head_weight() is matrix
+    with monkeypatch.context() as m:
+        m.setattr(HM.CausalLM, "head", lambda self, h: h)
+        assert model.head_weight() is None
+    with monkeypatch.context() as m:
+        m.setitem(model.__dict__, "head", lambda h: h)
+        assert model.head_weight() is None
+    if not tied:
+        with monkeypatch.context() as m:
+            m.setitem(model.lm_head.__dict__, "forward", lambda h: h)
+            assert model.head_weight() is None
+        with monkeypatch.context() as m:
+            m.setattr(torch.nn.Linear, "forward", lambda self, h: h)
+            assert model.head_weight() is None
+        nn = torch.nn.modules.module
+        for hook in (model.lm_head.register_forward_hook, model.lm_head.register_forward_pre_hook, nn.register_module_forward_hook, nn.register_module_forward_pre_hook,
+                     model.lm_head.register_full_backward_hook, nn.register_module_full_backward_hook):
+            handle = hook(lambda *a: None)
+            assert model.head_weight() is None, hook
+            handle.remove()
+    assert model.head_weight() is matrix
+    # and the product itself asks torch where a gradient, a transform or a mode would miss it
+    h, seen = torch.zeros(1, 1, 256, dtype=torch.bfloat16), []
+    monkeypatch.setitem(model.__dict__, "head", lambda t: seen.append(t.requires_grad) or t)
+    monkeypatch.setattr(model, "head_weight", lambda: matrix)
+    product = scmx.sc_decode.head_product(model)
+    product(h)                                  # the weight may want a gradient
+    with torch.no_grad():
+        torch.vmap(product)(h[None])
+    assert len(seen) == 2
