@@ -24,6 +24,8 @@ from . import sc_format as F
 from . import sc_kernels as S
 from .w4a8 import PackedWeight
 
+_SDPA = HM.sdpa      # the attention that this file may read head by head; any other, HM.sdpa replaced included, is called
+
 GROUPS = {"qkv": ["self_attn.q_proj", "self_attn.k_proj", "self_attn.v_proj"], "o": ["self_attn.o_proj"],
           "gu": ["mlp.gate_proj", "mlp.up_proj"], "down": ["mlp.down_proj"]}
 
@@ -65,7 +67,7 @@ def load_packed(cache_path, n_layers, fmt=F.DEFAULT):
 def attend_quant(sdpa, q, k, v, scale, Mp):
     """INT8 rows of the attention output.  Where torch leaves it head by head, the heads are read as column segments of the rows: the transposing
     copy before it took 18 us of a layer of 16 heads at 4096 tokens, 4.7 us at 333."""
-    (hq, L, d), heads = q.shape, sdpa is HM.sdpa
+    (hq, L, d), heads = q.shape, sdpa is _SDPA
     o = HM.sdpa_heads(q, k, v, scale, True) if heads else sdpa(q, k, v, scale, True)
     if heads and o.is_contiguous() and d % 8 == 0 and hq * d <= 8192:
         return S.act_quant_seg(o, Mp)

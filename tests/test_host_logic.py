@@ -203,3 +203,16 @@ def test_heads_that_want_the_call(scmx, monkeypatch, tied):
     with torch.no_grad():
         torch.vmap(product)(h[None])
     assert len(seen) == 2
+
+
+def test_replaced_attention_is_called(scmx, monkeypatch):
+    """A prompt's attention is read head by head only where it is this library's own function."""
+    HM, S = scmx.host_model, scmx.sc_kernels
+    monkeypatch.setattr(S, "act_quant", lambda x, rows: x)
+    monkeypatch.setattr(S, "act_quant_seg", lambda x, rows: x.transpose(0, 1).reshape(x.shape[1], -1))
+    q, answer = torch.randn(2, 3, 8), torch.randn(3, 16)
+    assert torch.allclose(scmx.fused_qwen3.attend_quant(HM.sdpa, q, q, q, 1.0, 128), HM.sdpa(q, q, q, 1.0, True))
+    own = lambda *a: answer      # noqa: E731
+    assert scmx.fused_qwen3.attend_quant(own, q, q, q, 1.0, 128) is answer
+    monkeypatch.setattr(HM, "sdpa", own)
+    assert scmx.fused_qwen3.attend_quant(HM.sdpa, q, q, q, 1.0, 128) is answer
