@@ -244,6 +244,18 @@ def require_cuda(*tensors):
             raise TypeError("expected contiguous CUDA tensors; this package has no CPU path")
 
 
+_sms = {}
+
+
+def sm_count():
+    """Multiprocessors of the current device, which the tile plans count waves of (the kernels' launches ask the same)."""
+    dev = torch._C._cuda_getDevice()
+    n = _sms.get(dev)
+    if n is None:
+        n = _sms[dev] = torch.cuda.get_device_properties(dev).multi_processor_count
+    return n
+
+
 _status = {}
 
 

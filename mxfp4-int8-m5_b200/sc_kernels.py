@@ -105,7 +105,7 @@ def _rmsnorm_quant(x, w, eps, Mp, want_n):
 
 
 @functools.lru_cache(maxsize=4096)
-def _ranges(M, N, K, n_sm=148):
+def _ranges(M, N, K, n_sm):
     """Ranges of K for a dense product whose 128 x 128 tiles leave most SMs idle.  Summing the ranges costs a launch of 3 us and their traffic,
     which only a long K repays: 256 x 2048 x 6144 takes 18.2 us in one piece and 12.7 us in four, 128 x 1024 x 3072 10.9 and 8.6 us, but
     256 x 2048 x 2048 9.0 and 9.4 us in two."""
@@ -113,7 +113,7 @@ def _ranges(M, N, K, n_sm=148):
 
 
 def _mm_i8(xq, wq, M, N, K, epi, xscale, wscale, res, out, splits=None):
-    splits = splits or (_ranges(M, N, K) if wscale is None or wscale.data_ptr() % 16 == 0 else 1)
+    splits = splits or (_ranges(M, N, K, _lib.sm_count()) if wscale is None or wscale.data_ptr() % 16 == 0 else 1)
     head = (_lib.ptr(xq), _lib.ptr(wq), M, N, K, epi, _lib.ptr(xscale), _lib.ptr(wscale), _lib.ptr(res), _lib.ptr(out))
     if splits > 1:
         part = torch.empty((splits, M, N), dtype=torch.int32, device=xq.device)

@@ -74,7 +74,7 @@ def _f32_tc(M, N, K):
 
 
 @functools.lru_cache(maxsize=4096)
-def _plan(M, N, K, splits, n_sm=148):
+def _plan(M, N, K, splits, n_sm):
     """(tile, ranges of K computed side by side) for a product with few output tiles: 4 us and 0.27 us for every step of 64 values that a CTA walks
     (77 x 4096 x 1024: 8.4 us, 77 x 1024 x 3072: 16.9 us), counting whole waves; summing ranges costs a launch, 2 us, and the traffic of
     the partial products (77 x 4096 x 1024 in three: 10 us, 77 x 1024 x 3072: 10.1 us).  (0, 1): leave it to the kernel."""
@@ -87,7 +87,7 @@ def _plan(M, N, K, splits, n_sm=148):
 
 
 @functools.lru_cache(maxsize=4096)
-def _plan_f32(M, N, K, splits, n_sm=148):
+def _plan_f32(M, N, K, splits, n_sm):
     """(tile, ranges of K) of a float32 product: steps of 64 values stage three parts of 128 + tile rows, about 5.5 ns a row and step; 5 us around them.
     Ranges cost a summing launch, about 3 us and their traffic.  300 x 6144 x 1024: 40 us as 128 x 128 tiles, 53 us as 128 x 64.  CTA pairs (tile 256), whose accumulators
     leave no room for a second set, are only run when asked for: 2048 x 2048 x 6144 300 us as 128 x 128 tiles, 436 us as pairs."""
@@ -144,7 +144,7 @@ class Linear:
         nout = self.N // 2 if act is not None and act.code == 2 else self.N
         y = empty_rows(M, nout, out_dtype, x.device)
         if tile == 0:
-            tile, splits = _plan(M, self.N, self.K, 1 if act is not None else splits)
+            tile, splits = _plan(M, self.N, self.K, 1 if act is not None else splits, _lib.sm_count())
         splits = splits or 1
         part = torch.empty(splits * M * ((self.N + 3) // 4 * 4), dtype=torch.float32, device=x.device) if splits > 1 else None
         _lib.mcall("scmx_gemm_bf16", _lib.ptr(x), _ld(x), _lib.ptr(self.w), self.w.shape[1], M, self.N, self.K, act.code if act else 0,
@@ -175,7 +175,7 @@ class Linear:
         y = empty_rows(M, nout, torch.float32, x.device)
         band = _band(self.N, self.K)
         if tile == 0:
-            tile, splits = _plan_f32(M, band, self.K, 1 if act is not None else splits)
+            tile, splits = _plan_f32(M, band, self.K, 1 if act is not None else splits, _lib.sm_count())
         splits = splits or 1
         scratch = torch.empty((M + band) * (192 * -(-self.K // 64) + 2), dtype=torch.bfloat16, device=x.device)
         part = torch.empty(splits * M * ((band + 3) // 4 * 4), dtype=torch.float32, device=x.device) if splits > 1 else None

@@ -216,3 +216,25 @@ def test_replaced_attention_is_called(scmx, monkeypatch):
     assert scmx.fused_qwen3.attend_quant(own, q, q, q, 1.0, 128) is answer
     monkeypatch.setattr(HM, "sdpa", own)
     assert scmx.fused_qwen3.attend_quant(HM.sdpa, q, q, q, 1.0, 128) is answer
+
+
+def test_plans_count_the_device(scmx, monkeypatch):
+    """Tiles and ranges of K are planned for the current device's multiprocessors, also after another device has been asked about."""
+    L, S, X = scmx._lib, scmx.sc_kernels, scmx.sc_mixers
+
+    class Of:
+        def __init__(self, dev):
+            self.multi_processor_count = (148, 20)[dev]
+
+    dev = [0]
+    monkeypatch.setattr(L, "_sms", {})
+    monkeypatch.setattr(torch._C, "_cuda_getDevice", lambda: dev[0])
+    monkeypatch.setattr(torch.cuda, "get_device_properties", Of)
+    plans = lambda: (S._ranges(256, 2048, 6144, L.sm_count()), X._plan(77, 1024, 3072, None, L.sm_count()), X._plan_f32(77, 1024, 3072, None, L.sm_count()))      # noqa: E731
+    large = plans()
+    assert large[0] == 4 and large[1][1] > 1 and large[2][1] > 1
+    dev[0] = 1
+    small = plans()
+    assert small[0] == 1 and small[1] != large[1] and small[2] != large[2]
+    dev[0] = 0
+    assert plans() == large
