@@ -153,15 +153,15 @@ int scmx_gemm_f32(const float* A, int64_t lda, const float* W, int64_t ldw, int6
  * Rows of W are zero padded to a multiple of 8 columns. */
 int scmx_gemv_x(const void* W, int64_t ldw, int dt, const float* x, int64_t N, int64_t K, int epi, float a_pos, float a_neg,
                 const float* conv_w, const float* conv_b, float* tail, int C, int taps, float* out, void* stream);
-/* A bfloat16 row x [K] (K a multiple of 8 up to 6400, 16-byte aligned) times bfloat16 W -> out [N], bfloat16 or float. */
-int scmx_gemv_bf16(const void* W, int64_t ldw, const void* x, int64_t N, int64_t K, void* out, int out_f32, void* stream);
-/* The same for an input row that is left in parts (K <= 2048, a multiple of 4; rows 16-byte aligned).  pro 1: r = x + mult y (y may be NULL), input r / rms(r) nw;
+/* scmx_gemv_x for an input row that is left in parts (K <= 2048, a multiple of 4; rows 16-byte aligned).  pro 1: r = x + mult y (y may be NULL), input r / rms(r) nw;
  * pro 2: r = x + nw y / rms(y); with n > 0 r goes to row n - 1 of the store (keep) and r = sum dwa[j] store[j] + dwa[n - 1] r; input r, or
  * r / rms(r) fw.  x_out receives r: another buffer than x and y. */
 int scmx_gemv_x_row(const void* W, int64_t ldw, int dt, const float* x, const float* y, const float* nw, int pro, float mult, float eps,
                     float* store, int64_t store_stride, const float* dwa, int n, int keep, const float* fw, float* x_out, int64_t N,
                     int64_t K, int epi, float a_pos, float a_neg, const float* conv_w, const float* conv_b, float* tail, int C, int taps,
                     float* out, void* stream);
+/* A bfloat16 row x [K] (K a multiple of 8 up to 6400, 16-byte aligned) times bfloat16 W -> out [N], bfloat16 or float. */
+int scmx_gemv_bf16(const void* W, int64_t ldw, const void* x, int64_t N, int64_t K, void* out, int out_f32, void* stream);
 
 #ifdef __cplusplus
 }

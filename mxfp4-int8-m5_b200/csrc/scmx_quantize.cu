@@ -230,8 +230,8 @@ __device__ __forceinline__ uint32_t e2m1_codes(const float (&t)[8]) {
     return w & (nz | 0x77777777u);
 }
 
-template <typename T> struct Raw8;      // eight elements as loaded
-template <> struct Raw8<float> {
+template <typename T> struct QuantRaw;      // eight elements as loaded
+template <> struct QuantRaw<float> {
     float4 a, b;
     __device__ __forceinline__ void load(const float* p) {
         a = reinterpret_cast<const float4*>(p)[0];
@@ -242,7 +242,7 @@ template <> struct Raw8<float> {
         x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
     }
 };
-template <> struct Raw8<uint16_t> {
+template <> struct QuantRaw<uint16_t> {
     uint4 w;
     __device__ __forceinline__ void load(const uint16_t* p) { w = *reinterpret_cast<const uint4*>(p); }
     __device__ __forceinline__ void zero() { w = make_uint4(0, 0, 0, 0); }
@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(1024) quantize_vec_kernel(const T* __restrict_
     __shared__ int red[2][2][32];
     const int tid = threadIdx.x;
     const bool in = tid < K / 8;
-    Raw8<T> raw;
+    QuantRaw<T> raw;
     raw.zero();
     if (in) raw.load(w + (int64_t)blockIdx.x * K + 8 * tid);
     int turn = 0;
@@ -384,7 +384,7 @@ __global__ void __launch_bounds__(1024) quantize_long_kernel(const T* __restrict
     const T* wr = w + n * K;
     int hi = INT_MIN, low = INT_MAX;
     float x[8];
-    Raw8<T> raw;
+    QuantRaw<T> raw;
     for (int v = tid; v - tid < nv; v += 1024) {
         raw.zero();
         if (v < nv) raw.load(wr + 8 * (int64_t)v);

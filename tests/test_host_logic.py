@@ -1,6 +1,7 @@
 """CPU: host-side logic of the package (layout helpers, Format checks), the C-ABI library's exports, and the
 argument validation every entry point performs before touching the GPU."""
 import ctypes
+import importlib.util
 import os
 import re
 
@@ -238,3 +239,15 @@ def test_plans_count_the_device(scmx, monkeypatch):
     assert small[0] == 1 and small[1] != large[1] and small[2] != large[2]
     dev[0] = 0
     assert plans() == large
+
+
+def test_structures_are_defined_once(scmx):
+    """The sources of one library share a namespace, so a structure of the same name in two of them would be two definitions of one class."""
+    spec = importlib.util.spec_from_file_location("scmx_build", os.path.join(ROOT, "mxfp4-int8-m5_b200", "build.py"))
+    build = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(build)
+    for which in build.LIBS:
+        where = {}
+        for path in set(build._deps(which)):
+            for name in set(re.findall(r"^\s*(?:template <[^>]*>\s*)?struct (\w+)(?:<[^;{]*>)?\s*\{", open(path).read(), re.M)):
+                assert where.setdefault(name, path) == path, (name, path, where[name])
