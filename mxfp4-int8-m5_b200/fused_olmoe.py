@@ -59,9 +59,11 @@ def pack_olmoe(model, cache_path=None, fmt=F.DEFAULT, on_device=False):
 
 class FusedOlmoe:
     def __init__(self, model, flat, tile_gu=None, tile_d=None, bk=None, two_pass="auto", sort="count", compiled=True):
-        """model: host_model.CausalLM (num_experts > 0) on the GPU; flat: pack_olmoe's dict.  two_pass=True decodes all
-        experts to INT8 once per call and runs the grouped GEMM on that (moe_mm_i8); "auto": once the average expert has
-        >= 256 rows (e2e/fused_olmoe.py:135-141).  The tile arguments are Metal tuning hints: accepted and ignored."""
+        """model: host_model.CausalLM (num_experts > 0) on the GPU; flat: pack_olmoe's dict.  Prompts whose average expert has fewer than
+        MoeBlock.FUSED_BELOW (480) rows run the grouped GEMMs on the packed weights; from there on, and with two_pass=True, the experts are decoded to INT8
+        first (moe_mm_i8): a layer ahead into two buffers kept for that where they fit (below), else once per call with two_pass=True or "auto" at >= 256 rows per
+        expert (e2e/fused_olmoe.py:135-141), in groups otherwise.  Formats, widths or numbers of experts that the packed-weight kernel does not take are
+        decoded at any length.  The tile arguments are Metal tuning hints: accepted and ignored."""
         assert sort == "count"
         self.model, self.args = model, model.args
         a = self.args
@@ -99,7 +101,7 @@ class FusedOlmoe:
                 setattr(layer.self_attn, path.split(".")[1], None)
             layer.mlp.switch_mlp = None
         # Expert weights of the NEXT layer are decoded to INT8 on a side stream while the current layer runs (two rotating
-        # buffer pairs), when the INT8 copy of one layer's experts is at most 1 GiB; the grouped GEMMs then read those
+        # buffer pairs, held from the start), when the INT8 copy of one layer's experts is at most 1 GiB; the grouped GEMMs of long prompts then read those
         # (moe_mm_i8).  Otherwise moe_mm decodes groups of experts between its own GEMM passes.
         F2, D = 2 * Fi, a.hidden_size
         self.prefetch = E * (F2 * D + D * Fi) <= (1 << 30)
@@ -135,7 +137,8 @@ class FusedOlmoe:
         """Whether the grouped GEMMs read the packed weights (scmx_moe_mm_w4) although the experts could be decoded ahead: MoeBlock's
         rule.  An expert's INT8 copy costs three passes over its bytes, which few rows do not repay: two layers of 64 experts of
         2048 x 1024 at 128 rows per expert take 592 us with the rest of a prompt against 765 us, the bits being the same."""
-        return (self.two_pass is not True and M_.FUSED_UNPACK and R // self.args.num_experts < MoeBlock.FUSED_BELOW and self.args.num_experts <= 512
+        asked = self.two_pass and self.two_pass != "auto"      # two passes at any length
+        return (not asked and M_.FUSED_UNPACK and R // self.args.num_experts < MoeBlock.FUSED_BELOW and self.args.num_experts <= 512
                 and all(_lib.lib().scmx_w4_supported(F.DEFAULT.c_struct(), k) for k in (self.args.hidden_size, self.args.intermediate_size)))
 
     def _decode_experts(self, i):

@@ -251,3 +251,12 @@ def test_structures_are_defined_once(scmx):
         for path in set(build._deps(which)):
             for name in set(re.findall(r"^\s*(?:template <[^>]*>\s*)?struct (\w+)(?:<[^;{]*>)?\s*\{", open(path).read(), re.M)):
                 assert where.setdefault(name, path) == path, (name, path, where[name])
+
+
+def test_two_passes_on_request(scmx):
+    """A mixture's prompts of few rows per expert run on packed weights unless two passes are asked for, by any true value."""
+    fused = scmx.fused_olmoe.FusedOlmoe.__new__(scmx.fused_olmoe.FusedOlmoe)
+    fused.args = scmx.host_model.ModelArgs(2048, 1024, 1, 16, 16, 128, num_experts=64, num_experts_per_tok=8)
+    for two_pass, packed in (("auto", True), (False, True), (True, False), (1, False), (np.True_, False)):
+        fused.two_pass = two_pass
+        assert fused._packed(64 * 479) is packed and not fused._packed(64 * 480)
