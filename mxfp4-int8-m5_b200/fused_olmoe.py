@@ -127,9 +127,10 @@ class FusedOlmoe:
         return M_.router_topk(logits.float(), self.args.num_experts_per_tok)
 
     def route_token(self, layer, xn):
-        """route for one row, in one kernel where the sizes allow."""
+        """route for one row, in one kernel where the sizes allow and `route` is this class's own."""
         w = layer.mlp.gate.weight
-        if w.dtype == xn.dtype == torch.bfloat16 and w.is_contiguous() and w.shape[1] % 8 == 0 and w.shape[0] <= 1024 and w.data_ptr() % 16 == 0:
+        own = type(self).route is _ROUTE and "route" not in self.__dict__
+        if own and w.dtype == xn.dtype == torch.bfloat16 and w.is_contiguous() and w.shape[1] % 8 == 0 and w.shape[0] <= 1024 and w.data_ptr() % 16 == 0:
             return M_.route_token(xn, w, self.args.num_experts_per_tok)
         return self.route(layer, xn, 1)
 
@@ -241,3 +242,6 @@ class FusedOlmoe:
 
 def load_fused_olmoe(model, cache_path=None, **kw):
     return FusedOlmoe(model, pack_olmoe(model, cache_path), **kw)
+
+
+_ROUTE = FusedOlmoe.route      # as this file defines it

@@ -260,3 +260,27 @@ def test_two_passes_on_request(scmx):
     for two_pass, packed in (("auto", True), (False, True), (True, False), (1, False), (np.True_, False)):
         fused.two_pass = two_pass
         assert fused._packed(64 * 479) is packed and not fused._packed(64 * 480)
+
+
+def test_replaced_router_is_called(scmx, monkeypatch):
+    """A decode step asks a `route` that was replaced on the object, in a subclass or in the class, not the kernel for one token."""
+    FO = scmx.fused_olmoe
+    monkeypatch.setattr(scmx.sc_moe, "route_token", lambda xn, w, k: "kernel")
+
+    class Own(FO.FusedOlmoe):
+        def route(self, layer, xn, M):
+            return "own"
+
+    class Layer:
+        class mlp:
+            gate = torch.nn.Linear(64, 8, bias=False, dtype=torch.bfloat16)
+
+    plain, own = (c.__new__(c) for c in (FO.FusedOlmoe, Own))
+    plain.args = own.args = scmx.host_model.ModelArgs(64, 128, 1, 1, 1, 64, num_experts=8, num_experts_per_tok=2)
+    xn = torch.zeros(1, 64, dtype=torch.bfloat16)
+    assert plain.route_token(Layer, xn) == "kernel" and own.route_token(Layer, xn) == "own"
+    plain.route = lambda layer, xn, M: "object"
+    assert plain.route_token(Layer, xn) == "object"
+    del plain.route
+    monkeypatch.setattr(FO.FusedOlmoe, "route", lambda self, layer, xn, M: "class")
+    assert plain.route_token(Layer, xn) == "class"
