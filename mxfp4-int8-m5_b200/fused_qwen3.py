@@ -165,7 +165,8 @@ class FusedQwen3:
     def _attention(self, i, at, c, src, xs, ws, L, Mp):
         """-> attention output (None unless it is recorded), its INT8 rows and their scales."""
         q, k, v = self._qkv(at, c, src, xs, ws, L)
-        if self.rot is True or (self.record is not None and i in self.record_layers):
+        own = type(self).act_q is not _ACT_Q or "act_q" in self.__dict__      # a quantizer of the caller's: it wants whole rows
+        if own or self.rot is True or (self.record is not None and i in self.record_layers):
             o = self.sdpa(q, k, v, at.scale, True)
             return (o, *self.act_q(o, Mp))
         return (None, *attend_quant(self.sdpa, q, k, v, at.scale, Mp))
@@ -264,3 +265,6 @@ def load_fused(model, cache_path=None, **kw):
     """Packs (or loads the cached pack of) a host_model.CausalLM and wraps it (e2e/fused_qwen3.py:312-337 without the
     checkpoint download)."""
     return FusedQwen3(model, pack_model(model, cache_path), **kw)
+
+
+_ACT_Q = FusedQwen3.act_q      # as this file defines it

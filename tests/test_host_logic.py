@@ -284,3 +284,28 @@ def test_replaced_router_is_called(scmx, monkeypatch):
     del plain.route
     monkeypatch.setattr(FO.FusedOlmoe, "route", lambda self, layer, xn, M: "class")
     assert plain.route_token(Layer, xn) == "class"
+
+
+def test_replaced_quantizer_is_called(scmx, monkeypatch):
+    """The attention output of a prompt goes to an `act_q` that was replaced on the object, in a subclass or in the class."""
+    FQ = scmx.fused_qwen3
+    monkeypatch.setattr(FQ, "attend_quant", lambda *a: ("kernel", "scales"))
+
+    class Own(FQ.FusedQwen3):
+        def act_q(self, x, Mp=None, nt=256, down=False):
+            return "own", "scales"
+
+    class At:
+        scale = 1.0
+
+    plain, own = (c.__new__(c) for c in (FQ.FusedQwen3, Own))
+    for f in (plain, own):
+        f.rot, f.record, f.record_layers, f.sdpa = False, None, (), lambda *a: "rows"
+        f._qkv = lambda *a: (None, None, None)
+    ask = lambda f: f._attention(0, At, None, None, None, None, 3, 128)[1]      # noqa: E731
+    assert ask(plain) == "kernel" and ask(own) == "own"
+    plain.act_q = lambda x, Mp: ("object", "scales")
+    assert ask(plain) == "object"
+    del plain.act_q
+    monkeypatch.setattr(FQ.FusedQwen3, "act_q", lambda self, x, Mp: ("class", "scales"))
+    assert ask(plain) == "class"
