@@ -26,6 +26,7 @@ import torch
 from . import _lib
 from . import sc_decode as G
 from . import sc_kernels as S
+from . import hybrid_mixers as MX
 from . import sc_mixers as X
 from . import sc_moe as M_
 
@@ -240,6 +241,11 @@ class DecodeOlmoe(_Decoder):
         return self.head(xn[None])
 
 
+def _row(row, in_parts):
+    """A row for its reader: as it is left, or joined."""
+    return row if in_parts or not isinstance(row, X.RowParts) else row.joined()
+
+
 class DecodeHybrid(_Decoder):
     """Built from a FusedHybrid.  Activations of a step are float32 vectors in buffers that live with the decoder."""
     replayable = True
@@ -262,6 +268,7 @@ class DecodeHybrid(_Decoder):
         self.bufs = [own[ly] for ly in fused.layers]
 
     def _mix(self, ly, b, x, c, pos_dev):
+        x = _row(x, MX.reads_parts(ly.mixer))
         return ly.mixer.w_o.vec(ly.mixer.step(self.f, x, c, b, pos_dev), out=self.y.view(-1))
 
     def _step(self, tok, cache, pos_dev):
@@ -269,7 +276,7 @@ class DecodeHybrid(_Decoder):
         f.ensure_positions(cache[0].capacity)
         assert pos_dev is not None or cache[0].offset < cache[0].capacity, "KV cache capacity exceeded"
         row = (self._prenorm if self.args.design.prenorm else self._postnorm)(tok.view(-1), cache, pos_dev)
-        return f.head.vec(row)[None, None]
+        return f.head.vec(_row(row, X.reads_parts(f.head)))[None, None]
 
     def _prenorm(self, tok, cache, pos_dev):
         f, (x, spare), y, mult = self.f, self.x, self.y, self.args.residual_mult
@@ -281,7 +288,7 @@ class DecodeHybrid(_Decoder):
             self._mix(ly, b, row, c, pos_dev)
             row, x, spare = X.RowParts(x, y, after if ly.w_up is None else ly.norm2, mult, f.eps, spare), spare, x
             if ly.w_up is not None:
-                ly.feed_forward_vec(row, b["u"], y.view(-1))
+                ly.feed_forward_vec(_row(row, ly.feed_reads_parts()), b["u"], y.view(-1))
                 row, x, spare = X.RowParts(x, y, after, mult, f.eps, spare), spare, x
         return row
 
@@ -297,7 +304,7 @@ class DecodeHybrid(_Decoder):
             norm = ly.norm1
             if ly.w_up is not None:
                 row, x, turn = X.RowParts(x, y, norm, 1.0, f.eps, self.x[turn], ()), self.x[turn], 1 - turn
-                ly.feed_forward_vec(row, b["u"], y.view(-1))
+                ly.feed_forward_vec(_row(row, ly.feed_reads_parts()), b["u"], y.view(-1))
                 norm = ly.norm2
             row = X.RowParts(x, y, norm, 1.0, f.eps, self.x[turn], (self.xs, ly.dwa, not last), f.final_norm if last else None)
             x, turn = self.x[turn], 1 - turn

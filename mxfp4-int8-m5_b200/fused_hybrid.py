@@ -36,6 +36,13 @@ class HybridLayer:
     def feed_forward_vec(self, x, u, y):
         return self.w_down.vec(self.w_up.vec(x, act=self.act, out=u)[:self.w_down.K], out=y)
 
+    def feed_reads_parts(self):
+        """Whether feed_forward_vec takes a row in parts (sc_mixers.RowParts)."""
+        return type(self).feed_forward_vec is _FEED and "feed_forward_vec" not in self.__dict__ and X.reads_parts(self.w_up)
+
+
+_FEED = HybridLayer.feed_forward_vec      # as this file defines it
+
 
 class FusedHybrid:
     def __init__(self, model, portion=4096):

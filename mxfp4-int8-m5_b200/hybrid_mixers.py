@@ -2,7 +2,8 @@
 (projections of the same input concatenated, small vectors float32) and the mixer's two paths,
 
     prefill(f, h, c)          a portion h [T, W] -> the input of the output projection [T, K]; cache c is read from c.offset on
-    step(f, x, c, b, pos)     one float32 row in the buffers b = buffers(dev); `pos` (int32 on the device) replaces c.offset
+    step(f, x, c, b, pos)     one float32 row in the buffers b = buffers(dev); `pos` (int32 on the device) replaces c.offset.  The classes here
+                              also take a row in parts (sc_mixers.RowParts), which w_in joins; any other step gets the row
 
 The caller applies w_o and advances the cache.  `f` is the fused_hybrid.FusedHybrid, which holds the rotation tables.
 
@@ -174,3 +175,9 @@ class LatentAttention(Mixer):
 
 CLASSES = {"mamba1": Mamba1, "retention": Retention, "attention": DiffAttention, "delta": Delta, "channel_delta": ChannelDelta,
            "latent_attention": LatentAttention}
+_STEPS = {c.step for c in CLASSES.values()}      # as this file defines them
+
+
+def reads_parts(mixer):
+    """Whether a mixer's step hands its row to one product and nowhere else, so that it may be left in parts: this file's own do."""
+    return type(mixer).step in _STEPS and "step" not in mixer.__dict__ and X.reads_parts(mixer.w_in)

@@ -153,6 +153,7 @@ class Linear:
         return y
 
     def _streams(self, x):
+        """One row as a stream of the weights; 6400 values are the widest rows that were timed, wider ones run as before."""
         return self.K <= 6400 and self.N % 8 == 0 and x.is_contiguous() and x.data_ptr() % 16 == 0
 
     def _call_f32(self, x, act, tile, splits):
@@ -214,6 +215,9 @@ class RowParts:
         self.x, self.y, self.w, self.mult, self.eps, self.x_out, self.average, self.final = x, y, w, mult, eps, x_out, average, final
 
     def fits(self, K):
+        """Two 16-byte pieces for each of a product's 256 threads.  Every CTA joins the whole row, an average over all layers' results included, and that still takes less
+        than the row kernels: step of a post-norm decoder with 32 layers of width 2048 1105 us, average by the row kernels 1155 us; 96 layers of 2048 3735 and 3769 us,
+        128 layers of 1024 3320 and 3767 us, 256 layers of 512 7.0 and 8.2 ms."""
         rows = (self.x, self.y, self.w, self.x_out, self.final, self.average[0] if self.average else None)
         return K <= 2048 and K % 4 == 0 and all(t is None or t.data_ptr() % 16 == 0 for t in rows)
 
@@ -231,6 +235,14 @@ class RowParts:
             return h.view(-1)
         res_norm(self.y, self.x, self.w, self.eps, self.x_out, average=self.average or None)
         return (self.x_out if self.final is None else norm_rows(self.x_out, self.final, self.eps, torch.float32)).view(-1)
+
+
+_VEC = Linear.vec      # as this file defines it
+
+
+def reads_parts(lin):
+    """Whether a product joins a row that is left in parts (a product of the caller's gets the row itself)."""
+    return type(lin) is Linear and Linear.vec is _VEC and "vec" not in lin.__dict__
 
 
 class _full_float32:

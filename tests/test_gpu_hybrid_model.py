@@ -222,3 +222,42 @@ def test_command_line_replay(scmx, tmp_path):
     assert sorted(os.listdir(out)) == ["0.f32", "2.f32"]
     got = [np.fromfile(out / f"{i}.f32", "<f4").reshape(-1, cfg["vocab"]) for i in (0, 2)]
     assert worst(got[0], want[[16, 2]]) < 2e-4 and worst(got[1], want[[19]]) < 2e-4
+
+
+@pytest.mark.parametrize("name", ["mixed", "attention"])
+def test_readers_of_the_callers(scmx, name):
+    """Mixers, feed-forwards, products and heads that a program puts in place of the library's get the row as a tensor, with the same answers."""
+    cfg = CONFIGS[name]
+    toks = tokens(cfg, 6)
+    want = Model(scmx, cfg, F32, 16).run(toks, [1] * 6)
+    m, X = Model(scmx, cfg, F32, 16), scmx.sc_mixers
+
+    class Product:
+        def __init__(self, lin):
+            self.lin = lin
+
+        def __getattr__(self, n):
+            return getattr(self.lin, n)
+
+        def __call__(self, *a, **k):
+            return self.lin(*a, **k)
+
+        def vec(self, x, **k):
+            assert torch.is_tensor(x) and x.shape == (self.lin.K,) and x.dtype == F32
+            return self.lin.vec(x, **k)
+
+    m.fused.head = Product(m.fused.head)
+    for i, ly in enumerate(m.fused.layers):
+        step, feed = ly.mixer.step, ly.feed_forward_vec
+        if i % 2:
+            ly.mixer.w_in = Product(ly.mixer.w_in)
+        else:
+            ly.mixer.step = lambda f, x, *a, step=step: step(f, x + 0, *a)
+        if ly.w_up is not None:
+            if i % 2:
+                ly.feed_forward_vec = lambda x, *a, feed=feed: feed(x + 0, *a)
+            else:
+                ly.w_up = Product(ly.w_up)
+    got = m.run(toks, [1] * 6)
+    assert worst(got, want) < 1e-4      # the row kernels' order of sums
+
