@@ -30,7 +30,7 @@ struct GvArgs {
 };
 
 constexpr int GV_ROWS = 2;
-constexpr int GV_PRO_MAXK = 2048;      // two 16-byte pieces per thread
+constexpr int GV_PRO_MAXK = 2048;      // two 16-byte pieces per thread; wider rows are joined by the row kernels
 
 // Weights are read once a token and are more than L2 holds in a model of some size: they leave it first, so that what a step comes back to (kernel
 // code, states, caches, activations) stays.  Without it kernels that run once a token began with a cold start of several us: generation of 8
@@ -335,6 +335,7 @@ extern "C" int scmx_gemv_x_row(const void* W, int64_t ldw, int dt, const float* 
     return gemv_x(W, ldw, dt, x, N, K, epi, a_pos, a_neg, conv_w, conv_b, tail, C, taps, out, a, stream);
 }
 
+// Rows of up to 6400 values.  Callers send wider ones to the products they used before, although a stream is ahead there too (4096 x 12288: 22 us, 31 us as a tile of 128 rows).
 static int row_product(const uint16_t* W, int64_t ldw, const uint16_t* x, int64_t N, int64_t K, void* out, int out_f32, void* stream) {
     SCMX_REQUIRE(W && x && out && N > 0 && K > 0 && N < (1ll << 30) && K % 8 == 0 && ldw % 8 == 0 && ldw >= K, SCMX_EINVAL, "row product: N=%lld K=%lld pitch %lld",
                  (long long)N, (long long)K, (long long)ldw);
@@ -346,6 +347,7 @@ static int row_product(const uint16_t* W, int64_t ldw, const uint16_t* x, int64_
     return run_gemv<bf16_t>(a, 4, (cudaStream_t)stream);
 }
 
+// One product under two names: scmx.h declares scmx_head_bf16, scmx_mixers.h declares scmx_gemv_bf16.
 extern "C" int scmx_head_bf16(const uint16_t* W, int64_t ldw, const uint16_t* x, int64_t N, int64_t K, uint16_t* out, void* stream) {
     return row_product(W, ldw, x, N, K, out, 0, stream);
 }
