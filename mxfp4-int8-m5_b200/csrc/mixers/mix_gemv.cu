@@ -1,9 +1,16 @@
 // Matrix-vector product of the decode step: out [N] = W [N, K] x, weights bfloat16 or float, x and out float32, float32
-// accumulation.  Each warp sums two rows at a time (or a slice of their columns) and keeps two sets of 8 weight loads of 16 bytes per lane
-// in flight across its rows; the first are issued before the previous kernel of the chain has finished (weights never change).
-// Epilogues: none; xIELU; the causal convolution + SiLU of the first C rows, whose carried inputs are shifted in place; gelu(gate) up
-// of rows that alternate 16 gate and 16 up rows (a warp owns one of each); a bfloat16 row in and out (the output head of the W4A8 decoders;
-// this file is part of both libraries).
+// accumulation.  Epilogues: none; xIELU; the causal convolution + SiLU of the first C rows, whose carried inputs are shifted in place;
+// gelu(gate) up of rows that alternate 16 gate and 16 up rows (a warp owns one of each); a bfloat16 row in and out (the output head of
+// the W4A8 decoders; this file is part of both libraries).
+//
+// Bound by the weights' bytes and by the latency of a link of the chain.  Every lane streams its pieces of the row pairs of its warp through a ring
+// of its own in shared memory (16-byte asynchronous copies, nothing shared and no barrier), filled before the kernel waits for its predecessor:
+// weights never change.  A CTA holds half of an SM's shared memory and few registers, so two products of a chain are resident together and the
+// next one's first 14 MB arrive while this one waits for its input, joins its row or reduces.  16 warps and two products an instruction: with 8 warps
+// a chunk's chain of dependent instructions, not memory, set the rate (131 MB 26 us; 33 us with one product an instruction).  Bulk copies of 2 KB, one
+// thread issuing for a warp, took a quarter longer than these copies.  With the weights in registers (two CTAs that filled the register file) memory stood still
+// between kernels: generation of 8 tokens 1486 -> 1280 us (hybrid, width 2048), 1445 -> 1229 us (fabezen, width 1024); the output head of 32000 x 2048
+// 27 -> 19.8 us in a chain of its own, 6.6 TB/s.
 #include "mix_common.cuh"
 
 namespace scmx {
@@ -14,6 +21,7 @@ struct GvArgs {
     float* out;             // [N]
     int64_t ldw;
     int N, K, ks;           // ks: warps that share a row (1, 2, 4 or 8)
+    int warps, slots;       // warps that stream weights, slots of a warp's ring
     float a_pos, a_neg;     // xIELU
     const float *cw, *cb;   // convolution weights [C, taps] and bias [C]
     float* tail;            // [C, taps - 1]
@@ -30,7 +38,10 @@ struct GvArgs {
 };
 
 constexpr int GV_ROWS = 2;
-constexpr int GV_PRO_MAXK = 2048;      // two 16-byte pieces per thread; wider rows are joined by the row kernels
+constexpr int GV_U = 2, GV_CP = 32 * GV_U, GV_SLOT = GV_ROWS * 16 * GV_CP;      // 16-byte pieces of a row per lane and per slot, bytes of a slot
+constexpr int GV_MAX_SLOTS = 3;
+constexpr int GV_THREADS = 512, GV_WARPS = GV_THREADS / 32;
+constexpr int GV_PRO_MAXK = 2048;      // a 16-byte piece per thread; wider rows are joined by the row kernels
 
 // Weights are read once a token and are more than L2 holds in a model of some size: they leave it first, so that what a step comes back to (kernel
 // code, states, caches, activations) stays.  Without it kernels that run once a token began with a cold start of several us: generation of 8
@@ -40,51 +51,49 @@ __device__ __forceinline__ uint64_t first_out() {
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
     return p;
 }
-__device__ __forceinline__ uint4 load_w(const void* p, uint64_t policy) {
-    uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "l"(policy));
-    return v;
+__device__ __forceinline__ void copy_w(uint32_t dst, const void* src, uint64_t policy) {
+    asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "l"(policy) : "memory");
+}
+__device__ __forceinline__ void copies_end() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// At most n - 1 of the thread's groups of copies are still on their way.
+__device__ __forceinline__ void copies_wait(int n) {
+    if (n == 3) asm volatile("cp.async.wait_group 2;" ::: "memory");
+    else if (n == 2) asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-template <typename T> struct Vec8;
-template <> struct Vec8<bf16_t> {
-    uint4 w;
-    __device__ __forceinline__ void load(const bf16_t* p, uint64_t policy) { w = load_w(p, policy); }
-    __device__ __forceinline__ void zero() { w = make_uint4(0, 0, 0, 0); }
-    __device__ __forceinline__ float dot(float4 lo, float4 hi, float s) const {
-        s = fmaf(bf16_lo(w.x), lo.x, s); s = fmaf(bf16_hi(w.x), lo.y, s); s = fmaf(bf16_lo(w.y), lo.z, s); s = fmaf(bf16_hi(w.y), lo.w, s);
-        s = fmaf(bf16_lo(w.z), hi.x, s); s = fmaf(bf16_hi(w.z), hi.y, s); s = fmaf(bf16_lo(w.w), hi.z, s); s = fmaf(bf16_hi(w.w), hi.w, s);
-        return s;
-    }
-};
-template <> struct Vec8<float> {
-    float4 a, b;
-    __device__ __forceinline__ void load(const float* p, uint64_t policy) {
-        const uint4 u = load_w(p, policy), v = load_w(p + 4, policy);
-        a = make_float4(__uint_as_float(u.x), __uint_as_float(u.y), __uint_as_float(u.z), __uint_as_float(u.w));
-        b = make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
-    }
-    __device__ __forceinline__ void zero() { a = b = make_float4(0, 0, 0, 0); }
-    __device__ __forceinline__ float dot(float4 lo, float4 hi, float s) const {
-        s = fmaf(a.x, lo.x, s); s = fmaf(a.y, lo.y, s); s = fmaf(a.z, lo.z, s); s = fmaf(a.w, lo.w, s);
-        s = fmaf(b.x, hi.x, s); s = fmaf(b.y, hi.y, s); s = fmaf(b.z, hi.z, s); s = fmaf(b.w, hi.w, s);
-        return s;
-    }
-};
+// The row in shared memory, in float4: with bfloat16 weights a 16-byte piece meets two of them, kept nv apart so that the lanes of a load are neighbours.
+template <typename T> __device__ __forceinline__ int x_place(int i, int nv);
+template <> __device__ __forceinline__ int x_place<bf16_t>(int i, int nv) { return (i & 1) * nv + (i >> 1); }
+template <> __device__ __forceinline__ int x_place<float>(int i, int) { return i; }
+// s += piece i of a row times x, two products per instruction (even and odd elements in the halves of s).
+template <typename T> __device__ __forceinline__ uint64_t dot_piece(const uint4& w, const ulonglong2* x, int nv, int i, uint64_t s);
+__device__ __forceinline__ uint64_t bf16_pair(uint32_t w) { return pack2(bf16_lo(w), bf16_hi(w)); }
+template <> __device__ __forceinline__ uint64_t dot_piece<bf16_t>(const uint4& w, const ulonglong2* x, int nv, int i, uint64_t s) {
+    const ulonglong2 lo = x[i], hi = x[nv + i];
+    s = fma2(bf16_pair(w.x), lo.x, s); s = fma2(bf16_pair(w.y), lo.y, s);
+    s = fma2(bf16_pair(w.z), hi.x, s); return fma2(bf16_pair(w.w), hi.y, s);
+}
+template <> __device__ __forceinline__ uint64_t dot_piece<float>(const uint4& w, const ulonglong2* x, int, int i, uint64_t s) {
+    const ulonglong2 v = x[i];
+    s = fma2(pack2(__uint_as_float(w.x), __uint_as_float(w.y)), v.x, s);
+    return fma2(pack2(__uint_as_float(w.z), __uint_as_float(w.w)), v.y, s);
+}
 
 // The residual and norm kernels between two products cost 2 - 5 us each in a chain of single rows, nearly all of it latency.  Every CTA computes
 // the whole row itself while its first weights arrive: a few reads from L2 and one or two sums over the CTA.
+template <typename T>
 __device__ __forceinline__ void gv_prologue(const GvArgs& a, float4* xs, int nv, float* red) {
     const int tid = threadIdx.x, quads = a.K >> 2;
     const bool first = blockIdx.x == 0;
-    float4 r[2], w[2], s[2];
+    constexpr int PIECES = GV_PRO_MAXK / 4 / GV_THREADS;
+    float4 r[PIECES], w[PIECES], s[PIECES];
     float ss = 0.0f;
     const float self = a.pro == 2 && a.n > 0 ? a.dwa[a.n - 1] : 1.0f;
     auto sq = [](const float4& v) { return v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w; };
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const int i = tid + 256 * k;
+    for (int k = 0; k < PIECES; ++k) {
+        const int i = tid + GV_THREADS * k;
         r[k] = w[k] = s[k] = make_float4(0, 0, 0, 0);
         if (i >= quads) continue;
         w[k] = ld4(a.nw + 4 * i);
@@ -102,8 +111,8 @@ __device__ __forceinline__ void gv_prologue(const GvArgs& a, float4* xs, int nv,
     if (a.pro == 2) {
         ss = 0.0f;
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const int i = tid + 256 * k;
+        for (int k = 0; k < PIECES; ++k) {
+            const int i = tid + GV_THREADS * k;
             if (i >= quads) continue;
             r[k] = make_float4(s[k].x + r[k].x * inv * w[k].x, s[k].y + r[k].y * inv * w[k].y, s[k].z + r[k].z * inv * w[k].z, s[k].w + r[k].w * inv * w[k].w);
             if (a.n > 0) {
@@ -126,175 +135,206 @@ __device__ __forceinline__ void gv_prologue(const GvArgs& a, float4* xs, int nv,
     const float scale = a.pro == 1 ? inv : a.fw != nullptr ? rms_inv_f32(block_sumf(ss, red), a.K, a.eps) : 1.0f;
     const bool norm = a.pro == 1 || a.fw != nullptr;
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const int i = tid + 256 * k;
+    for (int k = 0; k < PIECES; ++k) {
+        const int i = tid + GV_THREADS * k;
         if (i < 2 * nv) {
             float4 h = r[k];
             if (norm) h = make_float4(h.x * scale * w[k].x, h.y * scale * w[k].y, h.z * scale * w[k].z, h.w * scale * w[k].w);
-            xs[(i & 1) * nv + (i >> 1)] = h;      // zero above K
+            xs[x_place<T>(i, nv)] = h;      // zero above K
             if (first && a.x_out != nullptr && i < quads) *reinterpret_cast<float4*>(a.x_out + 4 * i) = r[k];
         }
     }
 }
 
 template <typename T, int EPI>
-__global__ void __launch_bounds__(256, 2) gemv_x_kernel(const GvArgs a) {
-    constexpr int U = sizeof(T) == 2 ? 4 : 2;          // vectors per lane and row in a set
-    extern __shared__ __align__(16) float4 xs[];       // [2][nv]: elements 0..3 and 4..7 of every vector of 8
-    __shared__ float part[2][8][GV_ROWS], red[33];
-    float* ys = reinterpret_cast<float*>(xs + 2 * ((a.K + 7) >> 3));      // EPI 2: products of this CTA's rows
+__global__ void __launch_bounds__(GV_THREADS, 2) gemv_x_kernel(const GvArgs a) {
+    constexpr int PER = 16 / sizeof(T);                // values of a 16-byte piece
+    // x: 2 nv float4 | partial sums of every (pair, slice) | the warps' rings (128-byte aligned)
+    extern __shared__ __align__(128) float4 xs[];
+    __shared__ float red[33];
     pdl_launch_dependents();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nv = (a.K + 7) >> 3, ks = a.ks, team = warp / ks, slice = warp - team * ks, teams = 8 / ks;
-    const int first = slice * 32 + lane, step = 32 * ks;
-    const int sets = (nv + U * step - 1) / (U * step);                 // of a row pair
-    // row pairs of this CTA: equal shares, dealt to its teams in turn
+    const int nv = (a.K + 7) >> 3, np = nv * (8 / PER), ks = a.ks, team = warp / ks, slice = warp - team * ks, teams = a.warps / ks;
+    const int slots = a.slots, chunks = (np + GV_CP - 1) / GV_CP;
+    // row pairs of this CTA: equal shares, dealt to its teams in turn; a team's warps share the chunks of a row
     const int all = (a.N + GV_ROWS - 1) / GV_ROWS;
     const int base = (int)((int64_t)all * blockIdx.x / gridDim.x), pairs = (int)((int64_t)all * (blockIdx.x + 1) / gridDim.x);
-    const int p0 = base + team, pstep = teams;
-    const T* W = static_cast<const T*>(a.W);
-    auto row_of = [&](int r0, int r) { return EPI == 3 ? 32 * (r0 >> 5) + ((r0 >> 1) & 15) + 16 * r : r0 + r; };
-    using Set = Vec8<T>[GV_ROWS][U];
+    const int c_lo = chunks * slice / ks, c_hi = chunks * (slice + 1) / ks;
+    float* part = reinterpret_cast<float*>(xs + 2 * nv);      // [pairs - base][ks][GV_ROWS]
+    const int part_bytes = ((int)((all + gridDim.x - 1) / gridDim.x) * ks * GV_ROWS * 4 + 127) & ~127;
+    const uint8_t* ring = reinterpret_cast<uint8_t*>(xs) + ((32 * nv + 127) & ~127) + part_bytes + (size_t)warp * slots * GV_SLOT + 16 * lane;
+    const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(ring), ring_end = ring_s + slots * GV_SLOT;
     const uint64_t policy = first_out();
-    Set wa, wb;
-    // the next set to load: of pair lp (done at pairs), from vector lv on
-    int lp = p0, lv = first;
-    auto fetch = [&](Set& w) {
-        const bool on = lp < pairs;
-        const int r0 = lp * GV_ROWS;
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-#pragma unroll
-            for (int r = 0; r < GV_ROWS; ++r) {
-                const int v = lv + u * step;
-                if (on && v < nv && r0 + r < a.N) w[r][u].load(W + (int64_t)row_of(r0, r) * a.ldw + 8 * (int64_t)v, policy);
-                else w[r][u].zero();
-            }
-        lv += U * step;
-        if (lv - first >= sets * U * step) {
-            lv = first;
-            lp += pstep;
-        }
+    auto row_of = [&](int p, int r) {                  // past the end (N odd): the last row again, its sum is not used
+        const int r0 = p * GV_ROWS;
+        return EPI == 3 ? 32 * (r0 >> 5) + ((r0 >> 1) & 15) + 16 * r : min(r0 + r, a.N - 1);
     };
-    fetch(wa);
-    fetch(wb);
+    // the next chunk to request: of pair ip, number ic; every request is one group of copies, empty ones past the end
+    const int p_first = warp < a.warps ? base + team : pairs;
+    int ip = p_first, ic = c_lo;
+    const uint8_t *g0 = nullptr, *g1 = nullptr;
+    auto row_start = [&]() {
+        const int64_t pitch = a.ldw * (int64_t)sizeof(T);
+        const uint8_t* w = static_cast<const uint8_t*>(a.W) + (int64_t)c_lo * (16 * GV_CP) + 16 * lane;
+        g0 = w + row_of(ip, 0) * pitch;
+        g1 = w + row_of(ip, 1) * pitch;
+    };
+    auto request = [&](uint32_t dst) {
+        if (ip < pairs) {
+            const int left = np - ic * GV_CP - lane;
+#pragma unroll
+            for (int u = 0; u < GV_U; ++u)
+                if (32 * u < left) {
+                    copy_w(dst + 512 * u, g0 + 512 * u, policy);
+                    copy_w(dst + 512 * (GV_U + u), g1 + 512 * u, policy);
+                }
+            g0 += 16 * GV_CP;
+            g1 += 16 * GV_CP;
+            if (++ic == c_hi) {
+                ic = c_lo;
+                ip += teams;
+                if (ip < pairs) row_start();
+            }
+        }
+        copies_end();
+    };
+    if (ip < pairs) row_start();
+    for (int i = 0; i < slots; ++i) request(ring_s + i * GV_SLOT);
+    // the convolution's weights of row `tid` of this CTA (EPI 2)
+    const int crow = GV_ROWS * base + tid, rows_end = min(GV_ROWS * pairs, a.N);
+    constexpr int RT = 4;                              // taps that a thread keeps in registers
+    const bool conv_early = EPI == 2 && a.taps <= RT && crow < min(rows_end, a.C);
+    float cw[RT], tl[RT], cb = 0.0f;
+    if (conv_early) {
+#pragma unroll
+        for (int j = 0; j < RT; ++j) cw[j] = j < a.taps ? a.cw[(int64_t)crow * a.taps + j] : 0.0f;
+        cb = a.cb == nullptr ? 0.0f : a.cb[crow];
+    }
     pdl_wait();
+    if (conv_early) {
+#pragma unroll
+        for (int j = 0; j < RT; ++j) tl[j] = j < a.taps - 1 ? a.tail[(int64_t)crow * (a.taps - 1) + j] : 0.0f;
+    }
     if (EPI == 4) {
-        for (int v = tid; v < nv; v += 256) {
+        for (int v = tid; v < nv; v += GV_THREADS) {
             float x[8];
             ld8(a.xh + 8 * v, x);
-            xs[v] = make_float4(x[0], x[1], x[2], x[3]);
-            xs[nv + v] = make_float4(x[4], x[5], x[6], x[7]);
+            xs[x_place<T>(2 * v, nv)] = make_float4(x[0], x[1], x[2], x[3]);
+            xs[x_place<T>(2 * v + 1, nv)] = make_float4(x[4], x[5], x[6], x[7]);
         }
     } else if (a.pro != 0) {
-        gv_prologue(a, xs, nv, red);
+        gv_prologue<T>(a, xs, nv, red);
     } else if ((a.K & 3) == 0 && ((uintptr_t)a.x & 15) == 0) {
 #pragma unroll 8
-        for (int i = tid; i < 2 * nv; i += 256)
-            xs[(i & 1) * nv + (i >> 1)] = 4 * i < a.K ? *reinterpret_cast<const float4*>(a.x + 4 * i) : make_float4(0, 0, 0, 0);
+        for (int i = tid; i < 2 * nv; i += GV_THREADS)
+            xs[x_place<T>(i, nv)] = 4 * i < a.K ? *reinterpret_cast<const float4*>(a.x + 4 * i) : make_float4(0, 0, 0, 0);
     } else {
-        for (int i = tid; i < nv * 8; i += 256) {
+        for (int i = tid; i < nv * 8; i += GV_THREADS) {
             const float x = i < a.K ? a.x[i] : 0.0f;
-            reinterpret_cast<float*>(xs + ((i >> 2) & 1) * nv + (i >> 3))[i & 3] = x;
+            reinterpret_cast<float*>(xs + x_place<T>(i >> 2, nv))[i & 3] = x;
         }
     }
     __syncthreads();
-    float s[GV_ROWS] = {};
-    int cp = p0, cv = first, turn = 0;
-    auto finish = [&]() {                               // row pair cp is summed
-        const int r0 = cp * GV_ROWS;
+    const ulonglong2* x2 = reinterpret_cast<const ulonglong2*>(xs);
+    uint32_t at = ring_s;
+    const uint8_t* w_at = ring;
+    for (int p = p_first; p < pairs; p += teams) {
+        uint64_t s0 = 0, s1 = 0;                       // two float32 sums each
+        for (int c = c_lo; c < c_hi; ++c) {
+            copies_wait(slots);
+            const int i = c * GV_CP + lane;
 #pragma unroll
-        for (int r = 0; r < GV_ROWS; ++r) s[r] = warp_sumf(s[r]);
-        if (ks > 1) {
-            if (lane == 0)
-#pragma unroll
-                for (int r = 0; r < GV_ROWS; ++r) part[turn][warp][r] = s[r];
-            // the team's warps meet once per pair; two sets of sums, so that the next pair's are not written over these
-            asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "r"(32 * ks) : "memory");
-            if (slice == 0)
-#pragma unroll
-                for (int r = 0; r < GV_ROWS; ++r) {
-                    s[r] = 0.0f;
-                    for (int i = 0; i < ks; ++i) s[r] += part[turn][warp + i][r];
+            for (int u = 0; u < GV_U; ++u)
+                if (i + 32 * u < np) {
+                    s0 = dot_piece<T>(*reinterpret_cast<const uint4*>(w_at + 512 * u), x2, nv, i + 32 * u, s0);
+                    s1 = dot_piece<T>(*reinterpret_cast<const uint4*>(w_at + 512 * (GV_U + u)), x2, nv, i + 32 * u, s1);
                 }
-            turn ^= 1;
-        }
-        if (slice == 0) {
-            if (EPI == 3) {
-                if (lane == 0) a.out[r0 >> 1] = gelu_tanh_f32(s[0]) * s[1];
-            } else {
-                const int row = r0 + lane;
-                if (lane < GV_ROWS && row < a.N) {
-                    float y = lane == 0 ? s[0] : s[1];
-                    if (EPI == 1) y = xielu_f32(y, a.a_pos, a.a_neg);
-                    if (EPI == 4 && a.outh != nullptr) a.outh[row] = f32_to_bf16(y);
-                    else if (EPI == 2 && row < a.C) ys[row - GV_ROWS * base] = y;
-                    else a.out[row] = y;
-                }
+            request(at);
+            at += GV_SLOT;
+            w_at += GV_SLOT;
+            if (at == ring_end) {
+                at = ring_s;
+                w_at = ring;
             }
         }
-#pragma unroll
-        for (int r = 0; r < GV_ROWS; ++r) s[r] = 0.0f;
-    };
-    auto consume = [&](Set& w) {
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int v = cv + u * step;
-            if (v < nv) {
-                const float4 lo = xs[v], hi = xs[nv + v];
-#pragma unroll
-                for (int r = 0; r < GV_ROWS; ++r) s[r] = w[r][u].dot(lo, hi, s[r]);
-            }
-        }
-        if (lp < pairs) fetch(w);
-        cv += U * step;
-        if (cv - first >= sets * U * step) {
-            finish();
-            cv = first;
-            cp += pstep;
-        }
-    };
-    while (cp < pairs) {
-        consume(wa);
-        if (cp >= pairs) break;
-        consume(wb);
+        const float2 a0 = unpack2(s0), a1 = unpack2(s1);
+        const float t0 = warp_sumf(a0.x + a0.y), t1 = warp_sumf(a1.x + a1.y);
+        if (lane < GV_ROWS) part[((p - base) * ks + slice) * GV_ROWS + lane] = lane == 0 ? t0 : t1;
     }
-    if (EPI == 2) {
-        // the convolution of all rows at once: its loads would otherwise be a chain in every row pair (33 MB of weights: 14 us, then 9)
-        __syncthreads();
-        const int row = GV_ROWS * base + tid;
-        for (int r = row; r < min(GV_ROWS * pairs, a.C); r += 256) {
-            const float y = ys[r - GV_ROWS * base];
-            const float* cw = a.cw + (int64_t)r * a.taps;
-            float* tl = a.tail + (int64_t)r * (a.taps - 1);
-            float c = fmaf(cw[a.taps - 1], y, a.cb == nullptr ? 0.0f : a.cb[r]);
-            for (int j = 0; j < a.taps - 1; ++j) {
-                c = fmaf(cw[j], tl[j], c);
-                tl[j] = j + 1 < a.taps - 1 ? tl[j + 1] : y;
+    __syncthreads();
+    auto total = [&](int i) {                          // row i of this CTA, in the order of its pairs
+        float y = 0.0f;
+        for (int k = 0; k < ks; ++k) y += part[((i >> 1) * ks + k) * GV_ROWS + (i & 1)];
+        return y;
+    };
+    if (EPI == 3) {
+        for (int i = tid; i < pairs - base; i += GV_THREADS) a.out[base + i] = gelu_tanh_f32(total(2 * i)) * total(2 * i + 1);
+        return;
+    }
+    for (int row = crow; row < rows_end; row += GV_THREADS) {
+        float y = total(row - GV_ROWS * base);
+        if (EPI == 1) y = xielu_f32(y, a.a_pos, a.a_neg);
+        if (EPI == 4 && a.outh != nullptr) {
+            a.outh[row] = f32_to_bf16(y);
+        } else if (EPI == 2 && row < a.C) {
+            float* t = a.tail + (int64_t)row * (a.taps - 1);
+            if (conv_early && row == crow) {
+                float c = cb;
+#pragma unroll
+                for (int j = 0; j < RT; ++j) c = j == a.taps - 1 ? fmaf(cw[j], y, c) : c;
+#pragma unroll
+                for (int j = 0; j < RT; ++j)
+                    if (j < a.taps - 1) {
+                        c = fmaf(cw[j], tl[j], c);
+                        t[j] = j + 1 < a.taps - 1 ? tl[j + 1 < RT ? j + 1 : 0] : y;
+                    }
+                a.out[row] = silu_f32(c);
+            } else {
+                const float* w = a.cw + (int64_t)row * a.taps;
+                float c = fmaf(w[a.taps - 1], y, a.cb == nullptr ? 0.0f : a.cb[row]);
+                for (int j = 0; j < a.taps - 1; ++j) {
+                    c = fmaf(w[j], t[j], c);
+                    t[j] = j + 1 < a.taps - 1 ? t[j + 1] : y;
+                }
+                a.out[row] = silu_f32(c);
             }
-            a.out[r] = silu_f32(c);
+        } else {
+            a.out[row] = y;
         }
     }
 }
 
 template <typename T>
 static int run_gemv(GvArgs a, int epi, cudaStream_t st) {
-    constexpr int U = sizeof(T) == 2 ? 4 : 2;
-    const int nv = (a.K + 7) / 8;
+    const int nv = (a.K + 7) / 8, np = nv * (int)sizeof(T) / 2, x_bytes = (nv * 32 + 127) & ~127;
     SCMX_REQUIRE(nv * 32 <= 200 * 1024, SCMX_ELIMIT, "gemv_x: K=%d", a.K);
-    // Persistent CTAs: x is staged once per CTA, and as many as stay resident (registers: two per SM) leave no wave of new ones that starts
-    // with nothing in flight.  Rows are shared by as many warps as still fill a set of loads each.
-    const int resident = (nv * 32 + 4096) * 2 <= 220 * 1024 ? 2 : 1;
-    int ks = 1;
-    while (ks < 8 && nv >= 2 * ks * 32 * U) ks *= 2;
-    a.ks = ks;
-    const int rows = 8 / ks * GV_ROWS, groups = (a.N + rows - 1) / rows, most = resident * sm_count();
-    const dim3 grid((unsigned)(groups < most ? groups : most)), block(256);
-    const size_t smem = (size_t)nv * 32 + (epi == 2 ? (size_t)4 * GV_ROWS * ((a.N / GV_ROWS + 1) / grid.x + 2) : 0);
-    SCMX_REQUIRE(smem <= 220 * 1024, SCMX_ELIMIT, "gemv_x: N=%d K=%d", a.N, a.K);
+    // One persistent CTA per SM, more where a CTA would have over 512 row pairs (its sums are kept in shared memory to the end).
+    const int all = (a.N + GV_ROWS - 1) / GV_ROWS, sms = sm_count();
+    const int by_rows = (all + 511) / 512, grid = by_rows > sms ? by_rows : all < sms ? all : sms;
+    const int ppc = (all + grid - 1) / grid;
+    // Rows are shared by the warps where that shortens the longest queue of chunks.
+    a.warps = x_bytes <= 184 * 1024 ? GV_WARPS : 4;                // very long rows leave room for few rings
+    const int chunks = (np + GV_CP - 1) / GV_CP;
+    int best = 1 << 30;
+    for (int k = 1; k <= a.warps && k <= chunks && ppc * k <= 1024; k *= 2) {
+        const int per = a.warps / k, cost = ((ppc + per - 1) / per) * ((chunks + k - 1) / k);
+        if (cost < best) {
+            best = cost;
+            a.ks = k;
+        }
+    }
+    // Three slots a warp, 96 KB a CTA: with the row and the sums half of an SM, so that the next product of a chain is resident beside this one.  Long rows leave
+    // fewer.
+    const int part = (ppc * a.ks * GV_ROWS * 4 + 127) & ~127;
+    auto ring = [&](int budget) { return (budget - x_bytes - part) / (a.warps * GV_SLOT); };
+    a.slots = ring(113 * 1024) >= 2 ? ring(113 * 1024) : ring(226 * 1024);
+    a.slots = a.slots > GV_MAX_SLOTS ? GV_MAX_SLOTS : a.slots < 1 ? 1 : a.slots;
+    if (a.slots > best) a.slots = best;
+    const size_t smem = (size_t)x_bytes + part + (size_t)a.slots * a.warps * GV_SLOT;
+    SCMX_REQUIRE(smem <= 226 * 1024, SCMX_ELIMIT, "gemv_x: N=%d K=%d", a.N, a.K);
     auto kernel = epi == 0 ? gemv_x_kernel<T, 0> : epi == 1 ? gemv_x_kernel<T, 1> : epi == 2 ? gemv_x_kernel<T, 2> : epi == 3 ? gemv_x_kernel<T, 3> : gemv_x_kernel<bf16_t, 4>;
     if (smem > 40 * 1024) SCMX_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    SCMX_PDL_OK("gemv_x_kernel", launch_pdl(kernel, grid, block, smem, st, a));
+    SCMX_PDL_OK("gemv_x_kernel", launch_pdl(kernel, dim3((unsigned)grid), dim3(GV_THREADS), smem, st, a));
     return SCMX_OK;
 }
 
