@@ -104,7 +104,9 @@ __global__ void __launch_bounds__(TA_THREADS, 1) diff_attn_tc_kernel(const __gri
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {          // the whole warp; `on` is the lane that issues
+            const uint32_t on = elect_lane();
+            bool ok = true;
             const uint32_t idesc_s = umma_idesc_bf16(128, 128);
             const uint32_t idesc_o = umma_idesc_bf16(128, (a.dv + 15) & ~15) | IDESC_B_MN;
             const int dsteps = (a.d + 15) / 16;
@@ -112,42 +114,42 @@ __global__ void __launch_bounds__(TA_THREADS, 1) diff_attn_tc_kernel(const __gri
                 for (int k = 0; k < dsteps; ++k) {
                     const uint32_t o = (k >> 2) * TA_TILE;
                     const uint64_t da = umma_desc(sbase + L::Q_OFF + m * KB * TA_TILE + o), db = umma_desc(sbase + L::K_OFF + (ks * 2 + m) * KB * TA_TILE + o);
-                    umma_bf16(tmem + 128 * m, da + 2 * (k & 3), db + 2 * (k & 3), idesc_s, k > 0);
+                    umma_bf16(on, tmem + 128 * m, da + 2 * (k & 3), db + 2 * (k & 3), idesc_s, k > 0);
                 }
-                umma_commit(b_s + 8 * m);
+                umma_commit(on, b_s + 8 * m);
             };
             do {
-                if (int w = mbar_wait(b_q, 0, abort_flag, a.wait_ns)) { fail = w == 1 ? 33 : -1; break; }
-                if (int w = mbar_wait(b_kf, 0, abort_flag, a.wait_ns)) { fail = w == 1 ? 33 : -1; break; }
+                if (!(ok = wait_warp(b_q, 0, abort_flag, a.wait_ns, 33, fail))) break;
+                if (!(ok = wait_warp(b_kf, 0, abort_flag, a.wait_ns, 33, fail))) break;
                 tc_fence_after();
                 scores(0, 0);
                 scores(1, 0);
-                umma_commit(b_ke);
-                for (int j = 0; j < nkt && fail == 0; ++j) {
+                umma_commit(on, b_ke);
+                for (int j = 0; j < nkt && ok; ++j) {
                     const int vs = j % VS, kn = (j + 1) % KS;
                     for (int m = 0; m < 2; ++m) {
-                        if (int w = mbar_wait(b_p + 8 * m, j & 1, abort_flag, a.wait_ns)) { fail = w == 1 ? 34 : -1; break; }
+                        if (!(ok = wait_warp(b_p + 8 * m, j & 1, abort_flag, a.wait_ns, 34, fail))) break;
                         if (m == 0)
-                            if (int w = mbar_wait(b_vf + 8 * vs, (j / VS) & 1, abort_flag, a.wait_ns)) { fail = w == 1 ? 33 : -1; break; }
+                            if (!(ok = wait_warp(b_vf + 8 * vs, (j / VS) & 1, abort_flag, a.wait_ns, 33, fail))) break;
                         tc_fence_after();
                         const uint64_t dv = umma_desc_mn(sbase + L::V_OFF + vs * VB * TA_TILE, TA_TILE);
 #pragma unroll
                         for (int k = 0; k < 8; ++k) {       // 16 keys: high and remainder terms, 8 columns each
                             const uint32_t pa = tmem + 128 * m + (k >> 1) * 32 + (k & 1) * 8;
-                            umma_bf16_ts(tmem + 256 + 128 * m, pa, dv + 128 * k, idesc_o, (j | k) != 0);
-                            umma_bf16_ts(tmem + 256 + 128 * m, pa + 16, dv + 128 * k, idesc_o, 1);
+                            umma_bf16_ts(on, tmem + 256 + 128 * m, pa, dv + 128 * k, idesc_o, (j | k) != 0);
+                            umma_bf16_ts(on, tmem + 256 + 128 * m, pa + 16, dv + 128 * k, idesc_o, 1);
                         }
                         if (j + 1 < nkt) {
                             if (m == 0)
-                                if (int w = mbar_wait(b_kf + 8 * kn, ((j + 1) / KS) & 1, abort_flag, a.wait_ns)) { fail = w == 1 ? 33 : -1; break; }
+                                if (!(ok = wait_warp(b_kf + 8 * kn, ((j + 1) / KS) & 1, abort_flag, a.wait_ns, 33, fail))) break;
                             tc_fence_after();
                             scores(m, kn);
-                            if (m == 1) umma_commit(b_ke + 8 * kn);
+                            if (m == 1) umma_commit(on, b_ke + 8 * kn);
                         }
-                        if (m == 1) umma_commit(b_ve + 8 * vs);
+                        if (m == 1) umma_commit(on, b_ve + 8 * vs);
                     }
                 }
-                if (fail == 0) umma_commit(b_o);
+                if (ok) umma_commit(on, b_o);
             } while (false);
         }
     } else {

@@ -860,7 +860,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1)
             return true;
         };
         auto done = [&]() {
-            umma_commit_on(on, b_e + 8 * st);
+            umma_commit(on, b_e + 8 * st);
             if (++st == DT_SLOTS) { st = 0; ph ^= 1; }
         };
         // D (+)= terms at `op` (per 32 values of K: 16 columns high, 16 remainder) times the K-major block pair at s, 64 of K
@@ -869,9 +869,9 @@ __global__ void __launch_bounds__(DT_THREADS, 1)
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const uint32_t x = op + (k >> 1) * 32 + (k & 1) * 8;
-                umma_bf16_ts_on(on, d, x, bh + 2 * k, idesc, k > 0 ? 1u : 1u - fresh);
-                umma_bf16_ts_on(on, d, x, bl + 2 * k, idesc, 1);
-                umma_bf16_ts_on(on, d, x + 16, bh + 2 * k, idesc, 1);
+                umma_bf16_ts(on, d, x, bh + 2 * k, idesc, k > 0 ? 1u : 1u - fresh);
+                umma_bf16_ts(on, d, x, bl + 2 * k, idesc, 1);
+                umma_bf16_ts(on, d, x + 16, bh + 2 * k, idesc, 1);
             }
         };
         bool ok = true;
@@ -884,7 +884,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1)
                 done();
             }
             if (!ok) break;
-            umma_commit_on(on, b_u);
+            umma_commit(on, b_u);
             const uint32_t o = tmem + DT_O + 64 * (c & 1);
             if (OUT && !wait(b_oe + 8 * (c & 1), ((c >> 1) & 1) ^ 1, 63)) break;
 #pragma unroll
@@ -907,20 +907,20 @@ __global__ void __launch_bounds__(DT_THREADS, 1)
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     const uint32_t u = tmem + DT_UP + (k >> 1) * 32 + (k & 1) * 8;
-                    umma_bf16_ts_on(on, tmem, u, eh + 128 * k, idesc_e, 1);
-                    umma_bf16_ts_on(on, tmem, u, el + 128 * k, idesc_e, 1);
-                    umma_bf16_ts_on(on, tmem, u + 16, eh + 128 * k, idesc_e, 1);
+                    umma_bf16_ts(on, tmem, u, eh + 128 * k, idesc_e, 1);
+                    umma_bf16_ts(on, tmem, u, el + 128 * k, idesc_e, 1);
+                    umma_bf16_ts(on, tmem, u + 16, eh + 128 * k, idesc_e, 1);
                 }
-                if (DB == 2) umma_commit_on(on, efree);
+                if (DB == 2) umma_commit(on, efree);
                 done();
             }
             if (!ok) break;
-            umma_commit_on(on, b_s);
+            umma_commit(on, b_s);
             if (!OUT) continue;
             if (!(ok = next())) break;
             split_product(o, tmem + DT_UP, 0);
             done();
-            umma_commit_on(on, b_of + 8 * (c & 1));
+            umma_commit(on, b_of + 8 * (c & 1));
         }
         if (!on) fail = fail > 0 ? -1 : fail;      // one lane reports
     } else {

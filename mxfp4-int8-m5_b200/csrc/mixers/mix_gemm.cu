@@ -179,36 +179,36 @@ __device__ __forceinline__ void gemm_bf16_body(const CUtensorMap& tmA, const CUt
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && leader) {
+        if (leader) {          // the whole warp; `on` is the lane that issues
+            const uint32_t on = elect_lane();
+            bool ok = true;
             constexpr uint32_t idesc = umma_idesc_bf16(TM_ROWS, BN);
             int stage = 0;
             uint32_t phase = 0, acc = 0, acc_phase = 0;
-            for (int t = worker; t < total && fail == 0; t += nworkers) {
-                const int w0 = PAIR ? mbar_wait_cluster(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, a.wait_ns)
-                                    : mbar_wait(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, a.wait_ns);
-                if (w0) { fail = w0 == 1 ? 2 : -1; break; }
+            for (int t = worker; t < total && ok; t += nworkers) {
+                if (!(ok = wait_warp<PAIR>(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, a.wait_ns, 2, fail))) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * BN;
                 const int sp = t / per_split;
                 const int num_kb = (int)((int64_t)all_kb * (sp + 1) / a.splits) - (int)((int64_t)all_kb * sp / a.splits);
                 for (int kb = 0; kb < num_kb; ++kb) {
-                    if (int w = mbar_wait(bar_full + 8 * stage, phase, abort_flag, a.wait_ns)) { fail = w == 1 ? 3 : -1; break; }
+                    if (!(ok = wait_warp(bar_full + 8 * stage, phase, abort_flag, a.wait_ns, 3, fail))) break;
                     tc_fence_after();
                     const uint32_t sa = sbase + stage * L::STAGE_BYTES, sb = sa + L::A_BYTES;
                     const uint64_t da = umma_desc(sa), db = umma_desc(sb);
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; ++k) {       // 16 values = 32 bytes of K per instruction
                         const uint64_t o = (uint64_t)(k * (UMMA_K >> 4));
-                        if (PAIR) umma_bf16_pair(d_tmem, da + o, db + o, idesc, (kb | k) != 0 ? 1u : 0u);
-                        else umma_bf16(d_tmem, da + o, db + o, idesc, (kb | k) != 0 ? 1u : 0u);
+                        if (PAIR) umma_bf16_pair(on, d_tmem, da + o, db + o, idesc, (kb | k) != 0 ? 1u : 0u);
+                        else umma_bf16(on, d_tmem, da + o, db + o, idesc, (kb | k) != 0 ? 1u : 0u);
                     }
-                    if (PAIR) umma_commit_pair(bar_empty + 8 * stage);
-                    else umma_commit(bar_empty + 8 * stage);
+                    if (PAIR) umma_commit_pair(on, bar_empty + 8 * stage);
+                    else umma_commit(on, bar_empty + 8 * stage);
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
                 }
-                if (fail) break;
-                if (PAIR) umma_commit_pair(bar_tfull + 8 * acc);
-                else umma_commit(bar_tfull + 8 * acc);
+                if (!ok) break;
+                if (PAIR) umma_commit_pair(on, bar_tfull + 8 * acc);
+                else umma_commit(on, bar_tfull + 8 * acc);
                 acc ^= 1;
                 if (acc == 0) acc_phase ^= 1;
             }

@@ -309,23 +309,23 @@ __device__ __forceinline__ void gemm_f32_body(const CUtensorMap& tmA, const CUte
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && leader) {
+        if (leader) {          // the whole warp; `on` is the lane that issues
+            const uint32_t on = elect_lane();
+            bool ok = true;
             constexpr uint32_t idesc = umma_idesc_bf16(TM_ROWS, BN);
             int stage = 0;
             uint32_t phase = 0, acc = 0, acc_phase = 0;
-            for (int t = worker; t < total && fail == 0; t += nworkers) {
+            for (int t = worker; t < total && ok; t += nworkers) {
                 const int sp = t / per_split, kb0 = first_kb(sp), kb1 = first_kb(sp + 1);
                 uint32_t d_tmem = 0;
                 for (int kb = kb0; kb < kb1; ++kb) {
                     const bool fresh = (kb - kb0) % GF_CHUNK == 0;
                     if (fresh) {
-                        const int w0 = PAIR ? mbar_wait_cluster(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, a.wait_ns)
-                                            : mbar_wait(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, a.wait_ns);
-                        if (w0) { fail = w0 == 1 ? 2 : -1; break; }
+                        if (!(ok = wait_warp<PAIR>(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, a.wait_ns, 2, fail))) break;
                         tc_fence_after();
                         d_tmem = tmem_base + acc * 2 * BN;
                     }
-                    if (int w = mbar_wait(bar_full + 8 * stage, phase, abort_flag, a.wait_ns)) { fail = w == 1 ? 3 : -1; break; }
+                    if (!(ok = wait_warp(bar_full + 8 * stage, phase, abort_flag, a.wait_ns, 3, fail))) break;
                     tc_fence_after();
                     const uint32_t sa = sbase + stage * L::STAGE_BYTES, sb = sa + 3 * L::A_BYTES;
 #pragma unroll
@@ -335,17 +335,17 @@ __device__ __forceinline__ void gemm_f32_body(const CUtensorMap& tmA, const CUte
 #pragma unroll
                         for (int k = 0; k < BK / UMMA_K; ++k) {
                             const uint64_t o = (uint64_t)(k * (UMMA_K >> 4));
-                            const uint32_t on = fresh && k == 0 && (i == 0 || i == 5) ? 0u : 1u, d = d_tmem + (i == 5 ? 0 : BN);
-                            if (PAIR) umma_bf16_pair(d, da + o, db + o, idesc, on);
-                            else umma_bf16(d, da + o, db + o, idesc, on);
+                            const uint32_t add = fresh && k == 0 && (i == 0 || i == 5) ? 0u : 1u, d = d_tmem + (i == 5 ? 0 : BN);
+                            if (PAIR) umma_bf16_pair(on, d, da + o, db + o, idesc, add);
+                            else umma_bf16(on, d, da + o, db + o, idesc, add);
                         }
                     }
-                    if (PAIR) umma_commit_pair(bar_empty + 8 * stage);
-                    else umma_commit(bar_empty + 8 * stage);
+                    if (PAIR) umma_commit_pair(on, bar_empty + 8 * stage);
+                    else umma_commit(on, bar_empty + 8 * stage);
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
                     if (kb + 1 == kb1 || (kb + 1 - kb0) % GF_CHUNK == 0) {
-                        if (PAIR) umma_commit_pair(bar_tfull + 8 * acc);
-                        else umma_commit(bar_tfull + 8 * acc);
+                        if (PAIR) umma_commit_pair(on, bar_tfull + 8 * acc);
+                        else umma_commit(on, bar_tfull + 8 * acc);
                         if (++acc == L::ACCS) { acc = 0; acc_phase ^= 1; }
                     }
                 }

@@ -131,18 +131,18 @@ __global__ void __launch_bounds__(LA_THREADS, 1)
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
                     if (k < steps) {
-                        umma_bf16_on(on, d, da + 2 * k, db + 2 * k, idesc_s, acc);
+                        umma_bf16(on, d, da + 2 * k, db + 2 * k, idesc_s, acc);
                         acc = 1;
                     }
             }
-            umma_commit_on(on, b_s + 8 * m);
+            umma_commit(on, b_s + 8 * m);
         };
         bool ok = wait(b_q, 0, 53) && wait(b_kf, 0, 53);
         if (ok) {
 #pragma unroll
             for (int m = 0; m < 2; ++m)
                 if (jlo >= lo[m] && jlo < hi[m]) scores(m, 0);
-            umma_commit_on(on, b_ke);
+            umma_commit(on, b_ke);
         }
         for (int j = jlo; j < jhi && ok; ++j) {
             const int i = j - jlo, vs = i % VS, kn = (i + 1) % KS;
@@ -156,17 +156,17 @@ __global__ void __launch_bounds__(LA_THREADS, 1)
 #pragma unroll
                     for (int k = 0; k < 8; ++k) {       // 16 keys: high and remainder terms, 8 columns each
                         const uint32_t pa = tmem + 128 * m + (k >> 1) * 32 + (k & 1) * 8;
-                        umma_bf16_ts_on(on, tmem + 256 + 128 * m, pa, dv + 128 * k, idesc_o, k > 0 ? 1u : (uint32_t)(j > lo[m]));
-                        umma_bf16_ts_on(on, tmem + 256 + 128 * m, pa + 16, dv + 128 * k, idesc_o, 1);
+                        umma_bf16_ts(on, tmem + 256 + 128 * m, pa, dv + 128 * k, idesc_o, k > 0 ? 1u : (uint32_t)(j > lo[m]));
+                        umma_bf16_ts(on, tmem + 256 + 128 * m, pa + 16, dv + 128 * k, idesc_o, 1);
                     }
-                    if (j + 1 == hi[m]) umma_commit_on(on, b_o + 8 * m);
+                    if (j + 1 == hi[m]) umma_commit(on, b_o + 8 * m);
                 }
                 if (j + 1 < jhi) {
                     if (m == 0 && !(ok = wait(b_kf + 8 * kn, ((i + 1) / KS) & 1, 53))) break;
                     if (j + 1 >= lo[m] && j + 1 < hi[m]) scores(m, kn);
-                    if (m == 1) umma_commit_on(on, b_ke + 8 * kn);
+                    if (m == 1) umma_commit(on, b_ke + 8 * kn);
                 }
-                if (m == 1) umma_commit_on(on, b_ve + 8 * vs);
+                if (m == 1) umma_commit(on, b_ve + 8 * vs);
             }
         }
         if (!on) fail = fail > 0 ? -1 : fail;      // one lane reports

@@ -164,20 +164,22 @@ __global__ void __launch_bounds__(RK_THREADS, 1) ret_chunk_kernel(const __grid_c
                 }
             }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {          // the whole warp; `on` is the lane that issues
+            const uint32_t on = elect_lane();
+            bool ok = true;
             constexpr uint32_t idesc = umma_idesc_bf16(128, 128) | IDESC_A_MN | IDESC_B_MN;
             for (int t = 0; t < ntile; ++t) {
-                if (int w = mbar_wait(b_full + 8 * t, 0, abort_flag, a.wait_ns)) { fail = w == 1 ? 41 : -1; break; }
+                if (!(ok = wait_warp(b_full + 8 * t, 0, abort_flag, a.wait_ns, 41, fail))) break;
                 tc_fence_after();
                 const uint32_t s = sbase + t * RK_TILE;
                 const uint64_t eh = umma_desc_mn(s, RT_BLK), el = umma_desc_mn(s + 2 * RT_BLK, RT_BLK), v = umma_desc_mn(s + 4 * RT_BLK, RT_BLK);
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
-                    umma_bf16(tmem, eh + 128 * k, v + 128 * k, idesc, (t | k) != 0);
-                    umma_bf16(tmem, el + 128 * k, v + 128 * k, idesc, 1);
+                    umma_bf16(on, tmem, eh + 128 * k, v + 128 * k, idesc, (t | k) != 0);
+                    umma_bf16(on, tmem, el + 128 * k, v + 128 * k, idesc, 1);
                 }
             }
-            if (fail == 0) umma_commit(b_done);
+            if (ok) umma_commit(on, b_done);
         }
     } else {
         int w = mbar_wait(b_done, 0, abort_flag, a.wait_ns);
@@ -312,35 +314,37 @@ __global__ void __launch_bounds__(RO_THREADS, 1)
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {          // the whole warp; `on` is the lane that issues
+            const uint32_t on = elect_lane();
+            bool ok = true;
             constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128), idesc_v = idesc_s | IDESC_B_MN;
             constexpr uint32_t idesc_64 = umma_idesc_bf16(128, 64) | IDESC_B_MN;
             int i = 0;
             auto next = [&](uint32_t& s) -> bool {
                 const int st = i % STAGES;
-                if (int w = mbar_wait(b_f + 8 * st, (i / STAGES) & 1, abort_flag, a.wait_ns)) { fail = w == 1 ? 44 : -1; return false; }
+                if (!(ok = wait_warp(b_f + 8 * st, (i / STAGES) & 1, abort_flag, a.wait_ns, 44, fail))) return false;
                 tc_fence_after();
                 s = ring + st * L::STAGE;
                 return true;
             };
-            auto done = [&]() { umma_commit(b_e + 8 * (i % STAGES)); ++i; };
+            auto done = [&]() { umma_commit(on, b_e + 8 * (i % STAGES)); ++i; };
             uint32_t s;
-            if (int w = mbar_wait(b_q, 0, abort_flag, a.wait_ns)) fail = w == 1 ? 44 : -1;
-            for (int t = 0; t < ntile && fail == 0; ++t) {
+            ok = wait_warp(b_q, 0, abort_flag, a.wait_ns, 44, fail);
+            for (int t = 0; t < ntile && ok; ++t) {
                 for (int b = 0; b < nkb; ++b) {
                     if (!next(s)) break;
                     const uint64_t qh = umma_desc(sbase + b * RT_BLK), ql = umma_desc(sbase + (KB + b) * RT_BLK), kh = umma_desc(s), kl = umma_desc(s + RT_BLK);
                     const int steps = min(4, (a.d - 64 * b + 15) / 16);
                     for (int k = 0; k < steps; ++k) {
-                        umma_bf16(tmem + 128 * t, qh + 2 * k, kh + 2 * k, idesc_s, (b | k) != 0);
-                        umma_bf16(tmem + 128 * t, qh + 2 * k, kl + 2 * k, idesc_s, 1);
-                        umma_bf16(tmem + 128 * t, ql + 2 * k, kh + 2 * k, idesc_s, 1);
+                        umma_bf16(on, tmem + 128 * t, qh + 2 * k, kh + 2 * k, idesc_s, (b | k) != 0);
+                        umma_bf16(on, tmem + 128 * t, qh + 2 * k, kl + 2 * k, idesc_s, 1);
+                        umma_bf16(on, tmem + 128 * t, ql + 2 * k, kh + 2 * k, idesc_s, 1);
                     }
                     done();
                 }
-                if (fail == 0) umma_commit(b_s + 8 * t);
+                if (ok) umma_commit(on, b_s + 8 * t);
             }
-            for (int r = 0; r < ndt && fail == 0; ++r)
+            for (int r = 0; r < ndt && ok; ++r)
                 for (int b = 0; b < nvb; ++b) {
                     if (!next(s)) break;
                     const uint64_t sh = umma_desc_mn(s, RT_BLK), sl = umma_desc_mn(s + RT_BLK, RT_BLK);
@@ -348,25 +352,25 @@ __global__ void __launch_bounds__(RO_THREADS, 1)
                     for (int k = 0; k < steps; ++k) {
                         const uint32_t qo = (2 * r + (k >> 2)) * RT_BLK;
                         const uint64_t qh = umma_desc(sbase + qo) + 2 * (k & 3), ql = umma_desc(sbase + KB * RT_BLK + qo) + 2 * (k & 3);
-                        umma_bf16(tmem + 384 + 64 * b, qh, sh + 128 * k, idesc_64, (r | k) != 0);
-                        umma_bf16(tmem + 384 + 64 * b, qh, sl + 128 * k, idesc_64, 1);
-                        umma_bf16(tmem + 384 + 64 * b, ql, sh + 128 * k, idesc_64, 1);
+                        umma_bf16(on, tmem + 384 + 64 * b, qh, sh + 128 * k, idesc_64, (r | k) != 0);
+                        umma_bf16(on, tmem + 384 + 64 * b, qh, sl + 128 * k, idesc_64, 1);
+                        umma_bf16(on, tmem + 384 + 64 * b, ql, sh + 128 * k, idesc_64, 1);
                     }
                     done();
                 }
-            for (int t = 0; t < ntile && fail == 0; ++t) {
-                if (int w = mbar_wait(b_p + 8 * t, 0, abort_flag, a.wait_ns)) { fail = w == 1 ? 44 : -1; break; }
+            for (int t = 0; t < ntile && ok; ++t) {
+                if (!(ok = wait_warp(b_p + 8 * t, 0, abort_flag, a.wait_ns, 44, fail))) break;
                 if (!next(s)) break;
                 const uint64_t v = umma_desc_mn(s, RT_BLK);
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
                     const uint32_t pa = tmem + 128 * t + (k >> 1) * 32 + (k & 1) * 8;
-                    umma_bf16_ts(tmem + 256, pa, v + 128 * k, idesc_v, (t | k) != 0);
-                    umma_bf16_ts(tmem + 256, pa + 16, v + 128 * k, idesc_v, 1);
+                    umma_bf16_ts(on, tmem + 256, pa, v + 128 * k, idesc_v, (t | k) != 0);
+                    umma_bf16_ts(on, tmem + 256, pa + 16, v + 128 * k, idesc_v, 1);
                 }
                 done();
             }
-            if (fail == 0) umma_commit(b_o);
+            if (ok) umma_commit(on, b_o);
         }
     } else {
         const int t = (warp - 2) >> 2, q = warp & 3, row = 32 * q + lane;

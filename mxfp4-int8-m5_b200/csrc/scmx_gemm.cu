@@ -103,29 +103,31 @@ __global__ void __launch_bounds__(CTA_THREADS, 1) gemm_i8_kernel(const __grid_co
         }
     } else if (warp == 1) {
         // ------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        {          // the whole warp; `on` is the lane that issues
+            const uint32_t on = elect_lane();
+            bool ok = true;
             constexpr uint32_t idesc = umma_idesc(BM, BN);
             int stage = 0;
             uint32_t phase = 0, acc = 0, acc_phase = 0;
-            for (int t = blockIdx.x; t < total && fail == 0; t += gridDim.x) {
-                if (int w = mbar_wait(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, a.wait_ns)) { fail = w == 1 ? 2 : -1; break; }
+            for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+                if (!(ok = wait_warp(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, a.wait_ns, 2, fail))) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * BN;
                 const int sp = t / tiles, num_kb = range_kb(a, all_kb, sp + 1) - range_kb(a, all_kb, sp);
                 for (int kb = 0; kb < num_kb; ++kb) {
-                    if (int w = mbar_wait(bar_full + 8 * stage, phase, abort_flag, a.wait_ns)) { fail = w == 1 ? 3 : -1; break; }
+                    if (!(ok = wait_warp(bar_full + 8 * stage, phase, abort_flag, a.wait_ns, 3, fail))) break;
                     tc_fence_after();
                     const uint32_t sa = sbase + stage * L::STAGE_BYTES, sb = sa + L::A_BYTES;
                     const uint64_t da = umma_desc(sa), db = umma_desc(sb);
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; ++k)
-                        umma_i8(d_tmem, da + (uint64_t)(k * (UMMA_K >> 4)), db + (uint64_t)(k * (UMMA_K >> 4)), idesc,
+                        umma_i8(on, d_tmem, da + (uint64_t)(k * (UMMA_K >> 4)), db + (uint64_t)(k * (UMMA_K >> 4)), idesc,
                                 (kb | k) != 0 ? 1u : 0u);
-                    umma_commit(bar_empty + 8 * stage);
+                    umma_commit(on, bar_empty + 8 * stage);
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
                 }
-                if (fail) break;
-                umma_commit(bar_tfull + 8 * acc);
+                if (!ok) break;
+                umma_commit(on, bar_tfull + 8 * acc);
                 acc ^= 1;
                 if (acc == 0) acc_phase ^= 1;
             }
@@ -281,29 +283,31 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CTA_THREADS, 1)
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && leader) {
+        if (leader) {          // the whole warp; `on` is the lane that issues
+            const uint32_t on = elect_lane();
+            bool ok = true;
             constexpr uint32_t idesc = umma_idesc(2 * BM, BN);
             int stage = 0;
             uint32_t phase = 0, acc = 0, acc_phase = 0;
-            for (int t = pair; t < total && fail == 0; t += npairs) {
-                if (int w = mbar_wait_cluster(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, a.wait_ns)) { fail = w == 1 ? 2 : -1; break; }
+            for (int t = pair; t < total && ok; t += npairs) {
+                if (!(ok = wait_warp<true>(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, a.wait_ns, 2, fail))) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * BN;
                 const int sp = t / tiles, num_kb = range_kb(a, all_kb, sp + 1) - range_kb(a, all_kb, sp);
                 for (int kb = 0; kb < num_kb; ++kb) {
-                    if (int w = mbar_wait(bar_full + 8 * stage, phase, abort_flag, a.wait_ns)) { fail = w == 1 ? 3 : -1; break; }
+                    if (!(ok = wait_warp(bar_full + 8 * stage, phase, abort_flag, a.wait_ns, 3, fail))) break;
                     tc_fence_after();
                     const uint32_t sa = sbase + stage * L::STAGE_BYTES, sb = sa + L::A_BYTES;
                     const uint64_t da = umma_desc(sa), db = umma_desc(sb);
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; ++k)
-                        umma_i8_pair(d_tmem, da + (uint64_t)(k * (UMMA_K >> 4)), db + (uint64_t)(k * (UMMA_K >> 4)), idesc,
+                        umma_i8_pair(on, d_tmem, da + (uint64_t)(k * (UMMA_K >> 4)), db + (uint64_t)(k * (UMMA_K >> 4)), idesc,
                                      (kb | k) != 0 ? 1u : 0u);
-                    umma_commit_pair(bar_empty + 8 * stage);
+                    umma_commit_pair(on, bar_empty + 8 * stage);
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
                 }
-                if (fail) break;
-                umma_commit_pair(bar_tfull + 8 * acc);
+                if (!ok) break;
+                umma_commit_pair(on, bar_tfull + 8 * acc);
                 acc ^= 1;
                 if (acc == 0) acc_phase ^= 1;
             }
