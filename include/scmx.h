@@ -218,6 +218,28 @@ int scmx_moe_mm_w4(const int8_t* xq, int64_t R, const uint32_t* codes, const uin
                    const int32_t* off, int E, int64_t N, int64_t K, const scmx_format* fmt, int epi, const float* xscale,
                    void* out, int32_t* status, void* stream);
 
+/* The same products on the tensor cores' 4-bit path (tcgen05 kind::mxf4): weights are read packed and expanded nowhere.  Activations are three
+ * planes of 4-bit digits to base eight, [3][drows][K / 2] bytes, x = d0 + 8 d1 + 64 d2, that scmx_digits makes from INT8 rows (dig row r = row tok[r], or
+ * row r without tok; ds[r] = xs[tok[r]] for r < R, either may be NULL).  Block factors, [E][ceil(N / 128)][K / 128][512] bytes, are made from the block
+ * codes u8 [E, N, K / 128] by scmx_f4_factors (several stacks in one launch).  Same INT32 totals bit for bit.  Format rule (scmx_f4_supported): the default format
+ * (e2m1 magnitudes, blocks of 32 times 1, 2, 4, 8), K % 128 == 0, K <= 10240; N % 32 == 0.  scmx_mm_f4 reads the first M of drows rows,
+ * scmx_moe_mm_f4 rows [off[e], off[e+1]) with expert e (E <= 512).  Status codes as scmx_mm_i8. */
+int scmx_f4_supported(const scmx_format* fmt, int64_t K);
+int scmx_digits(const int8_t* xq, const float* xs, const int32_t* tok, int64_t rows, int64_t R, int64_t K, uint32_t* dig, float* ds, void* stream);
+/* Row quantizer that writes digits: act_quant (nw NULL) or rmsnorm_quant of rows in nseg column segments (scmx_act_quant_seg; K <= 8192, K % 32 == 0), as
+ * digit planes [3][Mp][K / 2]; xq (INT8 rows) and xn (normalized rows) as well where given. */
+int scmx_row_quant_dig(const uint16_t* x, const uint16_t* nw, float eps, int64_t M, int64_t K, int64_t Mp, int nseg, int64_t seg_stride,
+                       int8_t* xq, uint32_t* dig, float* xs, uint16_t* xn, void* stream);
+typedef struct { const uint8_t* bcodes; uint8_t* factors; int64_t E, N, K; } scmx_f4_job;
+#define SCMX_F4_JOBS 8       /* stacks of matrices in one launch at most */
+int scmx_f4_factors(const scmx_f4_job* jobs, int n, void* stream);
+int scmx_mm_f4(const uint32_t* dig, int64_t drows, const uint32_t* codes, const uint8_t* factors, int64_t M, int64_t N, int64_t K,
+               const scmx_format* fmt, int epi, const float* xscale, const float* wscale, const uint16_t* res, void* out,
+               int32_t* status, void* stream);
+int scmx_moe_mm_f4(const uint32_t* dig, int64_t drows, int64_t R, const uint32_t* codes, const uint8_t* factors, const float* wscale,
+                   const int32_t* off, int E, int64_t N, int64_t K, const scmx_format* fmt, int epi, const float* xscale, void* out,
+                   int32_t* status, void* stream);
+
 /* scmx_moe_mm_w4 with the row-mapped epilogue of scmx_moe_mm_i8_ret (EPI 1; output row r stored at row ret_row[r] of
  * out_peers[ret_rank[r]]): the down GEMM of the expert-parallel block when the weights are read packed. */
 int scmx_moe_mm_w4_ret(const int8_t* xq, int64_t R, const uint32_t* codes, const uint8_t* bcodes, const float* wscale,

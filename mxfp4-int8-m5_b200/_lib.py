@@ -36,6 +36,11 @@ class ScmxGemvJob(ctypes.Structure):
                 ("K", ctypes.c_int32), ("epi", ctypes.c_int32), ("plan", ctypes.c_int32 * 15)]
 
 
+class ScmxF4Job(ctypes.Structure):
+    """Mirror of `scmx_f4_job` in include/scmx.h."""
+    _fields_ = [("bcodes", ctypes.c_void_p), ("factors", ctypes.c_void_p), ("E", ctypes.c_int64), ("N", ctypes.c_int64), ("K", ctypes.c_int64)]
+
+
 class ScmxError(RuntimeError):
     """A libscmx entry point returned a non-zero status."""
 
@@ -61,6 +66,12 @@ SIGNATURES = {
     "scmx_attn_decode": [c_vp, c_vp, c_vp, c_i64, c_vp, c_i64, c_float, c_int, c_int, c_int, c_int, c_vp, c_vp, c_vp, c_vp],
     "scmx_mm_i8": [c_vp, c_vp, c_i64, c_i64, c_i64, c_int, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp],
     "scmx_mm_i8_split": [c_vp, c_vp, c_i64, c_i64, c_i64, c_int, c_vp, c_vp, c_vp, c_vp, c_int, c_vp, c_vp, c_vp],
+    "scmx_f4_supported": [_FMT_P, c_i64],
+    "scmx_digits": [c_vp, c_vp, c_vp, c_i64, c_i64, c_i64, c_vp, c_vp, c_vp],
+    "scmx_row_quant_dig": [c_vp, c_vp, c_float, c_i64, c_i64, c_i64, c_int, c_i64, c_vp, c_vp, c_vp, c_vp, c_vp],
+    "scmx_f4_factors": [ctypes.POINTER(ScmxF4Job), c_int, c_vp],
+    "scmx_mm_f4": [c_vp, c_i64, c_vp, c_vp, c_i64, c_i64, c_i64, _FMT_P, c_int, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp],
+    "scmx_moe_mm_f4": [c_vp, c_i64, c_i64, c_vp, c_vp, c_vp, c_vp, c_int, c_i64, c_i64, _FMT_P, c_int, c_vp, c_vp, c_vp, c_vp],
     "scmx_w4_supported": [_FMT_P, c_i64],
     "scmx_mm_w4": [c_vp, c_vp, c_vp, c_i64, c_i64, c_i64, _FMT_P, c_int, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp],
     "scmx_moe_mm_w4": [c_vp, c_i64, c_vp, c_vp, c_vp, c_vp, c_int, c_i64, c_i64, _FMT_P, c_int, c_vp, c_vp, c_vp, c_vp],

@@ -228,6 +228,23 @@ __device__ __forceinline__ uint32_t quant4(float v0, float v1, float v2, float v
     return (b0 & 0xFFu) | ((b1 & 0xFFu) << 8) | ((b2 & 0xFFu) << 16) | (b3 << 24);
 }
 
+// Eight INT8 codes (two words) -> their balanced digits to base eight, x = d0 + 8 d1 + 64 d2 with -4 <= d0, d1 <= 3 and |d2| <= 2, one word of
+// eight e2m1 codes per digit (element i in bits 4 i .. 4 i + 3): a digit d is sign << 3 | |d|, the e2m1 number d / 2.
+// With t = x + 128 the digits plus four are (t + 36) mod 8, ((t + 36) / 8) mod 8 and (t + 36) / 64 + 2, taken from t / 4 + 41 so that bytes do not overflow.
+__device__ __forceinline__ uint32_t digit_codes(uint32_t lo, uint32_t hi) {        // digits plus four, a byte each
+    uint32_t e;
+    asm("prmt.b32 %0, %1, %2, 0x6420;" : "=r"(e) : "r"(lo | (lo >> 4)), "r"(hi | (hi >> 4)));
+    const uint32_t positive = ((e >> 2) & 0x11111111u) * 15u;
+    return (e & 0x33333333u & positive) | ((0xCCCCCCCCu - e) & ~positive);
+}
+__device__ __forceinline__ void digits8(uint32_t lo, uint32_t hi, uint32_t (&d)[3]) {
+    const uint32_t tl = lo ^ 0x80808080u, th = hi ^ 0x80808080u, M7 = 0x07070707u;
+    const uint32_t bl = ((tl >> 2) & 0x3F3F3F3Fu) + 0x29292929u, bh = ((th >> 2) & 0x3F3F3F3Fu) + 0x29292929u;
+    d[0] = digit_codes((tl & M7) ^ 0x04040404u, (th & M7) ^ 0x04040404u);
+    d[1] = digit_codes((bl >> 1) & M7, (bh >> 1) & M7);
+    d[2] = digit_codes((bl >> 4) & M7, (bh >> 4) & M7);
+}
+
 // Decode one 32-bit word of 8 packed codes to two words of 4 INT8 each, given per-block byte LUTs
 // (positive magnitudes already multiplied by the block multiplier, and their negations).
 __device__ __forceinline__ void decode_word(uint32_t w, uint32_t plo, uint32_t phi, uint32_t nlo, uint32_t nhi,

@@ -189,6 +189,19 @@ __device__ __forceinline__ uint2 pack8_i8(const int q[8]) {
     return o;
 }
 
+// Digit planes of the quantized rows (digits8), beside the INT8 rows or in their place: word v of row r and digit p at p * plane + r * (K / 8) + v.
+struct RowDigits {
+    uint32_t* p;         // or null
+    int64_t plane;
+    __device__ __forceinline__ void store(int64_t word, uint32_t lo, uint32_t hi) const {
+        if (p == nullptr) return;
+        uint32_t d[3];
+        digits8(lo, hi, d);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) p[i * plane + word] = d[i];
+    }
+};
+
 // WPR warps share a row (WPR = 1, 2 or 4; 8 / WPR rows per CTA): each lane holds MAXV vectors, vector v = (i * WPR + part) * 32 +
 // lane.  With few rows (one warp per row leaves an SM a dozen warps) splitting a row shortens every warp's dependent chain and
 // doubles the warps that hide it; the partial sums and maxima meet through shared memory behind a barrier of the row's warps.
@@ -196,7 +209,7 @@ template <int MAXV, bool NORM, int WPR>
 __global__ void __launch_bounds__(256) row_quant_warp_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ nw,
                                                              float eps, int64_t M, int64_t Mp, int K, RowSegs sg,
                                                              int8_t* __restrict__ xq, float* __restrict__ xs,
-                                                             uint16_t* __restrict__ xn) {
+                                                             uint16_t* __restrict__ xn, RowDigits dg) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ double s_ss[8];
@@ -212,7 +225,8 @@ __global__ void __launch_bounds__(256) row_quant_warp_kernel(const uint16_t* __r
         for (int i = 0; i < MAXV; ++i) {
             const int v = (i * WPR + part) * 32 + lane;
             if (v < nv) {
-                qrow[v] = make_uint2(0, 0);
+                if (xq) qrow[v] = make_uint2(0, 0);
+                dg.store(row * nv + v, 0, 0);
                 if (NORM && xn) reinterpret_cast<uint4*>(xn + row * K)[v] = make_uint4(0, 0, 0, 0);
             }
         }
@@ -277,7 +291,9 @@ __global__ void __launch_bounds__(256) row_quant_warp_kernel(const uint16_t* __r
         if (v < nv) {
             float f[8];
             unpack8(raw[i], f);
-            qrow[v] = make_uint2(quant4(f[0], f[1], f[2], f[3], qi), quant4(f[4], f[5], f[6], f[7], qi));
+            const uint32_t lo = quant4(f[0], f[1], f[2], f[3], qi), hi = quant4(f[4], f[5], f[6], f[7], qi);
+            if (xq) qrow[v] = make_uint2(lo, hi);
+            dg.store(row * nv + v, lo, hi);
         }
     }
     if (lane == 0 && part == 0) xs[row] = s;
@@ -287,7 +303,7 @@ __global__ void __launch_bounds__(256) row_quant_warp_kernel(const uint16_t* __r
 template <int MAXV, bool NORM>
 __global__ void __launch_bounds__(256) row_quant_block_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ nw,
                                                               float eps, int64_t M, int K, RowSegs sg, int8_t* __restrict__ xq,
-                                                              float* __restrict__ xs, uint16_t* __restrict__ xn) {
+                                                              float* __restrict__ xs, uint16_t* __restrict__ xn, RowDigits dg) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ float red[33];
@@ -300,7 +316,8 @@ __global__ void __launch_bounds__(256) row_quant_block_kernel(const uint16_t* __
         for (int i = 0; i < MAXV; ++i) {
             const int v = i * 256 + threadIdx.x;
             if (v < nv) {
-                qrow[v] = make_uint2(0, 0);
+                if (xq) qrow[v] = make_uint2(0, 0);
+                dg.store(row * nv + v, 0, 0);
                 if (NORM && xn) reinterpret_cast<uint4*>(xn + row * K)[v] = make_uint4(0, 0, 0, 0);
             }
         }
@@ -351,7 +368,9 @@ __global__ void __launch_bounds__(256) row_quant_block_kernel(const uint16_t* __
         if (v < nv) {
             float f[8];
             unpack8(raw[i], f);
-            qrow[v] = make_uint2(quant4(f[0], f[1], f[2], f[3], qi), quant4(f[4], f[5], f[6], f[7], qi));
+            const uint32_t lo = quant4(f[0], f[1], f[2], f[3], qi), hi = quant4(f[4], f[5], f[6], f[7], qi);
+            if (xq) qrow[v] = make_uint2(lo, hi);
+            dg.store(row * nv + v, lo, hi);
         }
     }
     if (threadIdx.x == 0) xs[row] = s;
@@ -359,7 +378,7 @@ __global__ void __launch_bounds__(256) row_quant_block_kernel(const uint16_t* __
 
 template <bool NORM>
 static bool launch_row_quant_warp(const uint16_t* x, const uint16_t* nw, float eps, int64_t M, int64_t Mp, int64_t K,
-                                  int nseg, int64_t seg_stride, int8_t* xq, float* xs, uint16_t* xn, cudaStream_t st) {
+                                  int nseg, int64_t seg_stride, int8_t* xq, float* xs, uint16_t* xn, cudaStream_t st, RowDigits dg = {}) {
     const unsigned grid = (unsigned)((Mp + 7) / 8);
     RowSegs sg;
     sg.w8 = (int)(K / nseg / 8);
@@ -372,14 +391,14 @@ static bool launch_row_quant_warp(const uint16_t* x, const uint16_t* nw, float e
     // kernel alone, launched back to back, prefers one warp per row): RMSNorm + INT8 with 4 warps per row 3.754 -> 3.705 ms per
     // step, act-quant with 2 warps per row a further 0.008 ms.
     const int wpr = (Mp <= 4096 && K > 1024 && K <= 2048) ? (NORM ? 4 : 2) : 1;     // 8 / 4 warps per row measured slower: 3.70 - 3.73 ms
-    if (Mp <= block_rows && K <= 2048) launch_pdl(row_quant_block_kernel<1, NORM>, dim3((unsigned)Mp), dim3(256), 0, st, x, nw, eps, M, (int)K, sg, xq, xs, xn);
-    else if (Mp <= block_rows && K <= 2048 * 4) launch_pdl(row_quant_block_kernel<4, NORM>, dim3((unsigned)Mp), dim3(256), 0, st, x, nw, eps, M, (int)K, sg, xq, xs, xn);
-    else if (wpr == 2 && K <= 256 * 8) launch_pdl(row_quant_warp_kernel<4, NORM, 2>, dim3((unsigned)((Mp + 3) / 4)), dim3(256), 0, st, x, nw, eps, M, Mp, (int)K, sg, xq, xs, xn);
-    else if (wpr == 4 && K <= 256 * 8) launch_pdl(row_quant_warp_kernel<2, NORM, 4>, dim3((unsigned)((Mp + 1) / 2)), dim3(256), 0, st, x, nw, eps, M, Mp, (int)K, sg, xq, xs, xn);
-    else if (K <= 256 * 4) launch_pdl(row_quant_warp_kernel<4, NORM, 1>, dim3(grid), dim3(256), 0, st, x, nw, eps, M, Mp, (int)K, sg, xq, xs, xn);
-    else if (K <= 256 * 8) launch_pdl(row_quant_warp_kernel<8, NORM, 1>, dim3(grid), dim3(256), 0, st, x, nw, eps, M, Mp, (int)K, sg, xq, xs, xn);
-    else if (K <= 256 * 16) launch_pdl(row_quant_warp_kernel<16, NORM, 1>, dim3(grid), dim3(256), 0, st, x, nw, eps, M, Mp, (int)K, sg, xq, xs, xn);
-    else if (K <= 2048 * 4) launch_pdl(row_quant_block_kernel<4, NORM>, dim3((unsigned)Mp), dim3(256), 0, st, x, nw, eps, M, (int)K, sg, xq, xs, xn);
+    if (Mp <= block_rows && K <= 2048) launch_pdl(row_quant_block_kernel<1, NORM>, dim3((unsigned)Mp), dim3(256), 0, st, x, nw, eps, M, (int)K, sg, xq, xs, xn, dg);
+    else if (Mp <= block_rows && K <= 2048 * 4) launch_pdl(row_quant_block_kernel<4, NORM>, dim3((unsigned)Mp), dim3(256), 0, st, x, nw, eps, M, (int)K, sg, xq, xs, xn, dg);
+    else if (wpr == 2 && K <= 256 * 8) launch_pdl(row_quant_warp_kernel<4, NORM, 2>, dim3((unsigned)((Mp + 3) / 4)), dim3(256), 0, st, x, nw, eps, M, Mp, (int)K, sg, xq, xs, xn, dg);
+    else if (wpr == 4 && K <= 256 * 8) launch_pdl(row_quant_warp_kernel<2, NORM, 4>, dim3((unsigned)((Mp + 1) / 2)), dim3(256), 0, st, x, nw, eps, M, Mp, (int)K, sg, xq, xs, xn, dg);
+    else if (K <= 256 * 4) launch_pdl(row_quant_warp_kernel<4, NORM, 1>, dim3(grid), dim3(256), 0, st, x, nw, eps, M, Mp, (int)K, sg, xq, xs, xn, dg);
+    else if (K <= 256 * 8) launch_pdl(row_quant_warp_kernel<8, NORM, 1>, dim3(grid), dim3(256), 0, st, x, nw, eps, M, Mp, (int)K, sg, xq, xs, xn, dg);
+    else if (K <= 256 * 16) launch_pdl(row_quant_warp_kernel<16, NORM, 1>, dim3(grid), dim3(256), 0, st, x, nw, eps, M, Mp, (int)K, sg, xq, xs, xn, dg);
+    else if (K <= 2048 * 4) launch_pdl(row_quant_block_kernel<4, NORM>, dim3((unsigned)Mp), dim3(256), 0, st, x, nw, eps, M, (int)K, sg, xq, xs, xn, dg);
     else return false;
     return true;
 }
@@ -827,6 +846,19 @@ extern "C" int scmx_rmsnorm_quant_seg(const uint16_t* x, const uint16_t* nw, flo
     return SCMX_OK;
 }
 
+extern "C" int scmx_row_quant_dig(const uint16_t* x, const uint16_t* nw, float eps, int64_t M, int64_t K, int64_t Mp, int nseg, int64_t seg_stride,
+                                  int8_t* xq, uint32_t* dig, float* xs, uint16_t* xn, void* stream) {
+    int rc = check_seg("row_quant_dig", M, K, Mp, nseg, seg_stride);
+    if (rc) return rc;
+    SCMX_REQUIRE(dig && xs && K % 32 == 0 && aligned16(x) && aligned16(dig) && (!nw || aligned16(nw)) && (!xq || aligned16(xq)) && (!xn || (nw && aligned16(xn))),
+                 SCMX_EINVAL, "row_quant_dig: K %% 32 == 0, buffers 16-byte aligned (K=%lld)", (long long)K);
+    if (Mp == 0) return SCMX_OK;
+    const RowDigits dg = {dig, Mp * (K / 8)};
+    if (nw) launch_row_quant_warp<true>(x, nw, eps, M, Mp, K, nseg, seg_stride, xq, xs, xn, (cudaStream_t)stream, dg);
+    else launch_row_quant_warp<false>(x, nullptr, 0.0f, M, Mp, K, nseg, seg_stride, xq, xs, nullptr, (cudaStream_t)stream, dg);
+    SCMX_LAUNCH_OK("row_quant kernel");
+    return SCMX_OK;
+}
 
 extern "C" int scmx_rot_quant(const uint16_t* x, const float* signs, int64_t M, int64_t K, int64_t Mp, int8_t* xq, float* xs,
                               void* stream) {

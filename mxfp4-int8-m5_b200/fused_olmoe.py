@@ -156,6 +156,47 @@ class FusedOlmoe:
             self._ready[i] = torch.cuda.Event()
             self._ready[i].record(self.side)
 
+    # rows per expert up to which a prompt runs on digit planes.  Two layers of 64 experts, us, packed grouped products / digit planes: 2048 x 1024, 2 rows per expert
+    # 427 / 250, 16 463 / 278, 128 571 / 515, 256 843 / 810, 375 1034 / 1085; 1024 x 512, 2 rows 233 / 166, 256 488 / 480, 375 616 / 634
+    F4_ROWS = 256
+
+    def _f4(self, L):
+        """Whether a prompt runs on digit planes and packed weights throughout (the tensor cores' 4-bit path, 1.5 times the tensor work of INT8 but no expansion): few
+        rows per expert, the default format, and this class's own methods."""
+        a = self.args
+        own = type(self).experts is _EXPERTS and "experts" not in self.__dict__
+        R = L * a.num_experts_per_tok
+        return (own and self.record is None and R // a.num_experts <= self.F4_ROWS and self._packed(R) and max(a.hidden_size, a.intermediate_size, self.layers[0][1]["o"].K) <= 8192
+                and M_.f4_fits(a.num_experts, a.hidden_size, a.intermediate_size, self.layers[0][1]["o"].K))
+
+    def _hidden_f4(self, h, cache, L):
+        """The blocks on digit planes: same bits as the products from INT8."""
+        a = self.args
+        H, d, D, E, Fi, nl = a.num_attention_heads, a.head_dim, a.hidden_size, a.num_experts, a.intermediate_size, len(self.layers)
+        R = L * a.num_experts_per_tok
+        dig, xs = S.quant_digits(h, self.layers[0][0].input_layernorm.weight, self.eps)
+        for i, (layer, ws, ex) in enumerate(self.layers):
+            at, c, wq, wo = layer.self_attn, cache[i], ws["qkv"], ws["o"]
+            fq, fo, fg, fd = M_.f4_factors((wq.bcodes, 1, wq.N, wq.K), (wo.bcodes, 1, wo.N, wo.K), (ex["gu"][1], E, 2 * Fi, D), (ex["down"][1], E, D, Fi))
+            y = S.mm_f4(dig, wq.codes, fq, xs, wq.wscale, 1)
+            q, kk, v = S.qkv_fullnorm_y(y, at.q_norm.weight, at.k_norm.weight, self.eps, L, H, d, rope=(self.inv_freq, c.offset, self.rope_cs), cache=c)
+            c.offset += L
+            dig, xs = attend_quant(self.sdpa, q, kk, v, at.scale, L, digits=True)
+            h = S.mm_f4(dig, wo.codes, fo, xs, wo.wscale, 2, res=h)
+            xq, xs, xn = S.rmsnorm_quant_n(h, layer.post_attention_layernorm.weight, self.eps, L)
+            inds, scores = self.route(layer, xn, L)
+            pos, tok, _, off, _, _ = M_.route_sort(inds, E, M_.TM)
+            dig, xs = M_.gather_digits(xq, xs, tok, R)
+            (cg, _, sg), (cd, _, sd) = ex["gu"], ex["down"]
+            act = M_.moe_mm_f4(dig, R, cg, fg, sg, off, 2 * Fi, 3, xs)
+            dig, xs = S.quant_digits(act)
+            yd = M_.moe_mm_f4(dig, R, cd, fd, sd, off, D, 1, xs)
+            nn = self.layers[i + 1][0].input_layernorm.weight if i + 1 < nl else self.model.model.norm.weight
+            h, xq, xs = M_.moe_combine(yd, pos, scores, h, nn, self.eps, L, quant=i + 1 < nl)
+            if i + 1 < nl:
+                dig, _ = M_.gather_digits(xq, None, None, L)
+        return h
+
     def experts(self, ex, xq, xs, inds, L, decoded=None):
         """INT8 rows + routing -> (sorted expert outputs yd bf16 [R, D], pos).  decoded: (gu8, dn8) INT8 copies of this
         layer's experts when they were decoded ahead."""
@@ -188,6 +229,9 @@ class FusedOlmoe:
         H, d, D = a.num_attention_heads, a.head_dim, a.hidden_size
         h = self.model.model.embed_tokens(ids)[0]
         L = h.shape[0]
+        if L > 0 and self._f4(L):
+            h = self._hidden_f4(h.contiguous(), cache, L)
+            return S.rmsnorm_quant_n(h, self.model.model.norm.weight, self.eps, L)[2][None]
         Mp = S.pad_rows(L)
         if Mp != L:
             h = torch.nn.functional.pad(h, (0, 0, 0, Mp - L))
@@ -244,4 +288,4 @@ def load_fused_olmoe(model, cache_path=None, **kw):
     return FusedOlmoe(model, pack_olmoe(model, cache_path), **kw)
 
 
-_ROUTE = FusedOlmoe.route      # as this file defines it
+_ROUTE, _EXPERTS = FusedOlmoe.route, FusedOlmoe.experts      # as this file defines them

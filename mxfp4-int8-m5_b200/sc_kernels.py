@@ -64,6 +64,31 @@ def act_quant_seg(xseg, Mp=None):
     return xq, xs
 
 
+def quant_digits(x, w=None, eps=0.0, segments=False):
+    """act_quant (w None) or rmsnorm_quant of x bf16 [M, K], or of rows in column segments [G, M, K / G], as digit planes for the products on
+    the tensor cores' 4-bit path: (int32 [3, M, K / 8], xscale f32 [M]).  K <= 8192, a multiple of 32."""
+    _lib.require_cuda(x, w)
+    G, M, ws = _bf16(x).shape if segments else (1, *_bf16(x).shape)
+    K = G * ws
+    dig = torch.empty((3, M, K // 8), dtype=torch.int32, device=x.device)
+    xs = torch.empty(M, dtype=torch.float32, device=x.device)
+    _lib.call("scmx_row_quant_dig", _lib.ptr(x), _lib.ptr(w), _eps(eps), M, K, M, G, M * ws if G > 1 else 0, None, _lib.ptr(dig), _lib.ptr(xs), None, _lib.stream())
+    return dig, xs
+
+
+def mm_f4(dig, codes, factors, xscale, wscale, epi, res=None):
+    """mm_epi of rows given as digit planes with packed weights and their block factors (sc_moe.f4_factors): same bits, no decoded weights.  epi 0: INT32."""
+    _lib.require_cuda(dig, codes, factors, xscale, wscale, res)
+    _, M, K8 = dig.shape
+    N, K = wscale.shape[0], K8 * 8
+    assert epi in (0, 1, 2, 3) and N % 32 == 0 and (epi != 2 or tuple(res.shape) == (M, N))
+    out = torch.empty((M, N), dtype=torch.int32, device=dig.device) if epi == 0 else \
+        torch.empty((M, N // 2 if epi == 3 else N), dtype=torch.bfloat16, device=dig.device)
+    _lib.call("scmx_mm_f4", _lib.ptr(dig), M, _lib.ptr(codes), _lib.ptr(factors), M, N, K, F.DEFAULT.c_struct(), epi, _lib.ptr(xscale), _lib.ptr(wscale),
+              _lib.ptr(res) if epi == 2 else None, _lib.ptr(out), _lib.ptr(_lib.status_buffer()), _lib.stream())
+    return out
+
+
 def rmsnorm_quant_seg(xseg, w, eps, Mp=None):
     """rmsnorm_quant of rows stored as column segments (see act_quant_seg)."""
     _lib.require_cuda(xseg, w)

@@ -83,6 +83,41 @@ def gather_rows(xq, xs, tok, R):
     return dq, ds
 
 
+def f4_fits(n_experts, *widths):
+    """Whether the products on digit planes (moe_mm_f4) take this many experts and these input widths in the current default format."""
+    return n_experts <= 512 and all(_lib.lib().scmx_f4_supported(F.DEFAULT.c_struct(), k) for k in widths)
+
+
+def gather_digits(xq, xs, tok, R):
+    """gather_rows as digit planes: (int32 [3, R, K / 8], scales [R]) of the rows tok[:R] (of xq itself without tok; no scales without xs)."""
+    _lib.require_cuda(xq, xs, tok)
+    K = xq.shape[1]
+    dig = torch.empty((3, R, K // 8), dtype=torch.int32, device=xq.device)
+    ds = torch.empty(R, dtype=torch.float32, device=xq.device) if xs is not None else None
+    _lib.call("scmx_digits", _lib.ptr(xq), _lib.ptr(xs), _lib.ptr(tok), R, R, K, _lib.ptr(dig), _lib.ptr(ds), _lib.stream())
+    return dig, ds
+
+
+def f4_factors(*mats):
+    """Block factors (scmx_f4_factors) of up to 8 stacks of packed matrices, each (block codes, matrices, N, K), in one launch -> a uint8 tensor per stack."""
+    _lib.require_cuda(*(m[0] for m in mats))
+    sizes = [e * -(-n // 128) * (k // 128) * 512 for _, e, n, k in mats]
+    out = torch.empty(sum(sizes), dtype=torch.uint8, device=mats[0][0].device).split(sizes)
+    jobs = (_lib.ScmxF4Job * len(mats))(*(_lib.ScmxF4Job(_lib.ptr(b), _lib.ptr(o), e, n, k) for (b, e, n, k), o in zip(mats, out)))
+    _lib.call("scmx_f4_factors", jobs, len(mats), _lib.stream())
+    return out
+
+
+def moe_mm_f4(dig, R, codes, factors, wscale, off, N, epi, xscale=None):
+    """moe_mm of rows given as digit planes, on the tensor cores' 4-bit path: same bits."""
+    _lib.require_cuda(dig, codes, factors, wscale, off, xscale)
+    E, K = wscale.shape[0], dig.shape[2] * 8
+    out = _out(R, N, epi, dig.device)
+    _lib.call("scmx_moe_mm_f4", _lib.ptr(dig), dig.shape[1], R, _lib.ptr(codes), _lib.ptr(factors), _lib.ptr(wscale), _lib.ptr(off), E, N, K, F.DEFAULT.c_struct(),
+              epi, _lib.ptr(xscale), _lib.ptr(out), _lib.ptr(_lib.status_buffer()), _lib.stream())
+    return out
+
+
 def _out(R, N, epi, dev):
     if epi == 0:
         return torch.empty((R, N), dtype=torch.int32, device=dev)
