@@ -394,17 +394,18 @@ typedef struct scmx_decode_layer {
 /* All layers of one batch-1 decode step in one cooperative launch: h bf16 [D] (in: the token's embedding, out: the residual
  * stream after the last layer) goes through n_layers of RMSNorm + INT8 -> q|k|v GEMV -> q/k head RMSNorm + rotary embedding
  * + cache append at row pos_dev[0] -> attention over pos_dev[0] + 1 positions -> o GEMV + residual -> RMSNorm + INT8 ->
- * gate|up GEMV with SwiGLU -> INT8 -> down GEMV + residual, the chain of e2e/decode.py:58-110, with grid-wide barriers
- * between the steps instead of kernel boundaries.  Same bits as scmx_rmsnorm_quant / scmx_gemv / scmx_qkv_norm /
+ * gate|up GEMV with SwiGLU -> INT8 -> down GEMV + residual, the chain of e2e/decode.py:58-110, rows travelling between the
+ * CTAs as packets that carry an epoch instead of kernel boundaries.  Same bits as scmx_rmsnorm_quant / scmx_gemv / scmx_qkv_norm /
  * scmx_attn_decode (with the same nsplit) / scmx_act_quant called in that order.
- * layers: device array; y bf16 [(hq + 2 hk) d], act bf16 [F], o bf16 [hq d], partials f32 [hq, nsplit, d + 2], barrier
- * uint32 [2] are scratch; counters int32 [hk] is scratch too (zeroed by every call on its stream); status int32 [1] receives 100 + k if barrier k timed out (0.5 s), after which the step's outputs are invalid.
- * Limits: d = 128; D, F and hq*d multiples of 1024 up to 6144; hq/hk in {1, 2, 4}; hk * nsplit <= number of SMs.
+ * layers: device array; scratch: scmx_decode_step_scratch bytes, 16-byte aligned, zero before its first use and then left to the steps that
+ * share it, which must not overlap; status int32 [1] receives 1000 + 5 layer + k if a wait timed out (0.5 s), k = 0 residual row, 1 q|k|v, 2 attention,
+ * 3 residual row after it, 4 feed-forward row, after which the step's outputs are invalid.
+ * Limits: d = 128; D, F and hq*d multiples of 1024 up to 6144; hq/hk in {1, 2, 4}; hk * nsplit <= number of SMs (64 to 256).
  * Not to be run concurrently with other work on the same device: the launch needs every SM. */
+int64_t scmx_decode_step_scratch(int D, int F, int hq, int hk, int d, int nsplit);
 int scmx_decode_step_dense(const scmx_decode_layer* layers, int n_layers, int D, int F, int hq, int hk, int d, float eps,
                            float scale, const float* inv_freq, const float* rope_table, int64_t rope_rows, int64_t capacity,
-                           const int32_t* pos_dev, uint16_t* h, uint16_t* y, uint16_t* act, uint16_t* o, float* partials,
-                           int nsplit, int32_t* counters, uint32_t* barrier, int32_t* status, void* stream);
+                           const int32_t* pos_dev, uint16_t* h, void* scratch, int nsplit, int32_t* status, void* stream);
 /* Output head of one row: out bf16 [N] = W bf16 [N, ldw] x, x bf16 [K], float32 sums.  K a multiple of 8 up to 6400, rows 16-byte aligned. */
 int scmx_head_bf16(const uint16_t* W, int64_t ldw, const uint16_t* x, int64_t N, int64_t K, uint16_t* out, void* stream);
 /* Greedy choice inside a captured decode step: *tok = out[*count] = index of the largest of V logits (bf16 or float; the lowest of equal ones, a

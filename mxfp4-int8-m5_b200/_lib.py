@@ -106,8 +106,8 @@ SIGNATURES = {
                               c_int, c_int, c_vp, c_vp, c_vp, c_vp],
     "scmx_moe_combine": [c_vp, c_vp, c_vp, c_vp, c_vp, c_float, c_i64, c_i64, c_i64, c_int, c_int, c_vp, c_vp, c_vp,
                          c_vp],
-    "scmx_decode_step_dense": [c_vp, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_vp, c_vp, c_i64, c_i64, c_vp,
-                               c_vp, c_vp, c_vp, c_vp, c_vp, c_int, c_vp, c_vp, c_vp, c_vp],
+    "scmx_decode_step_scratch": [c_int] * 6,
+    "scmx_decode_step_dense": [c_vp, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_vp, c_vp, c_i64, c_i64, c_vp, c_vp, c_vp, c_int, c_vp, c_vp],
     "scmx_set_decode_trace": [c_vp, c_int],
     "scmx_select_token": [c_vp, c_int, c_i64, c_vp, c_vp, c_vp, c_vp, c_i64, c_vp],
     "scmx_head_bf16": [c_vp, c_i64, c_vp, c_i64, c_i64, c_vp, c_vp],
@@ -167,7 +167,7 @@ MIXER_SIGNATURES = {
     "scmx_gemv_x": [c_vp, c_i64, c_int, c_vp, c_i64, c_i64, c_int, c_float, c_float, c_vp, c_vp, c_vp, c_int, c_int, c_vp, c_vp],
     "scmx_last_error_string": [],
 }
-_RESTYPE = {"scmx_last_error_string": ctypes.c_char_p, "scmx_retention_scratch": c_i64, "scmx_delta_scratch": c_i64}
+_RESTYPE = {"scmx_last_error_string": ctypes.c_char_p, "scmx_retention_scratch": c_i64, "scmx_delta_scratch": c_i64, "scmx_decode_step_scratch": c_i64}
 
 _lib = None
 _mixers = None
@@ -326,9 +326,14 @@ _GEMM_ROLES = {51: "latent attention producer waiting for a free key tile", 52: 
                12: "streaming GEMV consumer waiting for a tile", 20: "peer barrier waiting for another rank's flag"}
 
 
+_STEP_ROWS = ("input row", "q|k|v row", "attention output", "residual row after attention", "feed-forward row")
+
+
 def describe_status(code):
-    """Text for a status-word code: 1..5 GEMM roles, 11 / 12 streaming GEMV, 20 peer barrier, 100 + k = grid barrier k of
-    the one-kernel decode step."""
+    """Text for a status-word code: 1..5 GEMM roles, 11 / 12 streaming GEMV, 20 peer barrier, 100 + k grid barrier k, 1000 + 5 layer + k
+    row k of a layer of the one-kernel decode step."""
+    if code >= 1000:
+        return f"decode step: layer {(code - 1000) // 5} waiting for its {_STEP_ROWS[(code - 1000) % 5]}"
     if code >= 100:
         return f"decode step: grid barrier {code - 100} timed out"
     return _GEMM_ROLES.get(code, f"code {code}")

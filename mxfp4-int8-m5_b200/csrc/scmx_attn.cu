@@ -35,7 +35,8 @@ __global__ void __launch_bounds__(AD_THREADS) attn_decode_kernel(const AttnArgs 
     const int64_t t0 = (int64_t)split * chunk, t1 = t0 + chunk < T ? t0 + chunk : T;
     constexpr int stride = D + 2;
     attn_split<G, D>(a.q + (size_t)kvh * G * D, a.k + (size_t)kvh * a.cap * D, a.v + (size_t)kvh * a.cap * D, t0, t1, -1, nullptr,
-                     nullptr, a.scale, a.part + ((size_t)kvh * G * a.nsplit + split) * stride, (size_t)a.nsplit * stride, sm);
+                     nullptr, a.scale,
+                     [&](int g, int i, float v) { a.part[((size_t)(kvh * G + g) * a.nsplit + split) * stride + i] = v; }, sm);
     __threadfence();
     __syncthreads();
     if (tid == 0) s_ticket = atomicAdd(a.counters + kvh, 1);

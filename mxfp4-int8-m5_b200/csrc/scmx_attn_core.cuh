@@ -43,12 +43,11 @@ __device__ __forceinline__ void merge_state(float& m, float& l, float (&a)[E], f
 // One (key/value head, split) task, run by the first AD_THREADS threads of the CTA (every thread of the CTA must call it:
 // it contains __syncthreads).  q: bf16 [G][D] of the G query heads sharing this key/value head; kb / vb: the head's cache
 // rows [cap][D]; positions [t0, t1).  Position t_new (or -1) is read from knew / vnew (bf16 [D]) instead of the cache.
-// q, knew, vnew may point to shared or global memory.  Writes the G partial states to part + g * part_stride_g:
-// D unnormalized outputs, the running maximum (log2 domain), the running sum.
-template <int G, int D>
+// q, knew, vnew may point to shared or global memory.  put(g, i, value) stores the G partial states: D unnormalized outputs, the running
+// maximum (log2 domain), the running sum.
+template <int G, int D, typename Put>
 __device__ __forceinline__ void attn_split(const uint16_t* q, const uint16_t* kb, const uint16_t* vb, int64_t t0, int64_t t1,
-                                           int64_t t_new, const uint16_t* knew, const uint16_t* vnew, float scale, float* part,
-                                           size_t part_stride_g, AttnSmem<G, D>& sm) {
+                                           int64_t t_new, const uint16_t* knew, const uint16_t* vnew, float scale, Put put, AttnSmem<G, D>& sm) {
     constexpr int E = D / 8;                  // elements per lane
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, slot = lane >> 3, l8 = lane & 7;
     if (tid < AD_THREADS) {
@@ -157,11 +156,10 @@ __device__ __forceinline__ void attn_split(const uint16_t* q, const uint16_t* kb
                 ll += sm.ml[w][g][1] * c;
                 if (tid < D) av += sm.acc[w][g][tid] * c;
             }
-            float* p = part + (size_t)g * part_stride_g;
-            if (tid < D) p[tid] = av;
+            if (tid < D) put(g, tid, av);
             if (tid == 0) {
-                p[D] = mm;
-                p[D + 1] = ll;
+                put(g, D, mm);
+                put(g, D + 1, ll);
             }
         }
     }

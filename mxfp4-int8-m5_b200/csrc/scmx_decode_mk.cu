@@ -1,25 +1,32 @@
-// One decode step of a dense (Qwen3-style) stack as ONE persistent kernel: every SM keeps a CTA resident for the whole
-// step and the CTAs move through the phases of each layer together, separated by grid-wide barriers instead of kernel
-// boundaries.  A batch-1 step is a chain of ~10 tiny dependent kernels per layer; launched separately (even from a CUDA
-// graph, with programmatic dependent launch) each link costs a grid drain and a launch, about 5 us, while the weights it
-// reads would take 1 us at HBM speed.  Here a link costs one barrier and the activations are re-quantized redundantly by every
-// CTA in shared memory (instead of by a one-CTA kernel that everything waits for).  The phases are out-of-line functions with
-// short loops, one copy each: the kernel runs every phase once per layer, so straight-line unrolled code would be fetched
-// again from memory for every layer.
+// One decode step of a dense (Qwen3-style) stack as ONE persistent kernel: every SM keeps a CTA resident for the whole step and the CTAs move
+// through the phases of each layer together.  A batch-1 step is a chain of ~10 tiny dependent kernels per layer; launched separately each link
+// costs a grid drain and a launch, about 5 us, while the weights it reads would take 1 us at HBM speed.
 //
-// Per layer (5 barriers):
-//   P1  RMSNorm + INT8 of h (each CTA, shared memory; the first weight loads of every warp are already in flight) ->
-//       q|k|v GEMV rows spread over all warps -> y (bf16)
-//   P3  per (kv head, split) CTA: q/k RMSNorm + rotary embedding of the new token, cache append, attention over its
-//       positions -> partial softmax states; the last split of a kv head to finish combines them -> o
-//   P4  INT8 of o -> o-projection GEMV + residual -> h
-//   P5  RMSNorm + INT8 of h -> gate|up GEMV with SwiGLU -> act
-//   P6  INT8 of act -> down GEMV + residual -> h
-// Arithmetic: the device functions of the stand-alone kernels (row kernels, GEMV, q/k/v epilogue, decode attention), so the
-// step produces the same bits as the chain of those kernels.  Callers: e2e/decode.py:29-110 of the reference is the chain.
+// Per layer:
+//   P1  RMSNorm + INT8 of h (each CTA, shared memory) -> q|k|v rows -> y (bf16)
+//   P3  per (kv head, split) CTA: q/k RMSNorm + rotary embedding of the new token, cache append, attention over its positions -> partial
+//       softmax states; one CTA per query head combines its splits -> o
+//   P4  INT8 of o -> o-projection + residual -> h
+//   P5  RMSNorm + INT8 of h -> gate|up with SwiGLU -> act
+//   P6  INT8 of act -> down + residual -> h
 //
-// Every wait is bounded (MK_WAIT_NS): a CTA that gives up raises the abort word, writes the status word and returns; the
-// others see the abort word in their own waits and return too.  The launch is cooperative, so all CTAs are co-resident.
+// Bound by latency: what a link costs beyond its 4 us a layer of weights at HBM speed.  Two things keep it short.
+// (1) Rows travel between CTAs as packets of 8 bytes, 4 of data and 4 of an epoch (launch and layer) written by one store: a reader polls the packets
+//     themselves.  There is no barrier and no fence: a link is one store and one load through L2, about 1 us, where a grid barrier (fence, atomic,
+//     poll) and the load after it took 2.5 - 4 us.  A buffer is not rewritten before its readers are done, because every CTA has rows in
+//     every phase: who writes phase p of layer i + 1 has seen phase p - 1 complete, and so on back to phase p + 1 of layer i, whose rows were written after
+//     their CTAs had read phase p of layer i.
+// (2) Weights stream through rings in shared memory, one per warp, filled by asynchronous copies of the lanes that use them: the order of chunks is
+//     known from the start, so the ring runs ahead through phases and layers (170 KB per SM, most of a layer) while the CTA waits, joins or reduces.
+// Work item of a warp: 4 rows x 1024 columns; a row group's items are summed through shared memory (exact integers).
+// 8 layers of width 2048 at 1500 positions with the head: 342 us with grid barriers and weights in registers, 315 us here.  A layer (32 us): rows of q|k|v 2.3 (and 2.0
+// until the input row is there), attention 6.5, its combination and exchange 4.9, o 1.5, h 2.8, gate|up 5.4, act 1.7, down 3.7; two items at a time per warp changed
+// nothing (321), polling without a pause slowed the writers (375).
+// Arithmetic: the device functions of the stand-alone kernels (row kernels, GEMV, q/k/v epilogue, decode attention), so the step produces the
+// same bits as the chain of those kernels.  Callers: e2e/decode.py:29-110 of the reference is the chain.
+//
+// Every wait is bounded (MK_WAIT_NS): a thread that gives up raises the abort word and writes the status word; the others see the abort word in their
+// own waits; a CTA agrees on it at its next barrier and returns.  The launch is cooperative, so all CTAs are co-resident.
 #include "scmx_attn_core.cuh"
 #include "scmx_common.cuh"
 #include "scmx_gemv_core.cuh"
@@ -27,11 +34,15 @@
 
 namespace scmx {
 
-constexpr int MK_THREADS = 256;
+constexpr int MK_THREADS = 256;                       // the attention core wants 150 registers a thread: 384, 448 and 512 threads spill (357 - 375 us for the step below)
 constexpr int MK_WARPS = MK_THREADS / 32;
-constexpr int MK_MAXSTEPS = 6;                       // K <= 6144: a lane holds 32 codes of 4 rows per step
-constexpr int MK_MAXK = 1024 * MK_MAXSTEPS;
+constexpr int MK_MAXK = 6144;
 constexpr int MK_MAXHQ = 32;
+constexpr int MK_MAXROWS = 384;                      // output rows of a CTA in one phase at most (2 * 6144 rows on 32 SMs)
+constexpr int MK_CODES = 4 * 512, MK_CHUNK = MK_CODES + 32;      // bytes of an item: codes of 4 rows, their block codes
+constexpr int MK_SLOTS = 9;
+constexpr int MK_MAXLAYERS = 256;
+constexpr unsigned MK_BACKOFF_NS = 40;
 constexpr uint64_t MK_WAIT_NS = 500000000ull;        // 0.5 s
 
 struct MkArgs {
@@ -43,87 +54,79 @@ struct MkArgs {
     int64_t rope_rows, cap;
     const int32_t* pos_dev;
     uint16_t* h;          // bf16 [D] residual stream, in and out
-    uint16_t* y;          // bf16 [(hq + 2 hk) d]
-    uint16_t* act;        // bf16 [F]
-    float* part;          // f32 [hq, nsplit, d + 2]
-    uint16_t* o;          // bf16 [hq d] attention output
-    int32_t* counters;    // int32 [hk], zero at launch and left zero: arrivals of the splits of a kv head
-    uint32_t* bar;        // [0] arrivals, [1] abort word; both zero at launch
+    uint32_t* head;       // [0] epoch of the last launch, [1] abort word (zero at launch)
+    uint2 *xh[2], *xy, *xact, *xo, *xpart;      // packets: h after P6 / P4, y, act, o: {two bf16, epoch}; partial states [hq][nsplit][d + 2]: {float, epoch}
     int32_t* status;
     unsigned long long* trace;   // diagnostic: null, or CTA 0 stores its cycle counter at every phase boundary
     int n_trace;
-    int trace_barrier;           // diagnostic: every CTA stores its arrival time at this barrier (1-based) after the marks
 };
 
 struct MkSmem {
-    __align__(16) int8_t xq[MK_MAXK];
-    __align__(16) uint4 xn[MK_MAXK / 8];
-    float red[33];
-    double dred[33];
-    int ok;
+    __align__(16) int8_t xq[MK_MAXK];       // INT8 input row; of every 32 values the first 16 in the first half, the others in the second
+    int part[MK_MAXROWS * 6];               // [row group][step][4]
+    float ws[MK_MAXROWS];
+    float red[MK_WARPS];
+    double dred[MK_WARPS];
+    uint32_t res[MK_MAXROWS / 2];           // residual of the CTA's rows, two a word
 };
 
-__shared__ MkSmem sm;     // one instance per CTA, used by the out-of-line phase functions below
+__shared__ MkSmem sm;     // one instance per CTA
 
-// ---- grid-wide barrier ------------------------------------------------------------------------------------------------------
-__device__ __noinline__ bool grid_barrier(const MkArgs& a, uint32_t target) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(a.bar, 1u);
-        int good = 1;
-        uint64_t t0 = 0;
-        for (uint32_t it = 0;; ++it) {
-            uint32_t v;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
-            if (v >= target) break;
-            if ((it & 255u) == 255u) {
-                uint32_t ab;
-                asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(ab) : "l"(a.bar + 1) : "memory");
-                if (ab) { good = 0; break; }
-                const uint64_t now = globaltimer_ns();
-                if (!t0) t0 = now;
-                else if (now - t0 > MK_WAIT_NS) {
-                    atomicExch(a.bar + 1, 1u);
-                    atomicCAS((int*)a.status, 0, 100 + (int)(target / gridDim.x));   // which barrier gave up
-                    good = 0;
-                    break;
-                }
-            }
-        }
-        sm.ok = good;
+// ---- packets ------------------------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void put(uint2* p, uint32_t data, uint32_t epoch) {
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"((uint64_t)data | ((uint64_t)epoch << 32)) : "memory");
+}
+__device__ __forceinline__ uint2 get(const uint2* p) {
+    uint64_t v;
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return make_uint2((uint32_t)v, (uint32_t)(v >> 32));
+}
+// Two neighbouring packets; each is read whole.
+__device__ __forceinline__ void get2(const uint2* p, uint2& a, uint2& b) {
+    uint64_t x, y;
+    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "l"(p) : "memory");
+    a = make_uint2((uint32_t)x, (uint32_t)(x >> 32));
+    b = make_uint2((uint32_t)y, (uint32_t)(y >> 32));
+}
+// One turn of a wait: false once the limit has run out or another thread has given up.
+struct MkWait {
+    uint32_t turns = 0;
+    uint64_t t0 = 0;
+    __device__ __forceinline__ bool go_on(const MkArgs& a, int code) {
+        __nanosleep(MK_BACKOFF_NS);              // a row's readers are all CTAs: polling without a pause crowds out the writers
+        if ((++turns & 255u) != 0) return true;
+        uint32_t ab;
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(ab) : "l"(a.head + 1) : "memory");
+        if (ab) return false;
+        const uint64_t now = globaltimer_ns();
+        if (!t0) t0 = now;
+        if (now - t0 <= MK_WAIT_NS) return true;
+        atomicExch(a.head + 1, 1u);
+        atomicCAS(a.status, 0, code);
+        return false;
     }
-    __syncthreads();
-    return sm.ok != 0;
+};
+// Eight bf16 values, four packets; zero (and bad set) after a time-out.
+__device__ __forceinline__ uint4 get8(const MkArgs& a, const uint2* p, uint32_t epoch, int code, bool& bad) {
+    MkWait w;
+    for (;;) {
+        uint2 q[4];
+        get2(p, q[0], q[1]);
+        get2(p + 2, q[2], q[3]);
+        if (q[0].y == epoch && q[1].y == epoch && q[2].y == epoch && q[3].y == epoch) return make_uint4(q[0].x, q[1].x, q[2].x, q[3].x);
+        if (!w.go_on(a, code)) {
+            bad = true;
+            return make_uint4(0, 0, 0, 0);
+        }
+    }
 }
 
 __device__ __forceinline__ void mk_mark(const MkArgs& a, int& ti) {
     if (a.trace != nullptr && blockIdx.x == 0 && threadIdx.x == 0 && ti < a.n_trace) a.trace[ti] = (unsigned long long)clock64();
     ++ti;
 }
-// ---- activation prologues: bf16 row -> INT8 row in shared memory, returns the scale ------------------------------------------
-__device__ __forceinline__ uint4 ldcg4(const uint4* p) { return __ldcg(p); }
 
-// INT8 of the bf16 row staged in sm.xn (nv vectors of 8), arithmetic of act_quant; amax is this thread's partial maximum.
-__device__ __forceinline__ float quantize_staged(int nv, float amax) {
-    amax = block_max(amax, sm.red);
-    float s, qi;
-    quant_scale(amax, s, qi);
-    for (int v = threadIdx.x; v < nv; v += MK_THREADS) {
-        const uint4 r = sm.xn[v];
-        const uint32_t x[4] = {r.x, r.y, r.z, r.w};
-        float f[8];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            f[2 * j] = __uint_as_float(x[j] << 16);
-            f[2 * j + 1] = __uint_as_float(x[j] & 0xFFFF0000u);
-        }
-        reinterpret_cast<uint2*>(sm.xq)[v] = make_uint2(quant4(f[0], f[1], f[2], f[3], qi), quant4(f[4], f[5], f[6], f[7], qi));
-    }
-    __syncthreads();
-    return s;
-}
-
+// ---- input row of a phase: bf16 row -> INT8 row in shared memory, returns the scale ---------------------------------------------
 __device__ __forceinline__ float amax8(const uint4& r) {
     const uint32_t w[4] = {r.x, r.y, r.z, r.w};
     float m = 0.0f;
@@ -132,184 +135,193 @@ __device__ __forceinline__ float amax8(const uint4& r) {
     return m;
 }
 
-__device__ __forceinline__ float pro_act(const uint16_t* x, int K) {
-    const int nv = K / 8;
-    float amax = 0.0f;
-    for (int v = threadIdx.x; v < nv; v += MK_THREADS) {
-        const uint4 r = ldcg4(reinterpret_cast<const uint4*>(x) + v);
-        sm.xn[v] = r;
-        amax = fmaxf(amax, amax8(r));
-    }
-    return quantize_staged(nv, amax);
+// Sums and maxima over the CTA behind one barrier: every thread adds the warps' parts (a sum of squares is exact in 64 bits, so its order is free).
+__device__ __forceinline__ double mk_sum(double v) {
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) sm.dred[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = 0.0;
+#pragma unroll
+    for (int i = 0; i < MK_WARPS; ++i) v += sm.dred[i];
+    return v;
+}
+__device__ __forceinline__ float mk_max(float v) {
+    v = warp_max(v);
+    if ((threadIdx.x & 31) == 0) sm.red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = sm.red[0];
+#pragma unroll
+    for (int i = 1; i < MK_WARPS; ++i) v = fmaxf(v, sm.red[i]);
+    return v;
 }
 
-__device__ __forceinline__ float pro_norm(const uint16_t* x, const uint16_t* nw, float eps, int K) {
-    constexpr int NV = MK_MAXK / 8 / MK_THREADS;      // vectors of a thread
-    const int nv = K / 8;
-    double ss = 0.0;
-    uint4 nw_v[NV];                                    // requested together with the row: they are needed right after its sum
+// NORM: RMSNorm with weights nw first.  x: packets, or (x null) the plain row.  The arithmetic of act_quant / rmsnorm_quant.
+template <bool NORM>
+__device__ __forceinline__ float mk_input(const MkArgs& a, const uint2* x, const uint16_t* plain, uint32_t epoch, const uint16_t* nw, int K, int code, bool& bad) {
+    constexpr int NV = (MK_MAXK / 8 + MK_THREADS - 1) / MK_THREADS;      // vectors of a thread
+    const int nv = K / 8, tid = threadIdx.x;
+    uint4 r[NV], wv[NV];
 #pragma unroll
-    for (int i = 0; i < NV; ++i)
-        if ((int)threadIdx.x + MK_THREADS * i < nv) nw_v[i] = __ldg(reinterpret_cast<const uint4*>(nw) + threadIdx.x + MK_THREADS * i);
-    for (int v = threadIdx.x; v < nv; v += MK_THREADS) {
-        const uint4 r = ldcg4(reinterpret_cast<const uint4*>(x) + v);
-        sm.xn[v] = r;
-        const uint32_t w[4] = {r.x, r.y, r.z, r.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float f0 = __uint_as_float(w[j] << 16), f1 = __uint_as_float(w[j] & 0xFFFF0000u);
-            ss += sq_f64(f0) + sq_f64(f1);
-        }
+    for (int i = 0; i < NV; ++i) {
+        const int v = tid + MK_THREADS * i;
+        r[i] = wv[i] = make_uint4(0, 0, 0, 0);
+        if (NORM && v < nv) wv[i] = __ldg(reinterpret_cast<const uint4*>(nw) + v);
     }
-    ss = block_sum(ss, sm.dred);
-    const float inv = rms_inverse(ss, K, eps);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int v = tid + MK_THREADS * i;
+        if (v < nv) r[i] = x != nullptr ? get8(a, x + 4 * v, epoch, code, bad) : reinterpret_cast<const uint4*>(plain)[v];
+    }
     float amax = 0.0f;
+    if (NORM) {
+        double ss = 0.0;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {                             // the vectors this thread staged itself
-        const int v = threadIdx.x + MK_THREADS * i;
-        if (v >= nv) break;
-        const uint4 r = sm.xn[v], wv = nw_v[i];
-        const uint32_t x4[4] = {r.x, r.y, r.z, r.w}, w[4] = {wv.x, wv.y, wv.z, wv.w};
-        uint32_t o[4];
+        for (int i = 0; i < NV; ++i) {
+            const uint32_t w[4] = {r[i].x, r[i].y, r[i].z, r[i].w};
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const uint32_t t = pack_bf16x2(__fmul_rn(bf16_lo(x4[j]), inv), __fmul_rn(bf16_hi(x4[j]), inv));
-            o[j] = pack_bf16x2(__fmul_rn(bf16_lo(w[j]), bf16_lo(t)), __fmul_rn(bf16_hi(w[j]), bf16_hi(t)));
-            amax = fmaxf(amax, fmaxf(fabsf(bf16_lo(o[j])), fabsf(bf16_hi(o[j]))));
+            for (int j = 0; j < 4; ++j) ss += sq_f64(bf16_lo(w[j])) + sq_f64(bf16_hi(w[j]));
         }
-        sm.xn[v] = make_uint4(o[0], o[1], o[2], o[3]);
+        ss = mk_sum(ss);
+        const float inv = rms_inverse(ss, K, a.eps);
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const uint32_t x4[4] = {r[i].x, r[i].y, r[i].z, r[i].w}, w[4] = {wv[i].x, wv[i].y, wv[i].z, wv[i].w};
+            uint32_t o[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t t = pack_bf16x2(__fmul_rn(bf16_lo(x4[j]), inv), __fmul_rn(bf16_hi(x4[j]), inv));
+                o[j] = pack_bf16x2(__fmul_rn(bf16_lo(w[j]), bf16_lo(t)), __fmul_rn(bf16_hi(w[j]), bf16_hi(t)));
+            }
+            r[i] = make_uint4(o[0], o[1], o[2], o[3]);
+        }
     }
-    return quantize_staged(nv, amax);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) amax = fmaxf(amax, amax8(r[i]));
+    amax = mk_max(amax);
+    float s, qi;
+    quant_scale(amax, s, qi);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int v = tid + MK_THREADS * i;
+        if (v < nv) {
+            const uint32_t x4[4] = {r[i].x, r[i].y, r[i].z, r[i].w};
+            *reinterpret_cast<uint2*>(sm.xq + ((v >> 1) & 1) * (K / 2) + (v >> 2) * 16 + (v & 1) * 8) =
+                make_uint2(quant4(bf16_lo(x4[0]), bf16_hi(x4[0]), bf16_lo(x4[1]), bf16_hi(x4[1]), qi),
+                           quant4(bf16_lo(x4[2]), bf16_hi(x4[2]), bf16_lo(x4[3]), bf16_hi(x4[3]), qi));
+        }
+    }
+    return s;
 }
 
-// ---- GEMV: a warp computes 4 consecutive output rows over the whole K, in chunks of MK_UNROLL steps of 1024 codes -----------
-// The chunks of a warp (row group after row group) form one sequence that is software-pipelined: the loads of chunk i + 1
-// are issued before chunk i is expanded and accumulated, and nothing consumes a loaded value before all loads of its chunk
-// are issued.  epi 1: out[n] = T(acc xs ws); 2: out[n] = T(res[n] + T(..)); 3: SwiGLU of rows [g0 g1 u0 u1].
-constexpr int MK_UNROLL = 3;
+// ---- the warp's stream of weights -----------------------------------------------------------------------------------------------
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy4(uint32_t dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
 
-struct RowChunk {
-    uint4 w[MK_UNROLL][4];
-    uint32_t bc[MK_UNROLL];       // lane l: block-code byte (l >> 2) of the step, of row (l & 3)
+// At most n of the thread's groups of copies are still on their way.
+__device__ __forceinline__ void mk_copies_wait(int n) {
+    static_assert(MK_SLOTS == 9, "one case per slot");
+    switch (n) {
+        case 8: asm volatile("cp.async.wait_group 8;" ::: "memory"); break;
+        case 7: asm volatile("cp.async.wait_group 7;" ::: "memory"); break;
+        case 6: asm volatile("cp.async.wait_group 6;" ::: "memory"); break;
+        case 5: asm volatile("cp.async.wait_group 5;" ::: "memory"); break;
+        case 4: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
+        case 3: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
+        case 2: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
+        case 1: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
+        default: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
+    }
+}
+
+struct MkPhase {
+    int groups, steps;       // row groups in all, items per group
+    int base, count;         // the CTA's row groups: equal shares
+    uint32_t inv;            // item / steps = item * inv >> 16 for the items of a CTA
+    __device__ __forceinline__ int group_of(int item) const { return (int)(((uint32_t)item * inv) >> 16); }
 };
 
-__device__ __forceinline__ void load_chunk(RowChunk& c, const uint32_t* __restrict__ codes, const uint8_t* __restrict__ bcodes,
-                                           int n0, int s0, int steps, int wpr, int bcr, int lane) {
-#pragma unroll
-    for (int u = 0; u < MK_UNROLL; ++u) {
-        if (s0 + u < steps) {
-            const int k0 = ((s0 + u) * 32 + lane) * 32;
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                c.w[u][q] = ldg_stream(reinterpret_cast<const uint4*>(codes + (size_t)(n0 + q) * wpr + k0 / 8));
-            // the 32 lanes x 32 codes of a step span 8 block-code bytes per row: lane l fetches byte l >> 2 of row l & 3
-            c.bc[u] = __ldg(bcodes + (size_t)(n0 + (lane & 3)) * bcr + (s0 + u) * 8 + (lane >> 2));
-        }
-    }
-}
+// ---- the kernel's phases share this ------------------------------------------------------------------------------------------------
+struct MkStream {
+    const MkArgs& a;
+    const MkPhase* ph;
+    const unsigned long long* table;      // [layer][8]: codes and block codes of the four products
+    uint32_t ring;           // shared address of the warp's ring
+    int layer, phase, item;  // next item to request
+    uint32_t dst;
+    const uint32_t* codes;
+    const uint8_t* bcodes;
+    int lane, warp;
 
-__device__ __forceinline__ void compute_chunk(const RowChunk& c, const int8_t* xq, int s0, int steps, int lane, int (&tot)[4]) {
+    __device__ __forceinline__ void load_layer() {
+        codes = reinterpret_cast<const uint32_t*>(table[8 * layer + phase]);
+        bcodes = reinterpret_cast<const uint8_t*>(table[8 * layer + 4 + phase]);
+    }
+    // to the next phase in which the warp has an item
+    __device__ __forceinline__ void settle() {
+        bool moved = false;
+        while (layer < a.n_layers && item >= ph[phase].count * ph[phase].steps) {
+            item = warp;
+            moved = true;
+            if (++phase == 4) {
+                phase = 0;
+                ++layer;
+            }
+        }
+        if (moved && layer < a.n_layers) load_layer();
+    }
+    __device__ __forceinline__ void begin() {
+        layer = phase = 0;
+        item = warp;
+        dst = ring;
+        load_layer();
+        settle();
+    }
+    __device__ __forceinline__ void request() {
+        if (layer < a.n_layers) {
+            const MkPhase& p = ph[phase];
+            const int g = p.group_of(item), s = item - g * p.steps, row = 4 * (p.base + g);
+            const uint32_t* c = codes + ((size_t)row * p.steps + s) * 128 + 4 * lane;      // K / 8 = 128 steps words a row
+#pragma unroll
+            for (int q = 0; q < 4; ++q) copy16(dst + 512 * q + 16 * lane, c + (size_t)q * p.steps * 128);
+            // the 32 lanes x 32 codes of a step span 8 block-code bytes per row
+            if (lane < 8) copy4(dst + MK_CODES + 4 * lane, bcodes + ((size_t)(row + (lane >> 1)) * p.steps + s) * 8 + 4 * (lane & 1));
+            item += MK_WARPS;
+            settle();
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        dst += MK_CHUNK;
+        if (dst == ring + MK_SLOTS * MK_CHUNK) dst = ring;
+    }
+};
+
+// Totals of an item: 4 rows x 1024 columns.
+__device__ __forceinline__ void mk_item(const uint8_t* slot, const int8_t* xq, int half, int s, int lane, int (&tot)[4]) {
     const uint32_t mlo = 0x03020100u, mhi = 0x0C080604u;      // 2 x E2M1 magnitudes 0 1 2 3 | 4 6 8 12
+    const int blk = s * 32 + lane;
+    const uint4 xa = *reinterpret_cast<const uint4*>(xq + 16 * blk), xb = *reinterpret_cast<const uint4*>(xq + half + 16 * blk);
+    const uint32_t x[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
+    const int sh = 2 * (lane & 3);                            // the lane's 32-block inside its block-code byte
 #pragma unroll
-    for (int u = 0; u < MK_UNROLL; ++u) {
-        if (s0 + u < steps) {
-            const int k0 = ((s0 + u) * 32 + lane) * 32;
-            const uint4 xa = *reinterpret_cast<const uint4*>(xq + k0);
-            const uint4 xb = *reinterpret_cast<const uint4*>(xq + k0 + 16);
-            const uint32_t x[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
-            const int sh = ((k0 >> 5) & 3) * 2;               // the lane's 32-block inside its block-code byte
+    for (int q = 0; q < 4; ++q) {
+        const uint4 wv = *reinterpret_cast<const uint4*>(slot + 512 * q + 16 * lane);
+        const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w};
+        const uint32_t code = (slot[MK_CODES + 8 * q + (lane >> 2)] >> sh) & 3u;
+        // magnitudes of the positive and of the negative codes by sign-replicating byte permutes (a selector nibble with its top bit set yields the
+        // replicated top bit of the selected byte, 0 for a magnitude), two DP4A chains
+        int bp = 0, bn = 0;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const uint32_t ww[4] = {c.w[u][q].x, c.w[u][q].y, c.w[u][q].z, c.w[u][q].w};
-                const uint32_t code = (__shfl_sync(0xffffffffu, c.bc[u], (lane & ~3) | q) >> sh) & 3u;
-                // magnitudes of the positive and of the negative codes by sign-replicating byte permutes (a selector nibble with
-                // its top bit set yields the replicated top bit of the selected byte, 0 for a magnitude), two DP4A chains
-                int bp = 0, bn = 0;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const uint32_t w = ww[j], wx = w ^ 0x88888888u;
-                    bp = dp4a_ss(x[2 * j], prmt(mlo, mhi, w), bp);
-                    bn = dp4a_ss(x[2 * j], prmt(mlo, mhi, wx), bn);
-                    bp = dp4a_ss(x[2 * j + 1], prmt(mlo, mhi, w >> 16), bp);
-                    bn = dp4a_ss(x[2 * j + 1], prmt(mlo, mhi, wx >> 16), bn);
-                }
-                tot[q] += (bp - bn) << code;
-            }
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t w = ww[j], wx = w ^ 0x88888888u;
+            bp = dp4a_ss(x[2 * j], prmt(mlo, mhi, w), bp);
+            bn = dp4a_ss(x[2 * j], prmt(mlo, mhi, wx), bn);
+            bp = dp4a_ss(x[2 * j + 1], prmt(mlo, mhi, w >> 16), bp);
+            bn = dp4a_ss(x[2 * j + 1], prmt(mlo, mhi, wx >> 16), bn);
         }
-    }
-}
-
-// One GEMV phase: the warp's first chunk of weights is requested, then the CTA computes the INT8 input row in shared memory
-// (NORM: RMSNorm with weights nw first), then the chunks are consumed.  The weights do not depend on the activations, so
-// their first round trip to memory runs under the prologue.
-template <bool NORM>
-__device__ __noinline__ void run_phase(const uint32_t* __restrict__ codes, const uint8_t* __restrict__ bcodes,
-                                       const float* __restrict__ wscale, int N, int K, const uint16_t* x, const uint16_t* nw,
-                                       float eps, int epi, const uint16_t* res, uint16_t* out) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // row groups are dealt warp-major, so that a job with fewer groups than warps still uses every SM
-    const int gw = warp * gridDim.x + blockIdx.x, nw_ = gridDim.x * MK_WARPS;
-    const int steps = K / 1024, wpr = K / 8, bcr = K / 128, groups = N / 4;
-    const int8_t* xq = sm.xq;
-    const bool work = gw < groups;
-    RowChunk cur, nxt;
-    int grp = gw, s0 = 0;
-    // Scales and residual of a row group (lane r < 4: row r) are requested with its first codes: loaded where they are used, they cost every
-    // group a round trip to memory (with the norm weights and the cache positions requested early: 358 -> 345 us for 8 layers of 2048).
-    float ws = 0.0f, rs = 0.0f, ws_next = 0.0f, rs_next = 0.0f;
-    auto load_scales = [&](int g, float& w, float& r) {
-        if (lane < 4) {
-            w = __ldg(wscale + 4 * g + lane);
-            if (epi == 2) r = bf16_to_f32(__ldcg(res + 4 * g + lane));
-        }
-    };
-    if (work) {
-        load_chunk(cur, codes, bcodes, grp * 4, 0, steps, wpr, bcr, lane);
-        load_scales(grp, ws, rs);
-    }
-    const float xs = NORM ? pro_norm(x, nw, eps, K) : pro_act(x, K);     // every thread: contains CTA barriers
-    if (!work) return;
-    int tot[4] = {0, 0, 0, 0};
-    for (;;) {
-        // the chunk after this one: the next steps of the same rows, or the first steps of the warp's next row group
-        int ngrp = grp, ns0 = s0 + MK_UNROLL;
-        if (ns0 >= steps) {
-            ngrp = grp + nw_;
-            ns0 = 0;
-        }
-        const bool more = ngrp < groups;
-        if (more) {
-            load_chunk(nxt, codes, bcodes, ngrp * 4, ns0, steps, wpr, bcr, lane);
-            if (ngrp != grp) load_scales(ngrp, ws_next, rs_next);
-        }
-        compute_chunk(cur, xq, s0, steps, lane, tot);
-        if (ngrp != grp) {                                    // last chunk of the row group: reduce and write
-            const int n0 = grp * 4;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) tot[q] = warp_sum(tot[q]);
-            // every lane holds the four totals; lane r finishes row r (selects, not indexing: the totals stay in registers)
-            const int t_lo = (lane & 1) ? tot[1] : tot[0], t_hi = (lane & 1) ? tot[3] : tot[2];
-            if (epi == 3) {
-                const float wu = __shfl_down_sync(0xffffffffu, ws, 2);
-                if (lane < 2) {
-                    const float gg = scale_acc(t_lo, xs, ws);
-                    const float uu = scale_acc(t_hi, xs, wu);
-                    out[n0 / 2 + lane] = f32_to_bf16(swiglu_bf16(gg, uu));
-                }
-            } else if (lane < 4) {
-                float y = scale_acc(lane < 2 ? t_lo : t_hi, xs, ws);
-                if (epi == 2) y = __fadd_rn(rs, y);
-                out[n0 + lane] = f32_to_bf16(y);
-            }
-#pragma unroll
-            for (int q = 0; q < 4; ++q) tot[q] = 0;
-            ws = ws_next;
-            rs = rs_next;
-        }
-        if (!more) break;
-        cur = nxt;
-        grp = ngrp;
-        s0 = ns0;
+        tot[q] = (bp - bn) << code;
     }
 }
 
@@ -332,17 +344,13 @@ struct QkvSmem {
 };
 
 template <int G, int HD>
-__device__ __forceinline__ void qkv_prepare(QkvSmem<G, HD>& qs, const MkArgs& a, const scmx_decode_layer& L, int kvh, int64_t pos) {
+__device__ __forceinline__ void qkv_prepare(QkvSmem<G, HD>& qs, const MkArgs& a, const uint16_t* q_norm, const uint16_t* k_norm, int kvh, int64_t pos, uint32_t epoch,
+                                            int code, bool& bad) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int half = HD / 2, NE = (G + 2) * HD;
-    for (int e = tid; e < NE; e += MK_THREADS) {
-        const int hh = e / HD, dd = e - hh * HD;
-        const int src = hh < G ? (kvh * G + hh) * HD : (hh == G ? (a.hq + kvh) * HD : (a.hq + a.hk + kvh) * HD);
-        qs.vals[e] = bf16_to_f32(__ldcg(a.y + src + dd));
-    }
     for (int i = tid; i < HD; i += MK_THREADS) {
-        qs.wq[i] = L.q_norm[i];
-        qs.wk[i] = L.k_norm[i];
+        qs.wq[i] = q_norm[i];
+        qs.wk[i] = k_norm[i];
     }
     for (int i = tid; i < half; i += MK_THREADS) {
         if (a.rope_cs != nullptr && pos < a.rope_rows) {
@@ -355,6 +363,19 @@ __device__ __forceinline__ void qkv_prepare(QkvSmem<G, HD>& qs, const MkArgs& a,
             qs.cs[i] = (float)c;
             qs.sn[i] = (float)s;
         }
+    }
+    for (int e = 2 * tid; e < NE; e += 2 * MK_THREADS) {
+        const int hh = e / HD, dd = e - hh * HD;
+        const int src = hh < G ? (kvh * G + hh) * HD : (hh == G ? (a.hq + kvh) * HD : (a.hq + a.hk + kvh) * HD);
+        uint2 p;
+        MkWait w;
+        while ((p = get(a.xy + (src + dd) / 2)).y != epoch)
+            if (!w.go_on(a, code)) {
+                bad = true;
+                break;
+            }
+        qs.vals[e] = bf16_lo(p.x);
+        qs.vals[e + 1] = bf16_hi(p.x);
     }
     __syncthreads();
     for (int hh = warp; hh < G + 1; hh += MK_WARPS) {
@@ -388,14 +409,116 @@ __device__ __forceinline__ void qkv_prepare(QkvSmem<G, HD>& qs, const MkArgs& a,
     __syncthreads();
 }
 
-// ---- the kernel ------------------------------------------------------------------------------------------------------------
+// One (kv head, split) task of P3; out of line, so that its registers are its own.
 template <int G, int HD>
-__global__ void __launch_bounds__(MK_THREADS, 1) decode_step_kernel(const MkArgs a) {
+__device__ __noinline__ bool mk_attention(const MkArgs& a, const scmx_decode_layer& L, int kvh, int split, int64_t t0, int64_t t1, int64_t pos, uint32_t epoch, int code) {
     __shared__ QkvSmem<G, HD> qs;
     __shared__ AttnSmem<G, HD> as;
+    constexpr int stride = HD + 2;
+    const int tid = threadIdx.x;
+    const bool in_cache = pos < a.cap;
+    bool bad = false;
+    qkv_prepare<G, HD>(qs, a, L.q_norm, L.k_norm, kvh, pos, epoch, code, bad);
+    uint16_t* kc = L.k_cache + (size_t)kvh * a.cap * HD;
+    uint16_t* vc = L.v_cache + (size_t)kvh * a.cap * HD;
+    if (split == 0 && in_cache && tid < HD / 8) {
+        reinterpret_cast<uint4*>(kc + pos * HD)[tid] = reinterpret_cast<const uint4*>(qs.k)[tid];
+        reinterpret_cast<uint4*>(vc + pos * HD)[tid] = reinterpret_cast<const uint4*>(qs.v)[tid];
+    }
+    uint2* part = a.xpart + ((size_t)kvh * G * a.nsplit + split) * stride;
+    attn_split<G, HD>(qs.q, kc, vc, t0, t1, in_cache ? pos : -1, qs.k, qs.v, a.scale,
+                      [&](int g, int e, float v) { put(part + (size_t)g * a.nsplit * stride + e, __float_as_uint(v), epoch); }, as);
+    return bad;
+}
+
+// The splits of a query head (the arithmetic of attn_combine_cta): thread e owns output element e.
+template <int HD>
+__device__ __noinline__ bool mk_combine(const MkArgs& a, int head, int active, uint32_t epoch, int code) {
+    __shared__ float ml[32][2], coef[33];
+    constexpr int stride = HD + 2;
+    const int tid = threadIdx.x;
+    const uint2* p = a.xpart + (size_t)head * a.nsplit * stride;
+    bool bad = false;
+    __syncthreads();
+    if (tid < 2 * active) {                               // a split's last packets; its other ones were stored before, mostly
+        uint2 v;
+        MkWait w;
+        while ((v = get(p + (tid >> 1) * stride + HD + (tid & 1))).y != epoch)
+            if (!w.go_on(a, code)) {
+                bad = true;
+                break;
+            }
+        ml[tid >> 1][tid & 1] = __uint_as_float(v.x);
+    }
+    __syncthreads();
+    float v0[32];
+    if (tid < HD && !bad) {
+        MkWait w;
+        for (bool late = true; late;) {                   // all splits' packets are requested together
+            late = false;
+#pragma unroll
+            for (int s = 0; s < 32; ++s) {
+                v0[s] = 0.0f;
+                if (s < active) {
+                    const uint2 v = get(p + s * stride + tid);
+                    v0[s] = __uint_as_float(v.x);
+                    late |= v.y != epoch;
+                }
+            }
+            if (late && !w.go_on(a, code)) {
+                bad = true;
+                break;
+            }
+        }
+    }
+    if (tid >= HD && tid < HD + 32) {                     // the weights meanwhile, a split a lane
+        const int s = tid - HD;
+        const float ms = s < active ? ml[s][0] : -INFINITY, mm = warp_max(ms);
+        if (s < active) coef[s] = ms == -INFINITY ? 0.0f : exp2f(ms - mm);
+        __syncwarp();
+        if (s == 0) {
+            float ll = 0.0f;
+            for (int i = 0; i < active; ++i) ll += ml[i][1] * coef[i];
+            coef[32] = ll;
+        }
+    }
+    __syncthreads();
+    if (tid < HD) {
+        float av = 0.0f;
+#pragma unroll
+        for (int s = 0; s < 32; ++s)
+            if (s < active) av += v0[s] * coef[s];
+        const uint32_t b = f32_to_bf16(av / coef[32]), other = __shfl_down_sync(0xffffffffu, b, 1);      // whole warps
+        if ((tid & 1) == 0) put(a.xo + (head * HD + tid) / 2, b | (other << 16), epoch);
+    }
+    return bad;
+}
+
+// ---- the kernel ------------------------------------------------------------------------------------------------------------
+template <int G, int HD>
+__global__ void __launch_bounds__(MK_THREADS, 1) decode_step_kernel(const __grid_constant__ MkArgs a) {
+    extern __shared__ __align__(16) uint8_t rings[];
+    __shared__ MkPhase ph[4];
+    __shared__ scmx_decode_layer layer[2];        // this one and the next
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int D = a.D, F = a.F, QD = a.hq * HD, NQKV = (a.hq + 2 * a.hk) * HD;
-    uint32_t target = 0;
+    if (tid < 4) {
+        const int rows = tid == 0 ? NQKV : tid == 2 ? 2 * F : D, K = tid == 1 ? QD : tid == 3 ? F : D, g = rows / 4;
+        const int lo = (int)((int64_t)g * blockIdx.x / gridDim.x), hi = (int)((int64_t)g * (blockIdx.x + 1) / gridDim.x);
+        ph[tid] = {g, K / 1024, lo, hi - lo, 65536u / (uint32_t)(K / 1024) + 1u};
+    }
+    constexpr int LWORDS = (int)(sizeof(scmx_decode_layer) / 8);
+    if (tid < LWORDS) reinterpret_cast<unsigned long long*>(&layer[0])[tid] = reinterpret_cast<const unsigned long long*>(a.layers)[tid];
+    unsigned long long* table = reinterpret_cast<unsigned long long*>(rings + MK_WARPS * MK_SLOTS * MK_CHUNK);
+    for (int i = tid; i < 8 * a.n_layers; i += MK_THREADS)        // codes[4], bcodes[4] are the first words of a layer
+        table[i] = reinterpret_cast<const unsigned long long*>(a.layers + (i >> 3))[i & 7];
+    const uint32_t base_epoch = *reinterpret_cast<volatile const uint32_t*>(a.head);
+    __syncthreads();
+    MkStream st = {a, ph, table, (uint32_t)__cvta_generic_to_shared(rings) + warp * (MK_SLOTS * MK_CHUNK), 0, 0, 0, 0, nullptr, nullptr, lane, warp};
+    const uint8_t* ring = rings + warp * (MK_SLOTS * MK_CHUNK);
+    const uint8_t *slot = ring, *ring_end = ring + MK_SLOTS * MK_CHUNK;
+    st.begin();
+    for (int i = 0; i < MK_SLOTS; ++i) st.request();
 
     int64_t pos = a.pos_dev[0];
     pos = pos < 0 ? 0 : pos;
@@ -404,79 +527,156 @@ __global__ void __launch_bounds__(MK_THREADS, 1) decode_step_kernel(const MkArgs
     int64_t chunk;
     int active;
     attn_chunking(T, a.nsplit, chunk, active);
-    constexpr int stride = HD + 2;
-
+    const int kvh = blockIdx.x % a.hk, split = blockIdx.x / a.hk;
+    const bool attends = split < active;
+    const int64_t t0 = (int64_t)split * chunk, t1 = t0 + chunk < T ? t0 + chunk : T;
+    const int my_head = (int)gridDim.x - 1 - (int)blockIdx.x;      // query head whose splits this CTA combines
+    bool bad = false;
     int ti = 0;
-#define MK_MARK()                                                                                   \
-    do {                                                                                            \
-        mk_mark(a, ti);                                                                             \
-    } while (0)
-#define MK_BARRIER()                                          \
-    do {                                                      \
-        MK_MARK();                                            \
-        target += gridDim.x;                                  \
-        if (a.trace != nullptr && tid == 0 && (int)(target / gridDim.x) == a.trace_barrier)                      \
-            a.trace[a.n_trace + blockIdx.x] = globaltimer_ns();                                             \
-        if (!grid_barrier(a, target)) return;         \
-        MK_MARK();                                            \
-    } while (0)
+
+    auto gave_up = [&]() {                                         // the CTA agrees; copies in flight land before it leaves
+        if (!__syncthreads_or(bad)) return false;
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        return true;
+    };
+    // one product: the warp's items, summed per row group; the caller then finishes the rows.  Slots are refilled afterwards (refill), off the chain; in
+    // between only where a phase has more items than the ring.
+    int used = 0;
+    auto refill = [&]() {
+        for (; used > 0; --used) st.request();
+    };
+    auto items = [&](const MkPhase& p, int K) {
+        for (int it = warp; it < p.count * p.steps; it += MK_WARPS) {
+            const int g = p.group_of(it), s = it - g * p.steps;
+            if (used == MK_SLOTS) refill();
+            mk_copies_wait(MK_SLOTS - 1 - used);
+            __syncwarp();                                          // block codes were copied by other lanes
+            int tot[4];
+            mk_item(slot, sm.xq, K / 2, s, lane, tot);
+            __syncwarp();
+            ++used;
+            slot += MK_CHUNK;
+            if (slot == ring_end) slot = ring;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) tot[q] = __reduce_add_sync(0xffffffffu, tot[q]);
+            if (lane < 4) sm.part[(g * p.steps + s) * 4 + lane] = lane < 2 ? (lane ? tot[1] : tot[0]) : (lane == 3 ? tot[3] : tot[2]);
+        }
+    };
+    auto total = [&](const MkPhase& p, int r) {                    // row r of the CTA's
+        int t = 0;
+        for (int s = 0; s < p.steps; ++s) t += sm.part[((r >> 2) * p.steps + s) * 4 + (r & 3)];
+        return t;
+    };
+    // rows of a plain product or one with a residual: T(acc xs ws) (+ res), two a thread, as packets, and as a plain row if `plain`
+    auto finish = [&](const MkPhase& p, float xs, bool res, uint2* out, uint16_t* plain, uint32_t epoch) {
+        for (int r = 2 * tid; r < 4 * p.count; r += 2 * MK_THREADS) {
+            const int n = 4 * p.base + r;
+            float y0 = scale_acc(total(p, r), xs, sm.ws[r]), y1 = scale_acc(total(p, r + 1), xs, sm.ws[r + 1]);
+            if (res) {
+                const uint32_t h = sm.res[r >> 1];
+                y0 = __fadd_rn(bf16_lo(h), y0);
+                y1 = __fadd_rn(bf16_hi(h), y1);
+            }
+            const uint32_t two = pack_bf16x2(y0, y1);
+            put(out + (n >> 1), two, epoch);
+            if (plain != nullptr) *reinterpret_cast<uint32_t*>(plain + n) = two;
+        }
+    };
+    // scales and residual of the CTA's rows, requested before the input row is awaited (the residual's packets are complete long before)
+    auto ahead = [&](const MkPhase& p, const float* wscale, const uint2* res, const uint16_t* res_plain) {
+        for (int r = tid; r < 4 * p.count; r += MK_THREADS) {
+            const int n = 4 * p.base + r;
+            sm.ws[r] = __ldg(wscale + n);
+            if ((r & 1) == 0 && res != nullptr) sm.res[r >> 1] = get(res + (n >> 1)).x;
+            else if ((r & 1) == 0 && res_plain != nullptr) sm.res[r >> 1] = *reinterpret_cast<const uint32_t*>(res_plain + n);
+        }
+    };
 
     for (int li = 0; li < a.n_layers; ++li) {
-        const scmx_decode_layer L = a.layers[li];             // by value: the pointers sit in registers for the whole layer
+        const scmx_decode_layer& L = layer[li & 1];
+        if (li + 1 < a.n_layers && tid < LWORDS)              // read after several barriers
+            reinterpret_cast<unsigned long long*>(&layer[(li + 1) & 1])[tid] = reinterpret_cast<const unsigned long long*>(a.layers + li + 1)[tid];
+        const uint32_t epoch = base_epoch + 1 + li;
+        const int code = 1000 + 5 * li;
+        mk_mark(a, ti);
+        if (attends && tid < 2 && t1 > t0) {                  // the positions that this CTA will attend to
+            const int64_t te = t1 < T - 1 ? t1 : T - 1;
+            if (te > t0) prefetch_l2((tid ? L.v_cache : L.k_cache) + ((size_t)kvh * a.cap + t0) * HD, (uint32_t)(te - t0) * HD * 2);
+        }
         // P1: input RMSNorm + INT8, q|k|v projection
-        if (li > 0) MK_BARRIER();                             // h of the previous layer complete
-        {
-            const int kvh = blockIdx.x % a.hk, split = blockIdx.x / a.hk;
-            if (split < active && tid < 2) {                  // the positions that this CTA will attend to: 4.3 -> 3.7 us at 1500
-                const int64_t t0 = (int64_t)split * chunk, t1 = t0 + chunk < T - 1 ? t0 + chunk : T - 1;
-                if (t1 > t0) prefetch_l2((tid ? L.v_cache : L.k_cache) + ((size_t)kvh * a.cap + t0) * HD, (uint32_t)(t1 - t0) * HD * 2);
-            }
-        }
-        run_phase<true>(L.codes[0], L.bcodes[0], L.wscale[0], NQKV, D, a.h, L.ln_in, a.eps, 1, nullptr, a.y);
+        ahead(ph[0], L.wscale[0], nullptr, nullptr);
+        float xs = mk_input<true>(a, li > 0 ? a.xh[0] : nullptr, a.h, epoch - 1, L.ln_in, D, code, bad);
+        if (gave_up()) return;
+        mk_mark(a, ti);
+        items(ph[0], D);
+        __syncthreads();
+        finish(ph[0], xs, false, a.xy, nullptr, epoch);
+        refill();
+        mk_mark(a, ti);
         // P3: attention of one (kv head, split) per CTA
-        MK_BARRIER();
-        {
-            const int kvh = blockIdx.x % a.hk, split = blockIdx.x / a.hk;
-            if (split < active) {                             // uniform over the CTA
-                qkv_prepare<G, HD>(qs, a, L, kvh, pos);
-                MK_MARK();
-                uint16_t* kc = L.k_cache + (size_t)kvh * a.cap * HD;
-                uint16_t* vc = L.v_cache + (size_t)kvh * a.cap * HD;
-                if (split == 0 && in_cache && tid < HD / 8) {
-                    reinterpret_cast<uint4*>(kc + pos * HD)[tid] = reinterpret_cast<const uint4*>(qs.k)[tid];
-                    reinterpret_cast<uint4*>(vc + pos * HD)[tid] = reinterpret_cast<const uint4*>(qs.v)[tid];
-                }
-                const int64_t t0 = (int64_t)split * chunk, t1 = t0 + chunk < T ? t0 + chunk : T;
-                attn_split<G, HD>(qs.q, kc, vc, t0, t1, in_cache ? pos : -1, qs.k, qs.v, a.scale,
-                                  a.part + ((size_t)kvh * G * a.nsplit + split) * stride, (size_t)a.nsplit * stride, as);
-                MK_MARK();
-                // the last split of this kv head to finish combines them (the arithmetic of attn_combine) into o
-                __syncthreads();
-                if (tid == 0) {                               // one fence orders the CTA's partials before the ticket
-                    __threadfence();
-                    sm.ok = atomicAdd(a.counters + kvh, 1);
-                    __threadfence();
-                }
-                __syncthreads();
-                if (sm.ok == active - 1) {
-                    attn_combine_cta<G, HD>(a.part + (size_t)kvh * G * a.nsplit * stride, a.nsplit, active,
-                                            a.o + (size_t)kvh * G * HD, as);
-                    if (tid == 0) a.counters[kvh] = 0;
-                }
-            }
-        }
-        // P4: combine the splits, INT8 of o, o-projection + residual
-        MK_BARRIER();
-        run_phase<false>(L.codes[1], L.bcodes[1], L.wscale[1], D, QD, a.o, nullptr, 0.0f, 2, a.h, a.h);
+        if (attends) bad |= mk_attention<G, HD>(a, L, kvh, split, t0, t1, pos, epoch, code + 1);      // uniform over the CTA
+        mk_mark(a, ti);
+        if (my_head < a.hq) bad |= mk_combine<HD>(a, my_head, active, epoch, code + 2);
+        __syncthreads();                                      // sm.ws and the products are free
+        // P4: INT8 of o, o-projection + residual
+        ahead(ph[1], L.wscale[1], li > 0 ? a.xh[0] : nullptr, a.h);
+        xs = mk_input<false>(a, a.xo, nullptr, epoch, nullptr, QD, code + 2, bad);
+        if (gave_up()) return;
+        mk_mark(a, ti);
+        items(ph[1], QD);
+        __syncthreads();
+        finish(ph[1], xs, true, a.xh[1], nullptr, epoch);
+        refill();
+        mk_mark(a, ti);
+        __syncthreads();
         // P5: post-attention RMSNorm + INT8, gate|up projection with SwiGLU
-        MK_BARRIER();
-        run_phase<true>(L.codes[2], L.bcodes[2], L.wscale[2], 2 * F, D, a.h, L.ln_post, a.eps, 3, nullptr, a.act);
+        ahead(ph[2], L.wscale[2], nullptr, nullptr);
+        xs = mk_input<true>(a, a.xh[1], nullptr, epoch, L.ln_post, D, code + 3, bad);
+        if (gave_up()) return;
+        mk_mark(a, ti);
+        items(ph[2], D);
+        __syncthreads();
+        for (int g = tid; g < ph[2].count; g += MK_THREADS) {                  // a row group: two gate rows, two up rows
+            float v[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) v[r] = scale_acc(total(ph[2], 4 * g + r), xs, sm.ws[4 * g + r]);
+            put(a.xact + ph[2].base + g, pack_bf16x2(swiglu_bf16(v[0], v[2]), swiglu_bf16(v[1], v[3])), epoch);
+        }
+        refill();
+        mk_mark(a, ti);
+        __syncthreads();
         // P6: INT8 of act, down projection + residual
-        MK_BARRIER();
-        run_phase<false>(L.codes[3], L.bcodes[3], L.wscale[3], D, F, a.act, nullptr, 0.0f, 2, a.h, a.h);
+        ahead(ph[3], L.wscale[3], a.xh[1], nullptr);
+        xs = mk_input<false>(a, a.xact, nullptr, epoch, nullptr, F, code + 4, bad);
+        if (gave_up()) return;
+        mk_mark(a, ti);
+        items(ph[3], F);
+        __syncthreads();
+        finish(ph[3], xs, true, a.xh[0], li + 1 == a.n_layers ? a.h : nullptr, epoch);
+        refill();
+        __syncthreads();
     }
-#undef MK_BARRIER
-#undef MK_MARK
+    // every CTA has read the epoch: the last rows need all of them
+    if (blockIdx.x == 0 && tid == 0) a.head[0] = base_epoch + 1 + a.n_layers;
+}
+
+// Before a step: after one that gave up, its epochs must not come again.
+__global__ void mk_begin_kernel(uint32_t* head) {
+    if (head[1] != 0) {
+        head[0] += 1u << 16;
+        head[1] = 0;
+    }
+}
+
+// Bytes of the packet buffers, each 16-byte aligned, after 16 bytes of header.
+static size_t mk_scratch(int D, int F, int hq, int hk, int d, int nsplit, size_t (&off)[7]) {
+    const size_t n[6] = {(size_t)D / 2, (size_t)D / 2, (size_t)(hq + 2 * hk) * d / 2, (size_t)F / 2, (size_t)hq * d / 2, (size_t)hq * nsplit * (d + 2)};
+    size_t at = 16;
+    for (int i = 0; i < 6; ++i) {
+        off[i] = at;
+        at += (8 * n[i] + 15) & ~(size_t)15;
+    }
+    return off[6] = at;
 }
 
 }  // namespace scmx
@@ -491,12 +691,15 @@ extern "C" int scmx_set_decode_trace(unsigned long long* device_buf, int n) {
     return SCMX_OK;
 }
 
+extern "C" int64_t scmx_decode_step_scratch(int D, int F, int hq, int hk, int d, int nsplit) {
+    size_t off[7];
+    return D > 0 && F > 0 && hq > 0 && hk > 0 && d > 0 && nsplit > 0 ? (int64_t)mk_scratch(D, F, hq, hk, d, nsplit, off) : 0;
+}
+
 extern "C" int scmx_decode_step_dense(const scmx_decode_layer* layers, int n_layers, int D, int F, int hq, int hk, int d, float eps,
                                       float scale, const float* inv_freq, const float* rope_table, int64_t rope_rows,
-                                      int64_t capacity, const int32_t* pos_dev, uint16_t* h, uint16_t* y, uint16_t* act,
-                                      uint16_t* o, float* partials, int nsplit, int32_t* counters, uint32_t* barrier,
-                                      int32_t* status, void* stream) {
-    SCMX_REQUIRE(layers && pos_dev && h && y && act && o && partials && counters && barrier && status && inv_freq, SCMX_EINVAL, "decode_step: null buffer");
+                                      int64_t capacity, const int32_t* pos_dev, uint16_t* h, void* scratch, int nsplit, int32_t* status, void* stream) {
+    SCMX_REQUIRE(layers && pos_dev && h && scratch && status && inv_freq, SCMX_EINVAL, "decode_step: null buffer");
     SCMX_REQUIRE(n_layers > 0 && hq > 0 && hk > 0 && hq % hk == 0 && hq <= MK_MAXHQ, SCMX_EINVAL, "decode_step: hq=%d hk=%d", hq, hk);
     SCMX_REQUIRE(d == 128, SCMX_ELIMIT, "decode_step: head size %d (128)", d);
     const int G = hq / hk;
@@ -504,30 +707,41 @@ extern "C" int scmx_decode_step_dense(const scmx_decode_layer* layers, int n_lay
     SCMX_REQUIRE(D % 1024 == 0 && F % 1024 == 0 && (hq * d) % 1024 == 0 && D <= MK_MAXK && F <= MK_MAXK && hq * d <= MK_MAXK,
                  SCMX_ELIMIT, "decode_step: widths D=%d F=%d hq*d=%d must be multiples of 1024 up to %d", D, F, hq * d, MK_MAXK);
     SCMX_REQUIRE(capacity >= 1 && nsplit >= 1 && nsplit <= 32, SCMX_EINVAL, "decode_step: capacity=%lld nsplit=%d", (long long)capacity, nsplit);
+    SCMX_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & 15) == 0 && (reinterpret_cast<uintptr_t>(h) & 15) == 0, SCMX_EINVAL, "decode_step: unaligned buffer");
     static int coop_dev[64] = {};            // 0 unknown, 1 supported, -1 not: per device
     const int dev = current_device();
     SCMX_REQUIRE(dev >= 0, SCMX_ECUDA, "decode_step: no current CUDA device (ordinal 0..63)");
+    constexpr int RINGS = MK_WARPS * MK_SLOTS * MK_CHUNK + 64 * MK_MAXLAYERS;
+    SCMX_REQUIRE(n_layers <= MK_MAXLAYERS, SCMX_ELIMIT, "decode_step: %d layers (%d)", n_layers, MK_MAXLAYERS);
     if (!coop_dev[dev]) {
         int c = 0;
         SCMX_CUDA_OK(cudaDeviceGetAttribute(&c, cudaDevAttrCooperativeLaunch, dev));
+        SCMX_CUDA_OK(cudaFuncSetAttribute(decode_step_kernel<1, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, RINGS));
+        SCMX_CUDA_OK(cudaFuncSetAttribute(decode_step_kernel<2, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, RINGS));
+        SCMX_CUDA_OK(cudaFuncSetAttribute(decode_step_kernel<4, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, RINGS));
         coop_dev[dev] = c ? 1 : -1;
     }
     const int coop = coop_dev[dev] > 0, n_sm = sm_count();
     SCMX_REQUIRE(coop, SCMX_EDEVICE, "decode_step: the device does not support cooperative launches");
-    SCMX_REQUIRE(hk * nsplit <= n_sm, SCMX_EINVAL, "decode_step: hk * nsplit = %d exceeds the %d CTAs of the grid", hk * nsplit, n_sm);
+    // every CTA has rows in every phase, which the reuse of the packet buffers rests on (256 row groups at least)
+    SCMX_REQUIRE(hk * nsplit <= n_sm && hq <= n_sm && n_sm <= 256 && n_sm >= 4 * 6144 / MK_MAXROWS, SCMX_EINVAL,
+                 "decode_step: hk * nsplit = %d, hq = %d on the %d CTAs of the grid", hk * nsplit, hq, n_sm);
+    size_t off[7];
+    mk_scratch(D, F, hq, hk, d, nsplit, off);
+    uint8_t* sp = static_cast<uint8_t*>(scratch);
+    auto at = [&](int i) { return reinterpret_cast<uint2*>(sp + off[i]); };
     MkArgs a;
     a.layers = layers; a.n_layers = n_layers; a.D = D; a.F = F; a.hq = hq; a.hk = hk; a.nsplit = nsplit; a.eps = eps; a.scale = scale;
     a.inv_freq = inv_freq; a.rope_cs = rope_table; a.rope_rows = rope_table ? rope_rows : 0; a.cap = capacity; a.pos_dev = pos_dev;
-    a.h = h; a.y = y; a.act = act; a.o = o; a.counters = counters; a.part = partials; a.bar = barrier; a.status = status;
-    a.trace = g_trace; a.n_trace = g_n_trace & 0xFFFF; a.trace_barrier = g_n_trace >> 16;
+    a.h = h; a.head = reinterpret_cast<uint32_t*>(sp); a.xh[0] = at(0); a.xh[1] = at(1); a.xy = at(2); a.xact = at(3); a.xo = at(4); a.xpart = at(5); a.status = status;
+    a.trace = g_trace; a.n_trace = g_n_trace & 0xFFFF;
     cudaStream_t st = (cudaStream_t)stream;
-    SCMX_CUDA_OK(cudaMemsetAsync(barrier, 0, 2 * sizeof(uint32_t), st));
-    // tickets taken by a step that gave up on a barrier are not returned: start every step from zero
-    SCMX_CUDA_OK(cudaMemsetAsync(counters, 0, (size_t)hk * sizeof(int32_t), st));
+    mk_begin_kernel<<<1, 1, 0, st>>>(a.head);
+    SCMX_LAUNCH_OK("mk_begin_kernel");
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)n_sm);
     cfg.blockDim = dim3(MK_THREADS);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = RINGS;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;

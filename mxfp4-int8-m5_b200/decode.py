@@ -11,9 +11,9 @@ fuse_prologue selects where the per-token INT8 of a GEMV input is computed in th
 kernel); here both forms run the row kernel followed by the GEMV and give the same values, so the argument only keeps the
 signature.
 
-persistent=True (DecodeQwen3) runs all layers of a step as ONE cooperative kernel (scmx_decode_step_dense): the phases of a
-layer are separated by grid-wide barriers instead of kernel boundaries, each CTA re-quantizes the activations it needs in
-shared memory, and weight loads are issued ahead of the barriers.  Same bits as the chain of kernels; used where its limits
+persistent=True (DecodeQwen3) runs all layers of a step as ONE cooperative kernel (scmx_decode_step_dense): rows travel between
+the phases of a layer as packets instead of across kernel boundaries, each CTA re-quantizes the activations it needs in
+shared memory, and weights stream ahead of the phases.  Same bits as the chain of kernels; used where its limits
 hold (head size 128, widths multiples of 1024 up to 6144) and attention="kernel".
 
 DecodeHybrid is the same for hybrid decoders (fused_hybrid.FusedHybrid): GEMVs on bfloat16 or float32 weights with the mixers'
@@ -152,22 +152,18 @@ class DecodeQwen3(_Decoder):
             t.q_norm, t.k_norm = at.q_norm.weight.data_ptr(), at.k_norm.weight.data_ptr()
             t.k_cache, t.v_cache = c.k.data_ptr(), c.v.data_ptr()
         raw = np.frombuffer(ctypes.string_at(ctypes.addressof(table), ctypes.sizeof(table)), dtype=np.uint8).copy()
-        hq, hk, d = a.num_attention_heads, a.num_key_value_heads, a.head_dim
-        self._mk = dict(cache=cache, table=torch.from_numpy(raw).to(dev),
-                        y=torch.empty((hq + 2 * hk) * d, dtype=torch.bfloat16, device=dev),
-                        act=torch.empty(a.intermediate_size, dtype=torch.bfloat16, device=dev),
-                        o=torch.empty(hq * d, dtype=torch.bfloat16, device=dev),
-                        bar=torch.zeros(2, dtype=torch.int32, device=dev),
+        size = _lib.lib().scmx_decode_step_scratch(a.hidden_size, a.intermediate_size, a.num_attention_heads, a.num_key_value_heads, a.head_dim, self.attn.nsplit)
+        self._mk = dict(cache=cache, table=torch.from_numpy(raw).to(dev), scratch=torch.zeros(size, dtype=torch.uint8, device=dev),
                         status=torch.zeros(1, dtype=torch.int32, device=dev),
                         pos=torch.zeros(1, dtype=torch.int32, device=dev))
         return self._mk
 
     def check_status(self):
-        """Raises if a barrier of the persistent kernel timed out (synchronizes)."""
+        """Raises if a wait of the persistent kernel timed out (synchronizes)."""
         if self._mk is not None:
             st = int(self._mk["status"].item())
             if st:
-                raise _lib.ScmxError(f"persistent decode kernel gave up at barrier {st - 100}")
+                raise _lib.ScmxError(f"persistent decode kernel: {_lib.describe_status(st)}")
 
     def _step_persistent(self, tok, cache, pos_dev):
         f, a = self.f, self.args
@@ -179,8 +175,7 @@ class DecodeQwen3(_Decoder):
         h = self.model.model.embed_tokens(tok)[0].clone()     # [1, D]; the kernel updates it in place
         _lib.call("scmx_decode_step_dense", _lib.ptr(mk["table"]), len(f.layers), a.hidden_size, a.intermediate_size, hq, hk, d,
                   float(f.eps), float(f.layers[0][0].self_attn.scale), _lib.ptr(f.inv_freq), _lib.ptr(f.rope_cs),
-                  f.rope_cs.shape[0], cache[0].k.shape[1], _lib.ptr(pos_dev), _lib.ptr(h), _lib.ptr(mk["y"]), _lib.ptr(mk["act"]),
-                  _lib.ptr(mk["o"]), _lib.ptr(self.attn.part), self.attn.nsplit, _lib.ptr(self.attn.counters), _lib.ptr(mk["bar"]),
+                  f.rope_cs.shape[0], cache[0].k.shape[1], _lib.ptr(pos_dev), _lib.ptr(h), _lib.ptr(mk["scratch"]), self.attn.nsplit,
                   _lib.ptr(mk["status"]), _lib.stream())
         xn = S.rmsnorm_quant_n(h, self.model.model.norm.weight, f.eps, 1)[2]
         return self.head(xn[None])

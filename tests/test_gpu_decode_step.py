@@ -1,0 +1,55 @@
+"""GPU: the one-kernel decode step (decode_step_kernel: rows as packets, weights in rings) bit for bit against the chain of kernels: one, two and four query heads per
+key/value head, the smallest and the largest widths, one layer and several, positions on both sides of a split's edge, a full cache, and steps that share the scratch."""
+import importlib
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+CASES = [(1024, 1024, 1, 8, 8), (1024, 3072, 3, 8, 2), (2048, 6144, 2, 16, 8), (2048, 1024, 2, 32, 16), (3072, 2048, 2, 8, 4), (6144, 6144, 1, 16, 4)]
+
+
+@pytest.mark.parametrize("D,F,layers,hq,hk", CASES)
+def test_step_equals_chain(scmx, D, F, layers, hq, hk):
+    mod = lambda n: importlib.import_module(scmx.__name__ + "." + n)      # noqa: E731
+    HM, FQ, DEC = mod("host_model"), mod("fused_qwen3"), mod("decode")
+    model = HM.CausalLM(HM.ModelArgs(D, F, layers, hq, hk, 128, 1e-6, 1e6, 512, True)).init_random(seed=D + F, scale=0.05).cuda()
+    fused = FQ.FusedQwen3(model, FQ.pack_model(model, on_device=True))
+    chain, mk = DEC.DecodeQwen3(fused, persistent=False), DEC.DecodeQwen3(fused, persistent=True)
+    assert mk.persistent
+    g = torch.Generator(device="cuda").manual_seed(D)
+    for held, capacity in ((0, 40), (31, 40), (32, 40), (33, 34), (700, 720), (39, 40)):
+        pair = [fused.make_cache(capacity) for _ in range(2)]
+        for c, d in zip(*pair):
+            for to, other in ((c.k, d.k), (c.v, d.v)):
+                to.copy_(torch.randn(to.shape, generator=g, device="cuda").to(to.dtype))
+                other.copy_(to)
+            c.offset = d.offset = held
+        tok = torch.tensor([[held % 512]], device="cuda")
+        for _ in range(min(2, capacity - held)):      # twice on one cache: the second step follows the first one's epochs
+            a, b = chain.step(tok, pair[0]), mk.step(tok, pair[1])
+            assert torch.equal(a, b), (held, capacity)
+        mk.check_status()
+        for c, d in zip(*pair):
+            assert torch.equal(c.k, d.k) and torch.equal(c.v, d.v)
+
+
+def test_step_after_one_that_gave_up(scmx):
+    """The abort word of a step that gave up and its epochs do not reach the next one."""
+    mod = lambda n: importlib.import_module(scmx.__name__ + "." + n)      # noqa: E731
+    HM, FQ, DEC = mod("host_model"), mod("fused_qwen3"), mod("decode")
+    model = HM.CausalLM(HM.ModelArgs(1024, 1024, 2, 8, 4, 128, 1e-6, 1e6, 512, True)).init_random(seed=3, scale=0.05).cuda()
+    fused = FQ.FusedQwen3(model, FQ.pack_model(model, on_device=True))
+    chain, mk = DEC.DecodeQwen3(fused, persistent=False), DEC.DecodeQwen3(fused, persistent=True)
+    c1, c2 = fused.make_cache(16), fused.make_cache(16)
+    for x in c1 + c2:
+        x.k.zero_(), x.v.zero_()
+    tok = torch.tensor([[5]], device="cuda")
+    assert torch.equal(chain.step(tok, c1), mk.step(tok, c2))
+    head = mk._mk["scratch"][:8].view(torch.int32)
+    before = int(head[0])
+    head[1] = 1                                       # as a thread that ran out of time leaves it
+    assert torch.equal(chain.step(tok, c1), mk.step(tok, c2))
+    assert head.tolist() == [before + (1 << 16) + 3, 0]
+    mk.check_status()
