@@ -333,7 +333,13 @@ static int run_gemv(GvArgs a, int epi, cudaStream_t st) {
     const size_t smem = (size_t)x_bytes + part + (size_t)a.slots * a.warps * GV_SLOT;
     SCMX_REQUIRE(smem <= 226 * 1024, SCMX_ELIMIT, "gemv_x: N=%d K=%d", a.N, a.K);
     auto kernel = epi == 0 ? gemv_x_kernel<T, 0> : epi == 1 ? gemv_x_kernel<T, 1> : epi == 2 ? gemv_x_kernel<T, 2> : epi == 3 ? gemv_x_kernel<T, 3> : gemv_x_kernel<bf16_t, 4>;
-    if (smem > 40 * 1024) SCMX_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static bool configured[64][5] = {};
+    const int dev = current_device();
+    SCMX_REQUIRE(dev >= 0, SCMX_ECUDA, "no current CUDA device (ordinal 0..63)");
+    if (!configured[dev][epi]) {
+        SCMX_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+        configured[dev][epi] = true;
+    }
     SCMX_PDL_OK("gemv_x_kernel", launch_pdl(kernel, dim3((unsigned)grid), dim3(GV_THREADS), smem, st, a));
     return SCMX_OK;
 }

@@ -158,8 +158,8 @@ __global__ void __launch_bounds__(256) quantize_kernel(const T* __restrict__ w, 
 // squared errors of the candidates are taken in float32, where the scaled values and their distances to the grid are exact, so a sum is
 // off by at most 10 roundings of 2^-24; only where two sums are closer than that (one block in 7000 of bfloat16 normal values) or the
 // exponent leaves float32's range is the block decided in float64 as above, by the whole warp, so the packed bits are the same.
-// Bound by instructions (about 400 a lane and vector, against 6.6 us for the bytes), where the float64 form was bound by its compares
-// and conversions.  6144 x 2048 bfloat16 (44 MB in and out): 28 us against 107 us; with the float64 decision made by one lane 43 us, the
+// Bound by instructions (against 6.6 us for the bytes), where the float64 form was bound by its compares and conversions.  Products and sums are taken two at
+// a time; min, max and masks have no such form.  6144 x 2048 bfloat16 (44 MB in and out): 26.6 us (28.7 singly) against 107 us; with the float64 decision made by one lane 43 us, the
 // codes by seven compares instead of the conversion instruction 50 us.
 constexpr float QUANT_CLEAR = 4e-6f;      // relative distance of two float32 sums from which their order is certain (10 x 2^-24 each)
 constexpr float QUANT_LEAST = 1e-30f;     // and that of two sums so small that squares may have lost bits below float32's range
@@ -195,31 +195,75 @@ __device__ __noinline__ int block_exponent_f64(const T* p) {
     return best;
 }
 
-// Sum of the squared distances of the eight |t| to the nearest E2M1 value: adding 2^22 times the power of two below max(|t|, 1) rounds
-// to the grid's step there (which of two equally near values is taken does not matter here).  NaN gives NaN.
-template <bool SATURATES>
-__device__ __forceinline__ float grid_sq_err(const float (&t)[8], float scale) {
-    float s = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const float a = fabsf(t[i]) * scale;
-        const float p = __int_as_float(__float_as_int(fmaxf(a, 1.0f)) & 0x7F800000);
-        const float r = fmaf(p, -4194304.0f, fmaf(p, 4194304.0f, a));
-        const float d = __fsub_rn(SATURATES ? fminf(r, 6.0f) : r, a);
-        s = fmaf(d, d, s);
-    }
-    s += __shfl_xor_sync(0xffffffffu, s, 1);
-    s += __shfl_xor_sync(0xffffffffu, s, 2);
-    return s;
+// Packed float32 pairs: one instruction for two products or sums (min, max and masks stay single).
+__device__ __forceinline__ uint64_t q_pack(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 q_unpack(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t q_mul(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t q_fma(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
 }
 
-// Eight codes of t = x / 2^e.  The conversion instruction takes ties to the even code; here they go to the smaller magnitude, so a value
+// Sum of the squared distances of the eight a = |t| (in pairs) times `scale` to the nearest E2M1 value: adding 2^22 times the power of two below
+// max(a, 1) rounds to the grid's step there (which of two equally near values is taken does not matter here).  NaN gives NaN.
+template <bool SATURATES>
+__device__ __forceinline__ float grid_sq_err(const uint64_t (&t)[4], float scale) {
+    const uint64_t big = q_pack(4194304.0f, 4194304.0f), small = q_pack(-4194304.0f, -4194304.0f), neg = q_pack(-1.0f, -1.0f), sc = q_pack(scale, scale);
+    uint64_t s = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint64_t a = scale == 1.0f ? t[i] : q_mul(t[i], sc);
+        const float2 v = q_unpack(a);
+        const uint64_t p = q_pack(__int_as_float(__float_as_int(fmaxf(v.x, 1.0f)) & 0x7F800000), __int_as_float(__float_as_int(fmaxf(v.y, 1.0f)) & 0x7F800000));
+        uint64_t r = q_fma(p, small, q_fma(p, big, a));
+        if (SATURATES) {
+            const float2 u = q_unpack(r);
+            r = q_pack(fminf(u.x, 6.0f), fminf(u.y, 6.0f));
+        }
+        const uint64_t d = q_fma(a, neg, r);
+        s = q_fma(d, d, s);
+    }
+    const float2 two = q_unpack(s);
+    float e = two.x + two.y;
+    e += __shfl_xor_sync(0xffffffffu, e, 1);
+    e += __shfl_xor_sync(0xffffffffu, e, 2);
+    return e;
+}
+
+// Eight codes of t = x si, si = 1 / 2^e.  The conversion instruction takes ties to the even code; here they go to the smaller magnitude, so a value
 // whose low 16 bits are zero, which a tie is, first loses one unit in its last place (that reaches no other tie).  A negative value that
 // becomes zero has no sign.
-__device__ __forceinline__ uint32_t e2m1_codes(const float (&t)[8]) {
+template <typename T>
+__device__ __forceinline__ uint32_t e2m1_codes(const float (&x)[8], float si) {
     float u[8];
+    if (sizeof(T) == 2) {                     // of a bfloat16 value the low 16 bits are always zero
+        const uint64_t below = q_pack(si * 0.99999994f, si * 0.99999994f);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) u[i] = t[i] * ((__float_as_uint(t[i]) & 0xFFFFu) ? 1.0f : 0.99999994f);
+        for (int i = 0; i < 4; ++i) {
+            const float2 v = q_unpack(q_mul(q_pack(x[2 * i], x[2 * i + 1]), below));
+            u[2 * i] = v.x;
+            u[2 * i + 1] = v.y;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float t = x[i] * si;
+            u[i] = t * ((__float_as_uint(t) & 0xFFFFu) ? 1.0f : 0.99999994f);
+        }
+    }
     uint32_t w;
     asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
         "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\tcvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n\t"
@@ -263,9 +307,9 @@ __device__ __forceinline__ int block_exponent(const float (&x)[8], const T* p) {
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
     const int e0 = (__float_as_int(amax) >> 23) - 127 - 2;       // of a normal number; others leave the range below
     const float si = __int_as_float((127 - min(max(e0, -QUANT_EXP), QUANT_EXP)) << 23);
-    float t[8];
+    uint64_t t[4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) t[i] = x[i] * si;
+    for (int i = 0; i < 4; ++i) t[i] = q_mul(q_pack(fabsf(x[2 * i]), fabsf(x[2 * i + 1])), q_pack(si, si));
     float err = grid_sq_err<true>(t, 1.0f);
     const float em = 0.25f * grid_sq_err<true>(t, 2.0f), ep = 4.0f * grid_sq_err<false>(t, 0.5f);
     auto clear = [](float a, float b) { return fabsf(a - b) > fmaxf(QUANT_CLEAR * fmaxf(a, b), QUANT_LEAST); };
@@ -305,6 +349,7 @@ struct QuantOut {
 };
 
 // Codes of vector v of row n, whose block has exponent max(e, lo_c); the row's smallest exponent is lo.  Run by every lane of a warp.
+template <typename T>
 __device__ __forceinline__ void write_codes(const float (&x)[8], int e, int lo_c, int lo, int64_t n, int K, int v, const QuantOut& o) {
     const int nv = K / 8, eb = max(e, lo_c), shift = eb - lo;
     const bool in = v < nv;
@@ -312,12 +357,11 @@ __device__ __forceinline__ void write_codes(const float (&x)[8], int e, int lo_c
     const float sum = ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));      // finite: no element is NaN
     if (eb >= -QUANT_EXP && eb <= QUANT_EXP && fabsf(sum) < INFINITY) {
         const float si = __int_as_float((127 - eb) << 23);
-        float t[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) t[i] = x[i] * si;
-        word = e2m1_codes(t);
-        const uint32_t plo = 0x03020100u << shift, phi = 0x0C080604u << shift;
-        decode_word(word, plo, phi, lut_negate(plo), lut_negate(phi), q[0], q[1]);
+        word = e2m1_codes<T>(x, si);
+        if (o.qw) {
+            const uint32_t plo = 0x03020100u << shift, phi = 0x0C080604u << shift;
+            decode_word(word, plo, phi, lut_negate(plo), lut_negate(phi), q[0], q[1]);
+        }
     } else {
         const double si = scalbn(1.0, -eb);
 #pragma unroll 1
@@ -369,7 +413,7 @@ __global__ void __launch_bounds__(1024) quantize_vec_kernel(const T* __restrict_
         if (hi == INT_MIN) hi = 0;            // all-zero row
         const int lo_c = hi - 3, lo = max(low, lo_c);      // min over blocks of max(e, lo_c)
         if (tid == 0) write_row(n, lo, wscale, row_exp);
-        write_codes(x, e, lo_c, lo, n, K, tid, out);
+        write_codes<T>(x, e, lo_c, lo, n, K, tid, out);
     }
 }
 
@@ -403,7 +447,7 @@ __global__ void __launch_bounds__(1024) quantize_long_kernel(const T* __restrict
         raw.zero();
         if (v < nv) raw.load(wr + 8 * (int64_t)v);
         raw.widen(x);
-        write_codes(x, v < nv ? s_e[v >> 2] : INT_MIN, lo_c, lo, n, K, v, out);
+        write_codes<T>(x, v < nv ? s_e[v >> 2] : INT_MIN, lo_c, lo, n, K, v, out);
     }
 }
 
