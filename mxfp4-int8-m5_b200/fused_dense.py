@@ -32,38 +32,45 @@ class DecodeRing:
         self.bufs = [[torch.empty(n, dtype=torch.int8, device=device) for n in self.sizes] for _ in range(2)]
         self.overlap = overlap
         self.side = torch.cuda.Stream(device=device) if overlap else None
+        self._raw = self.side.cuda_stream if overlap else None
+        self._views = {}                                      # (buffer set, place, N, K) -> its INT8 view: a handful of shapes
+        # One event a buffer set and direction, recorded anew for every group (a wait is on the record before it), and streams named by handle: the launches of a
+        # prompt of 4 layers and 4096 tokens, 1230 us on the device, took the host 1850 us with streams entered and events created per weight, 1110 us so.
+        self._ready, self._done = ([torch.cuda.Event(), torch.cuda.Event()] for _ in range(2))
+        self._edge = torch.cuda.Event()                       # side after main at the start, main after side at the end
 
     def begin(self, seq):
         """seq: list of (codes, bcodes, wscale, N, K) in the order the GEMMs run."""
         self.seq, self._joined = seq, None
-        ng = -(-len(seq) // self.group)
-        self.ready, self.done = [None] * ng, [None] * ng
         self.main = torch.cuda.current_stream()
         if self.overlap:
-            self.side.wait_stream(self.main)
+            self._after(self.side, self.main, self._edge)
             self._decode_group(0)
+
+    @staticmethod
+    def _after(stream, other, event):
+        event.record(other)
+        stream.wait_event(event)
 
     def _view(self, g):
         _, _, _, N, K = self.seq[g]
         j, p = divmod(g, self.group)
-        assert N * K <= self.sizes[p]
-        return self.bufs[j % 2][p][:N * K].view(N, K)
+        key = (j % 2, p, N, K)
+        v = self._views.get(key)
+        if v is None:
+            assert N * K <= self.sizes[p]
+            v = self._views[key] = self.bufs[j % 2][p][:N * K].view(N, K)
+        return v
 
     def _decode_group(self, j):
         lo, hi = j * self.group, min((j + 1) * self.group, len(self.seq))
-        if not self.overlap:
-            for g in range(lo, hi):
-                codes, bc, _, N, K = self.seq[g]
-                S.unpack_i8(codes, bc, N, K, out=self._view(g))
-            return
-        with torch.cuda.stream(self.side):
-            if j >= 2:
-                self.side.wait_event(self.done[j - 2])       # the last GEMM that read this set of buffers
-            for g in range(lo, hi):
-                codes, bc, _, N, K = self.seq[g]
-                S.unpack_i8(codes, bc, N, K, out=self._view(g))
-            self.ready[j] = torch.cuda.Event()
-            self.ready[j].record(self.side)
+        if self.overlap and j >= 2:
+            self.side.wait_event(self._done[j % 2])          # the last GEMM that read this set of buffers
+        for g in range(lo, hi):
+            codes, bc, _, N, K = self.seq[g]
+            S.unpack_i8(codes, bc, N, K, out=self._view(g), stream=self._raw)
+        if self.overlap:
+            self._ready[j % 2].record(self.side)
 
     def join(self, g):
         """Make the main stream wait for the decode of g's group and start the next group's decode.  Called by weight() when
@@ -75,7 +82,7 @@ class DecodeRing:
         if self.overlap:
             if (j + 1) * self.group < len(self.seq):
                 self._decode_group(j + 1)                    # overlaps with the GEMMs of group j
-            self.main.wait_event(self.ready[j])
+            self.main.wait_event(self._ready[j % 2])
         else:
             self._decode_group(j)
 
@@ -88,13 +95,12 @@ class DecodeRing:
     def released(self, g):
         """Call right after launching GEMM g."""
         if self.overlap and (g % self.group == self.group - 1 or g == len(self.seq) - 1):
-            self.done[g // self.group] = torch.cuda.Event()
-            self.done[g // self.group].record(self.main)
+            self._done[g // self.group % 2].record(self.main)
 
     def end(self):
         self._joined = None
         if self.overlap:
-            self.main.wait_stream(self.side)
+            self._after(self.main, self.side, self._edge)
 
 
 class DenseStack:

@@ -140,7 +140,7 @@ class FusedOlmoe:
         2048 x 1024 at 128 rows per expert take 592 us with the rest of a prompt against 765 us, the bits being the same."""
         asked = self.two_pass and self.two_pass != "auto"      # two passes at any length
         return (not asked and M_.FUSED_UNPACK and R // self.args.num_experts < MoeBlock.FUSED_BELOW and self.args.num_experts <= 512
-                and all(_lib.lib().scmx_w4_supported(F.DEFAULT.c_struct(), k) for k in (self.args.hidden_size, self.args.intermediate_size)))
+                and all(_lib.lib().scmx_w4_supported(F.c_default(), k) for k in (self.args.hidden_size, self.args.intermediate_size)))
 
     def _decode_experts(self, i):
         """Layer i's experts -> INT8 in ring[i % 2] on the side stream; waits for the GEMMs that last read that pair."""

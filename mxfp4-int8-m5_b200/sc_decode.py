@@ -51,12 +51,12 @@ def gemv(xq, codes, bcodes, xscale, wscale, N, epi, dtype=torch.bfloat16, res=No
     if xbf is not None:
         _lib.require_cuda(nw)
         _lib.call("scmx_gemv_pro", _lib.ptr(xbf), pro, _lib.ptr(nw) if pro == 2 else None, S._eps(eps) if pro == 2 else 0.0,
-                  _lib.ptr(codes), _lib.ptr(bcodes), _lib.ptr(wscale), N, K, F.DEFAULT.c_struct(), epi,
+                  _lib.ptr(codes), _lib.ptr(bcodes), _lib.ptr(wscale), N, K, F.c_default(), epi,
                   _lib.ptr(res) if epi == 2 else None, _lib.ptr(eidx), nslot, -1 if shared is None else int(shared), xstride,
                   _lib.ptr(out), int(USE_PDL), _lib.stream())
     else:
         _lib.call("scmx_gemv", _lib.ptr(xq), _lib.ptr(xscale), _lib.ptr(codes), _lib.ptr(bcodes), _lib.ptr(wscale), N, K,
-                  F.DEFAULT.c_struct(), epi, _lib.ptr(res) if epi == 2 else None, _lib.ptr(eidx), nslot,
+                  F.c_default(), epi, _lib.ptr(res) if epi == 2 else None, _lib.ptr(eidx), nslot,
                   -1 if shared is None else int(shared), xstride, _lib.ptr(out), int(USE_PDL), _lib.stream())
     return out if eidx is None else out.reshape(S_, no)
 

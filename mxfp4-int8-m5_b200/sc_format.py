@@ -10,6 +10,7 @@ from_shift_layout, quantize) so that callers written against it keep working:
 
 `quantize` runs on the GPU (scmx_quantize_sc_mxfp4, float64 arithmetic); the layout helpers are host-side NumPy.
 """
+import functools
 from dataclasses import dataclass
 
 import numpy as np
@@ -52,6 +53,19 @@ class Format:
 
 
 DEFAULT = Format()
+
+
+@functools.lru_cache(maxsize=16)
+def _c_of(fmt):
+    return fmt.c_struct()
+
+
+def c_default():
+    """The C struct of DEFAULT, shared and only read: filling one in is a third of the host time of a small launch."""
+    try:
+        return _c_of(DEFAULT)
+    except TypeError:                 # fields given as lists: equal formats cannot be recognised
+        return DEFAULT.c_struct()
 
 
 def _or_fields(vals, bits):

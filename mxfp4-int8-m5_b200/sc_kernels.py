@@ -32,12 +32,14 @@ def _bf16(x):
     return x
 
 
-def unpack_i8(codes, bcodes, N, K, deps=(), out=None):
-    """Packed codes + block codes -> INT8 operand [N, K] (written into `out` when given)."""
+def unpack_i8(codes, bcodes, N, K, deps=(), out=None, stream=None):
+    """Packed codes + block codes -> INT8 operand [N, K] (written into `out` when given).  stream: a raw handle, for an `out` that is not allocated here."""
     _lib.require_cuda(codes, bcodes, out)
+    assert stream is None or out is not None
     wq = out if out is not None else torch.empty((N, K), dtype=torch.int8, device=codes.device)
     assert wq.dtype == torch.int8 and wq.numel() >= N * K
-    _lib.call("scmx_unpack_i8", _lib.ptr(codes), _lib.ptr(bcodes), N, K, F.DEFAULT.c_struct(), _lib.ptr(wq), _lib.stream())
+    _lib.call("scmx_unpack_i8", _lib.ptr(codes), _lib.ptr(bcodes), N, K, F.c_default(), _lib.ptr(wq),
+              _lib.stream() if stream is None else stream)
     return wq
 
 
@@ -84,7 +86,7 @@ def mm_f4(dig, codes, factors, xscale, wscale, epi, res=None):
     assert epi in (0, 1, 2, 3) and N % 32 == 0 and (epi != 2 or tuple(res.shape) == (M, N))
     out = torch.empty((M, N), dtype=torch.int32, device=dig.device) if epi == 0 else \
         torch.empty((M, N // 2 if epi == 3 else N), dtype=torch.bfloat16, device=dig.device)
-    _lib.call("scmx_mm_f4", _lib.ptr(dig), M, _lib.ptr(codes), _lib.ptr(factors), M, N, K, F.DEFAULT.c_struct(), epi, _lib.ptr(xscale), _lib.ptr(wscale),
+    _lib.call("scmx_mm_f4", _lib.ptr(dig), M, _lib.ptr(codes), _lib.ptr(factors), M, N, K, F.c_default(), epi, _lib.ptr(xscale), _lib.ptr(wscale),
               _lib.ptr(res) if epi == 2 else None, _lib.ptr(out), _lib.ptr(_lib.status_buffer()), _lib.stream())
     return out
 

@@ -85,7 +85,7 @@ def gather_rows(xq, xs, tok, R):
 
 def f4_fits(n_experts, *widths):
     """Whether the products on digit planes (moe_mm_f4) take this many experts and these input widths in the current default format."""
-    return n_experts <= 512 and all(_lib.lib().scmx_f4_supported(F.DEFAULT.c_struct(), k) for k in widths)
+    return n_experts <= 512 and all(_lib.lib().scmx_f4_supported(F.c_default(), k) for k in widths)
 
 
 def gather_digits(xq, xs, tok, R):
@@ -113,7 +113,7 @@ def moe_mm_f4(dig, R, codes, factors, wscale, off, N, epi, xscale=None):
     _lib.require_cuda(dig, codes, factors, wscale, off, xscale)
     E, K = wscale.shape[0], dig.shape[2] * 8
     out = _out(R, N, epi, dig.device)
-    _lib.call("scmx_moe_mm_f4", _lib.ptr(dig), dig.shape[1], R, _lib.ptr(codes), _lib.ptr(factors), _lib.ptr(wscale), _lib.ptr(off), E, N, K, F.DEFAULT.c_struct(),
+    _lib.call("scmx_moe_mm_f4", _lib.ptr(dig), dig.shape[1], R, _lib.ptr(codes), _lib.ptr(factors), _lib.ptr(wscale), _lib.ptr(off), E, N, K, F.c_default(),
               epi, _lib.ptr(xscale), _lib.ptr(out), _lib.ptr(_lib.status_buffer()), _lib.stream())
     return out
 
@@ -134,9 +134,9 @@ def moe_mm(xq, R, codes, bcodes, wscale, off, tstart, max_tiles, N, epi, xscale=
     E = wscale.shape[0]
     assert N % 32 == 0 and K % 16 == 0 and codes.numel() == E * N * K // 8
     out = _out(R, N, epi, xq.device)
-    if FUSED_UNPACK and E <= 512 and _lib.lib().scmx_w4_supported(F.DEFAULT.c_struct(), K):
+    if FUSED_UNPACK and E <= 512 and _lib.lib().scmx_w4_supported(F.c_default(), K):
         _lib.call("scmx_moe_mm_w4", _lib.ptr(xq), R, _lib.ptr(codes), _lib.ptr(bcodes), _lib.ptr(wscale), _lib.ptr(off), E, N, K,
-                  F.DEFAULT.c_struct(), epi, _lib.ptr(xscale), _lib.ptr(out), _lib.ptr(_lib.status_buffer()), _lib.stream())
+                  F.c_default(), epi, _lib.ptr(xscale), _lib.ptr(out), _lib.ptr(_lib.status_buffer()), _lib.stream())
         return out
     epp = min(EXPERTS_PER_PASS, E)
     need = 2 * epp * N * K
@@ -147,7 +147,7 @@ def moe_mm(xq, R, codes, bcodes, wscale, off, tstart, max_tiles, N, epi, xscale=
     buf = _scratch[key]
     base = (-buf.data_ptr()) % 1024
     _lib.call("scmx_moe_mm", _lib.ptr(xq), R, _lib.ptr(codes), _lib.ptr(bcodes), _lib.ptr(wscale), _lib.ptr(off),
-              _lib.ptr(tstart), E, N, K, F.DEFAULT.c_struct(), epi, _lib.ptr(xscale), _lib.ptr(out), TM, epp,
+              _lib.ptr(tstart), E, N, K, F.c_default(), epi, _lib.ptr(xscale), _lib.ptr(out), TM, epp,
               _lib.c_vp(buf.data_ptr() + base), need, _lib.ptr(_lib.status_buffer()), _lib.stream())
     return out
 

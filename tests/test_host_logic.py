@@ -309,3 +309,16 @@ def test_replaced_quantizer_is_called(scmx, monkeypatch):
     del plain.act_q
     monkeypatch.setattr(FQ.FusedQwen3, "act_q", lambda self, x, Mp: ("class", "scales"))
     assert ask(plain) == "class"
+
+
+def test_shared_format_struct(scmx):
+    """The struct handed to the kernels follows DEFAULT, is never the caller's own, and formats given as lists still work."""
+    F, S = scmx.sc_format, scmx.sc_kernels
+    old = F.DEFAULT
+    try:
+        for fmt in (F.Format(), F.Format(block=16, mult=(1, 2, 3, 4, 5, 6, 8, 10), bc_bits=4), F.Format(code_mag=[0, 1, 2, 3, 4, 6, 8, 12], mult=[1, 2, 4])):
+            S.set_format(fmt)
+            fmt.c_struct().block = 99
+            assert bytes(F.c_default()) == bytes(fmt.c_struct())
+    finally:
+        S.set_format(old)
