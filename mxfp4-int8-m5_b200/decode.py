@@ -14,7 +14,7 @@ signature.
 persistent=True (DecodeQwen3) runs all layers of a step as ONE cooperative kernel (scmx_decode_step_dense): rows travel between
 the phases of a layer as packets instead of across kernel boundaries, each CTA re-quantizes the activations it needs in
 shared memory, and weights stream ahead of the phases.  Same bits as the chain of kernels; used where its limits
-hold (head size 128, widths multiples of 1024 up to 6144) and attention="kernel".
+hold (head size 128, widths multiples of 1024 up to 6144, 256 layers) and attention="kernel".
 
 DecodeHybrid is the same for hybrid decoders (fused_hybrid.FusedHybrid): GEMVs on bfloat16 or float32 weights with the mixers'
 one-token kernels between them, float32 activations."""
@@ -135,7 +135,7 @@ class DecodeQwen3(_Decoder):
         fits = lambda n: n % 1024 == 0 and n <= 6144  # noqa: E731
         self.persistent = bool(persistent and self.attn is not None and a.head_dim == 128 and fits(a.hidden_size)
                                and fits(a.intermediate_size) and fits(a.num_attention_heads * a.head_dim)
-                               and a.num_attention_heads <= 32 and fused.fmt == type(fused.fmt)())
+                               and a.num_attention_heads <= 32 and a.num_hidden_layers <= 256 and fused.fmt == type(fused.fmt)())
 
     def _persistent_state(self, cache):
         """Layer table (device pointers of the packed weights, norms and this cache's tensors) and scratch buffers."""

@@ -129,3 +129,33 @@ def test_grouped_bits(scmx, counts, N, K):
         want = M_.moe_mm_i8(xp, R, wq.view(E * N, K), ws, off, ts, -(-R // M_.TM) + E, N, epi, xs)
         assert torch.equal(M_.moe_mm_f4(dig, R, c, fac, ws, off, N, epi, xs), want), epi
     scmx._lib.check_status()
+
+
+@pytest.mark.parametrize("kind,tokens", [("dense", 1), ("dense", 31), ("dense", 129), ("moe", 1), ("moe", 33), ("moe", 200)])
+def test_prompts_equal_both_ways(scmx, monkeypatch, kind, tokens):
+    """Prompts on digit planes against the INT8 products, at an empty cache and behind held positions: hidden states and cache rows bit for bit; a replaced attention is called."""
+    HM = scmx.host_model
+    if kind == "dense":
+        FU = scmx.fused_qwen3
+        model = HM.CausalLM(HM.ModelArgs(512, 768, 2, 4, 2, 128, 1e-6, 1e6, 512, True)).init_random(seed=4, scale=0.05).cuda()
+        f, cls, limits = FU.FusedQwen3(model, FU.pack_model(model, on_device=True)), FU.FusedQwen3, ("F4_TOKENS", "F4_TOKENS_SMALL")
+    else:
+        FU = scmx.fused_olmoe
+        model = HM.CausalLM(HM.ModelArgs(512, 256, 2, 4, 4, 128, 1e-5, 1e4, 512, False, 8, 2, False, "olmoe")).init_random(seed=4, scale=0.05).cuda()
+        f, cls, limits = FU.FusedOlmoe(model, FU.pack_olmoe(model)), FU.FusedOlmoe, ("F4_ROWS",)
+    ids = torch.randint(0, 512, (1, tokens), generator=torch.Generator().manual_seed(tokens)).cuda()
+    out = {}
+    for on in (True, False):
+        for n in limits:
+            monkeypatch.setattr(cls, n, 1 << 20 if on else -1)
+        assert f._f4(tokens) is on
+        cache, calls = f.make_cache(2 * tokens + 8), []
+        own = f.sdpa
+        hs = [f.hidden(ids, cache)]
+        f.sdpa = lambda *a: calls.append(1) or own(*a)
+        hs.append(f.hidden(ids, cache))
+        f.sdpa = own
+        assert len(calls) == 2
+        out[on] = hs + [x[:, :2 * tokens] for c in cache for x in (c.k, c.v)]
+    assert all(torch.equal(a, b) for a, b in zip(out[True], out[False]))
+    scmx._lib.check_status()

@@ -322,3 +322,40 @@ def test_shared_format_struct(scmx):
             assert bytes(F.c_default()) == bytes(fmt.c_struct())
     finally:
         S.set_format(old)
+
+
+@pytest.mark.parametrize("layers,one_kernel", [(1, True), (256, True), (257, False)])
+def test_decode_step_form(scmx, layers, one_kernel):
+    """A decoder with more layers than the one-kernel step's table holds takes the chain of kernels."""
+    from types import SimpleNamespace as NS
+    args = scmx.host_model.ModelArgs(1024, 1024, layers, 8, 4, 128, 1e-6, 1e6, 512, True)
+    fused = NS(epilogue="gemm", model=NS(), args=args, inv_freq=torch.zeros(64), fmt=scmx.sc_format.Format())
+    assert scmx.decode.DecodeQwen3(fused, head=lambda x: x).persistent is one_kernel
+
+
+def test_prompts_on_digit_planes(scmx):
+    """Which prompts of a dense decoder run on digit planes: few tokens, the default format, and none of the class's own steps replaced."""
+    from types import SimpleNamespace as NS
+    FQ, F, S = scmx.fused_qwen3, scmx.sc_format, scmx.sc_kernels
+
+    class Own(FQ.FusedQwen3):
+        def rms_q(self, h, nw, Mp=None):
+            return "own", "scales"
+
+    def make(cls=FQ.FusedQwen3, width=4096, K=2048, **kw):
+        f = cls.__new__(cls)
+        f.layers, f.epilogue, f.resident, f.rot, f.record = [(None, {g: NS(N=width, K=K) for g in FQ.GROUPS})], "gemm", False, False, None
+        f.__dict__.update(kw)
+        return f
+
+    limit, small = FQ.FusedQwen3.F4_TOKENS, FQ.FusedQwen3.F4_TOKENS_SMALL
+    assert [make()._f4(n) for n in (0, 1, limit, limit + 1)] == [False, True, True, False]
+    assert [make(width=1024)._f4(n) for n in (small, small + 1)] == [True, False]
+    assert not any(make(**kw)._f4(16) for kw in (dict(cls=Own), dict(K=2048 + 64), dict(K=10240), dict(epilogue="row"), dict(resident=True), dict(rot="down"),
+                                                 dict(record={}), dict(act_q=lambda x, Mp: None), dict(_rec=lambda *a: None)))
+    old = F.DEFAULT
+    try:
+        S.set_format(F.Format(block=16, mult=(1, 2, 3, 4, 5, 6, 8, 10), bc_bits=4))
+        assert not make()._f4(16)
+    finally:
+        S.set_format(old)
