@@ -376,7 +376,7 @@ int scmx_gemv_pro(const uint16_t* x, int pro, const uint16_t* nw, float eps, con
 
 /* ---- one decode step of a dense stack as a persistent kernel ------------------------------------------------------------- */
 
-/* Weights of one decoder layer for scmx_decode_step_dense: [0] q|k|v rows concatenated, [1] o, [2] gate|up with rows
+/* Weights of one decoder layer for scmx_decode_step: [0] q|k|v rows concatenated, [1] o, [2] gate|up with rows
  * interleaved for the SwiGLU epilogue, [3] down; SC-MXFP4 in the default format (block 32, shifts).  k_cache / v_cache:
  * bf16 [hk, capacity, d]. */
 typedef struct scmx_decode_layer {
@@ -403,21 +403,24 @@ typedef struct scmx_decode_layer {
  * Limits: d = 128; D, F and hq*d multiples of 1024 up to 6144; hq/hk in {1, 2, 4}; hk * nsplit <= number of SMs (64 to 256); 256 layers.
  * Not to be run concurrently with other work on the same device: the launch needs every SM. */
 int64_t scmx_decode_step_scratch(int D, int F, int hq, int hk, int d, int nsplit);
+int scmx_decode_step(const scmx_decode_layer* layers, int n_layers, int D, int F, int hq, int hk, int d, float eps,
+                     float scale, const float* inv_freq, const float* rope_table, int64_t rope_rows, int64_t capacity,
+                     const int32_t* pos_dev, uint16_t* h, void* scratch, int nsplit, int32_t* status, void* stream);
+/* scmx_decode_step with scratch that is allocated and zeroed in the stream's order by every call; y bf16 [(hq + 2 hk) d], act bf16 [F], o bf16 [hq d], partials
+ * f32 [hq, nsplit, d + 2], counters int32 [hk] and barrier uint32 [2] have to be given and are not touched. */
 int scmx_decode_step_dense(const scmx_decode_layer* layers, int n_layers, int D, int F, int hq, int hk, int d, float eps,
                            float scale, const float* inv_freq, const float* rope_table, int64_t rope_rows, int64_t capacity,
-                           const int32_t* pos_dev, uint16_t* h, void* scratch, int nsplit, int32_t* status, void* stream);
+                           const int32_t* pos_dev, uint16_t* h, uint16_t* y, uint16_t* act, uint16_t* o, float* partials,
+                           int nsplit, int32_t* counters, uint32_t* barrier, int32_t* status, void* stream);
 /* Output head of one row: out bf16 [N] = W bf16 [N, ldw] x, x bf16 [K], float32 sums.  K a multiple of 8 up to 6400, rows 16-byte aligned. */
 int scmx_head_bf16(const uint16_t* W, int64_t ldw, const uint16_t* x, int64_t N, int64_t K, uint16_t* out, void* stream);
 /* Greedy choice inside a captured decode step: *tok = out[*count] = index of the largest of V logits (bf16 or float; the lowest of equal ones, a
  * not-a-number value counts as the largest), *count += 1, *pos += 1.  Nothing is stored in out at cap or beyond.  In libscmx_mixers too. */
 int scmx_select_token(const void* logits, int is_f32, int64_t V, int64_t* tok, int32_t* pos, int32_t* count, int64_t* out, int64_t cap, void* stream);
-/* Diagnostic: while device_buf is set, CTA 0 of scmx_decode_step_dense stores its SM cycle counter in device_buf[0 .. n)
- * at every barrier entry and exit and, in the attention phase, after the q/k/v preparation and after the split's positions,
- * layer after layer; with
- * n_and_barrier = n | (b << 16), b > 0, every CTA also stores the global nanosecond timer at its arrival at barrier b
- * (1-based) in device_buf[n + CTA index].  device_buf: uint64 [n + number of SMs].  0 switches it off.  Process-wide; no
- * counterpart in the reference. */
-int scmx_set_decode_trace(unsigned long long* device_buf, int n_and_barrier);
+/* Diagnostic: while device_buf is set, CTA 0 of the one-kernel decode step stores its SM cycle counter in device_buf[0 .. n), n < 65536, at
+ * the ends of its phases, nine a layer: layer entered (the row before it done), input row there, q|k|v rows, attention, input row of o, o rows, input row of
+ * gate|up, gate|up rows, input row of down.  device_buf: uint64 [n].  0 switches it off.  Process-wide; no counterpart in the reference. */
+int scmx_set_decode_trace(unsigned long long* device_buf, int n);
 
 #ifdef __cplusplus
 }

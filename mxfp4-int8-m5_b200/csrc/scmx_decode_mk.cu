@@ -696,9 +696,9 @@ extern "C" int64_t scmx_decode_step_scratch(int D, int F, int hq, int hk, int d,
     return D > 0 && F > 0 && hq > 0 && hk > 0 && d > 0 && nsplit > 0 ? (int64_t)mk_scratch(D, F, hq, hk, d, nsplit, off) : 0;
 }
 
-extern "C" int scmx_decode_step_dense(const scmx_decode_layer* layers, int n_layers, int D, int F, int hq, int hk, int d, float eps,
-                                      float scale, const float* inv_freq, const float* rope_table, int64_t rope_rows,
-                                      int64_t capacity, const int32_t* pos_dev, uint16_t* h, void* scratch, int nsplit, int32_t* status, void* stream) {
+extern "C" int scmx_decode_step(const scmx_decode_layer* layers, int n_layers, int D, int F, int hq, int hk, int d, float eps,
+                                float scale, const float* inv_freq, const float* rope_table, int64_t rope_rows,
+                                int64_t capacity, const int32_t* pos_dev, uint16_t* h, void* scratch, int nsplit, int32_t* status, void* stream) {
     SCMX_REQUIRE(layers && pos_dev && h && scratch && status && inv_freq, SCMX_EINVAL, "decode_step: null buffer");
     SCMX_REQUIRE(n_layers > 0 && hq > 0 && hk > 0 && hq % hk == 0 && hq <= MK_MAXHQ, SCMX_EINVAL, "decode_step: hq=%d hk=%d", hq, hk);
     SCMX_REQUIRE(d == 128, SCMX_ELIMIT, "decode_step: head size %d (128)", d);
@@ -753,4 +753,24 @@ extern "C" int scmx_decode_step_dense(const scmx_decode_layer* layers, int n_lay
                            : cudaLaunchKernelEx(&cfg, decode_step_kernel<4, 128>, a);
     SCMX_PDL_OK("decode_step_kernel", e);
     return SCMX_OK;
+}
+
+// The step on scratch of its own, allocated and given back in the stream's order (a captured graph gets nodes for it).
+extern "C" int scmx_decode_step_dense(const scmx_decode_layer* layers, int n_layers, int D, int F, int hq, int hk, int d, float eps,
+                                      float scale, const float* inv_freq, const float* rope_table, int64_t rope_rows,
+                                      int64_t capacity, const int32_t* pos_dev, uint16_t* h, uint16_t* y, uint16_t* act, uint16_t* o,
+                                      float* partials, int nsplit, int32_t* counters, uint32_t* barrier, int32_t* status, void* stream) {
+    SCMX_REQUIRE(y && act && o && partials && counters && barrier, SCMX_EINVAL, "decode_step: null buffer");
+    const int64_t bytes = scmx_decode_step_scratch(D, F, hq, hk, d, nsplit);
+    SCMX_REQUIRE(bytes > 0 && nsplit <= 32, SCMX_EINVAL, "decode_step: D=%d F=%d hq=%d hk=%d d=%d nsplit=%d", D, F, hq, hk, d, nsplit);
+    cudaStream_t st = (cudaStream_t)stream;
+    void* scratch = nullptr;
+    SCMX_CUDA_OK(cudaMallocAsync(&scratch, (size_t)bytes, st));
+    const cudaError_t zero = cudaMemsetAsync(scratch, 0, (size_t)bytes, st);
+    const int rc = zero != cudaSuccess ? SCMX_OK
+                                       : scmx_decode_step(layers, n_layers, D, F, hq, hk, d, eps, scale, inv_freq, rope_table, rope_rows, capacity, pos_dev, h,
+                                                          scratch, nsplit, status, stream);
+    SCMX_CUDA_OK(cudaFreeAsync(scratch, st));
+    SCMX_CUDA_OK(zero);
+    return rc;
 }

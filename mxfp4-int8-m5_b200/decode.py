@@ -11,7 +11,7 @@ fuse_prologue selects where the per-token INT8 of a GEMV input is computed in th
 kernel); here both forms run the row kernel followed by the GEMV and give the same values, so the argument only keeps the
 signature.
 
-persistent=True (DecodeQwen3) runs all layers of a step as ONE cooperative kernel (scmx_decode_step_dense): rows travel between
+persistent=True (DecodeQwen3) runs all layers of a step as ONE cooperative kernel (scmx_decode_step): rows travel between
 the phases of a layer as packets instead of across kernel boundaries, each CTA re-quantizes the activations it needs in
 shared memory, and weights stream ahead of the phases.  Same bits as the chain of kernels; used where its limits
 hold (head size 128, widths multiples of 1024 up to 6144, 256 layers) and attention="kernel".
@@ -173,7 +173,7 @@ class DecodeQwen3(_Decoder):
             pos_dev.fill_(cache[0].offset)
         hq, hk, d = a.num_attention_heads, a.num_key_value_heads, a.head_dim
         h = self.model.model.embed_tokens(tok)[0].clone()     # [1, D]; the kernel updates it in place
-        _lib.call("scmx_decode_step_dense", _lib.ptr(mk["table"]), len(f.layers), a.hidden_size, a.intermediate_size, hq, hk, d,
+        _lib.call("scmx_decode_step", _lib.ptr(mk["table"]), len(f.layers), a.hidden_size, a.intermediate_size, hq, hk, d,
                   float(f.eps), float(f.layers[0][0].self_attn.scale), _lib.ptr(f.inv_freq), _lib.ptr(f.rope_cs),
                   f.rope_cs.shape[0], cache[0].k.shape[1], _lib.ptr(pos_dev), _lib.ptr(h), _lib.ptr(mk["scratch"]), self.attn.nsplit,
                   _lib.ptr(mk["status"]), _lib.stream())

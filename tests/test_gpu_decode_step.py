@@ -53,3 +53,34 @@ def test_step_after_one_that_gave_up(scmx):
     assert torch.equal(chain.step(tok, c1), mk.step(tok, c2))
     assert head.tolist() == [before + (1 << 16) + 3, 0]
     mk.check_status()
+
+
+def test_entry_with_scratch_of_its_own(scmx):
+    """scmx_decode_step_dense, which allocates its scratch, against scmx_decode_step: the residual row bit for bit, alone and from a captured graph; its other buffers are not touched."""
+    mod = lambda n: importlib.import_module(scmx.__name__ + "." + n)      # noqa: E731
+    HM, FQ, DEC, L = mod("host_model"), mod("fused_qwen3"), mod("decode"), scmx._lib
+    model = HM.CausalLM(HM.ModelArgs(1024, 2048, 2, 8, 4, 128, 1e-6, 1e6, 512, True)).init_random(seed=3, scale=0.05).cuda()
+    fused = FQ.FusedQwen3(model, FQ.pack_model(model, on_device=True))
+    dec, cache = DEC.DecodeQwen3(fused), fused.make_cache(16)
+    for x in cache:
+        x.k.normal_(), x.v.normal_()
+    mk, pos, nsplit = dec._persistent_state(cache), torch.tensor([7], dtype=torch.int32, device="cuda"), dec.attn.nsplit
+    h0 = torch.randn(1024, generator=torch.Generator(device="cuda").manual_seed(1), device="cuda").to(torch.bfloat16)
+    a, b = h0.clone(), h0.clone()
+    other = [torch.zeros(64, dtype=torch.int32, device="cuda") for _ in range(6)]
+    head = lambda h: (L.ptr(mk["table"]), 2, 1024, 2048, 8, 4, 128, 1e-6, 128 ** -0.5, L.ptr(fused.inv_freq), L.ptr(fused.rope_cs), fused.rope_cs.shape[0], 16,      # noqa: E731
+                      L.ptr(pos), L.ptr(h))
+    y, act, o, partials, counters, barrier = (L.ptr(x) for x in other)
+    dense = lambda: L.call("scmx_decode_step_dense", *head(b), y, act, o, partials, nsplit, counters, barrier, L.ptr(mk["status"]), L.stream())      # noqa: E731
+    L.call("scmx_decode_step", *head(a), L.ptr(mk["scratch"]), nsplit, L.ptr(mk["status"]), L.stream())
+    dense()
+    assert torch.equal(a, b) and not torch.equal(a, h0)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        dense()
+    for _ in range(2):
+        b.copy_(h0)
+        graph.replay()
+        assert torch.equal(a, b)
+    dec.check_status()
+    assert not any(bool(x.any()) for x in other)
