@@ -216,10 +216,14 @@ class DecodeOlmoe(_Decoder):
         H, d, D, eps = a.num_attention_heads, a.head_dim, a.hidden_size, f.eps
         F2, k = 2 * a.intermediate_size, a.num_experts_per_tok
         h = self.model.model.embed_tokens(tok)[0]
+        row = out = None
         for i, (layer, ws, ex) in enumerate(f.layers):
             at, c = layer.self_attn, cache[i]
             w, wo = ws["qkv"], ws["o"]
-            y = G.gemv(h, w.codes, w.bcodes, None, w.wscale, 3 * H * d, 1, pro=2, nw=layer.input_layernorm.weight, eps=eps)
+            if row is None:
+                y = G.gemv(h, w.codes, w.bcodes, None, w.wscale, 3 * H * d, 1, pro=2, nw=layer.input_layernorm.weight, eps=eps)
+            else:
+                y = G.gemv(row[0], w.codes, w.bcodes, row[1], w.wscale, 3 * H * d, 1)
             q, kk, v = S.qkv_fullnorm_y(y[None], at.q_norm.weight, at.k_norm.weight, eps, 1, H, d,
                                         rope=(f.inv_freq, c.offset, f.rope_cs), cache=c, pos_dev=pos_dev)
             o = self._attend(at, c, q, kk, v, pos_dev)
@@ -231,9 +235,14 @@ class DecodeOlmoe(_Decoder):
             (cg, bg, sg), (cd, bd, sd) = ex["gu"], ex["down"]
             act = G.gemv(xq, cg, bg, xs, sg, F2, 3, eidx=e, xstride=0)            # [k, F]
             yd = G.gemv(act, cd, bd, None, sd, D, 1, eidx=e, xstride=1, pro=1)    # [k, D], per-row INT8 in the prologue
-            h = M_.moe_combine(yd, self.pos, scores, h, pn, eps, 1, quant=False)[0]
-        xn = S.rmsnorm_quant_n(h, self.model.model.norm.weight, eps, 1)[2]
-        return self.head(xn[None])
+            # the sum of the experts' rows and the norm that follows: the next layer's INT8 row, or the output head's row
+            last = i + 1 == len(f.layers)
+            nn = self.model.model.norm.weight if last else f.layers[i + 1][0].input_layernorm.weight
+            if D <= 8192:
+                h, *row, out = M_.combine_norm(yd, self.pos, scores, h, nn, eps, quant=not last, normed=last)
+            else:
+                h = M_.moe_combine(yd, self.pos, scores, h, pn, eps, 1, quant=False)[0]
+        return self.head((S.rmsnorm_quant_n(h, self.model.model.norm.weight, eps, 1)[2] if out is None else out)[None])
 
 
 def _row(row, in_parts):
