@@ -179,6 +179,10 @@ int scmx_router_topk(const float* logits, int64_t M, int E, int topk, int32_t* i
                      float* scores_f32, void* stream);
 /* The router of one token in one kernel: logits bf16(W xn) (W bf16 [E, D], xn bf16 [D], 16-byte aligned, D % 8 == 0), then as scmx_router_topk. */
 int scmx_route_token(const uint16_t* xn, const uint16_t* W, int D, int E, int topk, int32_t* inds, uint16_t* scores, void* stream);
+/* The same of the row x before its RMSNorm (weights nw [D], D <= 8192), with the normalized row's INT8 row xq and scale xs: the bits of scmx_rmsnorm_quant and
+ * scmx_route_token one after the other. */
+int scmx_norm_route_token(const uint16_t* x, const uint16_t* nw, float eps, const uint16_t* W, int D, int E, int topk, int8_t* xq, float* xs, int32_t* inds,
+                          uint16_t* scores, void* stream);
 
 /* Row gather: dst_q[p] = xq[tok[p]] for p < rows_q, dst_s[p] = xs[tok[p]] for p < rows_s
  * (the `xq[tok_p], xs[tok_p[:R]]` of e2e/fused_olmoe.py:230). */

@@ -115,6 +115,7 @@ SIGNATURES = {
     "scmx_select_token": [c_vp, c_int, c_i64, c_vp, c_vp, c_vp, c_vp, c_i64, c_vp],
     "scmx_head_bf16": [c_vp, c_i64, c_vp, c_i64, c_i64, c_vp, c_vp],
     "scmx_route_token": [c_vp, c_vp, c_int, c_int, c_int, c_vp, c_vp, c_vp],
+    "scmx_norm_route_token": [c_vp, c_vp, c_float, c_vp, c_int, c_int, c_int, c_vp, c_vp, c_vp, c_vp, c_vp],
     "scmx_gemv_pro": [c_vp, c_int, c_vp, c_float, c_vp, c_vp, c_vp, c_i64, c_i64, _FMT_P, c_int, c_vp, c_vp, c_int, c_int, c_int,
                       c_vp, c_int, c_vp],
     "scmx_gemv_multi_plan": [c_vp, c_int, _FMT_P],

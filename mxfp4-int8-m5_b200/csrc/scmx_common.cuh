@@ -206,6 +206,21 @@ __device__ __forceinline__ float rms_inverse(double ss, int K, float eps) {
     return (float)(1.0 / sqrt((double)m));
 }
 
+// Eight elements of a row normalized in place: f[j] = T(w[j] * T(f[j] * inv)), T = round to bfloat16; returns them packed.
+// Roundings are taken two at a time (pack_bf16x2).
+__device__ __forceinline__ uint4 norm8(float (&f)[8], const uint4& wraw, float inv) {
+    const uint32_t w[4] = {wraw.x, wraw.y, wraw.z, wraw.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint32_t t = pack_bf16x2(__fmul_rn(f[2 * j], inv), __fmul_rn(f[2 * j + 1], inv));
+        o[j] = pack_bf16x2(__fmul_rn(bf16_lo(w[j]), bf16_lo(t)), __fmul_rn(bf16_hi(w[j]), bf16_hi(t)));
+        f[2 * j] = bf16_lo(o[j]);
+        f[2 * j + 1] = bf16_hi(o[j]);
+    }
+    return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
 // s = amax / 127, qi = s > 0 ? 1 / s : 0 in IEEE float32 (e2e/sc_kernels.py:221-222).
 __device__ __forceinline__ void quant_scale(float amax, float& s, float& qi) {
     s = __fdiv_rn(amax, 127.0f);

@@ -210,47 +210,109 @@ __global__ void __launch_bounds__(256) router_topk_kernel(const float* __restric
 // weights are requested while the previous kernel still runs, and the logits meet in the first CTA's shared memory.
 constexpr int RT_CTAS = 8, RT_WARPS = 8, RT_PRE = 8;
 
-template <int PER>
+__device__ __forceinline__ float rt_dot(const uint4& a, const uint4& b, float s) {
+    const uint32_t u[4] = {a.x, a.y, a.z, a.w}, v[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        s = fmaf(bf16_lo(u[k]), bf16_lo(v[k]), s);
+        s = fmaf(bf16_hi(u[k]), bf16_hi(v[k]), s);
+    }
+    return s;
+}
+// NV 0: x is the normalized row.  Else (D <= 2048 NV) x is the row before the norm with weights nw: every CTA normalizes it in shared memory, the last one
+// writes its INT8 row xq and scale xs, in place of a launch of the row quantizer before (generation of 8 tokens by two layers 1051 -> 1004 us).
+template <int PER, int NV>
 __global__ void __cluster_dims__(RT_CTAS, 1, 1) __launch_bounds__(32 * RT_WARPS)
-    route_token_kernel(const uint16_t* xn, const uint16_t* W, int D, int E, int topk, int32_t* inds, uint16_t* scores) {
-    __shared__ float lg[32 * PER];
+    route_token_kernel(const uint16_t* x, const uint16_t* nw, float eps, const uint16_t* W, int D, int E, int topk, int8_t* xq, float* xs, int32_t* inds,
+                       uint16_t* scores) {
+    constexpr int THREADS = 32 * RT_WARPS, NVS = NV > 0 ? NV : 1;
+    __shared__ float lg[32 * PER], red[33];
+    __shared__ double dred[33];
+    __shared__ uint4 row[NV > 0 ? THREADS * NV : 1];
     cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
     pdl_launch_dependents();
-    const int rank = (int)cl.block_rank(), lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nv = D / 8;
+    const int rank = (int)cl.block_rank(), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nv = D / 8;
     const int first = rank * RT_WARPS + warp;
-    uint4 pre[RT_PRE];
+    uint4 pre[RT_PRE], nwv[NVS];
 #pragma unroll
     for (int i = 0; i < RT_PRE; ++i)
         if (first < E && lane + 32 * i < nv) pre[i] = __ldg(reinterpret_cast<const uint4*>(W + (size_t)first * D) + lane + 32 * i);
+    if (NV > 0) {
+#pragma unroll
+        for (int i = 0; i < NVS; ++i) nwv[i] = tid + THREADS * i < nv ? __ldg(reinterpret_cast<const uint4*>(nw) + tid + THREADS * i) : make_uint4(0, 0, 0, 0);
+    }
     cl.sync();                              // every CTA of the cluster runs: its shared memory may be written
     pdl_wait();
-    const uint4* x4 = reinterpret_cast<const uint4*>(xn);
-    auto dot = [](const uint4& a, const uint4& b, float s) {
-        const uint32_t u[4] = {a.x, a.y, a.z, a.w}, v[4] = {b.x, b.y, b.z, b.w};
+    const uint4* x4 = reinterpret_cast<const uint4*>(x);
+    float amax = 0.0f;
+    if (NV > 0) {
+        uint4 r[NVS];
+        double ss = 0.0;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            s = fmaf(bf16_lo(u[k]), bf16_lo(v[k]), s);
-            s = fmaf(bf16_hi(u[k]), bf16_hi(v[k]), s);
+        for (int i = 0; i < NVS; ++i) r[i] = tid + THREADS * i < nv ? x4[tid + THREADS * i] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int i = 0; i < NVS; ++i) {
+            const uint32_t u[4] = {r[i].x, r[i].y, r[i].z, r[i].w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) ss += sq_f64(bf16_lo(u[j])) + sq_f64(bf16_hi(u[j]));
         }
-        return s;
-    };
+        const float inv = rms_inverse(block_sum(ss, dred), D, eps);
+#pragma unroll
+        for (int i = 0; i < NVS; ++i) {
+            const uint32_t u[4] = {r[i].x, r[i].y, r[i].z, r[i].w};
+            float f[8];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                f[2 * j] = bf16_lo(u[j]);
+                f[2 * j + 1] = bf16_hi(u[j]);
+            }
+            r[i] = norm8(f, nwv[i], inv);
+            if (tid + THREADS * i >= nv) continue;
+            row[tid + THREADS * i] = r[i];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(f[j]));
+        }
+        __syncthreads();
+        x4 = row;
+    }
     for (int e = first; e < E; e += RT_CTAS * RT_WARPS) {
         const uint4* w4 = reinterpret_cast<const uint4*>(W + (size_t)e * D);
         float s = 0.0f;
 #pragma unroll
         for (int i = 0; i < RT_PRE; ++i)
-            if (lane + 32 * i < nv) s = dot(e == first ? pre[i] : __ldg(w4 + lane + 32 * i), x4[lane + 32 * i], s);
-        for (int v = lane + 32 * RT_PRE; v < nv; v += 32) s = dot(__ldg(w4 + v), x4[v], s);
+            if (lane + 32 * i < nv) s = rt_dot(e == first ? pre[i] : __ldg(w4 + lane + 32 * i), x4[lane + 32 * i], s);
+        for (int v = lane + 32 * RT_PRE; v < nv; v += 32) s = rt_dot(__ldg(w4 + v), x4[v], s);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (lane == 0) *cl.map_shared_rank(&lg[e], 0) = rbf(s);
     }
     cl.sync();
+    if (NV > 0 && rank == RT_CTAS - 1) {
+        float s, qi;
+        quant_scale(block_max(amax, red), s, qi);
+#pragma unroll
+        for (int i = 0; i < NVS; ++i) {
+            const int v = tid + THREADS * i;
+            if (v >= nv) continue;
+            const uint4 o = row[v];
+            reinterpret_cast<uint2*>(xq)[v] = make_uint2(quant4(bf16_lo(o.x), bf16_hi(o.x), bf16_lo(o.y), bf16_hi(o.y), qi),
+                                                         quant4(bf16_lo(o.z), bf16_hi(o.z), bf16_lo(o.w), bf16_hi(o.w), qi));
+        }
+        if (tid == 0) xs[0] = s;
+    }
     if (rank != 0 || warp != 0) return;
     float p[PER];
 #pragma unroll
     for (int j = 0; j < PER; ++j) p[j] = j * 32 + lane < E ? lg[j * 32 + lane] : 0.0f;
     softmax_topk<PER>(p, E, topk, lane, inds, scores, nullptr);
+}
+
+template <int NV>
+static int run_route_token(const uint16_t* x, const uint16_t* nw, float eps, const uint16_t* W, int D, int E, int topk, int8_t* xq, float* xs, int32_t* inds,
+                           uint16_t* scores, cudaStream_t st) {
+    SCMX_PDL_OK("route_token_kernel", launch_pdl(E <= 64 ? route_token_kernel<2, NV> : E <= 256 ? route_token_kernel<8, NV> : route_token_kernel<32, NV>, dim3(RT_CTAS),
+                                                 dim3(32 * RT_WARPS), 0, st, x, nw, eps, W, D, E, topk, xq, xs, inds, scores));
+    return SCMX_OK;
 }
 
 }  // namespace scmx
@@ -305,9 +367,15 @@ extern "C" int scmx_route_token(const uint16_t* xn, const uint16_t* W, int D, in
     SCMX_REQUIRE(xn && W && inds && scores && E >= 1 && E <= 1024 && topk >= 1 && topk <= E, SCMX_EINVAL,
                  "route_token: need 1 <= topk <= E <= 1024 (E=%d topk=%d)", E, topk);
     SCMX_REQUIRE(D > 0 && D % 8 == 0 && (((uintptr_t)xn | (uintptr_t)W) & 15) == 0, SCMX_EINVAL, "route_token: D=%d, 16-byte aligned rows", D);
-    const dim3 grid(RT_CTAS), block(32 * RT_WARPS);
-    cudaStream_t st = (cudaStream_t)stream;
-    SCMX_PDL_OK("route_token_kernel", launch_pdl(E <= 64 ? route_token_kernel<2> : E <= 256 ? route_token_kernel<8> : route_token_kernel<32>, grid, block, 0, st,
-                                                 xn, W, D, E, topk, inds, scores));
-    return SCMX_OK;
+    return run_route_token<0>(xn, nullptr, 0.0f, W, D, E, topk, nullptr, nullptr, inds, scores, (cudaStream_t)stream);
+}
+
+extern "C" int scmx_norm_route_token(const uint16_t* x, const uint16_t* nw, float eps, const uint16_t* W, int D, int E, int topk, int8_t* xq, float* xs, int32_t* inds,
+                                     uint16_t* scores, void* stream) {
+    SCMX_REQUIRE(x && nw && W && xq && xs && inds && scores && E >= 1 && E <= 1024 && topk >= 1 && topk <= E, SCMX_EINVAL,
+                 "norm_route_token: need 1 <= topk <= E <= 1024 (E=%d topk=%d)", E, topk);
+    SCMX_REQUIRE(D > 0 && D % 8 == 0 && D <= 8192 && (((uintptr_t)x | (uintptr_t)nw | (uintptr_t)W | (uintptr_t)xq) & 15) == 0, SCMX_EINVAL,
+                 "norm_route_token: D=%d (a multiple of 8 up to 8192), 16-byte aligned rows", D);
+    return D <= 2048 ? run_route_token<1>(x, nw, eps, W, D, E, topk, xq, xs, inds, scores, (cudaStream_t)stream)
+                     : run_route_token<4>(x, nw, eps, W, D, E, topk, xq, xs, inds, scores, (cudaStream_t)stream);
 }

@@ -229,8 +229,7 @@ class DecodeOlmoe(_Decoder):
             o = self._attend(at, c, q, kk, v, pos_dev)
             h = G.gemv(o, wo.codes, wo.bcodes, None, wo.wscale, D, 2, res=h, pro=1)[None]
             pn = layer.post_attention_layernorm.weight
-            xq, xs, xn = S.rmsnorm_quant_n(h, pn, eps, 1)     # the router needs the bf16 normalized row too
-            inds, scores = f.route_token(layer, xn)
+            xq, xs, inds, scores = f.norm_route_token(layer, h)
             e = inds.reshape(-1)
             (cg, bg, sg), (cd, bd, sd) = ex["gu"], ex["down"]
             act = G.gemv(xq, cg, bg, xs, sg, F2, 3, eidx=e, xstride=0)            # [k, F]

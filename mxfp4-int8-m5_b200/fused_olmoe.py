@@ -128,11 +128,24 @@ class FusedOlmoe:
 
     def route_token(self, layer, xn):
         """route for one row, in one kernel where the sizes allow and `route` is this class's own."""
+        if self._route_kernel(layer, xn):
+            return M_.route_token(xn, layer.mlp.gate.weight, self.args.num_experts_per_tok)
+        return self.route(layer, xn, 1)
+
+    def _route_kernel(self, layer, x):
         w = layer.mlp.gate.weight
         own = type(self).route is _ROUTE and "route" not in self.__dict__
-        if own and w.dtype == xn.dtype == torch.bfloat16 and w.is_contiguous() and w.shape[1] % 8 == 0 and w.shape[0] <= 1024 and w.data_ptr() % 16 == 0:
-            return M_.route_token(xn, w, self.args.num_experts_per_tok)
-        return self.route(layer, xn, 1)
+        return own and w.dtype == x.dtype == torch.bfloat16 and w.is_contiguous() and w.shape[1] % 8 == 0 and w.shape[0] <= 1024 and w.data_ptr() % 16 == 0
+
+    def norm_route_token(self, layer, h):
+        """The norm before the experts, as INT8, and route_token of one row h [1, D]: (xq, xs, inds, scores), in one kernel where route_token takes its own and is this
+        class's."""
+        nw = layer.post_attention_layernorm.weight
+        own = type(self).route_token is _ROUTE_TOKEN and "route_token" not in self.__dict__
+        if own and h.shape[1] <= 8192 and self._route_kernel(layer, h):
+            return M_.norm_route_token(h, nw, self.eps, layer.mlp.gate.weight, self.args.num_experts_per_tok)
+        xq, xs, xn = S.rmsnorm_quant_n(h, nw, self.eps, 1)      # the router needs the bf16 normalized row too
+        return xq, xs, *self.route_token(layer, xn)
 
     def _packed(self, R):
         """Whether the grouped GEMMs read the packed weights (scmx_moe_mm_w4) although the experts could be decoded ahead: MoeBlock's
@@ -288,4 +301,4 @@ def load_fused_olmoe(model, cache_path=None, **kw):
     return FusedOlmoe(model, pack_olmoe(model, cache_path), **kw)
 
 
-_ROUTE, _EXPERTS = FusedOlmoe.route, FusedOlmoe.experts      # as this file defines them
+_ROUTE, _ROUTE_TOKEN, _EXPERTS = FusedOlmoe.route, FusedOlmoe.route_token, FusedOlmoe.experts      # as this file defines them

@@ -72,6 +72,18 @@ def route_token(xn, w, k):
     return inds, scores
 
 
+def norm_route_token(x, nw, eps, w, k):
+    """rmsnorm_quant_n of one row x bf16 [1, D], D <= 8192, and route_token of its result in one launch: (xq, xs, inds, scores)."""
+    _lib.require_cuda(x, nw, w)
+    (E, D), dev = w.shape, x.device
+    assert x.dtype == nw.dtype == w.dtype == torch.bfloat16 and x.numel() == D
+    xq, xs = torch.empty((1, D), dtype=torch.int8, device=dev), torch.empty(1, dtype=torch.float32, device=dev)
+    inds, scores = torch.empty((1, k), dtype=torch.int32, device=dev), torch.empty((1, k), dtype=torch.bfloat16, device=dev)
+    _lib.call("scmx_norm_route_token", _lib.ptr(x), _lib.ptr(nw), S._eps(eps), _lib.ptr(w), D, E, k, _lib.ptr(xq), _lib.ptr(xs), _lib.ptr(inds), _lib.ptr(scores),
+              _lib.stream())
+    return xq, xs, inds, scores
+
+
 def gather_rows(xq, xs, tok, R):
     """(xq[tok], xs[tok[:R]]): INT8 rows and scales of the sorted assignments (tok has R + tm entries)."""
     _lib.require_cuda(xq, xs, tok)

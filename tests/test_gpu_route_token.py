@@ -27,3 +27,14 @@ def test_route_token(scmx, E, D, k):
         assert (scores.float() - want_s.float()).abs().max() <= (step + 2.0 ** -7) * want_s.float().max()
     else:
         assert (inds != want_i).sum() <= 2
+
+
+@pytest.mark.parametrize("E,D,k", [(1, 8, 1), (63, 1024, 8), (64, 2048, 8), (65, 2056, 4), (257, 520, 3), (1024, 8192, 16)])
+def test_norm_route_token(scmx, E, D, k):
+    """With the norm before it: the bits of rmsnorm_quant_n and route_token one after the other, a zero row included."""
+    M_, S, g = scmx.sc_moe, scmx.sc_kernels, torch.Generator("cuda").manual_seed(E + D)
+    x, nw, w = (torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16) for s in ((1, D), (D,), (E, D)))
+    for row in (x, x * 1e-3, torch.zeros_like(x)):
+        xq, xs, xn = S.rmsnorm_quant_n(row, nw, 1e-5, 1)
+        want = (xq, xs, *M_.route_token(xn, w, k))
+        assert all(torch.equal(a, b) for a, b in zip(M_.norm_route_token(row, nw, 1e-5, w, k), want))

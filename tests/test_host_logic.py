@@ -286,6 +286,39 @@ def test_replaced_router_is_called(scmx, monkeypatch):
     assert plain.route_token(Layer, xn) == "class"
 
 
+def test_replaced_router_of_a_token_is_called(scmx, monkeypatch):
+    """Nor does a step's norm with the router pass by a `route` or `route_token` that was replaced."""
+    FO, S, M_ = scmx.fused_olmoe, scmx.sc_kernels, scmx.sc_moe
+    monkeypatch.setattr(M_, "norm_route_token", lambda *a: "kernel")
+    monkeypatch.setattr(S, "rmsnorm_quant_n", lambda h, w, eps, M: ("q", "s", h))
+
+    class Layer:
+        post_attention_layernorm = torch.nn.LayerNorm(64)
+
+        class mlp:
+            gate = torch.nn.Linear(64, 8, bias=False, dtype=torch.bfloat16)
+
+    class Own(FO.FusedOlmoe):
+        def route_token(self, layer, xn):
+            return "own", "scores"
+
+    def make(cls=FO.FusedOlmoe):
+        f = cls.__new__(cls)
+        f.args, f.eps = scmx.host_model.ModelArgs(64, 128, 1, 1, 1, 64, num_experts=8, num_experts_per_tok=2), 1e-5
+        return f
+
+    h, plain = torch.zeros(1, 64, dtype=torch.bfloat16), make()
+    assert plain.norm_route_token(Layer, h) == "kernel" and make(Own).norm_route_token(Layer, h) == ("q", "s", "own", "scores")
+    plain.route = lambda layer, xn, M: ("route", M)
+    assert plain.norm_route_token(Layer, h) == ("q", "s", "route", 1)
+    del plain.route
+    plain.route_token = lambda layer, xn: ("token", "scores")
+    assert plain.norm_route_token(Layer, h) == ("q", "s", "token", "scores")
+    del plain.route_token
+    monkeypatch.setattr(FO.FusedOlmoe, "route_token", lambda self, layer, xn: ("class", "scores"))
+    assert plain.norm_route_token(Layer, h) == ("q", "s", "class", "scores")
+
+
 def test_replaced_quantizer_is_called(scmx, monkeypatch):
     """The attention output of a prompt goes to an `act_q` that was replaced on the object, in a subclass or in the class."""
     FQ = scmx.fused_qwen3
