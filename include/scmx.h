@@ -306,10 +306,10 @@ int scmx_mm_i8_bcast(const int8_t* xq, const int8_t* wq, int64_t M, int64_t N, i
 int scmx_moe_mm_i8_ret(const int8_t* xq, int64_t R, const int8_t* wq, const float* wscale, const int32_t* off,
                        const int32_t* tstart, int E, int64_t N, int64_t K, const float* xscale, const int32_t* ret_rank,
                        const int32_t* ret_row, int world, void* const* out_peers, int tm, int32_t* status, void* stream);
-/* scmx_moe_combine of M rows with their RMSNorm (weights nw): h, and where given the normalized rows xn and their INT8 rows xq with scales xs, the bits of
- * scmx_moe_combine and scmx_rmsnorm_quant one after the other.  K a multiple of 8 up to 8192.  For the single rows of decode steps. */
+/* scmx_moe_combine of M rows with their RMSNorm (weights nw): h, and where given the normalized rows xn and their INT8 rows xq, their digit planes dig [3][M][K / 2]
+ * (scmx_digits) and scales xs, the bits of scmx_moe_combine and scmx_rmsnorm_quant one after the other.  K a multiple of 8 up to 8192. */
 int scmx_moe_combine_norm(const uint16_t* y, const int32_t* pos, const uint16_t* scores, const uint16_t* res, const uint16_t* nw, float eps, int64_t M,
-                          int64_t K, int topk, uint16_t* h, int8_t* xq, float* xs, uint16_t* xn, void* stream);
+                          int64_t K, int topk, uint16_t* h, int8_t* xq, uint32_t* dig, float* xs, uint16_t* xn, void* stream);
 
 /* scmx_moe_combine whose expert rows are READ from the GPUs that computed them (expert parallelism, "pull" form): y_peers[d]
  * is rank d's output buffer bf16 [world * cap, K] ordered by receive slot (source rank * cap + position among the rows that

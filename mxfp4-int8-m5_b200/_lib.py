@@ -106,7 +106,7 @@ SIGNATURES = {
                               c_int, c_int, c_vp, c_vp, c_vp, c_vp],
     "scmx_moe_combine": [c_vp, c_vp, c_vp, c_vp, c_vp, c_float, c_i64, c_i64, c_i64, c_int, c_int, c_vp, c_vp, c_vp,
                          c_vp],
-    "scmx_moe_combine_norm": [c_vp, c_vp, c_vp, c_vp, c_vp, c_float, c_i64, c_i64, c_int, c_vp, c_vp, c_vp, c_vp, c_vp],
+    "scmx_moe_combine_norm": [c_vp, c_vp, c_vp, c_vp, c_vp, c_float, c_i64, c_i64, c_int, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp],
     "scmx_decode_step_scratch": [c_int] * 6,
     "scmx_decode_step": [c_vp, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_vp, c_vp, c_i64, c_i64, c_vp, c_vp, c_vp, c_int, c_vp, c_vp],
     "scmx_decode_step_dense": [c_vp, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_vp, c_vp, c_i64, c_i64, c_vp,

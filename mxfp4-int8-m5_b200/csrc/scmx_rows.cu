@@ -574,12 +574,13 @@ __global__ void __launch_bounds__(256, 4) moe_combine_kernel(const uint16_t* __r
     if (threadIdx.x == 0) xs[row] = s;
 }
 
-// The combine of a token's step with the next norm: the row stays in registers, so the sum, the RMSNorm, its INT8 row and its bfloat16 row (the output head's
-// input) are one launch.  Bound by latency: a link of the chain less, generation of 8 tokens by two layers 1082 -> 1051 us.
+// The combine of a token's step, or of a prompt whose products take digit planes, with the next norm: the row stays in registers, so the sum, the RMSNorm, its INT8 row and its bfloat16 row (the output head's
+// input) are one launch.  Bound by latency: a link of the chain less, generation of 8 tokens by two layers 1082 -> 1051 us, prompts of 1024 tokens 508 -> 501 us.
 template <int NV>
 __global__ void __launch_bounds__(256) moe_combine_norm_kernel(const uint16_t* __restrict__ y, const int32_t* __restrict__ pos, const uint16_t* __restrict__ scores,
                                                                const uint16_t* __restrict__ res, const uint16_t* __restrict__ nw, float eps, int K, int topk,
-                                                               uint16_t* __restrict__ h, int8_t* __restrict__ xq, float* __restrict__ xs, uint16_t* __restrict__ xn) {
+                                                               uint16_t* __restrict__ h, int8_t* __restrict__ xq, RowDigits dg, float* __restrict__ xs,
+                                                               uint16_t* __restrict__ xn) {
     __shared__ float red[33], s_sc[32];
     __shared__ double dred[33];
     __shared__ const uint16_t* s_ptr[32];
@@ -652,7 +653,7 @@ __global__ void __launch_bounds__(256) moe_combine_norm_kernel(const uint16_t* _
 #pragma unroll
         for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(f[j]));
     }
-    if (xq == nullptr) return;
+    if (xq == nullptr && dg.p == nullptr) return;
     amax = block_max(amax, red);
     float s, qi;
     quant_scale(amax, s, qi);
@@ -662,7 +663,9 @@ __global__ void __launch_bounds__(256) moe_combine_norm_kernel(const uint16_t* _
         if (v >= nv) continue;
         float f[8];
         unpack8(r[i], f);
-        reinterpret_cast<uint2*>(xq + row * K)[v] = make_uint2(quant4(f[0], f[1], f[2], f[3], qi), quant4(f[4], f[5], f[6], f[7], qi));
+        const uint32_t lo = quant4(f[0], f[1], f[2], f[3], qi), hi = quant4(f[4], f[5], f[6], f[7], qi);
+        if (xq) reinterpret_cast<uint2*>(xq + row * K)[v] = make_uint2(lo, hi);
+        dg.store(row * nv + v, lo, hi);
     }
     if (tid == 0) xs[row] = s;
 }
@@ -856,15 +859,15 @@ extern "C" int scmx_moe_combine(const uint16_t* y, const int32_t* pos, const uin
 }
 
 extern "C" int scmx_moe_combine_norm(const uint16_t* y, const int32_t* pos, const uint16_t* scores, const uint16_t* res, const uint16_t* nw, float eps, int64_t M,
-                                     int64_t K, int topk, uint16_t* h, int8_t* xq, float* xs, uint16_t* xn, void* stream) {
+                                     int64_t K, int topk, uint16_t* h, int8_t* xq, uint32_t* dig, float* xs, uint16_t* xn, void* stream) {
     SCMX_REQUIRE(y && pos && scores && res && nw && h && M >= 0 && M < (1ll << 31) && K > 0 && K % 8 == 0 && K <= 8192, SCMX_EINVAL,
                  "moe_combine_norm: need K %% 8 == 0 and K <= 8192 (M=%lld K=%lld)", (long long)M, (long long)K);
     SCMX_REQUIRE(topk >= 1 && topk <= 32, SCMX_ELIMIT, "moe_combine_norm: topk=%d outside 1..32", topk);
-    SCMX_REQUIRE(aligned16(y) && aligned16(res) && aligned16(nw) && aligned16(h) && (!xq || (aligned16(xq) && xs)) && (!xn || aligned16(xn)), SCMX_EINVAL,
+    SCMX_REQUIRE(aligned16(y) && aligned16(res) && aligned16(nw) && aligned16(h) && (!xq || (aligned16(xq) && xs)) && (!dig || xs) && (!xn || aligned16(xn)), SCMX_EINVAL,
                  "moe_combine_norm: buffers must be 16-byte aligned");
     if (M == 0) return SCMX_OK;
     launch_pdl(K <= 2048 ? moe_combine_norm_kernel<1> : moe_combine_norm_kernel<4>, dim3((unsigned)M), dim3(256), 0, (cudaStream_t)stream, y, pos, scores, res, nw, eps,
-               (int)K, topk, h, xq, xs, xn);
+               (int)K, topk, h, xq, RowDigits{dig, M * (K / 8)}, xs, xn);
     SCMX_LAUNCH_OK("moe_combine_norm_kernel");
     return SCMX_OK;
 }

@@ -183,7 +183,7 @@ class FusedOlmoe:
                 and M_.f4_fits(a.num_experts, a.hidden_size, a.intermediate_size, self.layers[0][1]["o"].K))
 
     def _hidden_f4(self, h, cache, L):
-        """The blocks on digit planes: same bits as the products from INT8."""
+        """The blocks on digit planes and the final norm: same bits as the products from INT8."""
         a = self.args
         H, d, D, E, Fi, nl = a.num_attention_heads, a.head_dim, a.hidden_size, a.num_experts, a.intermediate_size, len(self.layers)
         R = L * a.num_experts_per_tok
@@ -204,11 +204,10 @@ class FusedOlmoe:
             act = M_.moe_mm_f4(dig, R, cg, fg, sg, off, 2 * Fi, 3, xs)
             dig, xs = S.quant_digits(act)
             yd = M_.moe_mm_f4(dig, R, cd, fd, sd, off, D, 1, xs)
-            nn = self.layers[i + 1][0].input_layernorm.weight if i + 1 < nl else self.model.model.norm.weight
-            h, xq, xs = M_.moe_combine(yd, pos, scores, h, nn, self.eps, L, quant=i + 1 < nl)
-            if i + 1 < nl:
-                dig, _ = M_.gather_digits(xq, None, None, L)
-        return h
+            last = i + 1 == nl
+            nn = self.model.model.norm.weight if last else self.layers[i + 1][0].input_layernorm.weight
+            h, dig, xs, xn = M_.combine_norm(yd, pos, scores, h, nn, self.eps, quant=False if last else "digits", normed=last)
+        return xn
 
     def experts(self, ex, xq, xs, inds, L, decoded=None):
         """INT8 rows + routing -> (sorted expert outputs yd bf16 [R, D], pos).  decoded: (gu8, dn8) INT8 copies of this
@@ -243,8 +242,7 @@ class FusedOlmoe:
         h = self.model.model.embed_tokens(ids)[0]
         L = h.shape[0]
         if L > 0 and self._f4(L):
-            h = self._hidden_f4(h.contiguous(), cache, L)
-            return S.rmsnorm_quant_n(h, self.model.model.norm.weight, self.eps, L)[2][None]
+            return self._hidden_f4(h.contiguous(), cache, L)[None]
         Mp = S.pad_rows(L)
         if Mp != L:
             h = torch.nn.functional.pad(h, (0, 0, 0, Mp - L))

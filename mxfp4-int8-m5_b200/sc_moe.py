@@ -199,14 +199,17 @@ def moe_combine(y, pos, scores, res, w, eps, M, quant=True):
 
 
 def combine_norm(y, pos, scores, res, w, eps, quant=True, normed=False):
-    """moe_combine(quant=False) of the rows of res [M, K], K <= 8192, and rmsnorm_quant_n of its result in one launch, for the rows of decode steps:
-    (h, xq, xs, xn), xq and xs None without quant, xn None unless normed."""
+    """moe_combine(quant=False) of the rows of res [M, K], K <= 8192, and rmsnorm_quant_n of its result in one launch: (h, xq, xs, xn), xq and xs None without quant,
+    xn None unless normed.  quant "digits": xq as digit planes (quant_digits)."""
     _lib.require_cuda(y, pos, scores, res, w)
-    (M, K), dev = res.shape, res.device
+    (M, K), dev, digits = res.shape, res.device, quant == "digits"
     assert y.dtype == scores.dtype == res.dtype == w.dtype == torch.bfloat16
     h = torch.empty((M, K), dtype=torch.bfloat16, device=dev)
-    xq, xs = (torch.empty((M, K), dtype=torch.int8, device=dev), torch.empty(M, dtype=torch.float32, device=dev)) if quant else (None, None)
+    xq = xs = None
+    if quant:
+        xq = torch.empty((3, M, K // 8), dtype=torch.int32, device=dev) if digits else torch.empty((M, K), dtype=torch.int8, device=dev)
+        xs = torch.empty(M, dtype=torch.float32, device=dev)
     xn = torch.empty((M, K), dtype=torch.bfloat16, device=dev) if normed else None
     _lib.call("scmx_moe_combine_norm", _lib.ptr(y), _lib.ptr(pos), _lib.ptr(scores), _lib.ptr(res), _lib.ptr(w), S._eps(eps), M, K, scores.shape[1], _lib.ptr(h),
-              _lib.ptr(xq), _lib.ptr(xs), _lib.ptr(xn), _lib.stream())
+              None if digits else _lib.ptr(xq), _lib.ptr(xq) if digits else None, _lib.ptr(xs), _lib.ptr(xn), _lib.stream())
     return h, xq, xs, xn

@@ -7,7 +7,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("M,topk", [(1, 8), (1, 1), (3, 9), (2, 32)])
-@pytest.mark.parametrize("K", [8, 1032, 2048, 2056, 8192])
+@pytest.mark.parametrize("K", [8, 1032, 2048, 2056, 4128, 8192])
 def test_bits(scmx, K, M, topk):
     M_, S = scmx.sc_moe, scmx.sc_kernels
     g = torch.Generator(device="cuda").manual_seed(K + 64 * M + topk)
@@ -26,3 +26,6 @@ def test_bits(scmx, K, M, topk):
     assert q is s is None and torch.equal(h, want) and torch.equal(n, xn)
     h, q, s, n = M_.combine_norm(y, pos, scores, res, w, 1e-5)
     assert n is None and torch.equal(q, xq) and torch.equal(s, xs)
+    if K % 32 == 0:
+        d, s = M_.combine_norm(y, pos, scores, res, w, 1e-5, quant="digits")[1:3]
+        assert torch.equal(d, M_.gather_digits(xq, None, None, M)[0]) and torch.equal(s, xs)
