@@ -32,6 +32,8 @@ from . import sc_moe as M_
 
 
 class _Decoder:
+    _mk = None                                                # persistent-kernel state, built per cache
+
     def __init__(self, fused, head, attention):
         self.f, self.model, self.args = fused, fused.model, fused.args
         self.head = G.head_product(fused.model if head == "model" else head)
@@ -42,7 +44,6 @@ class _Decoder:
         self.attention = attention
         self.attn = S.DecodeAttention(hq, hk, d, fused.inv_freq.device) if attention == "kernel" else None
         self._graph = None
-        self._mk = None                                       # persistent-kernel state, built per cache
 
     @property
     def replayable(self):
@@ -94,8 +95,9 @@ class _Decoder:
             torch.cuda.current_stream().wait_stream(s)
             for c, o in zip(cache, offsets):
                 c.offset = o
-            self._graph = (cache, g, tok_buf, pos, count, chosen, logits)
-        _, g, tok_buf, pos, count, chosen, _ = self._graph
+            self._graph = (cache, g, tok_buf, pos, count, chosen, logits, self._mk)
+        # the layer table, scratch and status word that the graph names live as long as it does, whatever cache was stepped on since
+        _, g, tok_buf, pos, count, chosen, _, self._mk = self._graph
         start = cache[0].offset
         assert start + n <= cache[0].capacity, "KV cache capacity exceeded"
         tok_buf.copy_(tok.reshape(1, 1))

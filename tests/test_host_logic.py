@@ -392,3 +392,48 @@ def test_prompts_on_digit_planes(scmx):
         assert not make()._f4(16)
     finally:
         S.set_format(old)
+
+
+def test_generation_keeps_what_its_graph_names(scmx, monkeypatch):
+    """Steps on other caches replace the one-kernel step's tables; those of a captured generation stay alive and are the decoder's again when it is replayed."""
+    import contextlib
+    import weakref
+    from types import SimpleNamespace as NS
+
+    class Stream:
+        def wait_stream(self, other):
+            pass
+
+    class Graph:
+        def replay(self):
+            assert self.table() is not None, "replayed on a table that was freed"
+
+    class Decoder(scmx.decode._Decoder):
+        replayable = True
+
+        def __init__(self):
+            self._graph = self._mk = None
+
+        def _step(self, tok, cache, pos):
+            if self._mk is None or self._mk["cache"] is not cache:
+                self._mk = dict(cache=cache, table=torch.zeros(4))
+            Graph.table = weakref.ref(self._mk["table"])
+            return torch.zeros(1, 1, 8)
+
+        def _select(self, *a):
+            pass
+
+    nothing = lambda *a, **kw: contextlib.nullcontext()      # noqa: E731
+    for name, fake in dict(Stream=lambda device: Stream(), current_stream=Stream, stream=nothing, synchronize=lambda: None, CUDAGraph=Graph, graph=nothing).items():
+        monkeypatch.setattr(torch.cuda, name, fake)
+    make = lambda: [NS(offset=3, capacity=16, carried=lambda: [])]      # noqa: E731
+    a, b, dec, tok = make(), make(), Decoder(), torch.zeros(1, 1, dtype=torch.long)
+    dec.generate(tok, a, 2)
+    first = dec._mk
+    table = Graph.table
+    dec.step(tok, b)
+    assert dec._mk is not first
+    del first
+    Graph.table = table
+    dec.generate(tok, a, 2)
+    assert dec._mk["table"] is table()
