@@ -407,7 +407,7 @@ typedef struct scmx_decode_layer {
  * CTAs as packets that carry an epoch instead of kernel boundaries.  Same bits as scmx_rmsnorm_quant / scmx_gemv / scmx_qkv_norm /
  * scmx_attn_decode (with the same nsplit) / scmx_act_quant called in that order.
  * layers: device array; scratch: scmx_decode_step_scratch bytes, 16-byte aligned, zero before its first use and then left to the steps that
- * share it, which must not overlap; status int32 [1] receives 1000 + 5 layer + k if a wait timed out (0.5 s), k = 0 residual row, 1 q|k|v, 2 attention,
+ * share it, which must not overlap; status int32 [1] receives 1000 + 5 layer + k if a wait ran out (scmx_set_wait_limit_ns), k = 0 residual row, 1 q|k|v, 2 attention,
  * 3 residual row after it, 4 feed-forward row, after which the step's outputs are invalid.
  * Limits: d = 128; D, F and hq*d multiples of 1024 up to 6144; hq/hk in {1, 2, 4}; hk * nsplit <= number of SMs (64 to 256); 256 layers.
  * Not to be run concurrently with other work on the same device: the launch needs every SM. */

@@ -25,7 +25,7 @@
 // Arithmetic: the device functions of the stand-alone kernels (row kernels, GEMV, q/k/v epilogue, decode attention), so the step produces the
 // same bits as the chain of those kernels.  Callers: e2e/decode.py:29-110 of the reference is the chain.
 //
-// Every wait is bounded (MK_WAIT_NS): a thread that gives up raises the abort word and writes the status word; the others see the abort word in their
+// Every wait is bounded (scmx_set_wait_limit_ns): a thread that gives up raises the abort word and writes the status word; the others see the abort word in their
 // own waits; a CTA agrees on it at its next barrier and returns.  The launch is cooperative, so all CTAs are co-resident.
 #include "scmx_attn_core.cuh"
 #include "scmx_common.cuh"
@@ -43,7 +43,6 @@ constexpr int MK_CODES = 4 * 512, MK_CHUNK = MK_CODES + 32;      // bytes of an 
 constexpr int MK_SLOTS = 9;
 constexpr int MK_MAXLAYERS = 256;
 constexpr unsigned MK_BACKOFF_NS = 40;
-constexpr uint64_t MK_WAIT_NS = 500000000ull;        // 0.5 s
 
 struct MkArgs {
     const scmx_decode_layer* layers;
@@ -57,6 +56,7 @@ struct MkArgs {
     uint32_t* head;       // [0] epoch of the last launch, [1] abort word (zero at launch)
     uint2 *xh[2], *xy, *xact, *xo, *xpart;      // packets: h after P6 / P4, y, act, o: {two bf16, epoch}; partial states [hq][nsplit][d + 2]: {float, epoch}
     int32_t* status;
+    uint64_t wait_ns;
     unsigned long long* trace;   // diagnostic: null, or CTA 0 stores its cycle counter at every phase boundary
     int n_trace;
 };
@@ -100,7 +100,7 @@ struct MkWait {
         if (ab) return false;
         const uint64_t now = globaltimer_ns();
         if (!t0) t0 = now;
-        if (now - t0 <= MK_WAIT_NS) return true;
+        if (now - t0 <= a.wait_ns) return true;
         atomicExch(a.head + 1, 1u);
         atomicCAS(a.status, 0, code);
         return false;
@@ -734,6 +734,7 @@ extern "C" int scmx_decode_step(const scmx_decode_layer* layers, int n_layers, i
     a.layers = layers; a.n_layers = n_layers; a.D = D; a.F = F; a.hq = hq; a.hk = hk; a.nsplit = nsplit; a.eps = eps; a.scale = scale;
     a.inv_freq = inv_freq; a.rope_cs = rope_table; a.rope_rows = rope_table ? rope_rows : 0; a.cap = capacity; a.pos_dev = pos_dev;
     a.h = h; a.head = reinterpret_cast<uint32_t*>(sp); a.xh[0] = at(0); a.xh[1] = at(1); a.xy = at(2); a.xact = at(3); a.xo = at(4); a.xpart = at(5); a.status = status;
+    a.wait_ns = g_wait_limit_ns;
     a.trace = g_trace; a.n_trace = g_n_trace & 0xFFFF;
     cudaStream_t st = (cudaStream_t)stream;
     mk_begin_kernel<<<1, 1, 0, st>>>(a.head);
