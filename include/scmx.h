@@ -2,7 +2,7 @@
  *
  * Conventions
  *   - Every pointer is a DEVICE pointer.  Nothing is allocated or freed across the ABI: outputs and scratch
- *     buffers are preallocated by the caller.
+ *     buffers are preallocated by the caller.  (One call allocates and frees in its stream's order: scmx_decode_step_dense.)
  *   - `stream` is a cudaStream_t passed as void*; all work is enqueued on it and nothing synchronises.
  *   - Return value: 0 on success, a negative SCMX_E* code otherwise; scmx_last_error_string() describes the last
  *     failure on the calling thread.  Shapes are validated on the host before anything is launched.
@@ -409,7 +409,8 @@ typedef struct scmx_decode_layer {
  * layers: device array; scratch: scmx_decode_step_scratch bytes, 16-byte aligned, zero before its first use and then left to the steps that
  * share it, which must not overlap; status int32 [1] receives 1000 + 5 layer + k if a wait ran out (scmx_set_wait_limit_ns), k = 0 residual row, 1 q|k|v, 2 attention,
  * 3 residual row after it, 4 feed-forward row, after which the step's outputs are invalid.
- * Limits: d = 128; D, F and hq*d multiples of 1024 up to 6144; hq/hk in {1, 2, 4}; hk * nsplit <= number of SMs (64 to 256); 256 layers.
+ * Limits: d = 128; D, F and hq*d multiples of 1024 up to 6144; hq/hk in {1, 2, 4}; hk * nsplit <= number of SMs; every SM gets rows of each product,
+ * at most 384 of one (32 to 256 SMs do for all widths).  More than 256 layers take a launch for every 256.
  * Not to be run concurrently with other work on the same device: the launch needs every SM. */
 int64_t scmx_decode_step_scratch(int D, int F, int hq, int hk, int d, int nsplit);
 int scmx_decode_step(const scmx_decode_layer* layers, int n_layers, int D, int F, int hq, int hk, int d, float eps,

@@ -27,6 +27,7 @@
 //
 // Every wait is bounded (scmx_set_wait_limit_ns): a thread that gives up raises the abort word and writes the status word; the others see the abort word in their
 // own waits; a CTA agrees on it at its next barrier and returns.  The launch is cooperative, so all CTAs are co-resident.
+#include <algorithm>
 #include "scmx_attn_core.cuh"
 #include "scmx_common.cuh"
 #include "scmx_gemv_core.cuh"
@@ -38,15 +39,17 @@ constexpr int MK_THREADS = 256;                       // the attention core want
 constexpr int MK_WARPS = MK_THREADS / 32;
 constexpr int MK_MAXK = 6144;
 constexpr int MK_MAXHQ = 32;
-constexpr int MK_MAXROWS = 384;                      // output rows of a CTA in one phase at most (2 * 6144 rows on 32 SMs)
+constexpr int MK_MAXROWS = 384;                      // output rows of a CTA in one phase at most: the widest phase, 12288 rows, on 32 SMs
 constexpr int MK_CODES = 4 * 512, MK_CHUNK = MK_CODES + 32;      // bytes of an item: codes of 4 rows, their block codes
 constexpr int MK_SLOTS = 9;
-constexpr int MK_MAXLAYERS = 256;
+constexpr int MK_MAXLAYERS = 256;                     // of one launch: its table of weights lies in shared memory
 constexpr unsigned MK_BACKOFF_NS = 40;
+constexpr int MK_MARKS = 9;                          // diagnostic marks of a layer
 
 struct MkArgs {
     const scmx_decode_layer* layers;
     int n_layers, D, F, hq, hk, nsplit;
+    int first;            // number of the first layer, for the status word
     float eps, scale;
     const float* inv_freq;
     const float* rope_cs;
@@ -530,7 +533,7 @@ __global__ void __launch_bounds__(MK_THREADS, 1) decode_step_kernel(const __grid
     const int kvh = blockIdx.x % a.hk, split = blockIdx.x / a.hk;
     const bool attends = split < active;
     const int64_t t0 = (int64_t)split * chunk, t1 = t0 + chunk < T ? t0 + chunk : T;
-    const int my_head = (int)gridDim.x - 1 - (int)blockIdx.x;      // query head whose splits this CTA combines
+    const int my_head = (int)gridDim.x - 1 - (int)blockIdx.x;      // query head whose splits this CTA combines (and every gridDim.x-th after it)
     bool bad = false;
     int ti = 0;
 
@@ -597,7 +600,7 @@ __global__ void __launch_bounds__(MK_THREADS, 1) decode_step_kernel(const __grid
         if (li + 1 < a.n_layers && tid < LWORDS)              // read after several barriers
             reinterpret_cast<unsigned long long*>(&layer[(li + 1) & 1])[tid] = reinterpret_cast<const unsigned long long*>(a.layers + li + 1)[tid];
         const uint32_t epoch = base_epoch + 1 + li;
-        const int code = 1000 + 5 * li;
+        const int code = 1000 + 5 * (a.first + li);
         mk_mark(a, ti);
         if (attends && tid < 2 && t1 > t0) {                  // the positions that this CTA will attend to
             const int64_t te = t1 < T - 1 ? t1 : T - 1;
@@ -616,7 +619,7 @@ __global__ void __launch_bounds__(MK_THREADS, 1) decode_step_kernel(const __grid
         // P3: attention of one (kv head, split) per CTA
         if (attends) bad |= mk_attention<G, HD>(a, L, kvh, split, t0, t1, pos, epoch, code + 1);      // uniform over the CTA
         mk_mark(a, ti);
-        if (my_head < a.hq) bad |= mk_combine<HD>(a, my_head, active, epoch, code + 2);
+        for (int head = my_head; head < a.hq; head += (int)gridDim.x) bad |= mk_combine<HD>(a, head, active, epoch, code + 2);
         __syncthreads();                                      // sm.ws and the products are free
         // P4: INT8 of o, o-projection + residual
         ahead(ph[1], L.wscale[1], li > 0 ? a.xh[0] : nullptr, a.h);
@@ -712,7 +715,6 @@ extern "C" int scmx_decode_step(const scmx_decode_layer* layers, int n_layers, i
     const int dev = current_device();
     SCMX_REQUIRE(dev >= 0, SCMX_ECUDA, "decode_step: no current CUDA device (ordinal 0..63)");
     constexpr int RINGS = MK_WARPS * MK_SLOTS * MK_CHUNK + 64 * MK_MAXLAYERS;
-    SCMX_REQUIRE(n_layers <= MK_MAXLAYERS, SCMX_ELIMIT, "decode_step: %d layers (%d)", n_layers, MK_MAXLAYERS);
     if (!coop_dev[dev]) {
         int c = 0;
         SCMX_CUDA_OK(cudaDeviceGetAttribute(&c, cudaDevAttrCooperativeLaunch, dev));
@@ -723,22 +725,20 @@ extern "C" int scmx_decode_step(const scmx_decode_layer* layers, int n_layers, i
     }
     const int coop = coop_dev[dev] > 0, n_sm = sm_count();
     SCMX_REQUIRE(coop, SCMX_EDEVICE, "decode_step: the device does not support cooperative launches");
-    // every CTA has rows in every phase, which the reuse of the packet buffers rests on (256 row groups at least)
-    SCMX_REQUIRE(hk * nsplit <= n_sm && hq <= n_sm && n_sm <= 256 && n_sm >= 4 * 6144 / MK_MAXROWS, SCMX_EINVAL,
-                 "decode_step: hk * nsplit = %d, hq = %d on the %d CTAs of the grid", hk * nsplit, hq, n_sm);
+    // Every CTA has rows in every phase, which the reuse of the packet buffers rests on, and no more than its tables hold.
+    const int qkv = (hq + 2 * hk) * d, most = std::max({qkv, 2 * F, D}) / 4, least = std::min({qkv, 2 * F, D}) / 4;
+    SCMX_REQUIRE(hk * nsplit <= n_sm && n_sm <= least && 4 * ((most + n_sm - 1) / n_sm) <= MK_MAXROWS, SCMX_EINVAL,
+                 "decode_step: hk * nsplit = %d, phases of %d to %d rows on the %d CTAs of the grid", hk * nsplit, 4 * least, 4 * most, n_sm);
     size_t off[7];
     mk_scratch(D, F, hq, hk, d, nsplit, off);
     uint8_t* sp = static_cast<uint8_t*>(scratch);
     auto at = [&](int i) { return reinterpret_cast<uint2*>(sp + off[i]); };
     MkArgs a;
-    a.layers = layers; a.n_layers = n_layers; a.D = D; a.F = F; a.hq = hq; a.hk = hk; a.nsplit = nsplit; a.eps = eps; a.scale = scale;
+    a.D = D; a.F = F; a.hq = hq; a.hk = hk; a.nsplit = nsplit; a.eps = eps; a.scale = scale;
     a.inv_freq = inv_freq; a.rope_cs = rope_table; a.rope_rows = rope_table ? rope_rows : 0; a.cap = capacity; a.pos_dev = pos_dev;
     a.h = h; a.head = reinterpret_cast<uint32_t*>(sp); a.xh[0] = at(0); a.xh[1] = at(1); a.xy = at(2); a.xact = at(3); a.xo = at(4); a.xpart = at(5); a.status = status;
     a.wait_ns = g_wait_limit_ns;
-    a.trace = g_trace; a.n_trace = g_n_trace & 0xFFFF;
     cudaStream_t st = (cudaStream_t)stream;
-    mk_begin_kernel<<<1, 1, 0, st>>>(a.head);
-    SCMX_LAUNCH_OK("mk_begin_kernel");
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)n_sm);
     cfg.blockDim = dim3(MK_THREADS);
@@ -749,10 +749,17 @@ extern "C" int scmx_decode_step(const scmx_decode_layer* layers, int n_layers, i
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaError_t e = G == 1 ? cudaLaunchKernelEx(&cfg, decode_step_kernel<1, 128>, a)
-                  : G == 2 ? cudaLaunchKernelEx(&cfg, decode_step_kernel<2, 128>, a)
-                           : cudaLaunchKernelEx(&cfg, decode_step_kernel<4, 128>, a);
-    SCMX_PDL_OK("decode_step_kernel", e);
+    for (int first = 0; first < n_layers; first += MK_MAXLAYERS) {
+        a.layers = layers + first; a.first = first; a.n_layers = std::min(n_layers - first, MK_MAXLAYERS);
+        const int marks = (g_n_trace & 0xFFFF) - MK_MARKS * first;
+        a.trace = marks > 0 ? g_trace + MK_MARKS * first : nullptr; a.n_trace = marks;
+        mk_begin_kernel<<<1, 1, 0, st>>>(a.head);
+        SCMX_LAUNCH_OK("mk_begin_kernel");
+        const cudaError_t e = G == 1   ? cudaLaunchKernelEx(&cfg, decode_step_kernel<1, 128>, a)
+                              : G == 2 ? cudaLaunchKernelEx(&cfg, decode_step_kernel<2, 128>, a)
+                                       : cudaLaunchKernelEx(&cfg, decode_step_kernel<4, 128>, a);
+        SCMX_PDL_OK("decode_step_kernel", e);
+    }
     return SCMX_OK;
 }
 

@@ -14,7 +14,7 @@ signature.
 persistent=True (DecodeQwen3) runs all layers of a step as ONE cooperative kernel (scmx_decode_step): rows travel between
 the phases of a layer as packets instead of across kernel boundaries, each CTA re-quantizes the activations it needs in
 shared memory, and weights stream ahead of the phases.  Same bits as the chain of kernels; used where its limits
-hold (head size 128, widths multiples of 1024 up to 6144, 256 layers) and attention="kernel".
+hold (head size 128, widths multiples of 1024 up to 6144, shares of rows that fit the multiprocessors) and attention="kernel".
 
 DecodeHybrid is the same for hybrid decoders (fused_hybrid.FusedHybrid): GEMVs on bfloat16 or float32 weights with the mixers'
 one-token kernels between them, float32 activations."""
@@ -137,7 +137,16 @@ class DecodeQwen3(_Decoder):
         fits = lambda n: n % 1024 == 0 and n <= 6144  # noqa: E731
         self.persistent = bool(persistent and self.attn is not None and a.head_dim == 128 and fits(a.hidden_size)
                                and fits(a.intermediate_size) and fits(a.num_attention_heads * a.head_dim)
-                               and a.num_attention_heads <= 32 and a.num_hidden_layers <= 256 and fused.fmt == type(fused.fmt)())
+                               and a.num_attention_heads <= 32 and fused.fmt == type(fused.fmt)()
+                               and (not torch.cuda.is_available() or self._shares_fit(a, self.attn.nsplit, _lib.sm_count())))
+
+    @staticmethod
+    def _shares_fit(a, nsplit, n_sm):
+        """Whether the one-kernel step takes n_sm multiprocessors, as a partition of the device may have fewer: each has rows of every product, at most
+        384 of one, and there is one for every split of every key/value head (scmx_decode_step)."""
+        hq, hk, d = a.num_attention_heads, a.num_key_value_heads, a.head_dim
+        groups = [n // 4 for n in ((hq + 2 * hk) * d, 2 * a.intermediate_size, a.hidden_size)]
+        return hk * nsplit <= n_sm <= min(groups) and 4 * -(-max(groups) // n_sm) <= 384
 
     def _persistent_state(self, cache):
         """Layer table (device pointers of the packed weights, norms and this cache's tensors) and scratch buffers."""

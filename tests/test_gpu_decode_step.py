@@ -35,6 +35,29 @@ def test_step_equals_chain(scmx, D, F, layers, hq, hk):
             assert torch.equal(c.k, d.k) and torch.equal(c.v, d.v)
 
 
+@pytest.mark.parametrize("layers", [256, 257, 600])
+def test_many_layers(scmx, layers):
+    """More layers than a launch's table holds: a launch for every 256, the residual row handed on; two layers' weights in turn, a cache for every layer."""
+    mod = lambda n: importlib.import_module(scmx.__name__ + "." + n)      # noqa: E731
+    HM, FQ, DEC = mod("host_model"), mod("fused_qwen3"), mod("decode")
+    model = HM.CausalLM(HM.ModelArgs(1024, 1024, 2, 8, 4, 128, 1e-6, 1e6, 512, True)).init_random(seed=9, scale=0.05).cuda()
+    fused = FQ.FusedQwen3(model, FQ.pack_model(model, on_device=True))
+    fused.layers = (fused.layers * layers)[:layers]
+    chain, mk = DEC.DecodeQwen3(fused, persistent=False), DEC.DecodeQwen3(fused, persistent=True)
+    pair = [sum((fused.make_cache(16) for _ in range(-(-layers // 2))), [])[:layers] for _ in range(2)]
+    g = torch.Generator(device="cuda").manual_seed(layers)
+    for c, d in zip(*pair):
+        for to, other in ((c.k, d.k), (c.v, d.v)):
+            to.copy_(torch.randn(to.shape, generator=g, device="cuda").to(to.dtype))
+            other.copy_(to)
+        c.offset = d.offset = 9
+    tok = torch.tensor([[11]], device="cuda")
+    for _ in range(2):
+        assert torch.equal(chain.step(tok, pair[0]), mk.step(tok, pair[1]))
+    mk.check_status()
+    assert all(torch.equal(c.k, d.k) and torch.equal(c.v, d.v) for c, d in zip(*pair))
+
+
 def test_step_after_one_that_gave_up(scmx):
     """The abort word of a step that gave up and its epochs do not reach the next one."""
     mod = lambda n: importlib.import_module(scmx.__name__ + "." + n)      # noqa: E731

@@ -357,13 +357,28 @@ def test_shared_format_struct(scmx):
         S.set_format(old)
 
 
-@pytest.mark.parametrize("layers,one_kernel", [(1, True), (256, True), (257, False)])
-def test_decode_step_form(scmx, layers, one_kernel):
-    """A decoder with more layers than the one-kernel step's table holds takes the chain of kernels."""
+@pytest.mark.parametrize("layers", [1, 256, 257])
+def test_decode_step_form(scmx, layers):
+    """The one-kernel step takes any number of layers."""
     from types import SimpleNamespace as NS
     args = scmx.host_model.ModelArgs(1024, 1024, layers, 8, 4, 128, 1e-6, 1e6, 512, True)
     fused = NS(epilogue="gemm", model=NS(), args=args, inv_freq=torch.zeros(64), fmt=scmx.sc_format.Format())
-    assert scmx.decode.DecodeQwen3(fused, head=lambda x: x).persistent is one_kernel
+    assert scmx.decode.DecodeQwen3(fused, head=lambda x: x).persistent
+
+
+def test_decode_step_on_fewer_multiprocessors(scmx, monkeypatch):
+    """A decoder on a partition of the device takes the chain of kernels where the one-kernel step would refuse its shares."""
+    from types import SimpleNamespace as NS
+    A, D = scmx.host_model.ModelArgs, scmx.decode.DecodeQwen3
+    narrow, wide = A(1024, 1024, 1, 8, 4, 128, 1e-6, 1e6, 512, True), A(6144, 6144, 1, 32, 8, 128, 1e-6, 1e6, 512, True)
+    fits = lambda a, nsplit: [n for n in (4, 8, 16, 31, 32, 63, 64, 148, 256, 257) if D._shares_fit(a, nsplit, n)]      # noqa: E731
+    assert fits(narrow, 1) == [8, 16, 31, 32, 63, 64, 148, 256] and fits(narrow, 32) == [148, 256]
+    assert fits(wide, 1) == [32, 63, 64, 148, 256, 257] and fits(wide, 18) == [148, 256, 257]
+    monkeypatch.setattr(torch.cuda, "is_available", lambda: True)
+    fused = NS(epilogue="gemm", model=NS(), args=narrow, inv_freq=torch.zeros(64), fmt=scmx.sc_format.Format())
+    for sms, one_kernel in ((148, True), (64, False)):      # 4 heads of 32 splits
+        monkeypatch.setattr(scmx._lib, "sm_count", lambda: sms)
+        assert D(fused, head=lambda x: x).persistent is one_kernel
 
 
 def test_prompts_on_digit_planes(scmx):
