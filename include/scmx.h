@@ -429,8 +429,10 @@ int scmx_head_bf16(const uint16_t* W, int64_t ldw, const uint16_t* x, int64_t N,
 int scmx_select_token(const void* logits, int is_f32, int64_t V, int64_t* tok, int32_t* pos, int32_t* count, int64_t* out, int64_t cap, void* stream);
 /* Diagnostic: while device_buf is set, CTA 0 of the one-kernel decode step stores its SM cycle counter in device_buf[0 .. n), n < 65536, at
  * the ends of its phases, nine a layer: layer entered (the row before it done), input row there, q|k|v rows, attention, input row of o, o rows, input row of
- * gate|up, gate|up rows, input row of down.  device_buf: uint64 [n].  0 switches it off.  Process-wide; no counterpart in the reference. */
-int scmx_set_decode_trace(unsigned long long* device_buf, int n);
+ * gate|up, gate|up rows, input row of down.  With n_and_link = n | (b << 16), b > 0, every CTA also stores the global nanosecond timer at its arrival at link b
+ * (1-based, five a layer: its q|k|v rows, attention and combination, o rows, gate|up rows, down rows done) in device_buf[n + CTA index].  device_buf: uint64 [n], or
+ * [n + number of SMs].  0 switches it off.  Process-wide; no counterpart in the reference. */
+int scmx_set_decode_trace(unsigned long long* device_buf, int n_and_link);
 
 #ifdef __cplusplus
 }

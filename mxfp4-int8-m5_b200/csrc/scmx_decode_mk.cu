@@ -62,6 +62,8 @@ struct MkArgs {
     uint64_t wait_ns;
     unsigned long long* trace;   // diagnostic: null, or CTA 0 stores its cycle counter at every phase boundary
     int n_trace;
+    unsigned long long* arrivals;      // diagnostic: null, or every CTA stores the global timer at its arrival at this link (1-based, five a layer)
+    int link;
 };
 
 struct MkSmem {
@@ -127,6 +129,10 @@ __device__ __forceinline__ uint4 get8(const MkArgs& a, const uint2* p, uint32_t 
 __device__ __forceinline__ void mk_mark(const MkArgs& a, int& ti) {
     if (a.trace != nullptr && blockIdx.x == 0 && threadIdx.x == 0 && ti < a.n_trace) a.trace[ti] = (unsigned long long)clock64();
     ++ti;
+}
+
+__device__ __forceinline__ void mk_arrive(const MkArgs& a, int link) {
+    if (a.arrivals != nullptr && threadIdx.x == 0 && link == a.link) a.arrivals[blockIdx.x] = globaltimer_ns();
 }
 
 // ---- input row of a phase: bf16 row -> INT8 row in shared memory, returns the scale ---------------------------------------------
@@ -600,7 +606,7 @@ __global__ void __launch_bounds__(MK_THREADS, 1) decode_step_kernel(const __grid
         if (li + 1 < a.n_layers && tid < LWORDS)              // read after several barriers
             reinterpret_cast<unsigned long long*>(&layer[(li + 1) & 1])[tid] = reinterpret_cast<const unsigned long long*>(a.layers + li + 1)[tid];
         const uint32_t epoch = base_epoch + 1 + li;
-        const int code = 1000 + 5 * (a.first + li);
+        const int code = 1000 + 5 * (a.first + li), link = code - 1000;
         mk_mark(a, ti);
         if (attends && tid < 2 && t1 > t0) {                  // the positions that this CTA will attend to
             const int64_t te = t1 < T - 1 ? t1 : T - 1;
@@ -614,12 +620,14 @@ __global__ void __launch_bounds__(MK_THREADS, 1) decode_step_kernel(const __grid
         items(ph[0], D);
         __syncthreads();
         finish(ph[0], xs, false, a.xy, nullptr, epoch);
+        mk_arrive(a, link + 1);
         refill();
         mk_mark(a, ti);
         // P3: attention of one (kv head, split) per CTA
         if (attends) bad |= mk_attention<G, HD>(a, L, kvh, split, t0, t1, pos, epoch, code + 1);      // uniform over the CTA
         mk_mark(a, ti);
         for (int head = my_head; head < a.hq; head += (int)gridDim.x) bad |= mk_combine<HD>(a, head, active, epoch, code + 2);
+        mk_arrive(a, link + 2);
         __syncthreads();                                      // sm.ws and the products are free
         // P4: INT8 of o, o-projection + residual
         ahead(ph[1], L.wscale[1], li > 0 ? a.xh[0] : nullptr, a.h);
@@ -629,6 +637,7 @@ __global__ void __launch_bounds__(MK_THREADS, 1) decode_step_kernel(const __grid
         items(ph[1], QD);
         __syncthreads();
         finish(ph[1], xs, true, a.xh[1], nullptr, epoch);
+        mk_arrive(a, link + 3);
         refill();
         mk_mark(a, ti);
         __syncthreads();
@@ -645,6 +654,7 @@ __global__ void __launch_bounds__(MK_THREADS, 1) decode_step_kernel(const __grid
             for (int r = 0; r < 4; ++r) v[r] = scale_acc(total(ph[2], 4 * g + r), xs, sm.ws[4 * g + r]);
             put(a.xact + ph[2].base + g, pack_bf16x2(swiglu_bf16(v[0], v[2]), swiglu_bf16(v[1], v[3])), epoch);
         }
+        mk_arrive(a, link + 4);
         refill();
         mk_mark(a, ti);
         __syncthreads();
@@ -656,6 +666,7 @@ __global__ void __launch_bounds__(MK_THREADS, 1) decode_step_kernel(const __grid
         items(ph[3], F);
         __syncthreads();
         finish(ph[3], xs, true, a.xh[0], li + 1 == a.n_layers ? a.h : nullptr, epoch);
+        mk_arrive(a, link + 5);
         refill();
         __syncthreads();
     }
@@ -752,7 +763,8 @@ extern "C" int scmx_decode_step(const scmx_decode_layer* layers, int n_layers, i
     for (int first = 0; first < n_layers; first += MK_MAXLAYERS) {
         a.layers = layers + first; a.first = first; a.n_layers = std::min(n_layers - first, MK_MAXLAYERS);
         const int marks = (g_n_trace & 0xFFFF) - MK_MARKS * first;
-        a.trace = marks > 0 ? g_trace + MK_MARKS * first : nullptr; a.n_trace = marks;
+        a.trace = g_trace && marks > 0 ? g_trace + MK_MARKS * first : nullptr; a.n_trace = marks;
+        a.link = g_n_trace >> 16; a.arrivals = a.link > 0 ? g_trace + (g_n_trace & 0xFFFF) : nullptr;
         mk_begin_kernel<<<1, 1, 0, st>>>(a.head);
         SCMX_LAUNCH_OK("mk_begin_kernel");
         const cudaError_t e = G == 1   ? cudaLaunchKernelEx(&cfg, decode_step_kernel<1, 128>, a)

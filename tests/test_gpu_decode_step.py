@@ -107,3 +107,31 @@ def test_entry_with_scratch_of_its_own(scmx):
         assert torch.equal(a, b)
     dec.check_status()
     assert not any(bool(x.any()) for x in other)
+
+
+@pytest.mark.parametrize("layers,link", [(2, 1), (2, 5), (2, 8), (258, 1286)])
+def test_trace_of_arrivals(scmx, layers, link):
+    """Both forms of the diagnostic: cycle counts of CTA 0 alone, and every CTA's arrival at one link, which lie between the marks of the step before and after it."""
+    mod = lambda n: importlib.import_module(scmx.__name__ + "." + n)      # noqa: E731
+    HM, FQ, DEC, L = mod("host_model"), mod("fused_qwen3"), mod("decode"), scmx._lib
+    model = HM.CausalLM(HM.ModelArgs(1024, 1024, 2, 8, 4, 128, 1e-6, 1e6, 512, True)).init_random(seed=3, scale=0.05).cuda()
+    fused = FQ.FusedQwen3(model, FQ.pack_model(model, on_device=True))
+    fused.layers = fused.layers * (layers // 2)
+    mk, cache = DEC.DecodeQwen3(fused), sum((fused.make_cache(16) for _ in range(layers // 2)), [])
+    tok, n, sms = torch.tensor([[5]], device="cuda"), 9 * layers, torch.cuda.get_device_properties(0).multi_processor_count
+    buf, lib = torch.zeros(n + sms + 1, dtype=torch.int64, device="cuda"), L.lib()
+    try:
+        for wanted in (0, link):
+            buf.zero_()
+            L.call("scmx_set_decode_trace", L.ptr(buf), n | wanted << 16)
+            mk.step(tok, cache)
+            marks, arrivals = buf[:n].tolist(), buf[n:n + sms].tolist()
+            assert all(a < b for a, b in zip(marks, marks[1:])) or layers > 256      # (another launch, another SM)
+            assert all(marks) and buf[-1] == 0
+            if wanted:
+                assert min(arrivals) > 0 and max(arrivals) - min(arrivals) < 10_000_000
+            else:
+                assert not any(arrivals)
+    finally:
+        lib.scmx_set_decode_trace(None, 0)
+    mk.check_status()
