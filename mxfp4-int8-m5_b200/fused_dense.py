@@ -14,11 +14,29 @@ from . import sc_kernels as S
 GROUPS = ("qkv", "o", "gu", "down")
 
 
+class PassOrder:
+    """Orders the passes over buffers that they share: one on another stream than the pass before waits for that one's end.  Passes in a captured graph are left to whoever
+    replays it."""
+
+    def __init__(self):
+        self._end, self._last = torch.cuda.Event(), None
+
+    def begin(self, stream):
+        if self._last is not None and self._last != stream and not torch.cuda.is_current_stream_capturing():
+            stream.wait_event(self._end)
+
+    def end(self, stream):
+        if not torch.cuda.is_current_stream_capturing():
+            self._end.record(stream)
+            self._last = stream
+
+
 class DecodeRing:
     """Schedules the 4-bit -> INT8 decode of a sequence of weights around the GEMMs that consume them.  The sequence is cut into
     groups of `group` consecutive weights; two rotating sets of scratch buffers hold the current and the next group.  The decode
     of group j + 1 is issued on a side stream when group j is joined, events in both directions (group decoded -> its GEMMs may
-    start; last GEMM of a group launched -> its buffers may be overwritten).  Capturable in a CUDA graph.
+    start; last GEMM of a group launched -> its buffers may be overwritten).  Capturable in a CUDA graph.  A pass on another stream
+    waits for the end of the pass before (PassOrder); replays of a graph are ordered against other passes by whoever replays it.
 
     group = 1 (the default) decodes weight g + 1 while GEMM g runs and joins the side stream before every GEMM: two buffers of
     one weight each, which stay in L2.  Larger groups join less often (group = 4: once per layer) but decode a whole layer in
@@ -38,11 +56,13 @@ class DecodeRing:
         # prompt of 4 layers and 4096 tokens, 1230 us on the device, took the host 1850 us with streams entered and events created per weight, 1110 us so.
         self._ready, self._done = ([torch.cuda.Event(), torch.cuda.Event()] for _ in range(2))
         self._edge = torch.cuda.Event()                       # side after main at the start, main after side at the end
+        self._order = PassOrder()
 
     def begin(self, seq):
         """seq: list of (codes, bcodes, wscale, N, K) in the order the GEMMs run."""
         self.seq, self._joined = seq, None
         self.main = torch.cuda.current_stream()
+        self._order.begin(self.main)
         if self.overlap:
             self._after(self.side, self.main, self._edge)
             self._decode_group(0)
@@ -101,6 +121,7 @@ class DecodeRing:
         self._joined = None
         if self.overlap:
             self._after(self.main, self.side, self._edge)
+        self._order.end(self.main)
 
 
 class DenseStack:

@@ -5,6 +5,7 @@ import torch
 
 from . import sc_kernels as S
 from . import sc_moe as M_
+from .fused_dense import PassOrder
 
 
 class MoeBlock:
@@ -29,7 +30,7 @@ class MoeBlock:
         elif self.early:
             self.gu8 = torch.empty((n_experts * 2 * F, D), dtype=torch.int8, device=dev)
             self.dn8 = torch.empty((n_experts * D, F), dtype=torch.int8, device=dev)
-            self.side = torch.cuda.Stream(device=dev)
+            self.side, self._order = torch.cuda.Stream(device=dev), PassOrder()
 
     # measured on B200 (64 experts, 2048 x 1024; half-block ms, packed-weight GEMMs / decode-then-GEMM): 128 rows per expert
     # 0.190 / 0.275, 256: 0.286 / 0.330, 384: 0.356 / 0.394, 448: 0.367 / 0.419, 512: 0.478 / 0.449 (past 512 rows an expert
@@ -42,6 +43,7 @@ class MoeBlock:
     def _start_decode(self):
         """Both expert sets -> INT8 on the side stream; returns the events the two GEMMs wait for."""
         main = torch.cuda.current_stream()
+        self._order.begin(main)
         self.side.wait_stream(main)                           # the previous step's GEMMs no longer read the buffers
         E, D, F = self.E, self.D, self.F
         with torch.cuda.stream(self.side):
@@ -74,7 +76,10 @@ class MoeBlock:
         if self.two_pass or self.early:
             if decoded is not None:
                 main.wait_event(decoded[1])
-            return M_.moe_mm_i8(xq2, R, self.dn8, self.dn[2], off, ts, mt, D, 1, xs2)
+            yd = M_.moe_mm_i8(xq2, R, self.dn8, self.dn[2], off, ts, mt, D, 1, xs2)
+            if decoded is not None:
+                self._order.end(main)
+            return yd
         return M_.moe_mm(xq2, R, *self.dn, off, ts, mt, D, 1, xs2)
 
     def step(self, h, logits):

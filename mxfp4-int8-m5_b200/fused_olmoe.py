@@ -18,6 +18,7 @@ from . import sc_decode as G
 from . import sc_format as F
 from . import sc_kernels as S
 from . import sc_moe as M_
+from .fused_dense import PassOrder
 from .fused_moe import MoeBlock
 from .fused_qwen3 import attend_quant
 from .w4a8 import PackedWeight
@@ -108,7 +109,7 @@ class FusedOlmoe:
         if self.prefetch:
             self.ring = [(torch.empty((E * F2, D), dtype=torch.int8, device=dev),
                           torch.empty((E * D, Fi), dtype=torch.int8, device=dev)) for _ in range(2)]
-            self.side = torch.cuda.Stream(device=dev)
+            self.side, self._order = torch.cuda.Stream(device=dev), PassOrder()
         self.inv_freq = S.rope_inv_freq(a.head_dim, a.rope_theta, dev)
         self.rope_cs = S.rope_table(self.inv_freq, 16384)          # cos / sin of the first positions, read by the q/k/v kernel
         self.record, self.record_layers = None, ()
@@ -252,6 +253,7 @@ class FusedOlmoe:
         ahead = self.prefetch and not self._packed(L * a.num_experts_per_tok)
         if ahead:
             self._ready, self._done = [None] * nl, [None] * nl
+            self._order.begin(main)
             self.side.wait_stream(main)
             self._decode_experts(0)
         xq, xs = S.rmsnorm_quant(h, self.layers[0][0].input_layernorm.weight, self.eps, Mp)
@@ -281,6 +283,7 @@ class FusedOlmoe:
                 self.record[(i, "experts")] = (h_in, xn, inds, scores, yd, pos, *rec)
         if ahead:
             main.wait_stream(self.side)
+            self._order.end(main)
         xn = S.rmsnorm_quant_n(h, self.model.model.norm.weight, self.eps, Mp)[2]
         return xn[:L][None]
 

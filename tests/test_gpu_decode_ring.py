@@ -1,5 +1,5 @@
-"""GPU: one decode ring used again and again: its events and views serve eager passes, a captured pass, a pass on another stream and sequences of other weights, with
-groups that do not divide the sequence, and the operand each product reads is the decoded weight (compared as integers)."""
+"""GPU: one decode ring used again and again: its events and views serve eager passes, a captured pass, passes on other streams that start while the last one still reads, and
+sequences of other weights, with groups that do not divide the sequence, and the operand each product reads is the decoded weight (compared as integers)."""
 import pytest
 import torch
 
@@ -21,11 +21,14 @@ def test_ring_serves_every_pass(scmx, group, count, overlap):
             seq.append((c, torch.randint(0, 256, (n, k // 128), generator=g, device="cuda").to(torch.uint8), None, n, k))
         return seq
 
-    def read(seq):
+    def read(seq, slow=False):
         ring.begin(seq)
         got = []
         for i in range(count):
-            got.append(ring.weight(i).clone())
+            w = ring.weight(i)
+            if slow:
+                torch.cuda._sleep(200_000)                # 0.1 ms: the host is through with the pass before its reads have begun
+            got.append(w.clone())
             ring.released(i)
         ring.end()
         return got
@@ -41,8 +44,9 @@ def test_ring_serves_every_pass(scmx, group, count, overlap):
         kept = read(seqs[1])
     graph.replay()
     torch.cuda.synchronize()
-    with torch.cuda.stream(side):
-        outs += [(read(seqs[0]), 0), (read(seqs[1]), 1)]
+    for stream in (torch.cuda.current_stream(), side, torch.cuda.current_stream()):      # no synchronization in between
+        with torch.cuda.stream(stream):
+            outs += [(read(seqs[0], True), 0), (read(seqs[1], True), 1)]
     torch.cuda.synchronize()
     graph.replay()
     torch.cuda.synchronize()

@@ -409,6 +409,62 @@ def test_prompts_on_digit_planes(scmx):
         S.set_format(old)
 
 
+class _Clock:
+    """Streams and events that know which operations they come after."""
+
+    class Stream:
+        cuda_stream = 0
+
+        def __init__(self, **kw):
+            self.before = set()
+
+        def do(self, op):
+            self.before.add(op)
+
+        def wait_event(self, e):
+            self.before |= e.before
+
+        def wait_stream(self, other):
+            self.before |= other.before
+
+    class Event:
+        before = frozenset()
+
+        def record(self, stream):
+            self.before = frozenset(stream.before)
+
+
+@pytest.mark.parametrize("overlap,group,count", [(True, 1, 1), (True, 1, 5), (True, 2, 5), (False, 1, 3)])
+def test_ring_on_another_stream(scmx, monkeypatch, overlap, group, count):
+    """A pass on another stream decodes into the ring's buffers only after every product of the pass before that read them, and so on to and fro."""
+    FD, S = scmx.fused_dense, scmx.sc_kernels
+    current, capturing = [None], [False]
+    for name, fake in dict(Stream=_Clock.Stream, Event=_Clock.Event, current_stream=lambda: current[0], is_current_stream_capturing=lambda: capturing[0]).items():
+        monkeypatch.setattr(torch.cuda, name, fake)
+    ring = FD.DecodeRing(64, "cpu", overlap, group)
+    readers, turn = {}, [0]
+
+    def unpack(codes, bc, N, K, out, stream):
+        on = ring.side if overlap else current[0]
+        if not capturing[0]:
+            assert readers.get(out.data_ptr(), set()) <= on.before
+        on.do(("decode", out.data_ptr(), turn[0]))
+
+    monkeypatch.setattr(S, "unpack_i8", unpack)
+    a, b, c = (_Clock.Stream() for _ in range(3))
+    for stream, captured in ((a, False), (a, False), (b, False), (c, True), (c, False), (a, False), (b, False)):
+        current[0], capturing[0] = stream, captured
+        ring.begin([(None, None, None, 8, 8)] * count)
+        for g in range(count):
+            turn[0] += 1
+            w = ring.weight(g).data_ptr()
+            stream.do(("read", w, turn[0]))
+            if not captured:
+                readers.setdefault(w, set()).add(("read", w, turn[0]))
+            ring.released(g)
+        ring.end()
+
+
 def test_generation_keeps_what_its_graph_names(scmx, monkeypatch):
     """Steps on other caches replace the one-kernel step's tables; those of a captured generation stay alive and are the decoder's again when it is replayed."""
     import contextlib
