@@ -334,10 +334,8 @@ _STEP_ROWS = ("input row", "q|k|v row", "attention output", "residual row after 
 
 
 def describe_status(code):
-    """Text for a status-word code: 1..5 GEMM roles, 11 / 12 streaming GEMV, 20 peer barrier, 100 + k grid barrier k, 1000 + 5 layer + k
-    row k of a layer of the one-kernel decode step."""
+    """Text for a status-word code: 1..6 GEMM roles, 11 / 12 streaming GEMV, 20 peer barrier, 31..64 kernels of the sequence mixers,
+    1000 + 5 layer + k row k of a layer of the one-kernel decode step."""
     if code >= 1000:
         return f"decode step: layer {(code - 1000) // 5} waiting for its {_STEP_ROWS[(code - 1000) % 5]}"
-    if code >= 100:
-        return f"decode step: grid barrier {code - 100} timed out"
     return _GEMM_ROLES.get(code, f"code {code}")

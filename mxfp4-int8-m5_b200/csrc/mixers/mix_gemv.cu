@@ -20,7 +20,7 @@ struct GvArgs {
     const float* x;         // [K]
     float* out;             // [N]
     int64_t ldw;
-    int N, K, ks;           // ks: warps that share a row (1, 2, 4 or 8)
+    int N, K, ks;           // ks: warps that share a row (1, 2, 4, 8 or 16)
     int warps, slots;       // warps that stream weights, slots of a warp's ring
     float a_pos, a_neg;     // xIELU
     const float *cw, *cb;   // convolution weights [C, taps] and bias [C]

@@ -139,8 +139,9 @@ def test_status_word_codes_have_texts(scmx):
     for code, word in ((1, "producer"), (2, "MMA"), (3, "MMA"), (4, "epilogue"), (6, "unpack"), (11, "GEMV"), (12, "GEMV"),
                        (20, "peer barrier")):
         assert word in L.describe_status(code), code
-    assert "grid barrier 3" in L.describe_status(103)
-    assert L.describe_status(77) == "code 77"
+    assert L.describe_status(1000) == "decode step: layer 0 waiting for its input row"
+    assert L.describe_status(1000 + 5 * 27 + 3) == "decode step: layer 27 waiting for its residual row after attention"
+    assert L.describe_status(77) == "code 77" and L.describe_status(103) == "code 103"
 
 
 def test_calls_that_torch_has_to_see(scmx):
