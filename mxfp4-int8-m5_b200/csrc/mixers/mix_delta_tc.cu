@@ -943,9 +943,11 @@ __global__ void __launch_bounds__(DT_THREADS, 1)
             uint32_t u[32];
 #pragma unroll
             for (int i = 0; i < 32; ++i) u[i] = in && !unit ? __float_as_uint(src[128 * i]) : 0u;
+            tmem_st32(tmem + DT_U + 32 * wg + lane_base, u);
+            // The buffer is given back after the store, whose operands are the loaded values.  An arrive does not wait for shared-memory loads on their way: behind a queue of
+            // loads of the carried state, the last tokens' were still there when the next chunk's copy landed (a wrong start of the second segment in half of all processes).
             __syncwarp();
             if (lane == 0) mbar_arrive(b_ve);
-            tmem_st32(tmem + DT_U + 32 * wg + lane_base, u);
             return true;
         };
         const bool go = wg >= 2 || bring_values(0);

@@ -185,6 +185,29 @@ def test_delta_segments(X, H, G, d, dv, channel, cuts):
     assert err(c.run(cuts, 2), o) < 5e-4 and err(c.state, S) < 5e-4
 
 
+@pytest.mark.parametrize("channel", [False, True])
+@pytest.mark.parametrize("H,T,dv", [(16, 2050, 128), (8, 1500, 128), (16, 1990, 64)])
+def test_delta_segments_repeat(X, H, T, dv, channel):
+    """Long portions from a carried state that lies in memory no cache holds, on buffers of other values: every pass has the bits of the first one, and those of the chunks one
+    after the other within rounding.  (A value buffer that was given back before its last loads had returned spoilt the second segment's start.)"""
+    c = DeltaCase(X, T, H, H, 128, dv, channel, BF, seed=6, strength=-5.0)
+    start = rnd(50, H, 128, dv, scale=0.3)
+    c.state.copy_(start)
+    chunks = c.run([190] * (T // 190) + ([T % 190] if T % 190 else []), 2)
+    want = None
+    for i in range(24):
+        keep = [torch.full((1 << 26,), i * 1e3, device="cuda") for _ in range(2)]      # 512 MB: out of L2, and what the pass's buffers hold
+        del keep
+        c.state = torch.empty(H, 128, dv, device="cuda")
+        c.state.copy_(start)
+        torch.full((1 << 26,), 1.0, device="cuda")
+        o = c.run([T], 2)
+        if want is None:
+            want = o, c.state
+            assert err(o, npy(chunks)) < 5e-4
+        assert torch.equal(o, want[0]) and torch.equal(c.state, want[1]), i
+
+
 def test_delta_far_value_is_read_back(X):
     """A value written once under its own key and asked for 700 tokens later, almost without decay."""
     for channel in (False, True):
