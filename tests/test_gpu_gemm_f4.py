@@ -1,5 +1,6 @@
 """GPU: the products on digit planes (gemm_f4_kernel: tcgen05 kind::mxf4) against the oracle's and the packed-weight GEMM's bits: edges of token tiles, of weight tiles of
-256 rows and of stages of 256 values, experts without rows, extreme codes (the largest sums the accumulators hold), every epilogue; and the digits themselves."""
+256 rows and of stages of 256 values, experts without rows, extreme codes (all of one sign, and the largest sums the accumulators hold), every epilogue; and the digits
+themselves."""
 import numpy as np
 import pytest
 import torch
@@ -64,7 +65,7 @@ def test_row_quantizer_digits(scmx, M, K):
 @pytest.mark.parametrize("extreme", [False, True])
 @pytest.mark.parametrize("M,N,K", [(1, 32, 128), (16, 256, 256), (17, 288, 384), (80, 512, 640), (81, 256, 1024), (161, 64, 2048), (640, 4096, 256), (33, 96, 10240)])
 def test_dense_bits(scmx, M, N, K, extreme):
-    """INT32 totals against 64-bit sums, the other epilogues against the packed-weight GEMM.  `extreme`: every product 127 * 96 of one sign, the largest accumulators."""
+    """INT32 totals against 64-bit sums, the other epilogues against the packed-weight GEMM.  `extreme`: every product 127 * 96 of one sign, the largest totals."""
     S, L, F, M_ = scmx.sc_kernels, scmx._lib, scmx.sc_format, scmx.sc_moe
     c, b, ws, g = _weights(1, N, K, M + N + K, extreme)
     xq = torch.randint(-127, 128, (M, K), generator=g, device="cuda").to(torch.int8)
@@ -87,8 +88,67 @@ def test_dense_bits(scmx, M, N, K, extreme):
     L.check_status()
 
 
+def _bits(x):
+    return x.contiguous().view(torch.int16 if x.dtype == torch.bfloat16 else torch.int32)
+
+
+def _compare(scmx, xq, c, b, ws, N, K, seed):
+    """Every epilogue, bit for bit (signs of zeros too), against the INT8 product, and the totals against 64-bit sums."""
+    S, M_ = scmx.sc_kernels, scmx.sc_moe
+    M, g = xq.shape[0], torch.Generator(device="cuda").manual_seed(seed)
+    dig, fac, wq = M_.gather_digits(xq, None, None, M)[0], M_.f4_factors((b, 1, N, K))[0], S.unpack_i8(c.view(-1), b.view(N, -1), N, K)
+    want = (xq.double() @ wq.double().T).long()
+    assert torch.equal(S.mm_f4(dig, c, fac, None, ws, 0).long(), want)
+    xs, res = torch.rand(M, generator=g, device="cuda") * 0.01, torch.randn(M, N, generator=g, device="cuda").to(torch.bfloat16)
+    pad = -(-M // 128) * 128 - M
+    xqp, xsp, resp = (torch.nn.functional.pad(t, (0, 0) * (t.dim() - 1) + (0, pad)) for t in (xq, xs, res))
+    for epi in (1, 2, 3):
+        ref = S.mm_epi(xqp, wq, xsp, ws, epi, res=resp if epi == 2 else None)[:M]
+        assert torch.equal(_bits(S.mm_f4(dig, c, fac, xs, ws, epi, res)), _bits(ref)), epi
+    scmx._lib.check_status()
+    return want
+
+
+@pytest.mark.parametrize("M,N,K", [(37, 128, 1024), (160, 256, 6144), (33, 64, 10240)])
+def test_low_bits_of_large_sums(scmx, M, N, K):
+    """Digits of -4 and -3 in the two lower planes times positive weights of every magnitude and block factor: plane sums between 2^15 and 2^22 whose low bits take every value
+    (a plane whose accumulator dropped one would show), and single rows of the values with the largest digits, -36 = (-4, -4, 0) and 92 = (-4, -4, 2), times 96."""
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    nib = torch.randint(0, 8, (N, K // 8, 8), generator=g, device="cuda")
+    nib[: N // 2, :, ::3] = 7                                   # half of the rows are heavy
+    c = (nib << torch.arange(0, 32, 4, device="cuda")).sum(-1).to(torch.int32)
+    b = torch.randint(0, 256, (1, N, K // 128), generator=g, device="cuda").to(torch.uint8)
+    b[:, : N // 2] |= 0xAA
+    c[0], b[0, 0] = 0x77777777, 255                             # one row of 96
+    x = torch.tensor([-36, -35, -28, -27], device="cuda", dtype=torch.int8)[torch.randint(0, 4, (M, K), generator=g, device="cuda")]
+    x[0], x[1], x[2], x[3], x[4] = -36, 92, -4, -32, 0
+    want = _compare(scmx, x, c, b, torch.rand(N, generator=g, device="cuda") * 1e-3 + 1e-5, N, K, M)
+    d0, d1 = (x.long() + 36) % 8 - 4, (x.long() + 36) // 8 % 8 - 4
+    wq = scmx.sc_kernels.unpack_i8(c.view(-1), b.view(N, -1), N, K).double()
+    for d in (d0, d1):
+        sums = (d.double() @ wq.T).long().abs()
+        assert int(sums.max()) == 384 * K and len(torch.unique(sums[5:] % 64)) == 64 and float((sums > 1 << 15).double().mean()) > 0.6
+    assert int(want.abs().max()) == 92 * 96 * K
+
+
+@pytest.mark.parametrize("K,N", [(5120, 128), (6144, 64), (10240, 192)])
+def test_totals_around_two_to_the_24th(scmx, K, N):
+    """Sums of the two lower planes on both sides of 2^24, where the epilogues go over to integers (36 * 96 * 4854 < 2^24 < 36 * 96 * 4855), with third planes of 0 and 2, and 64
+    columns of any sign and magnitude that move them by single units."""
+    c, b, ws, g = _weights(1, N, K, K, True)
+    c.view(N, K // 8)[:, -8:] = torch.randint(-2 ** 31, 2 ** 31 - 1, (N, 8), generator=g, device="cuda").to(torch.int32)
+    x = torch.zeros(40, K, dtype=torch.int8, device="cuda")
+    for r in range(40):
+        x[r, :4854 - 15 + 5 * (r % 8)] = -36 if r < 24 else 92
+        x[r, -64:] = torch.randint(-3, 4, (64,), generator=g, device="cuda").to(torch.int8)
+    _compare(scmx, x, c, b, ws.view(-1), N, K, K)
+    wq, low = scmx.sc_kernels.unpack_i8(c.view(-1), b.view(N, -1), N, K).double(), x.long() - 64 * ((x.long() + 36) // 64)
+    past = (low.double() @ wq.T).abs() - 2.0 ** 24
+    assert float(past.max()) > 0 > float(past.min()) and float(past.abs().min()) < 4000 and float(past.abs().max()) < 1 << 18
+
+
 def test_swiglu_of_every_gate(scmx):
-    """The epilogue's SiLU against sc_swiglu for all finite bfloat16 gates (equal), and not-a-number gates."""
+    """The epilogue's SiLU against sc_swiglu for all bfloat16 gates (finite and infinite ones equal), and scales that are infinite, not numbers or denormal against the INT8 product."""
     S, M_ = scmx.sc_kernels, scmx.sc_moe
     gate = torch.arange(65536, device="cuda").to(torch.int32).to(torch.int16).view(torch.bfloat16)
     K, N = 128, 64
@@ -101,6 +161,19 @@ def test_swiglu_of_every_gate(scmx):
     fin = torch.isfinite(gate.float())
     assert torch.equal(got[fin].view(torch.int16), want[fin].view(torch.int16)[:, None].expand(-1, N // 2))
     assert bool(torch.isnan(got[torch.isnan(gate)]).all())
+    inf = torch.isinf(gate.float())
+    assert torch.equal(got[inf].isnan(), want[inf].isnan()[:, None].expand(-1, N // 2))
+    assert torch.equal(got[inf].nan_to_num(7.0), want[inf].nan_to_num(7.0)[:, None].expand(-1, N // 2))
+    wq = S.unpack_i8(c.view(-1), b.view(N, 1), N, K)
+    scales = torch.tensor([float("inf"), float("-inf"), 3e38, -3e38, 1e-40, float("nan"), 1.0, 0.0], device="cuda").repeat(16)
+    for q in (1, 0, -1):
+        x8 = torch.zeros(128, K, dtype=torch.int8, device="cuda")
+        x8[:, 0] = q
+        for epi in (1, 3):
+            new = S.mm_f4(M_.gather_digits(x8, None, None, 128)[0], c.view(-1), M_.f4_factors((b, 1, N, K))[0], scales, torch.ones(N, device="cuda"), epi)
+            old = S.mm_epi(x8, wq, scales, torch.ones(N, device="cuda"), epi)
+            assert torch.equal(new.isnan(), old.isnan())
+            assert torch.equal(_bits(new[~new.isnan()]), _bits(old[~old.isnan()])), (q, epi)
 
 
 @pytest.mark.parametrize("N,K", [(256, 256), (320, 1024), (2048, 128)])
