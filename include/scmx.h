@@ -409,7 +409,7 @@ typedef struct scmx_decode_layer {
  * layers: device array; scratch: scmx_decode_step_scratch bytes, 16-byte aligned, zero before its first use and then left to the steps that
  * share it, which must not overlap; status int32 [1] receives 1000 + 5 layer + k if a wait ran out (scmx_set_wait_limit_ns), k = 0 residual row, 1 q|k|v, 2 attention,
  * 3 residual row after it, 4 feed-forward row, after which the step's outputs are invalid.
- * Limits: d = 128; D, F and hq*d multiples of 1024 up to 6144; hq/hk in {1, 2, 4}; hk * nsplit <= number of SMs; every SM gets rows of each product,
+ * Limits: d = 128; D, F and hq*d multiples of 1024 up to 6144; hq/hk in {1, 2, 4}; hk * nsplit and hq <= number of SMs; every SM gets rows of each product,
  * at most 384 of one (32 to 256 SMs do for all widths).  More than 256 layers take a launch for every 256.
  * Not to be run concurrently with other work on the same device: the launch needs every SM. */
 int64_t scmx_decode_step_scratch(int D, int F, int hq, int hk, int d, int nsplit);

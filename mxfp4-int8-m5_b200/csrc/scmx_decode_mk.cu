@@ -504,7 +504,8 @@ __device__ __noinline__ bool mk_combine(const MkArgs& a, int head, int active, u
 }
 
 // ---- the kernel ------------------------------------------------------------------------------------------------------------
-template <int G, int HD>
+// TRACE: the form that stores the diagnostic's times.  They cost the step of 8 layers 2 of 317 us, so the product's form has none of them.
+template <int G, int HD, bool TRACE>
 __global__ void __launch_bounds__(MK_THREADS, 1) decode_step_kernel(const __grid_constant__ MkArgs a) {
     extern __shared__ __align__(16) uint8_t rings[];
     __shared__ MkPhase ph[4];
@@ -539,7 +540,7 @@ __global__ void __launch_bounds__(MK_THREADS, 1) decode_step_kernel(const __grid
     const int kvh = blockIdx.x % a.hk, split = blockIdx.x / a.hk;
     const bool attends = split < active;
     const int64_t t0 = (int64_t)split * chunk, t1 = t0 + chunk < T ? t0 + chunk : T;
-    const int my_head = (int)gridDim.x - 1 - (int)blockIdx.x;      // query head whose splits this CTA combines (and every gridDim.x-th after it)
+    const int my_head = (int)gridDim.x - 1 - (int)blockIdx.x;      // query head whose splits this CTA combines
     bool bad = false;
     int ti = 0;
 
@@ -607,7 +608,7 @@ __global__ void __launch_bounds__(MK_THREADS, 1) decode_step_kernel(const __grid
             reinterpret_cast<unsigned long long*>(&layer[(li + 1) & 1])[tid] = reinterpret_cast<const unsigned long long*>(a.layers + li + 1)[tid];
         const uint32_t epoch = base_epoch + 1 + li;
         const int code = 1000 + 5 * (a.first + li), link = code - 1000;
-        mk_mark(a, ti);
+        if (TRACE) mk_mark(a, ti);
         if (attends && tid < 2 && t1 > t0) {                  // the positions that this CTA will attend to
             const int64_t te = t1 < T - 1 ? t1 : T - 1;
             if (te > t0) prefetch_l2((tid ? L.v_cache : L.k_cache) + ((size_t)kvh * a.cap + t0) * HD, (uint32_t)(te - t0) * HD * 2);
@@ -616,36 +617,36 @@ __global__ void __launch_bounds__(MK_THREADS, 1) decode_step_kernel(const __grid
         ahead(ph[0], L.wscale[0], nullptr, nullptr);
         float xs = mk_input<true>(a, li > 0 ? a.xh[0] : nullptr, a.h, epoch - 1, L.ln_in, D, code, bad);
         if (gave_up()) return;
-        mk_mark(a, ti);
+        if (TRACE) mk_mark(a, ti);
         items(ph[0], D);
         __syncthreads();
         finish(ph[0], xs, false, a.xy, nullptr, epoch);
-        mk_arrive(a, link + 1);
+        if (TRACE) mk_arrive(a, link + 1);
         refill();
-        mk_mark(a, ti);
+        if (TRACE) mk_mark(a, ti);
         // P3: attention of one (kv head, split) per CTA
         if (attends) bad |= mk_attention<G, HD>(a, L, kvh, split, t0, t1, pos, epoch, code + 1);      // uniform over the CTA
-        mk_mark(a, ti);
-        for (int head = my_head; head < a.hq; head += (int)gridDim.x) bad |= mk_combine<HD>(a, head, active, epoch, code + 2);
-        mk_arrive(a, link + 2);
+        if (TRACE) mk_mark(a, ti);
+        if (my_head < a.hq) bad |= mk_combine<HD>(a, my_head, active, epoch, code + 2);
+        if (TRACE) mk_arrive(a, link + 2);
         __syncthreads();                                      // sm.ws and the products are free
         // P4: INT8 of o, o-projection + residual
         ahead(ph[1], L.wscale[1], li > 0 ? a.xh[0] : nullptr, a.h);
         xs = mk_input<false>(a, a.xo, nullptr, epoch, nullptr, QD, code + 2, bad);
         if (gave_up()) return;
-        mk_mark(a, ti);
+        if (TRACE) mk_mark(a, ti);
         items(ph[1], QD);
         __syncthreads();
         finish(ph[1], xs, true, a.xh[1], nullptr, epoch);
-        mk_arrive(a, link + 3);
+        if (TRACE) mk_arrive(a, link + 3);
         refill();
-        mk_mark(a, ti);
+        if (TRACE) mk_mark(a, ti);
         __syncthreads();
         // P5: post-attention RMSNorm + INT8, gate|up projection with SwiGLU
         ahead(ph[2], L.wscale[2], nullptr, nullptr);
         xs = mk_input<true>(a, a.xh[1], nullptr, epoch, L.ln_post, D, code + 3, bad);
         if (gave_up()) return;
-        mk_mark(a, ti);
+        if (TRACE) mk_mark(a, ti);
         items(ph[2], D);
         __syncthreads();
         for (int g = tid; g < ph[2].count; g += MK_THREADS) {                  // a row group: two gate rows, two up rows
@@ -654,19 +655,19 @@ __global__ void __launch_bounds__(MK_THREADS, 1) decode_step_kernel(const __grid
             for (int r = 0; r < 4; ++r) v[r] = scale_acc(total(ph[2], 4 * g + r), xs, sm.ws[4 * g + r]);
             put(a.xact + ph[2].base + g, pack_bf16x2(swiglu_bf16(v[0], v[2]), swiglu_bf16(v[1], v[3])), epoch);
         }
-        mk_arrive(a, link + 4);
+        if (TRACE) mk_arrive(a, link + 4);
         refill();
-        mk_mark(a, ti);
+        if (TRACE) mk_mark(a, ti);
         __syncthreads();
         // P6: INT8 of act, down projection + residual
         ahead(ph[3], L.wscale[3], a.xh[1], nullptr);
         xs = mk_input<false>(a, a.xact, nullptr, epoch, nullptr, F, code + 4, bad);
         if (gave_up()) return;
-        mk_mark(a, ti);
+        if (TRACE) mk_mark(a, ti);
         items(ph[3], F);
         __syncthreads();
         finish(ph[3], xs, true, a.xh[0], li + 1 == a.n_layers ? a.h : nullptr, epoch);
-        mk_arrive(a, link + 5);
+        if (TRACE) mk_arrive(a, link + 5);
         refill();
         __syncthreads();
     }
@@ -729,17 +730,20 @@ extern "C" int scmx_decode_step(const scmx_decode_layer* layers, int n_layers, i
     if (!coop_dev[dev]) {
         int c = 0;
         SCMX_CUDA_OK(cudaDeviceGetAttribute(&c, cudaDevAttrCooperativeLaunch, dev));
-        SCMX_CUDA_OK(cudaFuncSetAttribute(decode_step_kernel<1, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, RINGS));
-        SCMX_CUDA_OK(cudaFuncSetAttribute(decode_step_kernel<2, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, RINGS));
-        SCMX_CUDA_OK(cudaFuncSetAttribute(decode_step_kernel<4, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, RINGS));
+        SCMX_CUDA_OK(cudaFuncSetAttribute(decode_step_kernel<1, 128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, RINGS));
+        SCMX_CUDA_OK(cudaFuncSetAttribute(decode_step_kernel<1, 128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, RINGS));
+        SCMX_CUDA_OK(cudaFuncSetAttribute(decode_step_kernel<2, 128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, RINGS));
+        SCMX_CUDA_OK(cudaFuncSetAttribute(decode_step_kernel<2, 128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, RINGS));
+        SCMX_CUDA_OK(cudaFuncSetAttribute(decode_step_kernel<4, 128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, RINGS));
+        SCMX_CUDA_OK(cudaFuncSetAttribute(decode_step_kernel<4, 128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, RINGS));
         coop_dev[dev] = c ? 1 : -1;
     }
     const int coop = coop_dev[dev] > 0, n_sm = sm_count();
     SCMX_REQUIRE(coop, SCMX_EDEVICE, "decode_step: the device does not support cooperative launches");
     // Every CTA has rows in every phase, which the reuse of the packet buffers rests on, and no more than its tables hold.
     const int qkv = (hq + 2 * hk) * d, most = std::max({qkv, 2 * F, D}) / 4, least = std::min({qkv, 2 * F, D}) / 4;
-    SCMX_REQUIRE(hk * nsplit <= n_sm && n_sm <= least && 4 * ((most + n_sm - 1) / n_sm) <= MK_MAXROWS, SCMX_EINVAL,
-                 "decode_step: hk * nsplit = %d, phases of %d to %d rows on the %d CTAs of the grid", hk * nsplit, 4 * least, 4 * most, n_sm);
+    SCMX_REQUIRE(hk * nsplit <= n_sm && hq <= n_sm && n_sm <= least && 4 * ((most + n_sm - 1) / n_sm) <= MK_MAXROWS, SCMX_EINVAL,
+                 "decode_step: hk * nsplit = %d, hq = %d, phases of %d to %d rows on the %d CTAs of the grid", hk * nsplit, hq, 4 * least, 4 * most, n_sm);
     size_t off[7];
     mk_scratch(D, F, hq, hk, d, nsplit, off);
     uint8_t* sp = static_cast<uint8_t*>(scratch);
@@ -767,9 +771,10 @@ extern "C" int scmx_decode_step(const scmx_decode_layer* layers, int n_layers, i
         a.link = g_n_trace >> 16; a.arrivals = a.link > 0 ? g_trace + (g_n_trace & 0xFFFF) : nullptr;
         mk_begin_kernel<<<1, 1, 0, st>>>(a.head);
         SCMX_LAUNCH_OK("mk_begin_kernel");
-        const cudaError_t e = G == 1   ? cudaLaunchKernelEx(&cfg, decode_step_kernel<1, 128>, a)
-                              : G == 2 ? cudaLaunchKernelEx(&cfg, decode_step_kernel<2, 128>, a)
-                                       : cudaLaunchKernelEx(&cfg, decode_step_kernel<4, 128>, a);
+        void (*kernel)(MkArgs) = G == 1   ? (g_trace ? decode_step_kernel<1, 128, true> : decode_step_kernel<1, 128, false>)
+                                 : G == 2 ? (g_trace ? decode_step_kernel<2, 128, true> : decode_step_kernel<2, 128, false>)
+                                          : (g_trace ? decode_step_kernel<4, 128, true> : decode_step_kernel<4, 128, false>);
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, a);
         SCMX_PDL_OK("decode_step_kernel", e);
     }
     return SCMX_OK;

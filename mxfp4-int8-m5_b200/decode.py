@@ -143,10 +143,10 @@ class DecodeQwen3(_Decoder):
     @staticmethod
     def _shares_fit(a, nsplit, n_sm):
         """Whether the one-kernel step takes n_sm multiprocessors, as a partition of the device may have fewer: each has rows of every product, at most
-        384 of one, and there is one for every split of every key/value head (scmx_decode_step)."""
+        384 of one, and there is one for every query head and every split of a key/value head (scmx_decode_step)."""
         hq, hk, d = a.num_attention_heads, a.num_key_value_heads, a.head_dim
         groups = [n // 4 for n in ((hq + 2 * hk) * d, 2 * a.intermediate_size, a.hidden_size)]
-        return hk * nsplit <= n_sm <= min(groups) and 4 * -(-max(groups) // n_sm) <= 384
+        return max(hk * nsplit, hq) <= n_sm <= min(groups) and 4 * -(-max(groups) // n_sm) <= 384
 
     def _persistent_state(self, cache):
         """Layer table (device pointers of the packed weights, norms and this cache's tensors) and scratch buffers."""
