@@ -261,18 +261,19 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemv_multi_kernel(const __grid_
 #pragma unroll
                 for (int r = 0; r < 4; ++r) tot[r] = accp[r] - accn[r];
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_empty + 8 * stage);       // this warp no longer reads the stage
-            if (++stage == GM_STAGES) { stage = 0; phase ^= 1; }
-            const int slot = it & 3;
-            ++it;
-            if (!active) continue;
             // sum over the warp: fold the 4 row totals while halving (6 shuffles); lane L ends with row 2*(L>>4&1) + (L>>3&1)
             const bool b4 = (lane & 16) != 0, b3 = (lane & 8) != 0;
             int va = b4 ? tot[2] : tot[0], sa = b4 ? tot[0] : tot[2];
             int vb = b4 ? tot[3] : tot[1], sb = b4 ? tot[1] : tot[3];
             va += __shfl_xor_sync(0xffffffffu, sa, 16);
             vb += __shfl_xor_sync(0xffffffffu, sb, 16);
+            // The stage is given back behind the first shuffles, which need every total: an arrive does not wait for shared-memory loads on their way, nor do the stage's next
+            // copies.  (A warp's loads return in their order, so the scale and the pointers asked for before are there too.)
+            if (lane == 0) mbar_arrive(bar_empty + 8 * stage);
+            if (++stage == GM_STAGES) { stage = 0; phase ^= 1; }
+            const int slot = it & 3;
+            ++it;
+            if (!active) continue;
             int vc = b3 ? vb : va;
             const int sc = b3 ? va : vb;
             vc += __shfl_xor_sync(0xffffffffu, sc, 8);
