@@ -175,15 +175,19 @@ class FusedQwen3:
 
     # ---- prompts on digit planes ----------------------------------------------------------------------------------------
     # 1.5 times the tensor work of the INT8 products, but weights are read packed, with nothing decoded beside the products.  Whole prompts of four layers, us, INT8 with
-    # overlapped decode / digit planes: width 2048, 16 tokens 308 / 238, 160 357 / 301, 333 382 / 362, 512 413 / 392, 700 473 / 466, 1024 534 / 572; width 1024 (12.6
-    # million weights a layer, whose decode hides), 16 tokens 236 / 185, 64 232 / 232, 160 262 / 273, 333 276 / 296.
-    F4_TOKENS, F4_TOKENS_SMALL, F4_LAYER = 640, 32, 1 << 25
+    # overlapped decode / digit planes.  By weights of a layer: 12.6 million (width 1024, whose decode hides) 16 tokens 214 / 165, 33 209 / 214, 160 242 / 255, 333 256 / 278; 28 million
+    # (1536) 40 tokens 225 / 197, 256 262 / 259, 512 302 / 322; 35.4 (1536, wide feed-forward) 400 tokens 341 / 332, 448 341 / 336, 512 334 / 346; 36.0 (1664) 512 tokens 367 / 348, 600
+    # 394 / 395, 640 387 / 398; 38.5 (1792) 600 tokens 376 / 376, 640 370 / 381; 44 (2048) 640 tokens 404 / 390; 50 (2048) 256 tokens 319 / 297, 640 415 / 407, 1024 534 / 572;
+    # 101 (3072) 640 tokens 764 / 659.
+    F4_TOKENS, F4_TOKENS_SMALL = 640, 32                                  # most tokens for large layers, and for small ones
+    F4_LAYERS = ((40 << 20, None), (34 << 20, 600), (32 << 20, 448))      # weights from which on it is F4_TOKENS, or so many
 
     def _f4(self, L):
         """Whether a prompt's products run on digit planes and packed weights (the tensor cores' 4-bit path): few tokens for the weights of a layer, the
         default format, and this class's own methods."""
         own = all(getattr(type(self), n) is f and n not in self.__dict__ for n, f in _OWN.items())
-        limit = self.F4_TOKENS if sum(w.N * w.K for w in self.layers[0][1].values()) >= self.F4_LAYER else self.F4_TOKENS_SMALL
+        weights = sum(w.N * w.K for w in self.layers[0][1].values())
+        limit = next((tokens or self.F4_TOKENS for least, tokens in self.F4_LAYERS if weights >= least), self.F4_TOKENS_SMALL)
         if not (own and 0 < L <= limit and self.epilogue == "gemm" and not self.resident and not self.rot and self.record is None):
             return False
         widths = {w.K for w in self.layers[0][1].values()}

@@ -398,7 +398,9 @@ def test_prompts_on_digit_planes(scmx):
         return f
 
     limit, small = FQ.FusedQwen3.F4_TOKENS, FQ.FusedQwen3.F4_TOKENS_SMALL
-    assert [make()._f4(n) for n in (0, 1, limit, limit + 1)] == [False, True, True, False]
+    assert [make(width=8192)._f4(n) for n in (0, 1, limit, limit + 1)] == [False, True, True, False]
+    for width, most in ((5120, limit), (5119, 600), (4352, 600), (4351, 448), (4096, 448), (4095, small)):      # weights of a layer: 4 x width x 2048
+        assert [make(width=width)._f4(n) for n in (most, most + 1)] == [True, False], width
     assert [make(width=1024)._f4(n) for n in (small, small + 1)] == [True, False]
     assert not any(make(**kw)._f4(16) for kw in (dict(cls=Own), dict(K=2048 + 64), dict(K=10240), dict(epilogue="row"), dict(resident=True), dict(rot="down"),
                                                  dict(record={}), dict(act_q=lambda x, Mp: None), dict(_rec=lambda *a: None)))
