@@ -19,7 +19,7 @@
 // (2) Weights stream through rings in shared memory, one per warp, filled by asynchronous copies of the lanes that use them: the order of chunks is
 //     known from the start, so the ring runs ahead through phases and layers (170 KB per SM, most of a layer) while the CTA waits, joins or reduces.
 // Work item of a warp: 4 rows x 1024 columns; a row group's items are summed through shared memory (exact integers).
-// 8 layers of width 2048 at 1500 positions with the head: 342 us with grid barriers and weights in registers, 315 us here.  A layer (32 us): rows of q|k|v 2.3 (and 2.0
+// 8 layers of width 2048 at 1500 positions with the head: 342 us with grid barriers and weights in registers, 312 us here.  A layer (32 us): rows of q|k|v 2.3 (and 2.0
 // until the input row is there), attention 6.5, its combination and exchange 4.9, o 1.5, h 2.8, gate|up 5.4, act 1.7, down 3.7; two items at a time per warp changed
 // nothing (321), polling without a pause slowed the writers (375).
 // Arithmetic: the device functions of the stand-alone kernels (row kernels, GEMV, q/k/v epilogue, decode attention), so the step produces the

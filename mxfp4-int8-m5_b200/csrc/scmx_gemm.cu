@@ -426,9 +426,9 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const Gem
 
 static int run_gemm(const int8_t* xq, int64_t a_rows, const int8_t* wq, int64_t b_rows, GemmArgs& a, cudaStream_t st) {
     // Dense products whose 128 x 128 tiles fit one wave of single CTAs run as those: more SMs share the operand traffic and a CTA's
-    // K loop moves 32 KB per step instead of 48 (384 x 2048 x 2048: 9.2 us, CTA pairs 11.9 us, 128 x 256 tiles 12.3 us; 128 x 12288 x 2048 11.3
-    // and 14.3 us).  Above that pairs while their 256 x 256 tiles fit one wave (512 x 6144 x 2048: 12.3 us, 128 x 128 tiles 14.9 us), 128 x 256
-    // tiles where only these do (384 x 12288 x 2048: 15.0 us, pairs 18.2 us), pairs for the rest.
+    // K loop moves 32 KB per step instead of 48 (in a chain, 384 x 2048 x 2048: 7.9 us, 128 x 256 tiles 12.2 us; 128 x 12288 x 2048 9.3
+    // and 13.4 us).  Above that pairs while their 256 x 256 tiles fit one wave (512 x 6144 x 2048: 11.7 us, 128 x 128 tiles 12.5 us), 128 x 256
+    // tiles where only these do (384 x 12288 x 2048: 13.7 us, 128 x 128 tiles 13.0 us since warps issue together; pairs 18.2 us before that), pairs for the rest.
     auto count = [&](int64_t tm, int64_t tn) { return (a.M + tm - 1) / tm * ((a.N + tn - 1) / tn); };
     const bool dense = a.E == 0 && a.bcast == 0 && a.ret_rank == nullptr;
     const bool small = dense && count(BM, 128) <= num_sms();

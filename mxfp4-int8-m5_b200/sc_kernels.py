@@ -134,8 +134,8 @@ def _rmsnorm_quant(x, w, eps, Mp, want_n):
 @functools.lru_cache(maxsize=4096)
 def _ranges(M, N, K, n_sm):
     """Ranges of K for a dense product whose 128 x 128 tiles leave most SMs idle.  Summing the ranges costs a launch of 3 us and their traffic,
-    which only a long K repays: 256 x 2048 x 6144 takes 18.2 us in one piece and 12.7 us in four, 128 x 1024 x 3072 10.9 and 8.6 us, but
-    256 x 2048 x 2048 9.0 and 9.4 us in two."""
+    which only a long K repays: in a chain, 256 x 2048 x 6144 takes 15.3 us in one piece and 11.1 us in four, 384 x 2048 x 6144 15.3 and 11.7 us in three, 128 x 1024 x 3072 8.9
+    and 8.0 us in four, but 256 x 2048 x 2048 7.9 and 8.7 us in two."""
     return max(1, min(4, n_sm // (-(-M // 128) * -(-N // 128)))) if K >= 3072 else 1
 
 

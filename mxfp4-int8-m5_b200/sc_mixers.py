@@ -75,9 +75,10 @@ def _f32_tc(M, N, K):
 
 @functools.lru_cache(maxsize=4096)
 def _plan(M, N, K, splits, n_sm):
-    """(tile, ranges of K computed side by side) for a product with few output tiles: 4 us and 0.27 us for every step of 64 values that a CTA walks
-    (77 x 4096 x 1024: 8.4 us, 77 x 1024 x 3072: 16.9 us), counting whole waves; summing ranges costs a launch, 2 us, and the traffic of
-    the partial products (77 x 4096 x 1024 in three: 10 us, 77 x 1024 x 3072: 10.1 us).  (0, 1): leave it to the kernel."""
+    """(tile, ranges of K computed side by side) for a product with few output tiles: 4 us and 0.27 us for every step of 64 values that a CTA walks, counting whole waves;
+    summing ranges costs a launch, 2 us, and the traffic of the partial products.  The rates are those of an issuing thread that ran alone; with whole warps it is 3 us and 0.2 us a
+    step, and the choices hold: in a chain, tiles of 64, 77 x 4096 x 1024 takes 6.6 us in one piece and 8.7 in three, 77 x 1024 x 3072 12.8 and in eight 7.1, 77 x 1024 x 1024 6.0
+    and in four 6.1, 300 x 2048 x 1024 6.8 and in three 9.1.  (0, 1): leave it to the kernel."""
     tm, kb = -(-M // 128), -(-K // 64)
     if tm * -(-N // 64) >= n_sm or splits == 1:
         return 0, splits or 1
@@ -89,7 +90,7 @@ def _plan(M, N, K, splits, n_sm):
 @functools.lru_cache(maxsize=4096)
 def _plan_f32(M, N, K, splits, n_sm):
     """(tile, ranges of K) of a float32 product: steps of 64 values stage three parts of 128 + tile rows, about 5.5 ns a row and step; 5 us around them.
-    Ranges cost a summing launch, about 3 us and their traffic.  300 x 6144 x 1024: 40 us as 128 x 128 tiles, 53 us as 128 x 64.  CTA pairs (tile 256), whose accumulators
+    Ranges cost a summing launch, about 3 us and their traffic.  300 x 6144 x 1024: 41 us as 128 x 128 tiles, 52 us as 128 x 64.  CTA pairs (tile 256), whose accumulators
     leave no room for a second set, are only run when asked for: 2048 x 2048 x 6144 300 us as 128 x 128 tiles, 436 us as pairs."""
     tm, kb = -(-M // 128), -(-K // 64)
 
